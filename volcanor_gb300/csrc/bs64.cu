@@ -14,50 +14,117 @@ namespace vlm {
 
 namespace {
 
-constexpr int kThreads64 = 128;  // targets per block
-constexpr int kTile64 = 32;      // records staged per shared-memory tile
+// FP64 partial sums.  A warp's FP64 instruction holds its quarter of the SM
+// for 64 cycles (half a lane a cycle), so the pair evaluations bound every
+// shape here and one warp per quarter already fills the unit; what a small
+// shape lacks is quarters.  So the evaluations of a chunk are spread over
+// threads and only its additions, which have to stay in record order, are
+// serial: a block of kThreads64 threads takes TT targets and evaluates
+// S = kThreads64 / TT consecutive records of them at once (thread = record s,
+// target t) into shared memory, then one warp adds the S contributions of
+// each (target, component) in record order -- the warps take turns, and a
+// block's other warps go on with the next batch's evaluations.  TT is chosen
+// per shape (pick_tile64): few targets and chunks get TT = 1 (a wing's 52
+// rings at 52 points: 52 blocks whose threads take a record each, 906 us in
+// one block of a thread per target before), many get TT = 8..32, whose
+// ordered additions use most of a warp.  Each contribution and each addition
+// is the reference's own, so the bits are those of one thread per target
+// (blade_vind_bywing / blade_vind_bywake, src/classdef.f90:1342-1513).
+constexpr int kThreads64 = 128;
+constexpr int kMaxTT = 32;
 
-// One block = kThreads64 targets x one chunk.  Each thread sums its target's
-// contributions over the chunk sequentially from zero (blade_vind_bywing /
-// blade_vind_bywake accumulation, src/classdef.f90:1342-1513).
+// One record's contribution (velocity times circulation) at target p; zero
+// for a record the reference skips, which leaves an ordered sum unchanged.
+__device__ __forceinline__ d3 rec_vind64(d3 p, const double* __restrict__ R) {
+  const int flags = (int)R[17];
+  const double g = R[16];
+  if ((flags & REC_SKIP) && !(fabs(g) > kEps)) return zero3();
+  if (flags & REC_FIL) return fil_vind64(p, mk3(R[0], R[1], R[2]), mk3(R[3], R[4], R[5]), R[12]) * g;
+  const d3 c[4] = {mk3(R[0], R[1], R[2]), mk3(R[3], R[4], R[5]), mk3(R[6], R[7], R[8]), mk3(R[9], R[10], R[11])};
+  return vr_vind64(p, c, R + 12) * g;
+}
+
+// Grid: (target tiles) x (runs of K consecutive chunks).  lgTT = log2(TT).
 __global__ void __launch_bounds__(kThreads64) k_partial64(const double* __restrict__ rec,
-                                                         const Chunk* __restrict__ chunks,
-                                                         const double* __restrict__ P, int M,
+                                                         const Chunk* __restrict__ chunks, int nchunks, int K,
+                                                         const double* __restrict__ P, int M, int lgTT,
                                                          double* __restrict__ part) {
-  __shared__ double tile[kTile64 * kRec64];
-  const Chunk ch = chunks[blockIdx.y];
-  const int m = blockIdx.x * kThreads64 + threadIdx.x;
-  const bool active = m < M;
-  d3 p = zero3();
-  if (active) p = mk3(P[3 * (size_t)m], P[3 * (size_t)m + 1], P[3 * (size_t)m + 2]);
-  d3 acc = zero3();
-  for (int t0 = 0; t0 < ch.rec_count; t0 += kTile64) {
-    const int nt = min(kTile64, ch.rec_count - t0);
+  __shared__ double C[kThreads64 * 3];  // contributions [s][component][t]
+  __shared__ double acc[3 * kMaxTT];    // the open chunk's sums [component][t]
+  const int TT = 1 << lgTT, S = kThreads64 >> lgTT;
+  const int t = threadIdx.x & (TT - 1), s = threadIdx.x >> lgTT;
+  const int m0 = blockIdx.x * TT;
+  const int m = min(m0 + t, M - 1);
+  int q = blockIdx.y * K;
+  const int qe = min(q + K, nchunks);
+  const int r0 = chunks[q].rec_begin;
+  const int r1 = chunks[qe - 1].rec_begin + chunks[qe - 1].rec_count;
+  const d3 p = mk3(P[3 * (size_t)m], P[3 * (size_t)m + 1], P[3 * (size_t)m + 2]);
+  if (threadIdx.x < 3 * TT) acc[threadIdx.x] = 0.0;
+  int qend = r0 + chunks[q].rec_count;  // end of the open chunk
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int f = r0, batch = 0; f < r1; f += S, ++batch) {
+    const int n = min(S, r1 - f);
+    d3 v = zero3();
+    if (s < n) v = rec_vind64(p, rec + (size_t)(f + s) * kRec64);
+    __syncthreads();  // the last batch's additions are done
+    double* c = C + 3 * TT * s + t;
+    c[0] = v.x;
+    c[TT] = v.y;
+    c[2 * TT] = v.z;
     __syncthreads();
-    const double* src = rec + (size_t)(ch.rec_begin + t0) * kRec64;
-    for (int k = threadIdx.x; k < nt * kRec64; k += kThreads64) tile[k] = src[k];
-    __syncthreads();
-    if (!active) continue;
-    for (int r = 0; r < nt; ++r) {
-      const double* R = tile + r * kRec64;
-      const int flags = (int)R[17];
-      const double g = R[16];
-      if ((flags & REC_SKIP) && !(fabs(g) > kEps)) continue;
-      d3 v;
-      if (flags & REC_FIL) {
-        v = fil_vind64(p, mk3(R[0], R[1], R[2]), mk3(R[3], R[4], R[5]), R[12]);
-      } else {
-        d3 c[4] = {mk3(R[0], R[1], R[2]), mk3(R[3], R[4], R[5]), mk3(R[6], R[7], R[8]), mk3(R[9], R[10], R[11])};
-        v = vr_vind64(p, c, R + 12);
+    const bool mine = warp == (batch & (kThreads64 / 32 - 1));
+    int qn = q, en = qend;
+    if (mine) {
+      for (int k = lane; k < 3 * TT; k += 32) {
+        double a = acc[k];
+        qn = q;
+        en = qend;
+        for (int i = 0; i < n; ++i) {
+          a = a + C[3 * TT * i + k];
+          if (f + i + 1 == en) {
+            const int mk = m0 + (k & (TT - 1));
+            if (mk < M) part[((size_t)qn * M + mk) * 3 + (k >> lgTT)] = a;
+            a = 0.0;
+            if (++qn < qe) en += chunks[qn].rec_count;
+          }
+        }
+        acc[k] = a;
       }
-      acc = acc + v * g;
     }
+    while (q < qe && qend <= f + n)
+      if (++q < qe) qend += chunks[q].rec_count;
   }
-  if (active) {
-    double* o = part + ((size_t)blockIdx.y * M + m) * 3;
-    o[0] = acc.x;
-    o[1] = acc.y;
-    o[2] = acc.z;
+}
+
+// TT and K for M targets, nchunks chunks of nrec records in all: the least
+// modelled time on a device of `sms` SMs.  Units: one FP64 instruction of a
+// warp, of which a quarter-SM does one at a time; a record costs kEval64 at 32
+// targets, an ordered addition 1.  A block's quarter does one warp's
+// evaluations per batch and, every fourth batch, the additions; a wave of
+// blocks is kWave64 per SM.
+constexpr int kEval64 = 509, kWave64 = 4;
+void pick_tile64(int M, int nchunks, int64_t nrec, int sms, int& lgTT, int& K) {
+  const double C = (double)nrec / nchunks;
+  double best = 0.0;
+  for (int lg = 0; (1 << lg) <= kMaxTT; ++lg) {
+    const int TT = 1 << lg, S = kThreads64 / TT;
+    const int64_t tiles = ((int64_t)M + TT - 1) / TT;
+    for (int k = 1;; k *= 2) {
+      const int64_t blocks = tiles * ((nchunks + k - 1) / k);
+      const double batches = std::max(1.0, std::ceil(std::min<double>(k, nchunks) * C / S));
+      const double perBatch = kEval64 + std::min<double>(S, C * std::min(k, nchunks)) * ((3 * TT + 31) / 32);
+      const double full = (double)blocks / ((double)sms * kWave64);
+      // below a wave the busiest SM decides, above it the average with half a block's tail
+      const double rounds = full <= 1.0 ? std::ceil((double)blocks / sms) : kWave64 * (full + 0.5);
+      const double T = rounds * batches * perBatch;
+      if (best == 0.0 || T < best * 0.999) {
+        best = T;
+        lgTT = lg;
+        K = k;
+      }
+      if (k >= nchunks || k >= 8) break;
+    }
   }
 }
 
@@ -287,12 +354,16 @@ int build_chunks(Group* groups, int ngroups, int chunk_size, Chunk* chunks, int 
   return nq;
 }
 
-void launch_partial64(const double* rec, const Chunk* chunks, int nchunks, const double* P, int M, double* part,
-                      cudaStream_t s) {
+void launch_partial64(const double* rec, const Chunk* chunks, int nchunks, int64_t nrec, const double* P, int M,
+                      double* part, cudaStream_t s) {
   if (M <= 0 || nchunks <= 0) return;
-  dim3 grid((M + kThreads64 - 1) / kThreads64, nchunks);
+  int lgTT = 0, K = 1;
+  pick_tile64(M, nchunks, nrec, device_sm_count(), lgTT, K);
+  // the grid's second dimension ends at 65535
+  K = std::max(K, (nchunks + 65534) / 65535);
+  dim3 grid((unsigned)(((int64_t)M + (1 << lgTT) - 1) >> lgTT), (unsigned)((nchunks + K - 1) / K));
   count_launch();
-  k_partial64<<<grid, kThreads64, 0, s>>>(rec, chunks, P, M, part);
+  k_partial64<<<grid, kThreads64, 0, s>>>(rec, chunks, nchunks, K, P, M, lgTT, part);
 }
 
 void launch_combine(const double* part, int M, const Group* groups, int ngroups, int mode, double* out,

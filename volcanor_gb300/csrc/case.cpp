@@ -521,7 +521,7 @@ struct Case {
     if (prec < 0) prec = opt.precision;
     const Chunk* ch = dChunks + e.coff;
     if (prec == VLM_PREC_FP64) {
-      launch_partial64(s.rec64, ch, e.nchunks, P, M, s.part, stream);
+      launch_partial64(s.rec64, ch, e.nchunks, e.nrec, P, M, s.part, stream);
     } else {
       const bool nearOn = prec == VLM_PREC_FP32_NEAR64;
       launch_pack32(s.rec64, e.nrec, nearOn ? opt.near_factor : 0.0, s.rec32, stream, s.edgeW);
@@ -1946,7 +1946,7 @@ struct Case {
       profileWork[1] = fils * M;
     }
     auto launch = [&]() {
-      if (opt.precision == VLM_PREC_FP64) launch_partial64(s.rec64, ch, pl.node.nchunks, s.targets, M, s.part, stream);
+      if (opt.precision == VLM_PREC_FP64) launch_partial64(s.rec64, ch, pl.node.nchunks, pl.node.nrec, s.targets, M, s.part, stream);
       else {
         VLM_CUDA(cudaMemsetAsync(s.err + 3, 0, sizeof(int), stream));
         launch_partial32(s.rec32, s.rec64, ch, pl.node.nchunks, pl.node.nrec, s.targets, M, s.part, s.err + 2,
@@ -2191,7 +2191,7 @@ struct Case {
       t.edgeW = nullptr;  // ring by ring: the probe's record count is not the plans'
       launch_gather(d, t, frame(fi), dg, (int)g.size(), rec, rN, rF, false, stream);
       if (opt.precision == VLM_PREC_FP64) {
-        launch_partial64(rec64, dc, nq, dP, (int)M, part, stream);
+        launch_partial64(rec64, dc, nq, rec, dP, (int)M, part, stream);
       } else {
         const bool nearOn = opt.precision == VLM_PREC_FP32_NEAR64;
         launch_pack32(rec64, rec, nearOn ? opt.near_factor : 0.0, rec32, stream);
@@ -2333,7 +2333,7 @@ void rings_device(const double* corners, const double* rvc, const double* gam, i
     if (fil) launch_fils_to_rec64(corners, rvc, gam, N, R.rec64, st);
     else launch_rings_to_rec64(corners, rvc, gam, N, R.rec64, st);
     if (precision == VLM_PREC_FP64) {
-      launch_partial64(R.rec64, R.chunks, nq, P, (int)M, R.part, st);
+      launch_partial64(R.rec64, R.chunks, nq, N, P, (int)M, R.part, st);
     } else {
       const bool nearOn = precision == VLM_PREC_FP32_NEAR64;
       launch_pack32(R.rec64, (int)N, nearOn ? 4.0 : 0.0, R.rec32, st);

@@ -164,9 +164,10 @@ int partial32_slots(int shape = 0);
 int device_sm_count();
 
 
-// FP64 reference-arithmetic partial sums: part[(q * M + m) * 3 + k].
-void launch_partial64(const double* rec, const Chunk* chunks, int nchunks, const double* P, int M, double* part,
-                      cudaStream_t s);
+// FP64 reference-arithmetic partial sums: part[(q * M + m) * 3 + k].  The
+// chunks follow one another in the record array and hold nrec records in all.
+void launch_partial64(const double* rec, const Chunk* chunks, int nchunks, int64_t nrec, const double* P, int M,
+                      double* part, cudaStream_t s);
 // FP32 pairs with FP64 accumulation over the nrec records the chunks cover.
 // When near_scratch is non-null (near_bytes = near_scratch_bytes(M, cap) for a list of cap
 // near pairs), the
