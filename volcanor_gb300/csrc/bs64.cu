@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "exact64.h"
 #include "vlm_bs.h"
 #include "vlm_math.h"
 
@@ -39,9 +40,9 @@ __device__ __forceinline__ d3 rec_vind64(d3 p, const double* __restrict__ R) {
   const int flags = (int)R[17];
   const double g = R[16];
   if ((flags & REC_SKIP) && !(fabs(g) > kEps)) return zero3();
-  if (flags & REC_FIL) return fil_vind64(p, mk3(R[0], R[1], R[2]), mk3(R[3], R[4], R[5]), R[12]) * g;
+  if (flags & REC_FIL) return exact64::fil_vind(p, mk3(R[0], R[1], R[2]), mk3(R[3], R[4], R[5]), R[12]) * g;
   const d3 c[4] = {mk3(R[0], R[1], R[2]), mk3(R[3], R[4], R[5]), mk3(R[6], R[7], R[8]), mk3(R[9], R[10], R[11])};
-  return vr_vind64(p, c, R + 12) * g;
+  return exact64::vr_vind(p, c, R + 12) * g;
 }
 
 // Grid: (target tiles) x (runs of K consecutive chunks).  lgTT = log2(TT).
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(kThreads64) k_partial64(const double* __restri
 // targets, an ordered addition 1.  A block's quarter does one warp's
 // evaluations per batch and, every fourth batch, the additions; a wave of
 // blocks is kWave64 per SM.
-constexpr int kEval64 = 509, kWave64 = 4;
+constexpr int kEval64 = 211, kWave64 = 4;
 void pick_tile64(int M, int nchunks, int64_t nrec, int sms, int& lgTT, int& K) {
   const double C = (double)nrec / nchunks;
   double best = 0.0;
