@@ -65,8 +65,8 @@ int main() {
       case 5: c[3].x = INFINITY; break;
       case 6: c[3].y = NAN; break;
     }
-    if (!same(vr_vind64(P, c, rv), exact64::vr_vind(P, c, rv))) return 3;
-    if (!same(fil_vind64(P, c[0], c[1], rv[0]), exact64::fil_vind(P, c[0], c[1], rv[0]))) return 4;
+    if (!same(vr_vind64(P, c, rv), exact64::vr_vind(Unit{1.0, -0.0}, P, c, rv))) return 3;
+    if (!same(fil_vind64(P, c[0], c[1], rv[0]), exact64::fil_vind(Unit{1.0, -0.0}, P, c[0], c[1], rv[0]))) return 4;
   }
   return 0;
 }

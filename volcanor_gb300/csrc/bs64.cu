@@ -17,42 +17,124 @@ namespace {
 
 // FP64 partial sums.  A warp's FP64 instruction holds its quarter of the SM
 // for 64 cycles (half a lane a cycle), so the pair evaluations bound every
-// shape here and one warp per quarter already fills the unit; what a small
-// shape lacks is quarters.  So the evaluations of a chunk are spread over
-// threads and only its additions, which have to stay in record order, are
-// serial: a block of kThreads64 threads takes TT targets and evaluates
-// S = kThreads64 / TT consecutive records of them at once (thread = record s,
-// target t) into shared memory, then one warp adds the S contributions of
-// each (target, component) in record order -- the warps take turns, and a
-// block's other warps go on with the next batch's evaluations.  TT is chosen
-// per shape (pick_tile64): few targets and chunks get TT = 1 (a wing's 52
-// rings at 52 points: 52 blocks whose threads take a record each, 906 us in
-// one block of a thread per target before), many get TT = 8..32, whose
-// ordered additions use most of a warp.  Each contribution and each addition
-// is the reference's own, so the bits are those of one thread per target
-// (blade_vind_bywing / blade_vind_bywake, src/classdef.f90:1342-1513).
-constexpr int kThreads64 = 128;
+// shape here; a few warps on an SM fill the unit, and what a small shape lacks
+// is quarters.  So the evaluations of a chunk are spread over threads and only
+// its additions, which have to stay in record order, are serial: a block takes TT targets and evaluates a batch of S = threads / TT
+// consecutive records of each at once into shared memory; one warp then adds
+// the S contributions of each (target, component) in record order -- the warps
+// take turns -- while all go on with the next batch.  Each contribution and each addition is the reference's own, so the bits are
+// those of one thread per target (blade_vind_bywing / blade_vind_bywake,
+// src/classdef.f90:1342-1513).
+//
+// A near-wake sheet's rings are listed column by column (L rows each): ring
+// r's corner 3 and edge 3 are ring r - 1's corner 2 and edge 1, its corner 1 and
+// edge 0 ring r - L's corner 2 and edge 2.  An edge run backwards has exactly
+// the negated velocity (every product and difference of vf_vind negates; only
+// the sign of a zero may differ), so a ring whose neighbours are at hand costs
+// one corner and two filaments, 111 FP64 instructions, instead of four and four,
+// 211.  Corner 2's unit vector and edge 2 of the last L records stay in shared
+// memory (48 bytes a target and row); share[r] says where the neighbours' hold
+// bit for bit (a dissipated core, a row that just moved or the sheet's border
+// breaks it, and a block's run of K chunks starts without neighbours), elsewhere
+// the ring evaluates its own.
+constexpr int kThreads64 = 128;          // rings one by one
+constexpr int kThreadsLattice64 = 256;  // sheets: the wider block shares a column's buffer among more warps
 constexpr int kMaxTT = 32;
+
+// A record's flags and the reference's |gam| > eps, read from the words of the
+// doubles: a conversion or a comparison would go through the FP64 unit.
+__device__ __forceinline__ bool is_fil(const double* R) {
+  const unsigned h = (unsigned)__double2hiint(R[17]);
+  return h == 0x3ff00000u || h == 0x40080000u;  // 1 or 3
+}
+__device__ __forceinline__ bool skipped(const double* R) {
+  const unsigned long long g = (unsigned long long)__double_as_longlong(R[16]) & 0x7fffffffffffffffull;
+  const unsigned long long lo = 0x3cb0000000000001ull;  // the number after kEps = 2^-52
+  return (unsigned)__double2hiint(R[17]) >= 0x40000000u && !(g - lo <= 0x7ff0000000000000ull - lo);
+}
+static_assert(REC_FIL == 1 && REC_SKIP == 2, "flag words");
+
+constexpr int kShareC3 = 1, kShareE3 = 2, kShareC1 = 4, kShareE0 = 8;
+__device__ __forceinline__ bool same_point(const double* a, const double* b) {
+  return __double_as_longlong(a[0]) == __double_as_longlong(b[0]) &&
+         __double_as_longlong(a[1]) == __double_as_longlong(b[1]) &&
+         __double_as_longlong(a[2]) == __double_as_longlong(b[2]);
+}
+__global__ void k_share64(const double* __restrict__ rec, int nrec, const Group* __restrict__ groups, int ngroups,
+                          int L, int* __restrict__ share) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= nrec) return;
+  int g = 0;
+  while (g + 1 < ngroups && r >= groups[g + 1].rec_begin) ++g;
+  const int first = groups[g].rec_begin;
+  const double* R = rec + (size_t)r * kRec64;
+  int b = 0;
+  if (!is_fil(R)) {
+    if (r - 1 >= first) {
+      const double* A = R - kRec64;
+      if (!is_fil(A) && same_point(R + 9, A + 6)) {
+        b |= kShareC3;
+        if (same_point(R, A + 3) && __double_as_longlong(R[15]) == __double_as_longlong(A[13])) b |= kShareE3;
+      }
+    }
+    if (r - L >= first) {
+      const double* A = R - (size_t)L * kRec64;
+      if (!is_fil(A) && same_point(R + 3, A + 6)) {
+        b |= kShareC1;
+        if (same_point(R, A + 9) && __double_as_longlong(R[12]) == __double_as_longlong(A[14])) b |= kShareE0;
+      }
+    }
+  }
+  share[r] = b;
+}
 
 // One record's contribution (velocity times circulation) at target p; zero
 // for a record the reference skips, which leaves an ordered sum unchanged.
-__device__ __forceinline__ d3 rec_vind64(d3 p, const double* __restrict__ R) {
-  const int flags = (int)R[17];
-  const double g = R[16];
-  if ((flags & REC_SKIP) && !(fabs(g) > kEps)) return zero3();
-  if (flags & REC_FIL) return exact64::fil_vind(p, mk3(R[0], R[1], R[2]), mk3(R[3], R[4], R[5]), R[12]) * g;
-  const d3 c[4] = {mk3(R[0], R[1], R[2]), mk3(R[3], R[4], R[5]), mk3(R[6], R[7], R[8]), mk3(R[9], R[10], R[11])};
-  return exact64::vr_vind(p, c, R + 12) * g;
+__device__ __forceinline__ d3 contribution64(const exact64::Unit& u, d3 p, const double* __restrict__ R) {
+  if (skipped(R)) return zero3();
+  d3 v;
+  if (is_fil(R)) {
+    v = exact64::fil_vind(u, p, mk3(R[0], R[1], R[2]), mk3(R[3], R[4], R[5]), R[12]);
+  } else {
+    const d3 c[4] = {mk3(R[0], R[1], R[2]), mk3(R[3], R[4], R[5]), mk3(R[6], R[7], R[8]), mk3(R[9], R[10], R[11])};
+    v = exact64::vr_vind(u, p, c, R + 12);
+  }
+  return exact64::mul(u, v, R[16]);
+}
+
+// The batch of n records from f whose contributions are in C added to the open
+// chunk's sums acc in record order, one (component, target) a lane of the warps
+// whose turn it is; q, qend: the open chunk and its end.
+template <int NT>
+__device__ __forceinline__ void add_batch64(const exact64::Unit& u, const double* C, double* acc, int turn, int lgTT,
+                                            int f, int n, int q, int qe, int qend, const Chunk* __restrict__ chunks,
+                                            int m0, int M, double* __restrict__ part) {
+  const int TT = 1 << lgTT;
+  const int lane = (threadIdx.x - 32 * (turn & (NT / 32 - 1))) & (NT - 1);
+  if (lane >= 3 * TT) return;
+  double a = acc[lane];
+  for (int i = 0; i < n;) {
+    const int e = min(n, qend - f);  // to the chunk's end
+#pragma unroll 4
+    for (; i < e; ++i) a = exact64::add(u, a, C[3 * TT * i + lane]);
+    if (f + i == qend) {
+      const int mk = m0 + (lane & (TT - 1));
+      if (mk < M) part[((size_t)q * M + mk) * 3 + (lane >> lgTT)] = a;
+      a = 0.0;
+      if (++q < qe) qend += chunks[q].rec_count;
+    }
+  }
+  acc[lane] = a;
 }
 
 // Grid: (target tiles) x (runs of K consecutive chunks).  lgTT = log2(TT).
-__global__ void __launch_bounds__(kThreads64) k_partial64(const double* __restrict__ rec,
-                                                         const Chunk* __restrict__ chunks, int nchunks, int K,
-                                                         const double* __restrict__ P, int M, int lgTT,
-                                                         double* __restrict__ part) {
-  __shared__ double C[kThreads64 * 3];  // contributions [s][component][t]
-  __shared__ double acc[3 * kMaxTT];    // the open chunk's sums [component][t]
+__global__ void __launch_bounds__(kThreads64) k_rings64(const double* __restrict__ rec, const Chunk* __restrict__ chunks,
+                                                       int nchunks, int K, const double* __restrict__ P, int M, int lgTT,
+                                                       double* __restrict__ part) {
+  __shared__ double C[2][3 * kThreads64];  // contributions of two batches [s][component][t]
+  __shared__ double acc[3 * kMaxTT];       // the open chunk's sums [component][t]
   const int TT = 1 << lgTT, S = kThreads64 >> lgTT;
+  const exact64::Unit u = exact64::load_unit();
   const int t = threadIdx.x & (TT - 1), s = threadIdx.x >> lgTT;
   const int m0 = blockIdx.x * TT;
   const int m = min(m0 + t, M - 1);
@@ -62,71 +144,187 @@ __global__ void __launch_bounds__(kThreads64) k_partial64(const double* __restri
   const int r1 = chunks[qe - 1].rec_begin + chunks[qe - 1].rec_count;
   const d3 p = mk3(P[3 * (size_t)m], P[3 * (size_t)m + 1], P[3 * (size_t)m + 2]);
   if (threadIdx.x < 3 * TT) acc[threadIdx.x] = 0.0;
-  int qend = r0 + chunks[q].rec_count;  // end of the open chunk
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int f = r0, batch = 0; f < r1; f += S, ++batch) {
-    const int n = min(S, r1 - f);
-    d3 v = zero3();
-    if (s < n) v = rec_vind64(p, rec + (size_t)(f + s) * kRec64);
-    __syncthreads();  // the last batch's additions are done
-    double* c = C + 3 * TT * s + t;
-    c[0] = v.x;
-    c[TT] = v.y;
-    c[2 * TT] = v.z;
-    __syncthreads();
-    const bool mine = warp == (batch & (kThreads64 / 32 - 1));
-    int qn = q, en = qend;
-    if (mine) {
-      for (int k = lane; k < 3 * TT; k += 32) {
-        double a = acc[k];
-        qn = q;
-        en = qend;
-        for (int i = 0; i < n; ++i) {
-          a = a + C[3 * TT * i + k];
-          if (f + i + 1 == en) {
-            const int mk = m0 + (k & (TT - 1));
-            if (mk < M) part[((size_t)qn * M + mk) * 3 + (k >> lgTT)] = a;
-            a = 0.0;
-            if (++qn < qe) en += chunks[qn].rec_count;
-          }
-        }
-        acc[k] = a;
-      }
+  int qend = r0 + chunks[q].rec_count;
+  const int nb = (r1 - r0 + S - 1) / S;
+  for (int b = 0; b <= nb; ++b) {
+    const int r = r0 + b * S + s;
+    if (r < r1) {
+      const d3 v = contribution64(u, p, rec + (size_t)r * kRec64);
+      double* c = C[b & 1] + 3 * TT * s + t;
+      c[0] = v.x;
+      c[TT] = v.y;
+      c[2 * TT] = v.z;
     }
-    while (q < qe && qend <= f + n)
-      if (++q < qe) qend += chunks[q].rec_count;
+    if (b > 0) {
+      const int f = r0 + (b - 1) * S, n = min(S, r1 - f);
+      add_batch64<kThreads64>(u, C[(b - 1) & 1], acc, b, lgTT, f, n, q, qe, qend, chunks, m0, M, part);
+      while (q < qe && qend <= f + n)
+        if (++q < qe) qend += chunks[q].rec_count;
+    }
+    __syncthreads();
   }
 }
 
-// TT and K for M targets, nchunks chunks of nrec records in all: the least
-// modelled time on a device of `sms` SMs.  Units: one FP64 instruction of a
-// warp, of which a quarter-SM does one at a time; a record costs kEval64 at 32
-// targets, an ordered addition 1.  A block's quarter does one warp's
-// evaluations per batch and, every fourth batch, the additions; a wave of
-// blocks is kWave64 per SM.
-constexpr int kEval64 = 211, kWave64 = 4;
-void pick_tile64(int M, int nchunks, int64_t nrec, int sms, int& lgTT, int& K) {
-  const double C = (double)nrec / nchunks;
-  double best = 0.0;
-  for (int lg = 0; (1 << lg) <= kMaxTT; ++lg) {
-    const int TT = 1 << lg, S = kThreads64 / TT;
-    const int64_t tiles = ((int64_t)M + TT - 1) / TT;
-    for (int k = 1;; k *= 2) {
-      const int64_t blocks = tiles * ((nchunks + k - 1) / k);
-      const double batches = std::max(1.0, std::ceil(std::min<double>(k, nchunks) * C / S));
-      const double perBatch = kEval64 + std::min<double>(S, C * std::min(k, nchunks)) * ((3 * TT + 31) / 32);
-      const double full = (double)blocks / ((double)sms * kWave64);
-      // below a wave the busiest SM decides, above it the average with half a block's tail
-      const double rounds = full <= 1.0 ? std::ceil((double)blocks / sms) : kWave64 * (full + 0.5);
-      const double T = rounds * batches * perBatch;
-      if (best == 0.0 || T < best * 0.999) {
-        best = T;
-        lgTT = lg;
-        K = k;
+// Between the first barrier of a batch and the second: corners 2 of the batch
+// and the contributions of the one before; between the second and the next
+// first: its edges and the additions of the one before.
+__global__ void __launch_bounds__(kThreadsLattice64) k_lattice64(const double* __restrict__ rec, const int* __restrict__ share,
+                                                         const Chunk* __restrict__ chunks, int nchunks, int K,
+                                                         const double* __restrict__ P, int M, int lgTT, int L,
+                                                         double* __restrict__ part) {
+  extern __shared__ double sm[];
+  constexpr int NT = kThreadsLattice64;
+  constexpr int B = 3 * NT;  // a batch's vectors in doubles, [s][component][t]
+  const int TT = 1 << lgTT, S = NT >> lgTT;
+  const int slots = L + S;
+  double* acc = sm;                 // the open chunk's sums [component][t]
+  double* C = acc + 3 * kMaxTT;     // contributions
+  double* O = C + B;         // edges 0 and 3 of the rings that do not share them
+  double* E1 = O + 2 * B;    // edge 1 of two batches
+  double* U = E1 + 2 * B;    // corner 2's unit vector of the last records [slot][component][t]
+  double* E2 = U + (size_t)3 * slots * TT;  // edge 2 of the last records
+  const exact64::Unit u = exact64::load_unit();
+  const int t = threadIdx.x & (TT - 1), s = threadIdx.x >> lgTT;
+  const int m0 = blockIdx.x * TT;
+  const int m = min(m0 + t, M - 1);
+  int q = blockIdx.y * K;
+  const int qe = min(q + K, nchunks);
+  const int r0 = chunks[q].rec_begin;
+  const int r1 = chunks[qe - 1].rec_begin + chunks[qe - 1].rec_count;
+  const d3 p = mk3(P[3 * (size_t)m], P[3 * (size_t)m + 1], P[3 * (size_t)m + 2]);
+  if (threadIdx.x < 3 * TT) acc[threadIdx.x] = 0.0;
+  int qend = r0 + chunks[q].rec_count;
+  auto put = [&](double* a, d3 v) {
+    a[0] = v.x;
+    a[TT] = v.y;
+    a[2 * TT] = v.z;
+  };
+  auto take = [&](const double* a) { return mk3(a[0], a[TT], a[2 * TT]); };
+  // what ring r shares with the rings of this run
+  auto shared_bits = [&](int r) {
+    int b = share[r];
+    if (r - 1 < r0) b &= ~(kShareC3 | kShareE3);
+    if (r - L < r0) b &= ~(kShareC1 | kShareE0);
+    return b;
+  };
+  const int nb = (r1 - r0 + S - 1) / S;
+  int slot = s, base = 0;  // this record's slot, and the first one's of the batch before
+  for (int b = 0; b <= nb; ++b) {
+    const int r = r0 + b * S + s, at = 3 * TT * s + t;
+    const double* R = rec + (size_t)r * kRec64;
+    const bool live = r < r1;
+    const bool fil = live && is_fil(R);
+    corner64 c2;
+    if (live && !fil) {
+      c2 = exact64::make_corner(u, p, mk3(R[6], R[7], R[8]));
+      put(U + 3 * TT * slot + t, c2.u);
+    }
+    const int f = r0 + (b - 1) * S, n = min(S, r1 - f);  // the batch before
+    if (b > 0) {
+      for (int i = threadIdx.x; i < 3 * TT * n; i += NT) {
+        const int si = (i >> lgTT) / 3, ri = f + si, ct = i - 3 * TT * si;
+        const double* Ri = rec + (size_t)ri * kRec64;
+        double v = O[i];
+        if (!is_fil(Ri)) {
+          const int sh = shared_bits(ri);
+          int at2 = base + si;
+          at2 -= at2 >= slots ? slots : 0;
+          if (sh & kShareE0) v = -E2[3 * TT * (at2 >= L ? at2 - L : at2 - L + slots) + ct];
+          const double* e1 = E1 + ((b - 1) & 1) * B;
+          const double e3 = !(sh & kShareE3) ? O[B + i] : si ? -e1[i - 3 * TT] : -E1[(b & 1) * B + 3 * TT * (S - 1) + ct];
+          v = exact64::add(u, exact64::add(u, exact64::add(u, v, e1[i]), E2[3 * TT * at2 + ct]), e3);
+        }
+        C[i] = skipped(Ri) ? 0.0 : exact64::mul(u, v, Ri[16]);
       }
-      if (k >= nchunks || k >= 8) break;
+      base += S;
+      base -= base >= slots ? slots : 0;
+    }
+    __syncthreads();
+    if (live) {
+      if (fil) {
+        put(O + at, exact64::fil_vind(u, p, mk3(R[0], R[1], R[2]), mk3(R[3], R[4], R[5]), R[12]));
+      } else {
+        const int sh = shared_bits(r);
+        const d3 p1 = mk3(R[3], R[4], R[5]), p3 = mk3(R[9], R[10], R[11]);
+        corner64 c1, c3;
+        if (sh & kShareC1) {
+          c1.r = exact64::sub(u, p, p1);
+          c1.u = take(U + 3 * TT * (slot >= L ? slot - L : slot - L + slots) + t);
+        } else {
+          c1 = exact64::make_corner(u, p, p1);
+        }
+        put(E1 + (b & 1) * B + at, exact64::vf_vind(u, c1, c2, R[13]));
+        if (sh & kShareC3) {
+          c3.r = exact64::sub(u, p, p3);
+          c3.u = take(U + 3 * TT * (slot ? slot - 1 : slots - 1) + t);
+        } else {
+          c3 = exact64::make_corner(u, p, p3);
+        }
+        put(E2 + 3 * TT * slot + t, exact64::vf_vind(u, c2, c3, R[14]));
+        if ((sh & (kShareE0 | kShareE3)) != (kShareE0 | kShareE3)) {
+          const corner64 c0 = exact64::make_corner(u, p, mk3(R[0], R[1], R[2]));
+          if (!(sh & kShareE0)) put(O + at, exact64::vf_vind(u, c0, c1, R[12]));
+          if (!(sh & kShareE3)) put(O + B + at, exact64::vf_vind(u, c3, c0, R[15]));
+        }
+      }
+    }
+    if (b > 0) {
+      add_batch64<NT>(u, C, acc, b, lgTT, f, n, q, qe, qend, chunks, m0, M, part);
+      while (q < qe && qend <= f + n)
+        if (++q < qe) qend += chunks[q].rec_count;
+    }
+    slot += S;
+    slot -= slot >= slots ? slots : 0;
+    __syncthreads();
+  }
+}
+
+// TT and K for M targets, nchunks chunks of nrec records in all, in sheets of L
+// rows (0: rings one by one): the least modelled time on a device of `sms` SMs.
+// A batch of a block that shares its quarters with w warps takes lat + w slope
+// cycles (fitted to sweeps over TT and K from 52 to 60000 targets and 52 to 12480
+// records; slope is its FP64 instructions, lat the chain of one evaluation),
+// a run's first column of a sheet's edges a half more, and an ordered addition
+// 90 in the warp whose turn it is.  Few targets and chunks get one target a
+// block (a wing's 52 rings at 52 points: 52 blocks whose threads take a record
+// each, 18 us; 906 us in one block of a thread per target), many get 4 to 16.
+struct Tile64 {
+  int lgTT = 0, K = 1;
+};
+constexpr size_t kSmemPerSm64 = 227 * 1024;
+inline size_t lattice_smem64(int lgTT, int L) {
+  const int TT = 1 << lgTT, nt = kThreadsLattice64;
+  return sizeof(double) * (3 * kMaxTT + (size_t)15 * nt + (size_t)6 * TT * (L + nt / TT));
+}
+Tile64 pick_tile64(int M, int nchunks, int64_t nrec, int L, int sms) {
+  const int nt = L > 0 ? kThreadsLattice64 : kThreads64;
+  const double C = (double)nrec / nchunks, wb = nt / 128;
+  double best = 0.0;
+  Tile64 T;
+  for (int lg = 0; (1 << lg) <= kMaxTT; ++lg) {
+    const int TT = 1 << lg, S = nt / TT;
+    const double tiles = (double)(((int64_t)M + TT - 1) / TT);
+    int bps = 5;  // by their registers
+    if (L > 0) bps = std::min<int>(2, (int)(kSmemPerSm64 / (lattice_smem64(lg, L) + 1024)));
+    if (bps < 1) break;
+    for (int k = 1;; k *= 2) {
+      const double runs = (nchunks + k - 1) / k, recs = std::min(k, nchunks) * C;
+      const double batches = std::ceil(recs / S) + 0.3;
+      const double lat = L > 0 ? 7700 : 11500, slope = L > 0 ? 8000 + 3200 * std::min(1.0, L / recs) : 13600;
+      const double add = 90.0 * std::min<double>(S, recs);
+      const double X = tiles * runs / sms;  // blocks per SM
+      double t;
+      if (X <= bps) t = batches * (lat + slope * wb * std::ceil(X) + add);
+      else t = (tiles * (nrec / (double)S + 0.8 * runs) / sms / bps + 0.15 * batches) * (lat + slope * wb * bps + add);
+      if (best == 0.0 || t < best * 0.999) {
+        best = t;
+        T.lgTT = lg;
+        T.K = k;
+      }
+      if (k >= nchunks || k >= 32) break;
     }
   }
+  return T;
 }
 
 __global__ void k_combine(const double* __restrict__ part, int M, const Group* __restrict__ groups, int ngroups,
@@ -355,16 +553,55 @@ int build_chunks(Group* groups, int ngroups, int chunk_size, Chunk* chunks, int 
   return nq;
 }
 
+namespace {
+dim3 grid64(const Tile64& T, int M, int nchunks, int& K) {
+  K = std::max(T.K, (nchunks + 65534) / 65535);  // the grid's second dimension ends at 65535
+  return dim3((unsigned)(((int64_t)M + (1 << T.lgTT) - 1) >> T.lgTT), (unsigned)((nchunks + K - 1) / K));
+}
+// the dynamic shared-memory opt-in is per device; set it once on each
+void lattice_attr64() {
+  static std::atomic<bool> attr[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && attr[dev].load(std::memory_order_acquire)) return;
+  cudaFuncSetAttribute(k_lattice64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemPerSm64);
+  if (dev >= 0 && dev < 64) attr[dev].store(true, std::memory_order_release);
+}
+void launch_rings64(const Tile64& T, const double* rec, const Chunk* chunks, int nchunks, const double* P, int M,
+                    double* part, cudaStream_t s) {
+  int K = 1;
+  const dim3 grid = grid64(T, M, nchunks, K);
+  k_rings64<<<grid, kThreads64, 0, s>>>(rec, chunks, nchunks, K, P, M, T.lgTT, part);
+}
+void launch_lattice64(const Tile64& T, const double* rec, const int* share, const Chunk* chunks, int nchunks, int L,
+                      const double* P, int M, double* part, cudaStream_t s) {
+  int K = 1;
+  const dim3 grid = grid64(T, M, nchunks, K);
+  k_lattice64<<<grid, kThreadsLattice64, lattice_smem64(T.lgTT, L), s>>>(rec, share, chunks, nchunks, K, P, M, T.lgTT,
+                                                                         L, part);
+}
+}  // namespace
+
 void launch_partial64(const double* rec, const Chunk* chunks, int nchunks, int64_t nrec, const double* P, int M,
                       double* part, cudaStream_t s) {
   if (M <= 0 || nchunks <= 0) return;
-  int lgTT = 0, K = 1;
-  pick_tile64(M, nchunks, nrec, device_sm_count(), lgTT, K);
-  // the grid's second dimension ends at 65535
-  K = std::max(K, (nchunks + 65534) / 65535);
-  dim3 grid((unsigned)(((int64_t)M + (1 << lgTT) - 1) >> lgTT), (unsigned)((nchunks + K - 1) / K));
   count_launch();
-  k_partial64<<<grid, kThreads64, 0, s>>>(rec, chunks, nchunks, K, P, M, lgTT, part);
+  launch_rings64(pick_tile64(M, nchunks, nrec, 0, device_sm_count()), rec, chunks, nchunks, P, M, part, s);
+}
+
+void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunks, int nrec, const Group* groups,
+                              int ngroups, int L, int* share, const double* P, int M, double* part, cudaStream_t s) {
+  // a sheet too tall for shared memory even with one target a block has no
+  // room for a column's edges
+  if (L <= 0 || lattice_smem64(0, L) + 1024 > kSmemPerSm64) {
+    launch_partial64(rec, chunks, nchunks, nrec, P, M, part, s);
+    return;
+  }
+  if (M <= 0 || nchunks <= 0) return;
+  lattice_attr64();
+  count_launches(2);
+  k_share64<<<(nrec + 255) / 256, 256, 0, s>>>(rec, nrec, groups, ngroups, L, share);
+  launch_lattice64(pick_tile64(M, nchunks, nrec, L, device_sm_count()), rec, share, chunks, nchunks, L, P, M, part, s);
 }
 
 void launch_combine(const double* part, int M, const Group* groups, int ngroups, int mode, double* out,

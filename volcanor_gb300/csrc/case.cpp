@@ -56,6 +56,7 @@ struct EvalPlan {
   int nrec = 0;
   int maxq = 0;   // most chunks of one group
   int shape = 0;  // FP32 kernel tile shape (launch_partial32)
+  int rows = 0;   // rows of its near-wake sheets (0: it has none)
 };
 struct StepPlan {
   int rowNear = 0, rowFar = 0;
@@ -173,6 +174,7 @@ struct Case {
     }
     e.ngroups = (int)hGroups.size() - e.goff;
     e.nrec = rec;
+    e.rows = farMode == 2 ? 0 : NW - (rowNear - 1);
     e.coff = (int)hChunks.size();
     std::vector<Chunk> tmp(rec + e.ngroups + 1);
     const int nq = force64 ? build_chunks(hGroups.data() + e.goff, e.ngroups, chunk64, tmp.data(), (int)tmp.size())
@@ -433,6 +435,7 @@ struct Case {
     s.rec64 = dalloc<double>((size_t)maxRecords * kRec64, scratchOwned);
     s.rec32 = dalloc<float>((size_t)maxRecords * kRec32, scratchOwned);
     s.edgeW = lattice() ? dalloc<double>((size_t)maxRecords * 4, scratchOwned) : nullptr;
+    s.share = opt.precision == VLM_PREC_FP64 ? dalloc<int>((size_t)maxRecords, scratchOwned) : nullptr;
     s.targets = dalloc<double>((size_t)maxTargets * 3, scratchOwned);
     s.outv = dalloc<double>((size_t)maxTargets * 3, scratchOwned);
     s.part = dalloc<double>((size_t)maxPart * 3, scratchOwned);
@@ -512,6 +515,12 @@ struct Case {
     count_launches(graphKernels);
   }
 
+  // FP64 chunk sums of plan e's gathered records at the M targets P
+  void partial64(const EvalPlan& e, const Chunk* ch, const double* P, int M) {
+    if (s.share) launch_partial64_lattice(s.rec64, ch, e.nchunks, e.nrec, dGroups + e.goff, e.ngroups, e.rows, s.share, P, M, s.part, stream);
+    else launch_partial64(s.rec64, ch, e.nchunks, e.nrec, P, M, s.part, stream);
+  }
+
   // one Biot-Savart evaluation of plan e (its records already gathered) at the
   // M targets P into out; prec -1 = the case's precision
   void evaluate(const EvalPlan& e, int M, int mode, const double* P = nullptr, double* out = nullptr, int prec = -1,
@@ -521,7 +530,7 @@ struct Case {
     if (prec < 0) prec = opt.precision;
     const Chunk* ch = dChunks + e.coff;
     if (prec == VLM_PREC_FP64) {
-      launch_partial64(s.rec64, ch, e.nchunks, e.nrec, P, M, s.part, stream);
+      partial64(e, ch, P, M);
     } else {
       const bool nearOn = prec == VLM_PREC_FP32_NEAR64;
       launch_pack32(s.rec64, e.nrec, nearOn ? opt.near_factor : 0.0, s.rec32, stream, s.edgeW);
@@ -1101,6 +1110,7 @@ struct Case {
     hGroups.insert(hGroups.end(), comb.begin(), comb.end());
     e.ngroups = (int)comb.size();
     e.nrec = rec;
+    e.rows = kind == 0 ? 0 : d.NW - (plans[k].rowNear - 1);
     e.coff = (int)hChunks.size();
     std::vector<Chunk> tmp(rec + e.ngroups + 1);
     const int nq = chunkTable(hGroups.data() + e.goff, e.ngroups, M, tmp.data(), (int)tmp.size());
@@ -1946,7 +1956,7 @@ struct Case {
       profileWork[1] = fils * M;
     }
     auto launch = [&]() {
-      if (opt.precision == VLM_PREC_FP64) launch_partial64(s.rec64, ch, pl.node.nchunks, pl.node.nrec, s.targets, M, s.part, stream);
+      if (opt.precision == VLM_PREC_FP64) partial64(pl.node, ch, s.targets, M);
       else {
         VLM_CUDA(cudaMemsetAsync(s.err + 3, 0, sizeof(int), stream));
         launch_partial32(s.rec32, s.rec64, ch, pl.node.nchunks, pl.node.nrec, s.targets, M, s.part, s.err + 2,

@@ -114,10 +114,13 @@ struct Root {
 constexpr uint32_t kSqrtLo = (1023u - 400u) << 20, kSqrtHi = (1023u + 400u) << 20;
 VLM_HD bool in_range(double x) { return high(x) - kSqrtLo < kSqrtHi - kSqrtLo; }
 constexpr uint32_t kDivLo = (1023u - 800u) << 20, kDivHi = (1023u + 700u) << 20;
-VLM_HD bool div_in_range(double a) {
+// whether a is +-0, told from its two words (a comparison of the whole would
+// become one on the FP64 unit)
+VLM_HD bool is_zero(double a) {
   const uint64_t u = bits(a);
-  return ((uint32_t)(u >> 32) & 0x7fffffffu) - kDivLo < kDivHi - kDivLo || (u << 1) == 0;
+  return (((uint32_t)(u >> 32) << 1) | (uint32_t)u) == 0u;
 }
+VLM_HD bool div_in_range(double a) { return (high(a) & 0x7fffffffu) - kDivLo < kDivHi - kDivLo || is_zero(a); }
 
 // sqrt(x), in_range(x)
 VLM_HD Root root_of(double x) {
@@ -175,41 +178,94 @@ VLM_HD double divide(double a, const Root& r, uint64_t Z) {
   if (rem2 < -(int64_t)r.N) --q;
   const uint32_t e = ((uint32_t)(u >> 52) & 0x7ffu) - (uint32_t)r.exp - up - 1u;
   const uint64_t w = (((uint64_t)e << 52) + q) | (u & 0x8000000000000000ull);
-  return (u << 1) == 0 ? a : from_bits(w);
+  return is_zero(a) ? a : from_bits(w);
 }
 
 // ---- the Biot-Savart functions of vlm_math.h with these roots and divisions ----
 // The same operations in the same order, so the same bits; numbers outside the
 // ranges above (a target on a corner, coordinates beyond 1e60) take
 // vlm_math.h's own functions.
+//
+// Every sum and product is a fused multiply-add of three registers, a 1 + b and
+// a b - 0, which round the same: the FP64 unit takes those in 64 cycles a warp
+// and quarter-SM, but an add, a multiply, or a fused multiply-add with a
+// constant operand in 76 (measured).  Unit holds the 1 and the -0 in registers
+// the compiler cannot see into; device code fills it with load_unit().
+struct Unit {
+  double one, nz;
+};
+#if defined(__CUDACC__)
+static __device__ double g_unit64[2] = {1.0, -0.0};
+__device__ __forceinline__ Unit load_unit() {
+  const volatile double* p = g_unit64;
+  Unit k;
+  k.one = p[0];
+  k.nz = p[1];
+  return k;
+}
+#endif
+VLM_HD double add(const Unit& k, double a, double b) {
+#if defined(__CUDA_ARCH__)
+  return __fma_rn(a, k.one, b);
+#else
+  (void)k;
+  return a + b;
+#endif
+}
+VLM_HD double mul(const Unit& k, double a, double b) {
+#if defined(__CUDA_ARCH__)
+  return __fma_rn(a, b, k.nz);
+#else
+  (void)k;
+  return a * b;
+#endif
+}
+VLM_HD double sub(const Unit& k, double a, double b) { return add(k, a, -b); }
+VLM_HD d3 add(const Unit& k, d3 a, d3 b) { return mk3(add(k, a.x, b.x), add(k, a.y, b.y), add(k, a.z, b.z)); }
+VLM_HD d3 sub(const Unit& k, d3 a, d3 b) { return mk3(sub(k, a.x, b.x), sub(k, a.y, b.y), sub(k, a.z, b.z)); }
+VLM_HD d3 mul(const Unit& k, d3 a, double s) { return mk3(mul(k, a.x, s), mul(k, a.y, s), mul(k, a.z, s)); }
+VLM_HD double dot(const Unit& k, d3 a, d3 b) {
+  return add(k, add(k, mul(k, a.x, b.x), mul(k, a.y, b.y)), mul(k, a.z, b.z));
+}
+VLM_HD d3 cross(const Unit& k, d3 a, d3 b) {
+  return mk3(sub(k, mul(k, a.y, b.z), mul(k, a.z, b.y)), sub(k, mul(k, a.z, b.x), mul(k, a.x, b.z)),
+             sub(k, mul(k, a.x, b.y), mul(k, a.y, b.x)));
+}
+// x > kEps^2 for x >= 0 or NaN (false), compared as integers
+VLM_HD bool above_eps2(double x) {
+  const uint64_t lo = 0x3970000000000000ull;  // 2^-104
+  return bits(x) - (lo + 1) <= 0x7ff0000000000000ull - (lo + 1);
+}
 
-VLM_HD corner64 make_corner(d3 P, d3 c) {
-  corner64 k;
-  k.r = P - c;
-  const double x = sumsq3(k.r);
-  if (in_range(x) && div_in_range(k.r.x) && div_in_range(k.r.y) && div_in_range(k.r.z)) {
+VLM_HD corner64 make_corner(const Unit& k, d3 P, d3 c) {
+  corner64 o;
+  o.r = sub(k, P, c);
+  const double x = dot(k, o.r, o.r);
+  if (in_range(x) && div_in_range(o.r.x) && div_in_range(o.r.y) && div_in_range(o.r.z)) {
     const Root n = root_of(x);
     // |r| > kEps = 2^-52
     if (n.exp > -52 || (n.exp == -52 && n.N > 0x10000000000000ull)) {
       const uint64_t Z = reciprocal(n);
-      k.u = mk3(divide(k.r.x, n, Z), divide(k.r.y, n, Z), divide(k.r.z, n, Z));
+      o.u = mk3(divide(o.r.x, n, Z), divide(o.r.y, n, Z), divide(o.r.z, n, Z));
     } else {
-      k.u = zero3();
+      o.u = zero3();
     }
   } else {
-    k.u = unit3(k.r);
+    o.u = unit3(o.r);
   }
-  return k;
+  return o;
 }
 VLM_HD double root(double x) { return in_range(x) ? value(root_of(x)) : sqrt(x); }
-VLM_HD d3 vf_vind(const corner64& a, const corner64& b, double rvc) {
-  const d3 r0 = a.r - b.r;
-  const d3 c = cross3(a.r, b.r);
-  const double c2 = dot3(c, c);
-  if (!(c2 > kEps * kEps)) return zero3();
-  const double d = dot3(r0, a.u - b.u);
-  const double den2 = pow4(rvc * root(sumsq3(r0))) + c2 * c2;
-  const d3 v = mk3((c.x * kInv4Pi) * d, (c.y * kInv4Pi) * d, (c.z * kInv4Pi) * d);
+VLM_HD d3 vf_vind(const Unit& k, const corner64& a, const corner64& b, double rvc) {
+  const d3 r0 = sub(k, a.r, b.r);
+  const d3 c = cross(k, a.r, b.r);
+  const double c2 = dot(k, c, c);
+  if (!above_eps2(c2)) return zero3();
+  const double d = dot(k, r0, sub(k, a.u, b.u));
+  const double s = mul(k, rvc, root(dot(k, r0, r0)));
+  const double s2 = mul(k, s, s);
+  const double den2 = add(k, mul(k, s2, s2), mul(k, c2, c2));
+  const d3 v = mul(k, mul(k, c, kInv4Pi), d);
   if (in_range(den2) && div_in_range(v.x) && div_in_range(v.y) && div_in_range(v.z)) {
     const Root n = root_of(den2);
     const uint64_t Z = reciprocal(n);
@@ -217,17 +273,19 @@ VLM_HD d3 vf_vind(const corner64& a, const corner64& b, double rvc) {
   }
   return v / sqrt(den2);
 }
-VLM_HD d3 vr_vind(d3 P, const d3* c, const double* rvc) {
-  const corner64 k0 = make_corner(P, c[0]), k1 = make_corner(P, c[1]);
-  d3 v = vf_vind(k0, k1, rvc[0]);
-  const corner64 k2 = make_corner(P, c[2]);
-  v = v + vf_vind(k1, k2, rvc[1]);
-  const corner64 k3 = make_corner(P, c[3]);
-  v = v + vf_vind(k2, k3, rvc[2]);
-  v = v + vf_vind(k3, k0, rvc[3]);
+VLM_HD d3 vr_vind(const Unit& k, d3 P, const d3* c, const double* rvc) {
+  const corner64 k0 = make_corner(k, P, c[0]), k1 = make_corner(k, P, c[1]);
+  d3 v = vf_vind(k, k0, k1, rvc[0]);
+  const corner64 k2 = make_corner(k, P, c[2]);
+  v = add(k, v, vf_vind(k, k1, k2, rvc[1]));
+  const corner64 k3 = make_corner(k, P, c[3]);
+  v = add(k, v, vf_vind(k, k2, k3, rvc[2]));
+  v = add(k, v, vf_vind(k, k3, k0, rvc[3]));
   return v;
 }
-VLM_HD d3 fil_vind(d3 P, d3 a, d3 b, double rvc) { return vf_vind(make_corner(P, a), make_corner(P, b), rvc); }
+VLM_HD d3 fil_vind(const Unit& k, d3 P, d3 a, d3 b, double rvc) {
+  return vf_vind(k, make_corner(k, P, a), make_corner(k, P, b), rvc);
+}
 
 }  // namespace exact64
 }  // namespace vlm

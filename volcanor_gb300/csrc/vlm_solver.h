@@ -105,6 +105,9 @@ struct DevState {
   // lattice-form edge weights of the gathered records ([rec][4]; null: the
   // records are evaluated ring by ring), written by the gather
   double* edgeW;
+  // FP64: which corners and filaments of a gathered record its neighbours
+  // share (launch_partial64_lattice; null in the FP32 precisions)
+  int* share;
   void* nearScratch;  // near-field grid scratch (null unless FP32 + FP64 near field)
   size_t nearBytes;
   long long* nacc;  // fixed-point near-field accumulators, zero between evaluations
