@@ -1,11 +1,20 @@
 // MLP engine of the learned far-wake surrogate (see mlp.h): FP32 CUDA-core
 // kernels for forward, backward and Adam, and the vlm_mlp_* C ABI.
 //
-// GEMM: C[M x N] = op(A)[M x K] op(B)[K x N] (+ bias, + tanh), 64 x 64 output
-// tile per 256-thread block, 4 x 4 outputs per thread, K in steps of 16
-// through shared memory.  Each output sums k = 0..K-1 in order, so results
-// (and the batch reductions of the weight gradients, which are GEMMs over the
-// batch) do not depend on the launch configuration.
+// GEMM: C[M x N] = op(A)[M x K] op(B)[K x N] (+ bias, + tanh; or times the
+// tanh derivative), 128 x 64 output tile per 256-thread block, 8 x 4 outputs per
+// thread (three 16-byte shared loads per 32 FMAs; 4 x 4 needed four), K in steps
+// of 16 through two shared buffers, the next step's global loads in flight behind
+// the FMAs.  Each output sums k = 0..K-1 in order, so results do not depend on
+// the launch configuration.
+//
+// The weight gradients are GEMMs over the batch (K = thousands of rows, M x N =
+// one or two tiles): one block each took 5.3 ms at 20000 rows.  They run in
+// slices of the batch, one block per tile and slice, whose sums (and the bias
+// gradients', summed from the same staged rows) one kernel adds in slice order.
+// The slices depend on the batch size and the network alone, so training is
+// reproducible.  20000 rows of a 12-128-128-128-3 network from host arrays:
+// 12.8 -> 0.40 ms, gradient error against 64 bits 2.1e-6 -> 4.3e-7.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -32,76 +41,98 @@ namespace {
     if (e_ != cudaSuccess) throw std::runtime_error(std::string("CUDA: ") + cudaGetErrorString(e_)); \
   } while (0)
 
-enum { EPI_NONE = 0, EPI_BIAS = 1, EPI_BIAS_TANH = 2 };
+enum { EPI_NONE = 0, EPI_BIAS = 1, EPI_BIAS_TANH = 2, EPI_TANH_BACK = 3 };
+constexpr int kBM = 128, kBN = 64, kBK = 16;
 
-template <bool TA, bool TB, int EPI>
+// bias: the row vector added (EPI_BIAS*); H: activations whose tanh derivative
+// 1 - H^2 multiplies the result (EPI_TANH_BACK, laid out as C).  SLICES: the
+// block sums rows kslice blockIdx.z .. of the K dimension only, into its own copy
+// of C (cstride floats apart), and with rowsum the column sums of A as well.
+template <bool TA, bool TB, int EPI, bool SLICES>
 __global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float* __restrict__ A, int lda,
                                               const float* __restrict__ B, int ldb, float* __restrict__ C, int ldc,
-                                              const float* __restrict__ bias) {
-  __shared__ float As[16][64 + 4];
-  __shared__ float Bs[16][64 + 4];
+                                              const float* __restrict__ bias, const float* __restrict__ H, int kslice,
+                                              int64_t cstride, float* __restrict__ rowsum) {
+  __shared__ __align__(16) float As[2][kBK][kBM + 4];
+  __shared__ __align__(16) float Bs[2][kBK][kBN + 4];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  float acc[4][4];
+  const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
+  const int kb = SLICES ? (int)blockIdx.z * kslice : 0, ke = SLICES ? min(K, kb + kslice) : K;
+  float acc[8][4], rs[8];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 8; ++i) {
+    rs[i] = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    for (int e = threadIdx.x; e < 1024; e += 256) {
-      int mm, kk;
-      if (TA) {
-        mm = e & 63;
-        kk = e >> 6;
-      } else {
-        kk = e & 15;
-        mm = e >> 4;
-      }
+  }
+  float ra[8], rb[4];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int e = threadIdx.x + 256 * q;
+      const int mm = TA ? e & (kBM - 1) : e >> 4, kk = TA ? e >> 7 : e & 15;
       const int gm = m0 + mm, gk = k0 + kk;
-      float a = 0.f;
-      if (gm < M && gk < K) a = TA ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk];
-      As[kk][mm] = a;
+      ra[q] = gm < M && gk < ke ? (TA ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk]) : 0.f;
     }
-    for (int e = threadIdx.x; e < 1024; e += 256) {
-      int nn, kk;
-      if (TB) {
-        kk = e & 15;
-        nn = e >> 4;
-      } else {
-        nn = e & 63;
-        kk = e >> 6;
-      }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = threadIdx.x + 256 * q;
+      const int nn = TB ? e >> 4 : e & (kBN - 1), kk = TB ? e & 15 : e >> 6;
       const int gn = n0 + nn, gk = k0 + kk;
-      float b = 0.f;
-      if (gn < N && gk < K) b = TB ? B[(size_t)gn * ldb + gk] : B[(size_t)gk * ldb + gn];
-      Bs[kk][nn] = b;
+      rb[q] = gn < N && gk < ke ? (TB ? B[(size_t)gn * ldb + gk] : B[(size_t)gk * ldb + gn]) : 0.f;
     }
-    __syncthreads();
+  };
+  auto stage = [&](int buf) {
 #pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      float a[4], b[4];
+    for (int q = 0; q < 8; ++q) {
+      const int e = threadIdx.x + 256 * q;
+      As[buf][TA ? e >> 7 : e & 15][TA ? e & (kBM - 1) : e >> 4] = ra[q];
+    }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
+    for (int q = 0; q < 4; ++q) {
+      const int e = threadIdx.x + 256 * q;
+      Bs[buf][TB ? e & 15 : e >> 6][TB ? e >> 4 : e & (kBN - 1)] = rb[q];
+    }
+  };
+  fetch(kb);
+  stage(0);
+  __syncthreads();
+  for (int k0 = kb, buf = 0; k0 < ke; k0 += kBK, buf ^= 1) {
+    const bool more = k0 + kBK < ke;
+    if (more) fetch(k0 + kBK);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
+    for (int kk = 0; kk < kBK; ++kk) {
+      float a[8], b[4];
+      *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 8]);
+      *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 8 + 4]);
+      *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&Bs[buf][kk][tx * 4]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 8; ++i) {
+        if (SLICES) rs[i] += a[i];
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+      }
     }
+    if (more) stage(buf ^ 1);
     __syncthreads();
   }
+  if (SLICES) C += (int64_t)blockIdx.z * cstride;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + ty * 4 + i;
+  for (int i = 0; i < 8; ++i) {
+    const int gm = m0 + ty * 8 + i;
     if (gm >= M) continue;
+    if (SLICES && n0 == 0 && tx == 0) rowsum[(int64_t)blockIdx.z * cstride + gm] = rs[i];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int gn = n0 + tx * 4 + j;
       if (gn >= N) continue;
       float c = acc[i][j];
-      if (EPI >= EPI_BIAS) c += bias[gn];
+      if (EPI == EPI_BIAS || EPI == EPI_BIAS_TANH) c += bias[gn];
       if (EPI == EPI_BIAS_TANH) c = tanhf(c);
+      if (EPI == EPI_TANH_BACK) {
+        const float h = H[(size_t)gm * ldc + gn];
+        c = c * (1.f - h * h);
+      }
       C[(size_t)gm * ldc + gn] = c;
     }
   }
@@ -109,29 +140,31 @@ __global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float* 
 
 template <bool TA, bool TB, int EPI>
 void gemm(cudaStream_t st, int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
-          const float* bias) {
+          const float* bias, const float* H = nullptr) {
   if (M <= 0 || N <= 0) return;
-  dim3 grid((N + 63) / 64, (M + 63) / 64);
+  dim3 grid((N + kBN - 1) / kBN, (M + kBM - 1) / kBM);
   count_launch();
-  k_gemm<TA, TB, EPI><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, bias);
+  k_gemm<TA, TB, EPI, false><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, H, 0, 0, nullptr);
 }
 
-// dH <- dH * (1 - H^2): gradient through tanh, in place
-__global__ void k_tanh_back(float* __restrict__ dH, const float* __restrict__ H, int64_t n) {
+// Rows of the batch a slice of the weight gradients sums: 128 (enough slices to
+// fill the device from about 10000 rows on), more when that made over 64 slices
+// or over 2^26 partial sums (a wide network's tiles fill the device by themselves).
+int slice_rows(int n, int64_t nparam) {
+  const int most = (int)std::max<int64_t>(1, std::min<int64_t>(64, ((int64_t)1 << 26) / nparam));
+  const int r = std::max(128, (n + most - 1) / most);
+  return (r + kBK - 1) / kBK * kBK;
+}
+
+// g[i] = the slices' sums added in slice order
+__global__ void k_sum_slices(const float* __restrict__ part, int64_t stride, int slices, int64_t n,
+                             float* __restrict__ g) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n) {
-    const float h = H[i];
-    dH[i] = dH[i] * (1.f - h * h);
-  }
-}
-
-// out[c] = sum over rows r (in order) of X[r * ld + c]
-__global__ void k_colsum(const float* __restrict__ X, int rows, int cols, int ld, float* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float s = 0.f;
-  for (int r = 0; r < rows; ++r) s += X[(size_t)r * ld + c];
-  out[c] = s;
+  if (i >= n) return;
+  float s = part[i];
+#pragma unroll 8
+  for (int k = 1; k < slices; ++k) s += part[(int64_t)k * stride + i];
+  g[i] = s;
 }
 
 // dY = 2 (Y - T) / (rows x cols); per-block partial sums of (Y - T)^2
@@ -239,9 +272,10 @@ bool Mlp::setTensorCores(bool on) {
 }
 
 void Mlp::destroy() {
-  for (float* q : {p, g, m, v, act, dact, loss, part})
+  for (float* q : {p, g, m, v, act, dact, loss, part, gpart})
     if (q) cudaFree(q);
-  p = g = m = v = act = dact = loss = part = nullptr;
+  p = g = m = v = act = dact = loss = part = gpart = nullptr;
+  gslices = 0;
   if (tcImg) cudaFree(tcImg);
   if (tcErr) cudaFree(tcErr);
   tcImg = nullptr;
@@ -307,23 +341,30 @@ void Mlp::grad(const float* X, const float* T, int n) {
   count_launch();
   k_sum_parts<<<1, 32, 0, st>>>(part, nb, 1.f / (float)ny, loss);
   // backward
+  const int rows = slice_rows(n, sh.nparam), slices = (n + rows - 1) / rows;
+  if (slices > gslices) {
+    if (gpart) MLP_CUDA(cudaFree(gpart));
+    gpart = nullptr;
+    gslices = 0;
+    MLP_CUDA(cudaMalloc(&gpart, sizeof(float) * (size_t)sh.nparam * slices));
+    gslices = slices;
+  }
   for (int l = sh.nl - 1; l >= 0; --l) {
     const int in = sh.sz[l], o = sh.sz[l + 1];
-    if (l < sh.nl - 1) {
-      const int64_t cnt = (int64_t)n * o;
-      count_launch();
-      k_tanh_back<<<(unsigned)((cnt + 255) / 256), 256, 0, st>>>(dZ, Hs[l + 1], cnt);
-    }
-    // dW = dZ^T H_prev, db = column sums of dZ
-    gemm<true, false, EPI_NONE>(st, o, in, n, dZ, o, Hs[l], in, g + sh.woff[l], in, nullptr);
+    // dW = dZ^T H_prev and db = column sums of dZ, in slices of the batch
+    dim3 grid((in + kBN - 1) / kBN, (o + kBM - 1) / kBM, slices);
     count_launch();
-    k_colsum<<<(o + 127) / 128, 128, 0, st>>>(dZ, n, o, o, g + sh.boff[l]);
+    k_gemm<true, false, EPI_NONE, true><<<grid, 256, 0, st>>>(o, in, n, dZ, o, Hs[l], in, gpart + sh.woff[l], in,
+                                                             nullptr, nullptr, rows, sh.nparam, gpart + sh.boff[l]);
     if (l > 0) {
       float* dH = (dZ == dact) ? dact + (size_t)cap * sh.maxw : dact;
-      gemm<false, false, EPI_NONE>(st, n, in, o, dZ, o, p + sh.woff[l], in, dH, in, nullptr);
+      // through the weights and the layer below's tanh
+      gemm<false, false, EPI_TANH_BACK>(st, n, in, o, dZ, o, p + sh.woff[l], in, dH, in, nullptr, Hs[l]);
       dZ = dH;
     }
   }
+  count_launch();
+  k_sum_slices<<<(unsigned)((sh.nparam + 255) / 256), 256, 0, st>>>(gpart, sh.nparam, slices, sh.nparam, g);
 }
 
 void Mlp::adam(float lr, float b1, float b2, float eps) {

@@ -58,6 +58,8 @@ struct Mlp {
   float* dact = nullptr;   // two [batch x maxw] gradient buffers
   float* loss = nullptr;   // [2]: loss of the last batch, scratch
   float* part = nullptr;   // per-block loss partials
+  float* gpart = nullptr;  // the gradient's sums over slices of the batch, gslices x nparam
+  int gslices = 0;
   int cap = 0;             // batch capacity of act / dact
   int64_t adamStep = 0;
   cudaStream_t st = nullptr;
