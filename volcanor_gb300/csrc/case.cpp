@@ -353,6 +353,7 @@ struct Case {
     s.AICinv = dalloc<double>((size_t)d.n * d.n, owned);
     s.LU = dalloc<double>((size_t)d.n * d.n, owned);
     s.piv = dalloc<int>(d.n, owned);
+    s.luPerm = dalloc<unsigned char>(lu_scratch_bytes(), owned);
     const size_t nring = (size_t)nb * std::max(NW, 1) * ns;
     s.nC = dalloc<double>(nring * 12, owned);
     s.nCP = dalloc<double>(nring * 12, owned);
@@ -1466,14 +1467,21 @@ struct Case {
     if (started) throw StatusError(VLM_ERR_STATE, "case already started");
     if (factored) return;
     launch_aic(d, s, frame(0), stream);
+    // the FP32 factors beside the FP64 ones: both only read the AIC
+    if (refine) {
+      VLM_CUDA(cudaEventRecord(evFork, stream));
+      VLM_CUDA(cudaStreamWaitEvent(side, evFork, 0));
+      launch_lu32(d, s, side);
+      VLM_CUDA(cudaEventRecord(evJoin, side));
+    }
     launch_lu_inverse(d, s, stream);
     launch_is_inverse(d, s, stream);
+    if (refine) VLM_CUDA(cudaStreamWaitEvent(stream, evJoin, 0));
     int err = 0;
     VLM_CUDA(cudaMemcpyAsync(&err, s.err, sizeof(int), cudaMemcpyDeviceToHost, stream));
     VLM_CUDA(cudaStreamSynchronize(stream));
     if (err == 10) throw StatusError(VLM_ERR_SINGULAR, "Matrix is numerically singular!");
     if (err == 11) throw StatusError(VLM_ERR_SINGULAR, "Computed AIC_inv does not seem to be correct within given tolerance");
-    if (refine) launch_lu32(d, s, stream);
     VLM_CUDA(cudaGetLastError());
     factored = true;
   }

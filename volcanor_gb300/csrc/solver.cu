@@ -718,178 +718,12 @@ __global__ void k_aic(Dims d, DevState s, const double* fr) {
   s.AIC[row + n * (size_t)col] = dot3(v, ld3(cp + 15));
 }
 
-// Right-looking LU with partial pivoting (first index of max |a|) in one block.
-__global__ void k_lu(Dims d, DevState s) {
-  const int n = d.n;
-  double* A = s.LU;
-  __shared__ double redv[1024];
-  __shared__ int redi[1024];
-  __shared__ int pk;
-  for (long e = threadIdx.x; e < (long)n * n; e += blockDim.x) A[e] = s.AIC[e];
-  __syncthreads();
-  for (int k = 0; k < n; ++k) {
-    double bv = -1.0;
-    int bi = n;
-    for (int i = k + threadIdx.x; i < n; i += blockDim.x) {
-      const double v = fabs(A[i + (size_t)n * k]);
-      if (v > bv || (v == bv && i < bi)) {
-        bv = v;
-        bi = i;
-      }
-    }
-    redv[threadIdx.x] = bv;
-    redi[threadIdx.x] = bi;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-      if (threadIdx.x < w) {
-        const double v = redv[threadIdx.x + w];
-        const int i = redi[threadIdx.x + w];
-        if (v > redv[threadIdx.x] || (v == redv[threadIdx.x] && i < redi[threadIdx.x])) {
-          redv[threadIdx.x] = v;
-          redi[threadIdx.x] = i;
-        }
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      pk = redi[0];
-      s.piv[k] = pk;
-      if (A[pk + (size_t)n * k] == 0.0) atomicExch(s.err, 10);
-    }
-    __syncthreads();
-    const int p = pk;
-    if (p != k)
-      for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const double a = A[k + (size_t)n * j];
-        A[k + (size_t)n * j] = A[p + (size_t)n * j];
-        A[p + (size_t)n * j] = a;
-      }
-    __syncthreads();
-    const double akk = A[k + (size_t)n * k];
-    for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x) A[i + (size_t)n * k] = A[i + (size_t)n * k] / akk;
-    __syncthreads();
-    const long m = n - k - 1;
-    for (long e = threadIdx.x; e < m * m; e += blockDim.x) {
-      const int i = k + 1 + (int)(e % m), j = k + 1 + (int)(e / m);
-      A[i + (size_t)n * j] = A[i + (size_t)n * j] - A[i + (size_t)n * k] * A[k + (size_t)n * j];
-    }
-    __syncthreads();
-  }
-}
-
-// X = A^-1 column by column: forward substitution on P e_c, then backward.
-__global__ void k_inv_cols(Dims d, DevState s) {
-  const int n = d.n;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  const double* A = s.LU;
-  double* X = s.AICinv + (size_t)n * c;
-  int pos = c;  // position of the 1 in P e_c after the row interchanges
-  for (int k = 0; k < n; ++k) {
-    const int pk = s.piv[k];
-    if (pos == k) pos = pk;
-    else if (pos == pk) pos = k;
-  }
-  for (int i = 0; i < n; ++i) {
-    double sum = i == pos ? 1.0 : 0.0;
-    for (int k = 0; k < i; ++k) sum = sum - A[i + (size_t)n * k] * X[k];
-    X[i] = sum;
-  }
-  for (int i = n - 1; i >= 0; --i) {
-    double sum = X[i];
-    for (int k = i + 1; k < n; ++k) sum = sum - A[i + (size_t)n * k] * X[k];
-    X[i] = sum / A[i + (size_t)n * i];
-  }
-}
-
 // ---- FP32 LU + FP64 iterative refinement ---------------------------------------
 // The AIC (FP64, assembled once like the reference) is factored in FP32 with
-// partial pivoting and inverted in FP32 (one unit column per thread); every
-// solve then refines in FP64: x <- x + inv32 (b - A x), the residual b - A x
-// in FP64.  ||I - inv32 A|| ~ cond(A) x 2^-24 << 1 for vortex-lattice AICs,
-// so each pass gains ~7 digits.
-__global__ void k_lu32(Dims d, DevState s) {
-  const int n = d.n;
-  float* A = s.LU32;
-  __shared__ float redv[1024];
-  __shared__ int redi[1024];
-  __shared__ int pk;
-  for (long e = threadIdx.x; e < (long)n * n; e += blockDim.x) A[e] = (float)s.AIC[e];
-  __syncthreads();
-  for (int k = 0; k < n; ++k) {
-    float bv = -1.f;
-    int bi = n;
-    for (int i = k + threadIdx.x; i < n; i += blockDim.x) {
-      const float v = fabsf(A[i + (size_t)n * k]);
-      if (v > bv || (v == bv && i < bi)) {
-        bv = v;
-        bi = i;
-      }
-    }
-    redv[threadIdx.x] = bv;
-    redi[threadIdx.x] = bi;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-      if (threadIdx.x < w) {
-        const float v = redv[threadIdx.x + w];
-        const int i = redi[threadIdx.x + w];
-        if (v > redv[threadIdx.x] || (v == redv[threadIdx.x] && i < redi[threadIdx.x])) {
-          redv[threadIdx.x] = v;
-          redi[threadIdx.x] = i;
-        }
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      pk = redi[0];
-      s.piv32[k] = pk;
-      if (A[pk + (size_t)n * k] == 0.f) atomicExch(s.err, 10);
-    }
-    __syncthreads();
-    const int p = pk;
-    if (p != k)
-      for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const float t = A[k + (size_t)n * j];
-        A[k + (size_t)n * j] = A[p + (size_t)n * j];
-        A[p + (size_t)n * j] = t;
-      }
-    __syncthreads();
-    const float akk = A[k + (size_t)n * k];
-    for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x) A[i + (size_t)n * k] = A[i + (size_t)n * k] / akk;
-    __syncthreads();
-    const long m = n - k - 1;
-    for (long e = threadIdx.x; e < m * m; e += blockDim.x) {
-      const int i = k + 1 + (int)(e % m), j = k + 1 + (int)(e / m);
-      A[i + (size_t)n * j] = fmaf(-A[i + (size_t)n * k], A[k + (size_t)n * j], A[i + (size_t)n * j]);
-    }
-    __syncthreads();
-  }
-}
-
-__global__ void k_inv32_cols(Dims d, DevState s) {
-  const int n = d.n;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  const float* A = s.LU32;
-  float* X = s.AICinv32 + (size_t)n * c;
-  int pos = c;
-  for (int k = 0; k < n; ++k) {
-    const int pk = s.piv32[k];
-    if (pos == k) pos = pk;
-    else if (pos == pk) pos = k;
-  }
-  for (int i = 0; i < n; ++i) {
-    float sum = i == pos ? 1.f : 0.f;
-    for (int k = 0; k < i; ++k) sum = fmaf(-A[i + (size_t)n * k], X[k], sum);
-    X[i] = sum;
-  }
-  for (int i = n - 1; i >= 0; --i) {
-    float sum = X[i];
-    for (int k = i + 1; k < n; ++k) sum = fmaf(-A[i + (size_t)n * k], X[k], sum);
-    X[i] = sum / A[i + (size_t)n * i];
-  }
-}
-
+// partial pivoting and inverted in FP32 (factor.cu); every solve then refines
+// in FP64: x <- x + inv32 (b - A x), the residual b - A x in FP64.
+// ||I - inv32 A|| ~ cond(A) x 2^-24 << 1 for vortex-lattice AICs, so each pass
+// gains ~7 digits.
 // Solve AIC gamVec = -RHS by refinement (one block); records the final
 // relative residual max|b - A x| / max|b| in s.luRes[0] and flags err[1]
 // when it stays above 1e-9.
@@ -964,19 +798,6 @@ __global__ void k_solve_refine(Dims d, DevState s) {
   __syncthreads();
   if (d.axisym)
     for (int t = d.npan + threadIdx.x; t < d.nb * d.npan; t += blockDim.x) s.wGam[t] = s.wGam[t % d.npan];
-}
-
-// libMath.f90:428-458 (tolerance 1E-04 single precision)
-__global__ void k_is_inverse(Dims d, DevState s) {
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const long n = d.n;
-  if (t >= n * n) return;
-  const int i = (int)(t % n), j = (int)(t / n);
-  double sum = 0.0;
-  for (int k = 0; k < n; ++k) sum = sum + s.AIC[i + n * (size_t)k] * s.AICinv[k + n * (size_t)j];
-  const double tol = (double)1e-4f;
-  const bool bad = (i != j) ? (sum > tol) : (sum - 1.0 > tol);
-  if (bad) atomicExch(s.err, 11);
 }
 
 // ---- circulation solve (main.f90:522-603) ------------------------------------
@@ -1671,29 +1492,12 @@ void launch_aic(const Dims& d, const DevState& s, const double* frame, cudaStrea
   count_launch();
   k_aic<<<nblk(n, 128), 128, 0, st>>>(d, s, frame);
 }
-void launch_lu_inverse(const Dims& d, const DevState& s, cudaStream_t st) {
-  count_launch();
-  k_lu<<<1, 1024, 0, st>>>(d, s);
-  count_launch();
-  k_inv_cols<<<nblk(d.n, 64), 64, 0, st>>>(d, s);
-}
-void launch_is_inverse(const Dims& d, const DevState& s, cudaStream_t st) {
-  const long n = (long)d.n * d.n;
-  count_launch();
-  k_is_inverse<<<nblk(n, 256), 256, 0, st>>>(d, s);
-}
 void launch_solve(const Dims& d, const DevState& s, const double* frame, bool withWake, cudaStream_t st) {
   count_launch();
   k_rhs<<<nblk(d.nbC * d.npan, 128), 128, 0, st>>>(d, s, frame, withWake ? 1 : 0);
   count_launch();
   if (s.LU32) k_solve_refine<<<1, 1024, 0, st>>>(d, s);
   else k_solve<<<1, 1024, 0, st>>>(d, s);
-}
-void launch_lu32(const Dims& d, const DevState& s, cudaStream_t st) {
-  count_launch();
-  k_lu32<<<1, 1024, 0, st>>>(d, s);
-  count_launch();
-  k_inv32_cols<<<nblk(d.n, 64), 64, 0, st>>>(d, s);
 }
 void launch_step_begin(const Dims& d, const DevState& s, cudaStream_t st) {
   count_launch();

@@ -78,6 +78,7 @@ struct DevState {
   double *wGam, *gamPrev, *gamVec, *gamVecPrev, *RHS, *velCP, *velCPTotal;
   double *AIC, *AICinv, *LU;
   int* piv;
+  void* luPerm;  // lu_scratch_bytes(): a panel's interchanges (FP64, FP32)
   // FP32 LU + FP64 refinement (null when the solve uses the FP64 inverse)
   float *LU32, *AICinv32;
   int* piv32;
@@ -169,6 +170,7 @@ void launch_scatter_nodes(const Dims& d, const DevState& s, const double* frame,
 
 // ---- circulation and loads -----------------------------------------------
 void launch_aic(const Dims& d, const DevState& s, const double* frame, cudaStream_t st);
+size_t lu_scratch_bytes();
 void launch_lu_inverse(const Dims& d, const DevState& s, cudaStream_t st);
 void launch_is_inverse(const Dims& d, const DevState& s, cudaStream_t st);
 // FP32 LU with partial pivoting of the AIC and its FP32 inverse (solves then
