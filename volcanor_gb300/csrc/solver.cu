@@ -5,6 +5,10 @@
 // element, exactly the IEEE operations of the reference routine it restates.
 #include <math.h>
 
+#include <algorithm>
+#include <atomic>
+
+#include "exact64.h"
 #include "vlm_math.h"
 #include "vlm_solver.h"
 
@@ -714,7 +718,7 @@ __global__ void k_aic(Dims d, DevState s, const double* fr) {
   const double* cp = panRec(d, fr, row / d.npan, row % d.npan);
   const double* w = panRec(d, fr, col / d.npan, col % d.npan);
   d3 c[4] = {ld3(w), ld3(w + 3), ld3(w + 6), ld3(w + 9)};
-  const d3 v = vr_vind64(ld3(cp + 12), c, s.wRvc + 4 * (size_t)col);
+  const d3 v = exact64::vr_vind(exact64::load_unit(), ld3(cp + 12), c, s.wRvc + 4 * (size_t)col);
   s.AIC[row + n * (size_t)col] = dot3(v, ld3(cp + 15));
 }
 
@@ -724,68 +728,64 @@ __global__ void k_aic(Dims d, DevState s, const double* fr) {
 // in FP64: x <- x + inv32 (b - A x), the residual b - A x in FP64.
 // ||I - inv32 A|| ~ cond(A) x 2^-24 << 1 for vortex-lattice AICs, so each pass
 // gains ~7 digits.
-// Solve AIC gamVec = -RHS by refinement (one block); records the final
-// relative residual max|b - A x| / max|b| in s.luRes[0] and flags err[1]
-// when it stays above 1e-9.
+// Solve AIC gamVec = -RHS by refinement; records the final relative residual
+// max|b - A x| / max|b| in s.luRes[0] and flags err[1] when it stays above 1e-9.
+// One cluster of kSolveBlocks blocks, a warp per row of the two products (lanes
+// over the columns, then a butterfly), x and r in global memory between them: on
+// one SM the FP64 product alone was n^2 / 2 cycles a pass (290 us at n = 300).
 constexpr int kRefinePasses = 3;
-__global__ void k_solve_refine(Dims d, DevState s) {
+constexpr int kSolveBlocks = 8;
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__global__ void __cluster_dims__(kSolveBlocks, 1, 1) __launch_bounds__(1024) k_solve_refine(Dims d, DevState s) {
   const int n = d.n;
-  __shared__ double red[1024];
-  double* b = s.RHS;
-  double* x = s.refX;
-  double* r = s.refR;
-  if (d.axisym)
-    for (int i = d.npan + threadIdx.x; i < n; i += blockDim.x) b[i] = b[i % d.npan];
-  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row0 = warp * kSolveBlocks + blockIdx.x, rows = 32 * kSolveBlocks;
+  const double* rhs = s.RHS;
+  volatile double* x = s.refX;
+  volatile double* r = s.refR;
+  __shared__ double red[32];
+  // b = -RHS (under axisymmetry blade 1's for every blade), and its largest magnitude, in every block
+  auto b = [&](int i) { return -1.0 * rhs[d.axisym ? i % d.npan : i]; };
+  auto block_max = [&](double v) {
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    __syncthreads();
+    if (lane == 0) red[warp] = v;
+    __syncthreads();
+    v = red[lane];
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+  };
   double bmax = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    b[i] = -1.0 * b[i];
-    x[i] = 0.0;
-    r[i] = b[i];
-    bmax = fmax(bmax, fabs(b[i]));
-  }
-  red[threadIdx.x] = bmax;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + w]);
-    __syncthreads();
-  }
-  bmax = red[0];
-  __syncthreads();
-  // one warp per row for both products, lanes over the columns, then a
-  // butterfly: latency of n/32 multiply-adds instead of n
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  double rmax = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) bmax = fmax(bmax, fabs(b(i)));
+  bmax = block_max(bmax);
   for (int pass = 0; pass < kRefinePasses; ++pass) {
-    // x += inv32 r  (FP32 products of the FP32-rounded residual, FP64 update)
-    for (int i = warp; i < n; i += nwarps) {
+    // x += inv32 r  (FP32 products of the FP32-rounded residual, FP64 update); r = b at first
+    for (int i = row0; i < n; i += rows) {
       float z = 0.f;
-      for (int j = lane; j < n; j += 32) z = fmaf(s.AICinv32[i + (size_t)n * j], (float)r[j], z);
+#pragma unroll 4
+      for (int j = lane; j < n; j += 32) z = fmaf(s.AICinv32[i + (size_t)n * j], (float)(pass ? r[j] : b(j)), z);
       for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-      if (lane == 0) x[i] += (double)z;
+      if (lane == 0) x[i] = (pass ? x[i] : 0.0) + (double)z;
     }
-    __syncthreads();
+    cluster_sync();
     // r = b - A x in FP64
-    rmax = 0.0;
-    for (int i = warp; i < n; i += nwarps) {
+    for (int i = row0; i < n; i += rows) {
       double ax = 0.0;
+#pragma unroll 4
       for (int j = lane; j < n; j += 32) ax = fma(s.AIC[i + (size_t)n * j], x[j], ax);
       for (int o = 16; o > 0; o >>= 1) ax += __shfl_xor_sync(0xffffffffu, ax, o);
-      if (lane == 0) {
-        r[i] = b[i] - ax;
-        rmax = fmax(rmax, fabs(r[i]));
-      }
+      if (lane == 0) r[i] = b(i) - ax;
     }
-    __syncthreads();
+    cluster_sync();
   }
-  red[threadIdx.x] = rmax;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + w]);
-    __syncthreads();
-  }
-  const double rel = bmax > 0.0 ? red[0] / bmax : red[0];
+  if (blockIdx.x != 0) return;
+  double rmax = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) rmax = fmax(rmax, fabs(r[i]));
+  rmax = block_max(rmax);
   if (threadIdx.x == 0) {
+    const double rel = bmax > 0.0 ? rmax / bmax : rmax;
     s.luRes[0] = rel;
     if (!(rel <= 1e-9)) atomicExch(s.err + 1, 12);
   }
@@ -793,11 +793,14 @@ __global__ void k_solve_refine(Dims d, DevState s) {
     s.gamVecPrev[i] = s.gamVec[i];
     s.gamVec[i] = x[i];
   }
-  __syncthreads();
-  for (int t = threadIdx.x; t < d.nbC * d.npan; t += blockDim.x) s.wGam[t] = s.gamVec[t];
+  // RHS keeps the reference's sign change (and, under axisymmetry, blade 1's rows in every blade)
   __syncthreads();
   if (d.axisym)
-    for (int t = d.npan + threadIdx.x; t < d.nb * d.npan; t += blockDim.x) s.wGam[t] = s.wGam[t % d.npan];
+    for (int i = d.npan + threadIdx.x; i < n; i += blockDim.x) s.RHS[i] = s.RHS[i % d.npan];
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) s.RHS[i] = -1.0 * s.RHS[i];
+  for (int t = threadIdx.x; t < d.nb * d.npan; t += blockDim.x)
+    if (t < d.nbC * d.npan || d.axisym) s.wGam[t] = x[d.axisym ? t % d.npan : t];
 }
 
 // ---- circulation solve (main.f90:522-603) ------------------------------------
@@ -851,88 +854,90 @@ struct ChunkAcc1 {
   __device__ double result() const { return (C > 0 && cnt > 0) ? tot + part : tot; }
 };
 
+// Sums over the rings of a rotor's blades at one collocation point, one block
+// per point: every thread evaluates a ring (the four edges in vr_vind's order)
+// and leaves its terms in shared memory -- the ring's (((f0 + f1) + f2) + f3) gam,
+// its bound pair's (f1 + f3) gam and, on the trailing edge, f1 gam -- and the
+// first lanes of two warps add them in the reference's order, one component a
+// lane, so that only additions are serial.  (Formed by three threads between the
+// additions, those terms were two thirds of the kernel: 340 us at 300 points.)
+//   bound: per blade s = 0, s + the pair's term panel by panel (spanwise
+//          stations outer), s - the trailing-edge terms; blades added to 0
+//          (rotor_vind_bywing_boundVortices, src/classdef.f90:1376-1393, 4445-4457)
+//   wing:  per blade the rings' terms in summation blocks; blades added to 0
+constexpr int kVcThreads = 256;
+inline size_t velcp_smem(int ns) { return sizeof(double) * 3 * (2 * (size_t)kVcThreads + ns); }
+template <bool WING>
+__device__ void ring_sums(const Dims& d, const DevState& s, const double* fr, d3 P, int sumChunk, double* sm,
+                          double& bound, double& wing) {
+  double* ring = sm;                      // [ring of the batch][component]
+  double* pair = ring + 3 * kVcThreads;
+  double* te = pair + 3 * kVcThreads;     // [station][component]
+  const exact64::Unit u = exact64::load_unit();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  bound = wing = 0.0;
+  for (int b = 0; b < d.nb; ++b) {
+    double sb = 0.0;
+    ChunkAcc1 acc(sumChunk);
+    for (int p0 = 0; p0 < d.npan; p0 += kVcThreads) {
+      const int n = min(kVcThreads, d.npan - p0), p = p0 + (int)threadIdx.x;
+      if (p < d.npan) {
+        const double* w = panRec(d, fr, b, p);
+        const double* rv = s.wRvc + 4 * ((size_t)b * d.npan + p);
+        const double g = s.wGam[(size_t)b * d.npan + p];
+        const corner64 c1 = exact64::make_corner(u, P, ld3(w + 3)), c2 = exact64::make_corner(u, P, ld3(w + 6));
+        const d3 f1 = exact64::vf_vind(u, c1, c2, rv[1]);
+        const corner64 c0 = exact64::make_corner(u, P, ld3(w)), c3 = exact64::make_corner(u, P, ld3(w + 9));
+        const d3 f3 = exact64::vf_vind(u, c3, c0, rv[3]);
+        if (WING) {
+          const d3 f0 = exact64::vf_vind(u, c0, c1, rv[0]), f2 = exact64::vf_vind(u, c2, c3, rv[2]);
+          st3(ring + 3 * threadIdx.x, (((f0 + f1) + f2) + f3) * g);
+        }
+        st3(pair + 3 * threadIdx.x, (f1 + f3) * g);
+        if (p % d.nc == d.nc - 1) st3(te + 3 * (p / d.nc), f1 * g);
+      }
+      __syncthreads();
+      if (lane < 3) {
+        if (WING && warp == 0)
+          for (int i = 0; i < n; ++i) acc.add(ring[3 * i + lane]);
+        if (warp == 1) {
+#pragma unroll 4
+          for (int i = 0; i < n; ++i) sb = sb + pair[3 * i + lane];
+          if (p0 + n == d.npan)
+            for (int j = 0; j < d.ns; ++j) sb = sb - te[3 * j + lane];
+        }
+      }
+      __syncthreads();
+    }
+    if (warp == 1) bound = bound + sb;
+    wing = wing + acc.result();
+  }
+}
 
-// Velocity at collocation point t including the wing's own induced velocity
-// minus its bound vortices (src/classdef.f90 calc_force's velCPTotal): one
-// block per collocation point.  The block's threads evaluate, batch by
-// batch, one stream of items over all blades -- per blade the four filament
-// velocities of every panel, then the trailing-edge filament of every
-// section (times its circulation), padded to a multiple of 4 -- into shared
-// memory, and the terms are formed and added in the reference's
-// order: the ring term ((f1 + f2) + f3) + f4 is vr_vind's sum, the bound pair
-// f2 + f4 and the trailing-edge f2 are the single-filament calls, all of
-// which evaluate the same filament function on the same corners.  Threads
-// 0..2 do the ordered sums of the x, y, z components.
-constexpr int kVcItems = 256;  // items per batch (a multiple of 4)
+// Velocity at the collocation points including the wing's own induced velocity
+// minus its bound vortices (src/classdef.f90 calc_force's velCPTotal).
 // fb (coupled rotors, else null): the bound-vortex velocity of every rotor
 // at this rotor's collocation points, [rotor][point][xyz]; the entry of this
 // rotor (self) is computed here.  velCPTotal = velCP - bound of every rotor in
 // rotor order + this rotor's wing (src/main.f90:636-652).
-__global__ void __launch_bounds__(256) k_velcp_total(Dims d, DevState s, const double* fr, int sumChunk,
-                                                     const double* fb, int nrs, int self) {
-  __shared__ double F[kVcItems * 3];
+__global__ void __launch_bounds__(kVcThreads) k_velcp_total(Dims d, DevState s, const double* fr, int sumChunk,
+                                                            const double* fb, int nrs, int self) {
+  extern __shared__ double sm[];
+  __shared__ double bnd[3];
   const int t = blockIdx.x;
-  if (t >= d.nbC * d.npan) return;
   const d3 P = ld3(panRec(d, fr, t / d.npan, t % d.npan) + 12);
-  const int nf = 4 * d.npan, nte = (d.ns + 3) & ~3, per = nf + nte;
-  const int total = d.nb * per;
-  // threads 0..2 each sum one component (the d3 sums are component-wise, so
-  // the bits equal those of one thread summing d3 values)
+  double bound, wing;
+  ring_sums<true>(d, s, fr, P, sumChunk, sm, bound, wing);
+  if (threadIdx.x >= 32 && threadIdx.x < 35) bnd[threadIdx.x - 32] = bound;
+  __syncthreads();
   const int c = threadIdx.x;
-  double bound = 0.0, wing = 0.0, sb = 0.0;
-  ChunkAcc1 acc(sumChunk);
-  for (int i0 = 0; i0 < total; i0 += kVcItems) {
-    const int n = min(kVcItems, total - i0);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const int it = i0 + i, b = it / per, o = it % per;
-      d3 v = zero3();
-      if (o < nf) {
-        const int p = o >> 2, k = o & 3;
-        const double* w = panRec(d, fr, b, p);
-        v = vf_vind64(make_corner64(P, ld3(w + 3 * k)), make_corner64(P, ld3(w + 3 * ((k + 1) & 3))),
-                      s.wRvc[4 * ((size_t)b * d.npan + p) + k]);
-      } else if (o - nf < d.ns) {
-        const int p = (d.nc - 1) + d.nc * (o - nf);
-        const double* w = panRec(d, fr, b, p);
-        v = vf_vind64(make_corner64(P, ld3(w + 3)), make_corner64(P, ld3(w + 6)),
-                      s.wRvc[4 * ((size_t)b * d.npan + p) + 1]) *
-            s.wGam[(size_t)b * d.npan + p];
-      }
-      st3(F + 3 * i, v);
-    }
-    __syncthreads();
-    if (c < 3) {
-      for (int i = 0; i < n;) {
-        const int it = i0 + i, b = it / per, o = it % per;
-        if (o < nf) {
-          const int p = o >> 2;
-          const double g = s.wGam[(size_t)b * d.npan + p];
-          const double f0 = F[3 * i + c], f1 = F[3 * i + 3 + c], f2 = F[3 * i + 6 + c], f3 = F[3 * i + 9 + c];
-          sb = sb + (f1 + f3) * g;
-          acc.add((((f0 + f1) + f2) + f3) * g);
-          i += 4;
-        } else {
-          if (o - nf < d.ns) sb = sb - F[3 * i + c];
-          if (o == per - 1) {
-            // the blade's sums are complete
-            bound = bound + sb;
-            wing = wing + acc.result();
-            sb = 0.0;
-            acc = ChunkAcc1(sumChunk);
-          }
-          i += 1;
-        }
-      }
-    }
-    __syncthreads();
-  }
   if (c < 3) {
     double v = s.velCP[3 * (size_t)t + c];
     if (fb) {
       const size_t M = (size_t)d.nbC * d.npan;
-      for (int jr = 0; jr < nrs; ++jr) v = v - (jr == self ? bound : fb[3 * (jr * M + t) + c]);
+      for (int jr = 0; jr < nrs; ++jr) v = v - (jr == self ? bnd[c] : fb[3 * (jr * M + t) + c]);
     } else {
-      v = v - bound;
+      v = v - bnd[c];
     }
     v = v + wing;
     s.velCPTotal[3 * (size_t)t + c] = v;
@@ -940,36 +945,15 @@ __global__ void __launch_bounds__(256) k_velcp_total(Dims d, DevState s, const d
 }
 
 // Bound vortices of rotor (ds, ss, frs) at the collocation points of rotor
-// (dt, frt) (rotor_vind_bywing_boundVortices, src/classdef.f90:1376-1393,
-// 4445-4457): per blade, s = 0, s + (filament 2 + filament 4) gam over the
-// panels (spanwise stations outer), s - filament 2 gam of the trailing-edge
-// panels, blades added to 0 in order.  One thread per point.
-__global__ void k_bound_foreign(Dims dt, const double* frt, Dims ds, DevState ss, const double* frs,
-                                double* out) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= dt.nbC * dt.npan) return;
+// (dt, frt), one block per point (a thread per point: 309 us at 16 panels).
+__global__ void __launch_bounds__(kVcThreads) k_bound_foreign(Dims dt, const double* frt, Dims ds, DevState ss,
+                                                              const double* frs, double* out) {
+  extern __shared__ double sm[];
+  const int t = blockIdx.x;
   const d3 P = ld3(panRec(dt, frt, t / dt.npan, t % dt.npan) + 12);
-  d3 bound = zero3();
-  for (int b = 0; b < ds.nb; ++b) {
-    d3 sb = zero3();
-    for (int p = 0; p < ds.npan; ++p) {
-      const double* w = panRec(ds, frs, b, p);
-      const double* rv = ss.wRvc + 4 * ((size_t)b * ds.npan + p);
-      const double g = ss.wGam[(size_t)b * ds.npan + p];
-      const d3 f1 = vf_vind64(make_corner64(P, ld3(w + 3)), make_corner64(P, ld3(w + 6)), rv[1]);
-      const d3 f3 = vf_vind64(make_corner64(P, ld3(w + 9)), make_corner64(P, ld3(w)), rv[3]);
-      sb = sb + (f1 + f3) * g;
-    }
-    for (int j = 0; j < ds.ns; ++j) {
-      const int p = (ds.nc - 1) + ds.nc * j;
-      const double* w = panRec(ds, frs, b, p);
-      sb = sb - vf_vind64(make_corner64(P, ld3(w + 3)), make_corner64(P, ld3(w + 6)),
-                          ss.wRvc[4 * ((size_t)b * ds.npan + p) + 1]) *
-                    ss.wGam[(size_t)b * ds.npan + p];
-    }
-    bound = bound + sb;
-  }
-  st3(out + 3 * (size_t)t, bound);
+  double bound, wing;
+  ring_sums<false>(ds, ss, frs, P, 0, sm, bound, wing);
+  if (threadIdx.x >= 32 && threadIdx.x < 35) out[3 * (size_t)t + threadIdx.x - 32] = bound;
 }
 
 // ---- image rotors (src/classdef.f90:4990-5131) ------------------------------
@@ -1496,7 +1480,7 @@ void launch_solve(const Dims& d, const DevState& s, const double* frame, bool wi
   count_launch();
   k_rhs<<<nblk(d.nbC * d.npan, 128), 128, 0, st>>>(d, s, frame, withWake ? 1 : 0);
   count_launch();
-  if (s.LU32) k_solve_refine<<<1, 1024, 0, st>>>(d, s);
+  if (s.LU32) k_solve_refine<<<kSolveBlocks, 1024, 0, st>>>(d, s);
   else k_solve<<<1, 1024, 0, st>>>(d, s);
 }
 void launch_step_begin(const Dims& d, const DevState& s, cudaStream_t st) {
@@ -1526,18 +1510,31 @@ void launch_mirror_wake(const Dims& d, const DevState& dst, const DevState& src,
 }
 void launch_solve_only(const Dims& d, const DevState& s, cudaStream_t st) {
   count_launch();
-  if (s.LU32) k_solve_refine<<<1, 1024, 0, st>>>(d, s);
+  if (s.LU32) k_solve_refine<<<kSolveBlocks, 1024, 0, st>>>(d, s);
   else k_solve<<<1, 1024, 0, st>>>(d, s);
+}
+// shared memory for up to 8192 stations (the most panels a rotor has)
+static void velcp_attr() {
+  static std::atomic<bool> attr[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && attr[dev].load(std::memory_order_acquire)) return;
+  const int most = (int)velcp_smem(8192);
+  cudaFuncSetAttribute(k_velcp_total, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  cudaFuncSetAttribute(k_bound_foreign, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (dev >= 0 && dev < 64) attr[dev].store(true, std::memory_order_release);
 }
 void launch_bound_foreign(const Dims& dt, const double* frameT, const Dims& ds, const DevState& ss,
                           const double* frameS, double* out, cudaStream_t st) {
   count_launch();
-  k_bound_foreign<<<nblk(dt.nbC * dt.npan, 64), 64, 0, st>>>(dt, frameT, ds, ss, frameS, out);
+  velcp_attr();
+  k_bound_foreign<<<dt.nbC * dt.npan, kVcThreads, velcp_smem(ds.ns), st>>>(dt, frameT, ds, ss, frameS, out);
 }
 void launch_loads(const Dims& d, const DevState& s, const double* frame, int sumChunk, int iter, cudaStream_t st,
                   const double* foreignBound, int nrs, int self) {
   count_launch();
-  k_velcp_total<<<d.nbC * d.npan, 256, 0, st>>>(d, s, frame, sumChunk, foreignBound, nrs, self);
+  velcp_attr();
+  k_velcp_total<<<d.nbC * d.npan, kVcThreads, velcp_smem(d.ns), st>>>(d, s, frame, sumChunk, foreignBound, nrs, self);
   count_launch();
   k_loads<<<1, 256, 0, st>>>(d, s, frame, iter);
 }
