@@ -223,8 +223,8 @@ __device__ __forceinline__ void rec_lat_pair(const float4* __restrict__ R4, cons
 // add / mul / fma below is one instruction for the two lanes, each lane
 // rounded exactly as the scalar instruction (.rn, .ftz as the unit's
 // -ftz=true).  The scalar functions above are rewritten only where a
-// negation would need its own instruction: -(a b) as (-a) b with the exactly
-// negated corner vector c - P, -(t - e) as e - t; both exact, so every lane
+// negation would need its own instruction: -(a b) as (-a) b or a (-b) with an
+// exactly negated corner vector, -(t - e) as e - t; all exact, so every lane
 // carries the scalar path's bits (k_near_fix recomputes those).
 typedef unsigned long long f2;
 __device__ __forceinline__ f2 f2pack(float a, float b) {
@@ -257,68 +257,79 @@ __device__ __forceinline__ f2 f2rsqrt(f2 a) {
   return f2pack(rsqrtf(x), rsqrtf(y));
 }
 
-// corner_vector for both targets: r = P - c, 1/|r|
-__device__ __forceinline__ void corner_pair(f2 px, f2 py, f2 pz, float cx, float cy, float cz, f2& rx, f2& ry, f2& rz,
-                                            f2& inv) {
-  rx = f2sub(px, f2splat(cx));
-  ry = f2sub(py, f2splat(cy));
-  rz = f2sub(pz, f2splat(cz));
-  inv = f2rsqrt(f2fma(rx, rx, f2fma(ry, ry, f2fma(rz, rz, f2splat(kS2Min)))));
-}
+// -a: two sign flips on the integer pipe, where a packed subtraction c - P
+// would take the FMA pipe that bounds the kernel
+__device__ __forceinline__ f2 f2neg(f2 a) { return a ^ 0x8000000080000000ull; }
 
-// fil_fp32 for both targets; (cxk, cyk, czk) is corner K itself, whose
-// negated corner vector c - P the cross product takes
-template <int K>
-__device__ __forceinline__ void fil_pair(const RecView& v, f2 px, f2 py, f2 pz, float cxk, float cyk, float czk,
-                                         f2 rxk, f2 ryk, f2 rzk, f2 invk, f2 rxj, f2 ryj, f2 rzj, f2 invj, f2& ax,
-                                         f2& ay, f2& az) {
-  const f2 nrxk = f2sub(f2splat(cxk), px), nryk = f2sub(f2splat(cyk), py), nrzk = f2sub(f2splat(czk), pz);
-  const f2 kx = f2fma(ryk, rzj, f2mul(nrzk, ryj));
-  const f2 ky = f2fma(rzk, rxj, f2mul(nrxk, rzj));
-  const f2 kz = f2fma(rxk, ryj, f2mul(nryk, rxj));
+// Corner vector r = P - c and 1/|r| for both targets.
+struct CornerPair {
+  f2 x, y, z, inv;
+};
+__device__ __forceinline__ CornerPair corner_pair(f2 px, f2 py, f2 pz, float cx, float cy, float cz) {
+  CornerPair r;
+  r.x = f2sub(px, f2splat(cx));
+  r.y = f2sub(py, f2splat(cy));
+  r.z = f2sub(pz, f2splat(cz));
+  r.inv = f2rsqrt(f2fma(r.x, r.x, f2fma(r.y, r.y, f2fma(r.z, r.z, f2splat(kS2Min)))));
+  return r;
+}
+struct NegCorner {
+  f2 x, y, z;
+};
+__device__ __forceinline__ NegCorner neg_corner(const CornerPair& r) { return {f2neg(r.x), f2neg(r.y), f2neg(r.z)}; }
+
+// fil_fp32 for both targets, corner k = (rk) -> j = (rj); n is the negated
+// vector of corner k (NEGK) or of corner j, whichever two filaments share.
+template <int K, bool NEGK>
+__device__ __forceinline__ void fil_pair(const RecView& v, const CornerPair& rk, const CornerPair& rj,
+                                         const NegCorner& n, f2& ax, f2& ay, f2& az) {
+  const f2 kx = f2fma(rk.y, rj.z, NEGK ? f2mul(n.z, rj.y) : f2mul(rk.z, n.y));
+  const f2 ky = f2fma(rk.z, rj.x, NEGK ? f2mul(n.x, rj.z) : f2mul(rk.x, n.z));
+  const f2 kz = f2fma(rk.x, rj.y, NEGK ? f2mul(n.y, rj.x) : f2mul(rk.y, n.x));
   const f2 c2 = f2fma(kx, kx, f2fma(ky, ky, f2mul(kz, kz)));
-  const f2 tt = f2fma(f2splat(v.ex[K]), rxk, f2fma(f2splat(v.ey[K]), ryk, f2mul(f2splat(v.ez[K]), rzk)));
-  const f2 d = f2fma(tt, invk, f2mul(f2sub(f2splat(v.eev[K]), tt), invj));
+  const f2 tt = f2fma(f2splat(v.ex[K]), rk.x, f2fma(f2splat(v.ey[K]), rk.y, f2mul(f2splat(v.ez[K]), rk.z)));
+  const f2 d = f2fma(tt, rk.inv, f2mul(f2sub(f2splat(v.eev[K]), tt), rj.inv));
   const f2 f = f2mul(d, f2rsqrt(f2fma(c2, c2, f2splat(v.a4v[K]))));
   ax = f2fma(f, kx, ax);
   ay = f2fma(f, ky, ay);
   az = f2fma(f, kz, az);
 }
 
-// ring_fp32 for both targets (all four edges)
+// ring_fp32 for both targets (all four edges): 104 packed FMA-pipe
+// instructions, the negated vectors of corners 0 and 2 serving two edges each
 __device__ __forceinline__ void ring_pair(const float4* __restrict__ R4, const float (&cx)[4], const float (&cy)[4],
                                           const float (&cz)[4], f2 px, f2 py, f2 pz, f2& ax, f2& ay, f2& az) {
   RecView v;
   load_view(R4, v);
-  f2 rx[4], ry[4], rz[4], inv[4];
+  CornerPair r[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) corner_pair(px, py, pz, cx[k], cy[k], cz[k], rx[k], ry[k], rz[k], inv[k]);
-  fil_pair<0>(v, px, py, pz, cx[0], cy[0], cz[0], rx[0], ry[0], rz[0], inv[0], rx[1], ry[1], rz[1], inv[1], ax, ay, az);
-  fil_pair<1>(v, px, py, pz, cx[1], cy[1], cz[1], rx[1], ry[1], rz[1], inv[1], rx[2], ry[2], rz[2], inv[2], ax, ay, az);
-  fil_pair<2>(v, px, py, pz, cx[2], cy[2], cz[2], rx[2], ry[2], rz[2], inv[2], rx[3], ry[3], rz[3], inv[3], ax, ay, az);
-  fil_pair<3>(v, px, py, pz, cx[3], cy[3], cz[3], rx[3], ry[3], rz[3], inv[3], rx[0], ry[0], rz[0], inv[0], ax, ay, az);
+  for (int k = 0; k < 4; ++k) r[k] = corner_pair(px, py, pz, cx[k], cy[k], cz[k]);
+  const NegCorner n0 = neg_corner(r[0]), n2 = neg_corner(r[2]);
+  fil_pair<0, true>(v, r[0], r[1], n0, ax, ay, az);
+  fil_pair<1, false>(v, r[1], r[2], n2, ax, ay, az);
+  fil_pair<2, true>(v, r[2], r[3], n2, ax, ay, az);
+  fil_pair<3, false>(v, r[3], r[0], n0, ax, ay, az);
 }
 
-// rec_lat_pair<2> with packed pairs
+// rec_lat_pair<2> with packed pairs: 58 packed FMA-pipe instructions for an
+// interior ring, corner 1's negated vector serving both edges
 __device__ __forceinline__ void rec_lat_packed(const float4* __restrict__ R4, const float (&cx)[4],
                                                const float (&cy)[4], const float (&cz)[4], f2 px, f2 py, f2 pz, f2& ax,
                                                f2& ay, f2& az) {
   RecView v;
   load_view(R4, v);
-  f2 rx[4], ry[4], rz[4], inv[4];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) corner_pair(px, py, pz, cx[k], cy[k], cz[k], rx[k], ry[k], rz[k], inv[k]);
-  fil_pair<0>(v, px, py, pz, cx[0], cy[0], cz[0], rx[0], ry[0], rz[0], inv[0], rx[1], ry[1], rz[1], inv[1], ax, ay, az);
-  fil_pair<1>(v, px, py, pz, cx[1], cy[1], cz[1], rx[1], ry[1], rz[1], inv[1], rx[2], ry[2], rz[2], inv[2], ax, ay, az);
+  const CornerPair r0 = corner_pair(px, py, pz, cx[0], cy[0], cz[0]);
+  const CornerPair r1 = corner_pair(px, py, pz, cx[1], cy[1], cz[1]);
+  const CornerPair r2 = corner_pair(px, py, pz, cx[2], cy[2], cz[2]);
+  const NegCorner n1 = neg_corner(r1);
+  fil_pair<0, false>(v, r0, r1, n1, ax, ay, az);
+  fil_pair<1, true>(v, r1, r2, n1, ax, ay, az);
   const bool t2 = v.a4v[2] >= 0.f, t3 = v.a4v[3] >= 0.f;
   if (t2 || t3) {
-    corner_pair(px, py, pz, cx[3], cy[3], cz[3], rx[3], ry[3], rz[3], inv[3]);
-    if (t2)
-      fil_pair<2>(v, px, py, pz, cx[2], cy[2], cz[2], rx[2], ry[2], rz[2], inv[2], rx[3], ry[3], rz[3], inv[3], ax, ay,
-                  az);
-    if (t3)
-      fil_pair<3>(v, px, py, pz, cx[3], cy[3], cz[3], rx[3], ry[3], rz[3], inv[3], rx[0], ry[0], rz[0], inv[0], ax, ay,
-                  az);
+    const CornerPair r3 = corner_pair(px, py, pz, cx[3], cy[3], cz[3]);
+    const NegCorner n3 = neg_corner(r3);
+    if (t2) fil_pair<2, false>(v, r2, r3, n3, ax, ay, az);
+    if (t3) fil_pair<3, true>(v, r3, r0, n3, ax, ay, az);
   }
 }
 
