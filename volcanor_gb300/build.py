@@ -2,8 +2,8 @@
 
 FP64 translation units (bs64.cu, solver.cu, factor.cu, incr.cu) are compiled with -fmad=false and
 the host units with -ffp-contract=off so that every FP64 operation rounds as
-in the reference arithmetic; the FP32 kernel unit (bs32.cu) keeps FMA
-contraction and flushes FP32 denormals (-ftz=true), which lets rsqrtf map to
+in the reference arithmetic; the FP32 kernel units (bs32.cu, gather.cu) keep FMA
+contraction and flush FP32 denormals (-ftz=true), which lets rsqrtf map to
 a single MUFU instruction.  Compilation runs in parallel and takes well under a minute.
 """
 from __future__ import annotations
@@ -20,7 +20,7 @@ LIB = BUILD / "libvlm_gb300.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 CU_EXACT = ["bs64.cu", "solver.cu", "factor.cu", "incr.cu"]
-CU_FAST = ["bs32.cu"]
+CU_FAST = ["bs32.cu", "gather.cu"]
 CU_PLAIN = ["noalloc.cu", "mlp.cu", "mlp_tc.cu", "surrogate.cu", "peak.cu"]
 CXX = ["wing.cpp", "case.cpp", "plan.cpp"]
 

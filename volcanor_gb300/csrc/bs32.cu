@@ -40,6 +40,7 @@
 #include <climits>
 #include <atomic>
 
+#include "pack32.h"
 #include "vlm_bs.h"
 #include "vlm_math.h"
 
@@ -991,61 +992,20 @@ __global__ void k_wait_probe(uint32_t limit, int* out) {
   out[0] = mbar_wait(&bar, 0, limit) ? 0 : 1;  // 1: the limit expired, as it must
 }
 
-// FP64 record -> FP32 record.  The edge vectors are differenced in FP64
-// (nearby corners cancel) and rounded once; everything else is FP32 (the
-// record is FP32; GB300's FP64 rate would make this kernel latency-bound).
-// With edge weights ew (lattice form) edge k carries ew[k] and is active iff
-// ew[k] != 0; without, every filament of a record carries its gam unless the
-// record is skipped (|gam| <= eps with REC_SKIP), a single filament only its
-// first.  Inactive edges 2 and 3 are marked for the kernel to skip.
+// FP64 records -> FP32 records, four lanes a record (pack32.h).
 __global__ void k_pack32(const double* __restrict__ rec64, int nrec, double near_factor, float* __restrict__ rec32,
                          const double* __restrict__ ew) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nrec) return;
-  const double* R = rec64 + (size_t)i * kRec64;
-  float* o = rec32 + (size_t)i * kRec32;
+  const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const bool live = q < (size_t)nrec * 4;
+  const size_t i = live ? q >> 2 : 0;
+  const int k = (int)(q & 3);
+  const double* R = rec64 + i * kRec64;
   const int flags = (int)R[17];
-  const double g = R[16];
-  const bool skipped = (flags & REC_SKIP) && !(fabs(g) > kEps);
   const bool fil = flags & REC_FIL;
-  const double* EW = ew ? ew + 4 * (size_t)i : nullptr;
-  // corner k (FP64) and core radius of filament k
-  double cx[4], cy[4], cz[4];
-  float rv[4];
-  for (int k = 0; k < 4; ++k) {
-    const int src = fil ? (k == 1 || k == 2 ? 1 : 0) : k;
-    cx[k] = R[3 * src];
-    cy[k] = R[3 * src + 1];
-    cz[k] = R[3 * src + 2];
-    rv[k] = fil ? (k == 0 ? (float)R[12] : 0.f) : (float)R[12 + k];
-  }
-  const float nf = (float)near_factor;
-  const float w = (float)(g * kInv4Pi);
-  for (int k = 0; k < 4; ++k) {
-    const int j = (k + 1) & 3;
-    const bool act = EW ? EW[k] != 0.0 : (!fil || k == 0) && !skipped;
-    const float ex = (float)(cx[j] - cx[k]), ey = (float)(cy[j] - cy[k]), ez = (float)(cz[j] - cz[k]);
-    const float ee = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-    const float sk = rv[k] * sqrtf(ee);
-    const float s2 = sk * sk;
-    o[3 * k] = (float)cx[k];
-    o[3 * k + 1] = (float)cy[k];
-    o[3 * k + 2] = (float)cz[k];
-    const float wk = act ? (EW ? (float)(EW[k] * kInv4Pi) : w) : 0.f;
-    o[12 + 3 * k] = wk * ex;
-    o[12 + 3 * k + 1] = wk * ey;
-    o[12 + 3 * k + 2] = wk * ez;
-    o[24 + k] = wk * ee;
-    o[28 + k] = EW && k >= 2 && !act ? -1.f : fmaxf(s2 * s2, 1e-36f);
-    const bool on = act && nf > 0.f;
-    const float nfs = nf * sk;
-    o[32 + k] = on ? nfs * nfs : -1.f;
-    // -s < e.r1 < |e|^2 + s, multiplied by w_k
-    const float blo = -nfs * wk, bhi = (ee + nfs) * wk;
-    o[36 + k] = on ? fminf(blo, bhi) : 0.f;
-    o[40 + k] = on ? fmaxf(blo, bhi) : 0.f;
-  }
-  o[44] = o[45] = o[46] = o[47] = 0.f;
+  const int src = fil ? (k == 1 || k == 2 ? 1 : 0) : k;
+  const double g = R[16], rv = fil && k ? 0.0 : R[12 + k];
+  pack_edge32(mk3(R[3 * src], R[3 * src + 1], R[3 * src + 2]), rv, g, flags, ew != nullptr,
+              ew ? ew[4 * i + k] : 0.0, k, (float)near_factor, live ? rec32 + i * kRec32 : nullptr);
 }
 
 }  // namespace
@@ -1054,7 +1014,7 @@ void launch_pack32(const double* rec64, int nrec, double near_factor, float* rec
                    const double* ew) {
   if (nrec <= 0) return;
   count_launch();
-  k_pack32<<<(nrec + 255) / 256, 256, 0, s>>>(rec64, nrec, near_factor, rec32, ew);
+  k_pack32<<<(unsigned)(((size_t)nrec * 4 + 255) / 256), 256, 0, s>>>(rec64, nrec, near_factor, rec32, ew);
 }
 
 // The compiled tile shapes: {targets per thread, stages, blocks per SM}.

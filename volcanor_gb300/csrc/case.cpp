@@ -434,7 +434,7 @@ struct Case {
     for (void* p : scratchOwned) cudaFree(p);
     scratchOwned.clear();
     s.rec64 = dalloc<double>((size_t)maxRecords * kRec64, scratchOwned);
-    s.rec32 = dalloc<float>((size_t)maxRecords * kRec32, scratchOwned);
+    s.rec32 = opt.precision != VLM_PREC_FP64 ? dalloc<float>((size_t)maxRecords * kRec32, scratchOwned) : nullptr;
     s.edgeW = lattice() ? dalloc<double>((size_t)maxRecords * 4, scratchOwned) : nullptr;
     s.share = opt.precision == VLM_PREC_FP64 ? dalloc<int>((size_t)maxRecords, scratchOwned) : nullptr;
     s.targets = dalloc<double>((size_t)maxTargets * 3, scratchOwned);
@@ -522,6 +522,19 @@ struct Case {
     else launch_partial64(s.rec64, ch, e.nchunks, e.nrec, P, M, s.part, stream);
   }
 
+  // near zones of the FP32 records
+  double nearFactor() const { return opt.precision == VLM_PREC_FP32_NEAR64 ? opt.near_factor : 0.0; }
+  // the records of plan e (packed for the FP32 precisions), with targets of
+  // `kind` (GatherTargets) into P, and the near-pair count reset
+  void gather(const EvalPlan& e, const double* fr, int rN, int rF, bool pred, int kind = 0, double* P = nullptr, int M = 0) {
+    GatherTargets tg;
+    tg.kind = kind;
+    tg.P = P;
+    tg.M = M;
+    tg.zero[0] = s.err + 3;
+    launch_gather(d, s, fr, dGroups + e.goff, e.ngroups, e.nrec, rN, rF, pred, nearFactor(), tg, stream);
+  }
+
   // one Biot-Savart evaluation of plan e (its records already gathered) at the
   // M targets P into out; prec -1 = the case's precision
   void evaluate(const EvalPlan& e, int M, int mode, const double* P = nullptr, double* out = nullptr, int prec = -1,
@@ -534,8 +547,6 @@ struct Case {
       partial64(e, ch, P, M);
     } else {
       const bool nearOn = prec == VLM_PREC_FP32_NEAR64;
-      launch_pack32(s.rec64, e.nrec, nearOn ? opt.near_factor : 0.0, s.rec32, stream, s.edgeW);
-      VLM_CUDA(cudaMemsetAsync(s.err + 3, 0, sizeof(int), stream));
       launch_partial32(s.rec32, s.rec64, ch, e.nchunks, e.nrec, P, M, s.part, s.err + 2,
                        nearOn ? s.nearScratch : nullptr, s.nearBytes, s.nacc, stream, s.edgeW, e.shape,
                        opt.nbody_slots > 0 ? nullptr : &nearOv);  // a batch's cases already run side by side
@@ -715,9 +726,7 @@ struct Case {
         changed = true;
         continue;
       }
-      if (which == 0) launch_node_targets(d, s, pl.rowNear, pl.rowFar, false, s.targets, stream);
-      else launch_cp_targets(d, frame(k), s.targets, stream);
-      launch_gather(d, s, frame(k), dGroups + e.goff, e.ngroups, e.nrec, pl.rowNear, pl.rowFar, false, stream);
+      gather(e, frame(k), pl.rowNear, pl.rowFar, false, which == 0 ? 2 : 1, s.targets, M);
       launch_pack32(s.rec64, e.nrec, 0.0, s.rec32, stream, s.edgeW);
       std::vector<Group> g0(hGroups.begin() + e.goff, hGroups.begin() + e.goff + e.ngroups);
       const int cap = e.nrec + e.ngroups + 1;
@@ -897,14 +906,22 @@ struct Case {
   }
   // the predicted targets and records beside the current ones, and the
   // comparison (counts and per-tile offsets)
-  void incrDiff(int k, int M) {
+  // (rec32, when not null, receives the predicted records packed)
+  void incrDiff(int k, int M, float* rec32) {
     const StepPlan& pl = plans[k];
     const EvalPlan& e = pl.node;
-    launch_node_targets(d, s, pl.rowNear, pl.rowFar, true, tgtP, stream);
     DevState sp = s;
     sp.rec64 = recP;
     sp.edgeW = s.edgeW ? ewP : nullptr;
-    launch_gather(d, sp, stepFrame(k), dGroups + e.goff, e.ngroups, e.nrec, pl.rowNear, pl.rowFar, true, stream);
+    sp.rec32 = rec32;
+    GatherTargets tg;
+    tg.kind = 2;
+    tg.P = tgtP;
+    tg.M = M;
+    tg.zero[0] = s.err + 3;
+    tg.zero[1] = incrCtl + 1;
+    launch_gather(d, sp, stepFrame(k), dGroups + e.goff, e.ngroups, e.nrec, pl.rowNear, pl.rowFar, true, nearFactor(),
+                  tg, stream);
     launch_diff_count(recP, s.rec64, kRec64, sp.edgeW, s.edgeW, e.nrec, incrBlk, incrCnt, stream);
     launch_diff_count(tgtP, s.targets, 3, nullptr, nullptr, M, incrBlk + incr_diff_blocks(e.nrec), incrCnt + 1,
                       stream);
@@ -919,7 +936,7 @@ struct Case {
     ip.M = M;
     if (M > 0 && e.nrec > 0) {
       allocIncrBase();
-      incrDiff(k, M);
+      incrDiff(k, M, nullptr);
       int cnt[2] = {0, 0};
       VLM_CUDA(cudaMemcpyAsync(cnt, incrCnt, sizeof(cnt), cudaMemcpyDeviceToHost, stream));
       VLM_CUDA(cudaStreamSynchronize(stream));
@@ -986,7 +1003,7 @@ struct Case {
     const EvalPlan& e = plans[k].node;
     const bool nearOn = opt.precision == VLM_PREC_FP32_NEAR64;
     const double nf = nearOn ? opt.near_factor : 0.0;
-    incrDiff(k, M);
+    incrDiff(k, M, ip.mRec32);
     const double* ew = s.edgeW ? ewP : nullptr;
     launch_moved_targets(tgtP, s.targets, M, incrBlk + incr_diff_blocks(e.nrec), incrCnt + 1, ip.tIdx, ip.tPos,
                          ip.mcap, s.err + 2, stream);
@@ -998,8 +1015,6 @@ struct Case {
       VLM_CUDA(cudaEventRecord(incrFork, stream));
       VLM_CUDA(cudaStreamWaitEvent(incrStream, incrFork, 0));
     }
-    launch_pack32(recP, e.nrec, nf, ip.mRec32, ms, ew);
-    VLM_CUDA(cudaMemsetAsync(incrCtl + 1, 0, sizeof(int), ms));
     launch_partial32(ip.mRec32, recP, ip.mC, ip.mq, e.nrec, ip.tPos, ip.mcap, ip.mPart, incrCtl, ip.mNear,
                      ip.mNearBytes, ip.mNacc, ms, ew, 0, side ? &incrOv : nullptr);
     launch_combine_unordered(ip.mPart, ip.mcap, ip.mG, ip.mng, ip.mmaxq, 0, ip.tOut, ms);
@@ -1010,7 +1025,6 @@ struct Case {
     launch_delta_records(recP, s.rec64, ew, s.edgeW, e.nrec, incrBlk, incrCnt, ip.dRec, ip.dEw, ip.dcap, s.err + 2,
                          stream);
     launch_pack32(ip.dRec, ip.dcap, nf, s.rec32, stream, ip.dEw);
-    VLM_CUDA(cudaMemsetAsync(s.err + 3, 0, sizeof(int), stream));
     launch_partial32(s.rec32, ip.dRec, ip.dC, ip.dq, ip.dcap, s.targets, M, ip.dPart, s.err + 2,
                      nearOn ? s.nearScratch : nullptr, s.nearBytes, ip.dNacc, stream, ip.dEw, 0,
                      side ? &nearOv : nullptr, true);
@@ -1142,23 +1156,40 @@ struct Case {
   }
 
   // the records of every source rotor at step k (frame fk), each from its own state
-  void sysGather(const SysEval& se, int k, bool pred, int fk) {
+  // (and this rotor's targets of `kind`)
+  void sysGather(const SysEval& se, int k, bool pred, int fk, int kind, int M) {
+    bool placed = false;
     for (int i = 0; i < se.nseg; ++i) {
       const SysSeg& g = hSegs[se.soff + i];
       const Case& o = *sys[g.jr];
       DevState sj = o.s;
       sj.rec64 = s.rec64 + (size_t)g.recOff * kRec64;
       sj.edgeW = s.edgeW ? s.edgeW + 4 * (size_t)g.recOff : nullptr;
+      sj.rec32 = s.rec32 ? s.rec32 + (size_t)g.recOff * kRec32 : nullptr;
+      GatherTargets tg;
+      tg.zero[0] = s.err + 3;
+      if (g.jr == self) {
+        tg.kind = kind;
+        tg.P = s.targets;
+        tg.M = M;
+        placed = true;
+      }
       launch_gather(o.d, sj, o.frame(fk), dGroups + g.lgoff, g.lng, g.nrec, o.plans[k].rowNear, o.plans[k].rowFar,
-                    pred, stream);
+                    pred, nearFactor(), tg, stream);
+    }
+    if (!placed) {  // this rotor is no source (the initial solution): targets alone
+      GatherTargets tg;
+      tg.kind = kind;
+      tg.P = s.targets;
+      tg.M = M;
+      launch_gather(d, s, frame(fk), dGroups, 0, 0, plans[k].rowNear, plans[k].rowFar, pred, 0.0, tg, stream);
     }
   }
   // velCP and the RHS at step k (frame k; k = 0: the initial solution)
   void sysRhsPhase(int k) {
     const SysEval& se = k == 0 ? sysStart : sysRhs[k];
     const int Mcp = d.nbC * d.npan;
-    launch_cp_targets(d, frame(k), s.targets, stream);
-    sysGather(se, k, false, k);
+    sysGather(se, k, false, k, 1, Mcp);
     evaluate(se.e, Mcp, 3, nullptr, sysOut, -1, se.nterms);
     launch_rhs_terms(d, s, frame(k), sysOut, se.nterms, stream);
   }
@@ -1311,8 +1342,7 @@ struct Case {
     const int M = d.nbC * d.npan + nodes;
     const int rNprev = plans[k - 1].rowNear;
     launch_surr_targets(d, s, frame(k - 1), rNprev, plans[k].rowFar, 0, stride, offset, nodes, surr.sP, stream);
-    launch_gather(d, s, frame(k - 1), dGroups + e.goff, e.ngroups, e.nrec, plans[k].rowNear, plans[k].rowFar, false,
-                  stream);
+    gather(e, frame(k - 1), plans[k].rowNear, plans[k].rowFar, false);
     evaluate(e, M, 2, surr.sP, surr.sV, prec);
     launch_surr_features(d, s, frame(k - 1), surr.sP, M, surr.invR, farFill(plans[k].rowFar), plans[k].rowFar,
                          youngAt(k), false, surr.desc, surr.fX, stream);
@@ -1429,31 +1459,27 @@ struct Case {
   }
   void evalNodesFull(int k, bool pred, int M) {
     const StepPlan& pl = plans[k];
-    launch_node_targets(d, s, pl.rowNear, pl.rowFar, pred, s.targets, stream);
     if (member) {
       const SysEval& se = sysNode[k];
-      sysGather(se, k, pred, k);
+      sysGather(se, k, pred, k, 2, M);
       evaluate(se.e, M, 0, nullptr, nullptr, -1, se.nterms);
     } else if (surr.on && surr.useNow) {
       // near-wake nodes: direct without the far wake + the network's far-wake
       // velocity; far-wake nodes: + the direct far-wake sum
       const SurrPlans& sp = splans[k];
-      launch_gather(d, s, stepFrame(k), dGroups + sp.nodeNoFar.goff, sp.nodeNoFar.ngroups, sp.nodeNoFar.nrec, pl.rowNear,
-                    pl.rowFar, pred, stream);
+      gather(sp.nodeNoFar, stepFrame(k), pl.rowNear, pl.rowFar, pred, 2, s.targets, M);
       evaluate(sp.nodeNoFar, M, 0);
       // every far-wake node, young or old, sums the old far wake directly
       const int Mf = d.nbC * farRows(pl.rowFar);
       launch_surr_far_targets(d, s, pl.rowFar, 0, pred, surr.farP, stream);
-      launch_gather(d, s, stepFrame(k), dGroups + sp.farFar.goff, sp.farFar.ngroups, sp.farFar.nrec, pl.rowNear, pl.rowFar,
-                    pred, stream);
+      gather(sp.farFar, stepFrame(k), pl.rowNear, pl.rowFar, pred);
       evaluate(sp.farFar, Mf, 2, surr.farP, surr.outFar);
       launch_surr_features(d, s, frame(pred ? k : k - 1), s.targets, M, surr.invR, farFill(pl.rowFar), pl.rowFar,
                            youngAt(k), pred, surr.desc, surr.fX, stream);
       surr.net.forward(surr.fX, M, surr.fY);
       launch_surr_merge_nodes(d, pl.rowNear, pl.rowFar, 0, M, surr.fY, surr.scale, surr.outFar, s.outv, stream);
     } else {
-      launch_gather(d, s, stepFrame(k), dGroups + pl.node.goff, pl.node.ngroups, pl.node.nrec, pl.rowNear, pl.rowFar,
-                    pred, stream);
+      gather(pl.node, stepFrame(k), pl.rowNear, pl.rowFar, pred, 2, s.targets, M);
       evaluate(pl.node, M, 0);
     }
   }
@@ -1527,17 +1553,16 @@ struct Case {
     const double* fr = stepFrame(k);
     if (d.NW > 0) {
       const int Mcp = d.nbC * d.npan;
-      launch_cp_targets(d, fr, s.targets, stream);
       if (surr.on && surr.useNow) {
         const EvalPlan& e = splans[k].rhsNoFar;
-        launch_gather(d, s, fr, dGroups + e.goff, e.ngroups, e.nrec, rN, rF, false, stream);
+        gather(e, fr, rN, rF, false, 1, s.targets, Mcp);
         evaluate(e, Mcp, 1);
         launch_surr_features(d, s, frame(k - 1), s.targets, Mcp, surr.invR, farFill(rF), rF, youngAt(k), false,
                              surr.desc, surr.fX, stream);
         surr.net.forward(surr.fX, Mcp, surr.fY);
         launch_surr_add(Mcp, surr.fY, surr.scale, s.outv, stream);
       } else {
-        launch_gather(d, s, fr, dGroups + pl.rhs.goff, pl.rhs.ngroups, pl.rhs.nrec, rN, rF, false, stream);
+        gather(pl.rhs, fr, rN, rF, false, 1, s.targets, Mcp);
         evaluate(pl.rhs, Mcp, 1);
       }
       launch_solve(d, s, fr, true, stream);
@@ -1938,12 +1963,8 @@ struct Case {
     VLM_CUDA(cudaMemcpyAsync(s.frames + (size_t)k * d.fl.size, hFrames + (size_t)k * d.fl.size,
                              sizeof(double) * d.fl.size, cudaMemcpyHostToDevice, stream));
     const int M = node_target_count(d, pl.rowNear, pl.rowFar);
-    launch_node_targets(d, s, pl.rowNear, pl.rowFar, false, s.targets, stream);
-    launch_gather(d, s, frame(k), dGroups + pl.node.goff, pl.node.ngroups, pl.node.nrec, pl.rowNear, pl.rowFar, false,
-                  stream);
+    gather(pl.node, frame(k), pl.rowNear, pl.rowFar, false, 2, s.targets, M);
     const Chunk* ch = dChunks + pl.node.coff;
-    const double nf = opt.precision == VLM_PREC_FP32_NEAR64 ? opt.near_factor : 0.0;
-    if (opt.precision != VLM_PREC_FP64) launch_pack32(s.rec64, pl.node.nrec, nf, s.rec32, stream, s.edgeW);
     // the work the FP32 kernel executes per target (9 flop per corner vector,
     // 35 per filament): a whole ring 4 + 4; a lattice-form record 3 corners
     // and edges 0, 1, plus corner c3 and edges 2 / 3 where they carry
@@ -2207,16 +2228,17 @@ struct Case {
       DevState t = s;
       t.rec64 = rec64;
       t.edgeW = nullptr;  // ring by ring: the probe's record count is not the plans'
-      launch_gather(d, t, frame(fi), dg, (int)g.size(), rec, rN, rF, false, stream);
+      t.rec32 = opt.precision == VLM_PREC_FP64 ? nullptr : rec32;
+      GatherTargets tg;
+      tg.zero[0] = s.err + 3;
+      launch_gather(d, t, frame(fi), dg, (int)g.size(), rec, rN, rF, false, nearFactor(), tg, stream);
       if (opt.precision == VLM_PREC_FP64) {
         launch_partial64(rec64, dc, nq, rec, dP, (int)M, part, stream);
       } else {
         const bool nearOn = opt.precision == VLM_PREC_FP32_NEAR64;
-        launch_pack32(rec64, rec, nearOn ? opt.near_factor : 0.0, rec32, stream);
         const size_t nb = nearOn ? near_scratch_bytes((int)M, (size_t)std::min<int64_t>(64 * M + (1 << 16), 1 << 26)) : 1;
         unsigned char* ns = dalloc<unsigned char>(nb, tmpOwned);
         long long* nacc = dalloc<long long>(nearOn ? (size_t)M * nq * 3 : 1, tmpOwned);
-        VLM_CUDA(cudaMemsetAsync(s.err + 3, 0, sizeof(int), stream));
         launch_partial32(rec32, rec64, dc, nq, rec, dP, (int)M, part, s.err + 2, nearOn ? ns : nullptr, nb, nacc,
                          stream);
       }

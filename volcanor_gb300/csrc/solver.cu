@@ -9,6 +9,7 @@
 #include <atomic>
 
 #include "exact64.h"
+#include "state_dev.h"
 #include "vlm_math.h"
 #include "vlm_solver.h"
 
@@ -16,21 +17,6 @@ namespace vlm {
 
 namespace {
 
-__device__ __forceinline__ d3 ld3(const double* p) { return mk3(p[0], p[1], p[2]); }
-__device__ __forceinline__ void st3(double* p, d3 v) {
-  p[0] = v.x;
-  p[1] = v.y;
-  p[2] = v.z;
-}
-__device__ __forceinline__ size_t ringI(const Dims& d, int b, int i, int j) {
-  return (size_t)b * d.NW * d.ns + i + (size_t)d.NW * j;
-}
-__device__ __forceinline__ size_t velI(const Dims& d, int b, int i, int j) {
-  return (size_t)b * d.NW * (d.ns + 1) + i + (size_t)d.NW * j;
-}
-__device__ __forceinline__ const double* panRec(const Dims& d, const double* fr, int b, int p) {
-  return fr + d.fl.pan + ((size_t)b * d.npan + p) * kPan;
-}
 __device__ __forceinline__ m33 frameT(const Dims& d, const double* fr, int b) {
   const double* t = fr + d.fl.rot + 10 + 9 * (b - 1);
   m33 T;
@@ -530,50 +516,6 @@ __global__ void k_order2(Dims d, DevState s, int rowNear, int rowFar, int phase)
   }
 }
 
-// ---- targets ----------------------------------------------------------------
-constexpr int kTileRows = 16, kTileCols = 4;
-__device__ __forceinline__ void decode_node(const Dims& d, int rowNear, int rowFar, int m, int& b, int& far, int& i,
-                                            int& j) {
-  const int rowsN = d.NW - (rowNear - 1);
-  const int rowsF = max(d.NF - (rowFar - 1), 0);
-  const int per = rowsN * (d.ns + 1) + rowsF;
-  b = m / per;
-  const int l = m % per;
-  if (l < rowsN * (d.ns + 1)) {
-    // tiles of kTileRows rows x kTileCols span stations, tile by tile: a run
-    // of 32 consecutive targets (one warp's lanes in the FP32 kernel) is a
-    // compact patch of the wake sheet, so few source rings come near any of
-    // them
-    far = 0;
-    const int band = l / (kTileRows * (d.ns + 1));
-    const int br = min(kTileRows, rowsN - band * kTileRows);
-    const int o = l - band * kTileRows * (d.ns + 1);
-    const int tc = o / (br * kTileCols);
-    const int q = o - tc * br * kTileCols;
-    i = rowNear - 1 + band * kTileRows + q % br;
-    j = tc * kTileCols + q / br;
-  } else {
-    far = 1;
-    j = 0;
-    i = rowFar - 1 + (l - rowsN * (d.ns + 1));
-  }
-}
-__global__ void k_node_targets(Dims d, DevState s, int rowNear, int rowFar, int pred, int M, double* P) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= M) return;
-  int b, far, i, j;
-  decode_node(d, rowNear, rowFar, m, b, far, i, j);
-  const double* nc = pred ? s.nCP : s.nC;
-  d3 p;
-  if (!far) p = j < d.ns ? ld3(nc + ringI(d, b, i, j) * 12 + 3) : ld3(nc + ringI(d, b, i, d.ns - 1) * 12 + 6);
-  else p = ld3((pred ? s.fCP : s.fC) + ((size_t)b * d.NF + i) * 6);
-  st3(P + 3 * (size_t)m, p);
-}
-__global__ void k_cp_targets(Dims d, const double* fr, double* P) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= d.nbC * d.npan) return;
-  st3(P + 3 * (size_t)m, ld3(panRec(d, fr, m / d.npan, m % d.npan) + 12));
-}
 __global__ void k_scatter_nodes(Dims d, DevState s, const double* fr, int rowNear, int rowFar, int pred,
                                 double initWakeVel, int addInit, int M) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
@@ -588,125 +530,6 @@ __global__ void k_scatter_nodes(Dims d, DevState s, const double* fr, int rowNea
   }
   double* dst = far ? s.vF[pred ? 4 : 0] + 3 * ((size_t)b * d.NF + i) : s.vN[pred ? 4 : 0] + 3 * velI(d, b, i, j);
   st3(dst, v);
-}
-
-// ---- source gather ----------------------------------------------------------
-// Lattice form of near-wake ring (b, i, j) (i the absolute row): the edge
-// weights of its record (see vlm_bs.h).  Ring (i, j-1)'s edge 2 runs from
-// its c2 to its c3, which are ring (i, j)'s c1 and c0, so with equal cores
-// the two filaments are one with the circulation difference; likewise ring
-// (i+1, j)'s edge 3 (its c3 -> c0 = ring (i, j)'s c2 -> c1).  Circulations
-// at or below eps count as zero (the skip of blade_vind_bywake,
-// src/classdef.f90:1452-1466).
-__device__ __forceinline__ bool same3(const double* a, const double* b) {
-  return a[0] == b[0] && a[1] == b[1] && a[2] == b[2];
-}
-__device__ void lattice_weights(const Dims& d, const DevState& s, const double* nc, int b, int i, int j, int rowNear,
-                                double* W) {
-  auto gam = [&](size_t r) {
-    const double g = s.nGam[r];
-    return fabs(g) > kEps ? g : 0.0;
-  };
-  // streamwise edge between stations: ring (i, jj-1) edge 2 == ring (i, jj) edge 0
-  auto mergeS = [&](int jj) {
-    const size_t a = ringI(d, b, i, jj - 1), c = ringI(d, b, i, jj);
-    return same3(nc + 12 * a + 9, nc + 12 * c) && same3(nc + 12 * a + 6, nc + 12 * c + 3) &&
-           s.nRvc[4 * a + 2] == s.nRvc[4 * c];
-  };
-  // spanwise edge between rows: ring (ii, j) edge 1 == ring (ii+1, j) edge 3
-  auto mergeC = [&](int ii) {
-    const size_t a = ringI(d, b, ii, j), c = ringI(d, b, ii + 1, j);
-    return same3(nc + 12 * c, nc + 12 * a + 3) && same3(nc + 12 * c + 9, nc + 12 * a + 6) &&
-           s.nRvc[4 * c + 3] == s.nRvc[4 * a + 1];
-  };
-  const double G = gam(ringI(d, b, i, j));
-  W[0] = j > 0 && mergeS(j) ? G - gam(ringI(d, b, i, j - 1)) : G;
-  W[1] = i + 1 < d.NW && mergeC(i) ? G - gam(ringI(d, b, i + 1, j)) : G;
-  W[2] = j + 1 < d.ns && mergeS(j + 1) ? 0.0 : G;
-  W[3] = i > rowNear - 1 && mergeC(i - 1) ? 0.0 : G;
-}
-
-__global__ void k_gather(Dims d, DevState s, const double* fr, const Group* groups, int ngroups, int nrec,
-                         int rowNear, int rowFar, int pred) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nrec) return;
-  int g = 0;
-  while (g + 1 < ngroups && t >= groups[g + 1].rec_begin) ++g;
-  const Group G = groups[g];
-  const int l0 = t - G.rec_begin;
-  const int b = G.blade;
-  double* R = s.rec64 + (size_t)t * kRec64;
-  if (G.kind == 0) {
-    const int j = l0 / d.nc, i = l0 % d.nc;
-    const int p = i + d.nc * j;
-    const double* w = panRec(d, fr, b, p);
-    for (int k = 0; k < 12; ++k) R[k] = w[k];
-    for (int k = 0; k < 4; ++k) R[12 + k] = s.wRvc[4 * ((size_t)b * d.npan + p) + k];
-    R[16] = s.wGam[(size_t)b * d.npan + p];
-    R[17] = 0.0;
-    if (s.edgeW)
-      for (int k = 0; k < 4; ++k) s.edgeW[4 * (size_t)t + k] = R[16];  // wing rings: no eps skip
-    return;
-  }
-  const int rowsN = d.NW - (rowNear - 1);
-  const int nNear = rowsN * d.ns;
-  const int hs = rowFar <= d.NF ? d.ns : 0;
-  const double* nc = pred ? s.nCP : s.nC;
-  // a far-only group (pad[0] = 1) lists the far filaments alone, from the
-  // pad[1]-th active one
-  const int l = G.pad[0] ? l0 + nNear + hs + G.pad[1] : l0;
-  if (l < nNear) {
-    const int j = l / rowsN, i = rowNear - 1 + l % rowsN;
-    const size_t r = ringI(d, b, i, j);
-    for (int k = 0; k < 12; ++k) R[k] = nc[12 * r + k];
-    for (int k = 0; k < 4; ++k) R[12 + k] = s.nRvc[4 * r + k];
-    R[16] = s.nGam[r];
-    R[17] = (double)REC_SKIP;
-    if (s.edgeW) lattice_weights(d, s, nc, b, i, j, rowNear, s.edgeW + 4 * (size_t)t);
-  } else if (l < nNear + hs) {
-    const size_t r = ringI(d, b, d.NW - 1, l - nNear);
-    for (int k = 0; k < 6; ++k) R[k] = nc[12 * r + 3 + k];
-    for (int k = 6; k < 12; ++k) R[k] = 0.0;
-    R[12] = s.nRvc[4 * r + 1];
-    R[13] = R[14] = R[15] = 0.0;
-    R[16] = -s.nGam[r];
-    R[17] = (double)REC_FIL;
-    if (s.edgeW) {
-      double* W = s.edgeW + 4 * (size_t)t;
-      W[0] = R[16];
-      W[1] = W[2] = W[3] = 0.0;
-    }
-  } else if (l >= nNear + hs + (rowFar <= d.NF ? d.NF - rowFar + 1 : 0)) {
-    // prescribed far wake (classdef.f90:1471-1476): single filaments
-    const int i = l - nNear - hs - (d.NF - rowFar + 1);
-    const size_t pb = (size_t)pred * d.nb + b;
-    const double* f = s.pfC + (pb * kPresc + i) * 6;
-    for (int k = 0; k < 6; ++k) R[k] = f[k];
-    for (int k = 6; k < 12; ++k) R[k] = 0.0;
-    R[12] = s.pfRvc[pb];
-    R[13] = R[14] = R[15] = 0.0;
-    R[16] = s.pfGam[pb];
-    R[17] = (double)(REC_FIL | REC_SKIP);
-    if (s.edgeW) {
-      double* W = s.edgeW + 4 * (size_t)t;
-      W[0] = fabs(R[16]) > kEps ? R[16] : 0.0;
-      W[1] = W[2] = W[3] = 0.0;
-    }
-  } else {
-    const size_t f = (size_t)b * d.NF + rowFar - 1 + (l - nNear - hs);
-    const double* fc = pred ? s.fCP : s.fC;
-    for (int k = 0; k < 6; ++k) R[k] = fc[6 * f + k];
-    for (int k = 6; k < 12; ++k) R[k] = 0.0;
-    R[12] = s.fRvc[f];
-    R[13] = R[14] = R[15] = 0.0;
-    R[16] = s.fGam[f];
-    R[17] = (double)(REC_FIL | REC_SKIP);
-    if (s.edgeW) {
-      double* W = s.edgeW + 4 * (size_t)t;
-      W[0] = fabs(R[16]) > kEps ? R[16] : 0.0;
-      W[1] = W[2] = W[3] = 0.0;
-    }
-  }
 }
 
 // ---- AIC and its inverse (classdef.f90:4151-4179, libMath.f90:48-83) ---------
@@ -1443,25 +1266,6 @@ int node_target_count(const Dims& d, int rowNear, int rowFar) {
   const int rowsN = d.NW - (rowNear - 1);
   const int rowsF = d.NF - (rowFar - 1) > 0 ? d.NF - (rowFar - 1) : 0;
   return d.nbC * (rowsN * (d.ns + 1) + rowsF);
-}
-void launch_node_targets(const Dims& d, const DevState& s, int rowNear, int rowFar, bool pred, double* P,
-                         cudaStream_t st) {
-  const int M = node_target_count(d, rowNear, rowFar);
-  if (M > 0) {
-    count_launch();
-    k_node_targets<<<nblk(M, 256), 256, 0, st>>>(d, s, rowNear, rowFar, pred ? 1 : 0, M, P);
-  }
-}
-void launch_cp_targets(const Dims& d, const double* frame, double* P, cudaStream_t st) {
-  count_launch();
-  k_cp_targets<<<nblk(d.nbC * d.npan, 128), 128, 0, st>>>(d, frame, P);
-}
-void launch_gather(const Dims& d, const DevState& s, const double* frame, const Group* groups, int ngroups, int nrec,
-                   int rowNear, int rowFar, bool pred, cudaStream_t st) {
-  if (nrec > 0) {
-    count_launch();
-    k_gather<<<nblk(nrec, 256), 256, 0, st>>>(d, s, frame, groups, ngroups, nrec, rowNear, rowFar, pred ? 1 : 0);
-  }
 }
 void launch_scatter_nodes(const Dims& d, const DevState& s, const double* frame, int rowNear, int rowFar, bool pred,
                           double initWakeVel, cudaStream_t st) {

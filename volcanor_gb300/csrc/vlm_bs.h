@@ -38,13 +38,9 @@ constexpr int REC_SKIP = 2;
 //            [30], [31] are -1 when edge 2 / edge 3 carries no circulation
 //            (the kernel then skips it and, if both, corner c3's vector)
 //   [32..35] near-field threshold on |r1 x r2|^2: (near_factor rvc_k |e_k|)^2, -1 if off
-//   [36..39] lower near-field bound on (w_k e_k).r1
-//   [40..43] upper near-field bound on (w_k e_k).r1
-//   [44..47] unused (zero; pads the record to 192 B)
+//   [36..47] unused (never read; they pad the record to 192 B)
 // A pair is near when the target lies within near_factor core radii of the
-// filament SEGMENT: |r1 x r2|^2 < [32+k] and -s < e.r1 < |e|^2 + s with
-// s = near_factor rvc_k |e_k|; the second test is stored multiplied by w_k,
-// so [36+k] < (w_k e_k).r1 < [40+k] (bounds swapped when w_k < 0).
+// filament SEGMENT.
 constexpr int kRec32 = 48;
 
 // Lattice form (FP32 paths): a near-wake lattice has every interior

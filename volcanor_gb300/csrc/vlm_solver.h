@@ -158,12 +158,20 @@ void launch_order2(const Dims& d, const DevState& s, int rowNear, int rowFar, cu
 // ---- Biot-Savart evaluations ---------------------------------------------
 // targets: wake nodes of blades < nbC (count returned by node_target_count)
 int node_target_count(const Dims& d, int rowNear, int rowFar);
-void launch_node_targets(const Dims& d, const DevState& s, int rowNear, int rowFar, bool pred, double* P,
-                         cudaStream_t st);
-void launch_cp_targets(const Dims& d, const double* frame, double* P, cudaStream_t st);
-// record gather for the given groups (kind 0 wing, kind 1 wake)
+// what a gather writes beside the records: the targets (kind 1: collocation
+// points, 2: wake nodes) and up to two counters to zero
+struct GatherTargets {
+  int kind = 0;
+  double* P = nullptr;
+  int M = 0;
+  int* zero[2] = {nullptr, nullptr};
+};
+// records of the given groups (kind 0 wing, kind 1 wake) into s.rec64, their
+// lattice weights into s.edgeW and their FP32 records, with near zones of
+// nearFactor core radii (0: none), into s.rec32, each where not null
 void launch_gather(const Dims& d, const DevState& s, const double* frame, const Group* groups, int ngroups,
-                   int nrec, int rowNear, int rowFar, bool pred, cudaStream_t st);
+                   int nrec, int rowNear, int rowFar, bool pred, double nearFactor, const GatherTargets& tg,
+                   cudaStream_t st);
 // node velocities from outv (0 + v), plus the initial wake velocity terms
 void launch_scatter_nodes(const Dims& d, const DevState& s, const double* frame, int rowNear, int rowFar, bool pred,
                           double initWakeVel, cudaStream_t st);
