@@ -30,8 +30,8 @@
 // (k_near_find).  For every listed pair k_near_fix recomputes the FP32
 // kernel's own contribution bit for bit (same
 // inline arithmetic, same FP32 inputs) and adds FP64 value - FP32
-// contribution to order-independent fixed-point accumulators, which
-// k_near_apply folds into the chunk partial sums.  The result equals summing
+// contribution to order-independent fixed-point accumulators, which the
+// combiner folds into the chunk partial sums.  The result equals summing
 // the far pairs in FP32 and the near pairs in FP64, up to the FP32 rounding
 // of the tile sums that held the near terms.
 #include <stdint.h>
@@ -971,17 +971,6 @@ __global__ void k_near_fix(const NearPair* __restrict__ near, int near_cap, cons
 
 __global__ void k_set_flag(int* ctl, int code) { atomicExch(ctl, code); }
 
-// part += nacc / 2^44, and nacc back to zero for the next evaluation.
-__global__ void k_near_apply(double* __restrict__ part, long long* __restrict__ nacc, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const long long a = nacc[i];
-    if (a != 0) {
-      part[i] += (double)a * (1.0 / kNearScale);
-      nacc[i] = 0;
-    }
-  }
-}
-
 // Self-test of the bounded waits: one thread waits on an mbarrier that
 // nothing arrives on, with a short limit; the wait must give up and report.
 __global__ void k_wait_probe(uint32_t limit, int* out) {
@@ -1087,7 +1076,7 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
   }
   // With ov, the near-field detection and FP64 correction (which read only
   // the records and targets) run on ov->stream alongside the pair kernel;
-  // the fold into the partial sums waits for both.
+  // what follows on s (the fold into the partial sums) waits for both.
   cudaStream_t ns = s;
   if (nearOn && ov) {
     cudaEventRecord(ov->fork, s);
@@ -1117,9 +1106,6 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
       cudaEventRecord(ov->join, ns);
       cudaStreamWaitEvent(s, ov->join, 0);
     }
-    const size_t n = (size_t)M * nchunks * 3;
-    count_launch();
-    k_near_apply<<<(unsigned)std::min<size_t>((n + 255) / 256, (size_t)8 * sms), 256, 0, s>>>(part, nacc, n);
     return;
   }
   if (!reuse_grid) {
@@ -1141,9 +1127,6 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
     cudaEventRecord(ov->join, ns);
     cudaStreamWaitEvent(s, ov->join, 0);
   }
-  const size_t n = (size_t)M * nchunks * 3;
-  count_launch();
-  k_near_apply<<<(unsigned)std::min<size_t>((n + 255) / 256, (size_t)8 * sms), 256, 0, s>>>(part, nacc, n);
 }
 
 // A host without a usable device still plans (sizes are queried before any

@@ -327,81 +327,73 @@ Tile64 pick_tile64(int M, int nchunks, int64_t nrec, int L, int sms) {
   return T;
 }
 
-__global__ void k_combine(const double* __restrict__ part, int M, const Group* __restrict__ groups, int ngroups,
-                          int mode, double* __restrict__ out) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= M) return;
-  d3 wing = zero3(), wake = zero3();
-  for (int g = 0; g < ngroups; ++g) {
-    const Group G = groups[g];
-    d3 gs = zero3();
-    int q = G.chunk_begin;
-    const int qe = G.chunk_begin + G.chunk_count;
-    // loads issued 16 at a time (the adds stay in chunk order): a collocation-
-    // point evaluation has few targets and hundreds of chunks
+// One component of a target's chunk partials -> group sums -> the result, a
+// thread (ORDERED) or G lanes per (target, component).
+//
+// ORDERED (FP64): each group's partials in chunk order, loads 16 at a time (a
+// collocation-point evaluation has few targets and hundreds of chunks).
+// Else (FP32 paths, whose summation order is free): G a power of two <= 32;
+// lane l adds partials l, l + G, ... in order, then a butterfly over the G
+// lanes.  The tree has a fixed shape, so the result is reproducible run to
+// run.  nacc: the near field's fixed-point corrections of the same partials,
+// folded in on the way and zeroed (a pass of their own over the partials before).
+// (One lane's 3 components in turn were 16 us at 16 targets, an FP64 addition
+// being 64 cycles; each component has its own lanes now.)
+template <bool ORDERED>
+__device__ __forceinline__ double group_sum(const double* __restrict__ part, long long* __restrict__ nacc, int M,
+                                            const Group& g, size_t mc, int l, int G, bool live) {
+  const size_t stride = 3 * (size_t)M;
+  double s = 0.0;
+  if (ORDERED) {
+    const double* p = part + g.chunk_begin * stride + mc;
+    int q = 0;
     constexpr int kB = 16;
-    for (; q + kB <= qe; q += kB) {
-      d3 buf[kB];
+    for (; q + kB <= g.chunk_count; q += kB, p += kB * stride) {
+      double buf[kB];
 #pragma unroll
-      for (int i = 0; i < kB; ++i) {
-        const double* pp = part + ((size_t)(q + i) * M + m) * 3;
-        buf[i] = mk3(pp[0], pp[1], pp[2]);
-      }
+      for (int i = 0; i < kB; ++i) buf[i] = p[i * stride];
 #pragma unroll
-      for (int i = 0; i < kB; ++i) gs = gs + buf[i];
+      for (int i = 0; i < kB; ++i) s = s + buf[i];
     }
-    for (; q < qe; ++q) {
-      const double* pp = part + ((size_t)q * M + m) * 3;
-      gs = gs + mk3(pp[0], pp[1], pp[2]);
-    }
-    if (G.kind == 0) wing = wing + gs;
-    else wake = wake + gs;
+    for (; q < g.chunk_count; ++q, p += stride) s = s + p[0];
+    return s;
   }
-  d3 v;
-  if (mode == 0) v = zero3() + (wing + wake);
-  else if (mode == 1) v = wake;
-  else v = wing + wake;
-  out[3 * (size_t)m] = v.x;
-  out[3 * (size_t)m + 1] = v.y;
-  out[3 * (size_t)m + 2] = v.z;
+  if (live)
+    for (int q = g.chunk_begin + l; q < g.chunk_begin + g.chunk_count; q += G) {
+      double p = part[q * stride + mc];
+      if (nacc) {
+        const long long a = nacc[q * stride + mc];
+        if (a != 0) {
+          p += (double)a * (1.0 / kNearScale);
+          nacc[q * stride + mc] = 0;
+        }
+      }
+      s = s + p;
+    }
+  for (int o = G >> 1; o > 0; o >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, o, G);
+  return s;
 }
 
-// Unordered combine (FP32 paths, whose summation order is free): G lanes
-// per target (G a power of two <= 32); lane l of a target adds chunk
-// partials l, l + G, ... of a group in order, then a butterfly over the G
-// lanes.  The tree has a fixed shape, so the result is reproducible run to
-// run; the serial chain is chunks/G adds long.
-__global__ void k_combine_tree(const double* __restrict__ part, int M, const Group* __restrict__ groups, int ngroups,
-                               int mode, int G, double* __restrict__ out) {
+// mode 0 (wake nodes): out = 0 + (wing + wake); 1: wake; 2: wing + wake.
+// ADD: out = out + that.
+template <bool ORDERED, bool ADD>
+__global__ void k_combine(const double* __restrict__ part, long long* __restrict__ nacc, int M,
+                          const Group* __restrict__ groups, int ngroups, int mode, int G, double* __restrict__ out) {
   const size_t gt = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  const int m = (int)(gt / G), l = (int)(gt % G);
-  const bool live = m < M;  // dead lanes still take part in the shuffles
-  d3 wing = zero3(), wake = zero3();
+  const size_t mc = gt / G;
+  const int l = (int)(gt % G);
+  const bool live = mc < 3 * (size_t)M;  // dead lanes still take part in the shuffles
+  if (ORDERED && !live) return;
+  double wing = 0.0, wake = 0.0;
   for (int g = 0; g < ngroups; ++g) {
-    const Group G_ = groups[g];
-    d3 gs = zero3();
-    if (live)
-      for (int q = G_.chunk_begin + l; q < G_.chunk_begin + G_.chunk_count; q += G) {
-        const double* pp = part + ((size_t)q * M + m) * 3;
-        gs = gs + mk3(pp[0], pp[1], pp[2]);
-      }
-    for (int o = G >> 1; o > 0; o >>= 1) {
-      gs.x = gs.x + __shfl_xor_sync(0xffffffffu, gs.x, o, G);
-      gs.y = gs.y + __shfl_xor_sync(0xffffffffu, gs.y, o, G);
-      gs.z = gs.z + __shfl_xor_sync(0xffffffffu, gs.z, o, G);
-    }
-    if (G_.kind == 0) wing = wing + gs;
-    else wake = wake + gs;
+    const Group gr = groups[g];
+    const double s = group_sum<ORDERED>(part, nacc, M, gr, mc, l, G, live);
+    if (gr.kind == 0) wing = wing + s;
+    else wake = wake + s;
   }
-  if (live && l == 0) {
-    d3 v;
-    if (mode == 0) v = zero3() + (wing + wake);
-    else if (mode == 1) v = wake;
-    else v = wing + wake;
-    out[3 * (size_t)m] = v.x;
-    out[3 * (size_t)m + 1] = v.y;
-    out[3 * (size_t)m + 2] = v.z;
-  }
+  if (!live || l != 0) return;
+  const double v = mode == 0 ? 0.0 + (wing + wake) : mode == 1 ? wake : wing + wake;
+  out[mc] = ADD ? out[mc] + v : v;
 }
 
 // Coupled rotors: the groups carry the index of the sum they belong to
@@ -412,92 +404,42 @@ __global__ void k_combine_tree(const double* __restrict__ part, int M, const Gro
 // out[t][m] = 0 + the term's groups in order, one per-rotor wake or wing
 // sum each, which the RHS adds to velCP in turn.  With a single term, mode 0
 // equals k_combine's mode 0 bit for bit.
-__device__ __forceinline__ void term_done(int mode, int t, int M, int m, d3& v, d3& wing, d3& wake, d3& ts,
-                                          double* out) {
-  if (mode == 0) {
-    v = v + (wing + wake);
-  } else {
-    double* o = out + 3 * ((size_t)t * M + m);
-    o[0] = ts.x;
-    o[1] = ts.y;
-    o[2] = ts.z;
-  }
-  wing = wake = ts = zero3();
-}
-
-__global__ void k_combine_terms(const double* __restrict__ part, int M, const Group* __restrict__ groups,
-                                int ngroups, int mode, double* __restrict__ out) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= M || ngroups <= 0) return;
-  d3 v = zero3(), wing = zero3(), wake = zero3(), ts = zero3();
-  int t = groups[0].term;
-  for (int g = 0; g < ngroups; ++g) {
-    const Group G = groups[g];
-    if (G.term != t) {
-      term_done(mode, t, M, m, v, wing, wake, ts, out);
-      t = G.term;
-    }
-    d3 gs = zero3();
-    for (int q = G.chunk_begin; q < G.chunk_begin + G.chunk_count; ++q) {
-      const double* pp = part + ((size_t)q * M + m) * 3;
-      gs = gs + mk3(pp[0], pp[1], pp[2]);
-    }
-    if (mode == 0) {
-      if (G.kind == 0) wing = wing + gs;
-      else wake = wake + gs;
-    } else {
-      ts = ts + gs;
-    }
-  }
-  term_done(mode, t, M, m, v, wing, wake, ts, out);
-  if (mode == 0) {
-    out[3 * (size_t)m] = v.x;
-    out[3 * (size_t)m + 1] = v.y;
-    out[3 * (size_t)m + 2] = v.z;
-  }
-}
-
-// The same with k_combine_tree's fixed-shape tree per group (FP32 paths).
-__global__ void k_combine_terms_tree(const double* __restrict__ part, int M, const Group* __restrict__ groups,
-                                     int ngroups, int mode, int G, double* __restrict__ out) {
+template <bool ORDERED>
+__global__ void k_combine_terms(const double* __restrict__ part, long long* __restrict__ nacc, int M,
+                                const Group* __restrict__ groups, int ngroups, int mode, int G,
+                                double* __restrict__ out) {
   const size_t gt = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  const int m = (int)(gt / G), l = (int)(gt % G);
-  const bool live = m < M;
-  if (ngroups <= 0) return;
-  d3 v = zero3(), wing = zero3(), wake = zero3(), ts = zero3();
+  const size_t mc = gt / G;
+  const int l = (int)(gt % G);
+  const bool live = mc < 3 * (size_t)M;
+  if (ORDERED && !live) return;
+  double v = 0.0, wing = 0.0, wake = 0.0, ts = 0.0;
   int t = groups[0].term;
+  auto done = [&]() {
+    if (mode == 0) v = v + (wing + wake);
+    else if (live && l == 0) out[3 * (size_t)M * t + mc] = ts;
+    wing = wake = ts = 0.0;
+  };
   for (int g = 0; g < ngroups; ++g) {
-    const Group G_ = groups[g];
-    if (G_.term != t) {
-      if (live && l == 0) term_done(mode, t, M, m, v, wing, wake, ts, out);
-      t = G_.term;
+    const Group gr = groups[g];
+    if (gr.term != t) {
+      done();
+      t = gr.term;
     }
-    d3 gs = zero3();
-    if (live)
-      for (int q = G_.chunk_begin + l; q < G_.chunk_begin + G_.chunk_count; q += G) {
-        const double* pp = part + ((size_t)q * M + m) * 3;
-        gs = gs + mk3(pp[0], pp[1], pp[2]);
-      }
-    for (int o = G >> 1; o > 0; o >>= 1) {
-      gs.x = gs.x + __shfl_xor_sync(0xffffffffu, gs.x, o, G);
-      gs.y = gs.y + __shfl_xor_sync(0xffffffffu, gs.y, o, G);
-      gs.z = gs.z + __shfl_xor_sync(0xffffffffu, gs.z, o, G);
-    }
-    if (mode == 0) {
-      if (G_.kind == 0) wing = wing + gs;
-      else wake = wake + gs;
-    } else {
-      ts = ts + gs;
-    }
+    const double s = group_sum<ORDERED>(part, nacc, M, gr, mc, l, G, live);
+    if (mode != 0) ts = ts + s;
+    else if (gr.kind == 0) wing = wing + s;
+    else wake = wake + s;
   }
-  if (live && l == 0) {
-    term_done(mode, t, M, m, v, wing, wake, ts, out);
-    if (mode == 0) {
-      out[3 * (size_t)m] = v.x;
-      out[3 * (size_t)m + 1] = v.y;
-      out[3 * (size_t)m + 2] = v.z;
-    }
-  }
+  done();
+  if (mode == 0 && live && l == 0) out[mc] = v;
+}
+
+// lanes per (target, component): about 8 chunk partials each, at most a warp
+inline int tree_lanes(int max_chunks) {
+  int G = 1;
+  while (G < 32 && G * 8 < max_chunks) G <<= 1;
+  return G;
 }
 
 __global__ void k_rings_to_rec64(const double* __restrict__ corners, const double* __restrict__ rvc,
@@ -608,32 +550,32 @@ void launch_combine(const double* part, int M, const Group* groups, int ngroups,
                     cudaStream_t s) {
   if (M <= 0) return;
   count_launch();
-  k_combine<<<(M + 127) / 128, 128, 0, s>>>(part, M, groups, ngroups, mode, out);
+  k_combine<true, false><<<(unsigned)((3 * (size_t)M + 127) / 128), 128, 0, s>>>(part, nullptr, M, groups, ngroups,
+                                                                                mode, 1, out);
 }
 
-void launch_combine_unordered(const double* part, int M, const Group* groups, int ngroups, int max_chunks, int mode,
-                              double* out, cudaStream_t s) {
+void launch_combine_unordered(const double* part, long long* nacc, int M, const Group* groups, int ngroups,
+                              int max_chunks, int mode, double* out, cudaStream_t s, bool add) {
   if (M <= 0) return;
-  // about 8 chunk partials per lane, at most a warp per target
-  int G = 1;
-  while (G < 32 && G * 8 < max_chunks) G <<= 1;
-  const size_t threads = (size_t)M * G;
+  const int G = tree_lanes(max_chunks);
+  const unsigned blocks = (unsigned)((3 * (size_t)M * G + 255) / 256);
   count_launch();
-  k_combine_tree<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(part, M, groups, ngroups, mode, G, out);
+  if (add) k_combine<false, true><<<blocks, 256, 0, s>>>(part, nacc, M, groups, ngroups, mode, G, out);
+  else k_combine<false, false><<<blocks, 256, 0, s>>>(part, nacc, M, groups, ngroups, mode, G, out);
 }
 
-void launch_combine_terms(const double* part, int M, const Group* groups, int ngroups, int max_chunks, int mode,
-                          bool ordered, double* out, cudaStream_t s) {
+void launch_combine_terms(const double* part, long long* nacc, int M, const Group* groups, int ngroups,
+                          int max_chunks, int mode, bool ordered, double* out, cudaStream_t s) {
   if (M <= 0 || ngroups <= 0) return;
   count_launch();
   if (ordered) {
-    k_combine_terms<<<(M + 127) / 128, 128, 0, s>>>(part, M, groups, ngroups, mode, out);
+    k_combine_terms<true><<<(unsigned)((3 * (size_t)M + 127) / 128), 128, 0, s>>>(part, nullptr, M, groups, ngroups,
+                                                                                 mode, 1, out);
     return;
   }
-  int G = 1;
-  while (G < 32 && G * 8 < max_chunks) G <<= 1;
-  const size_t threads = (size_t)M * G;
-  k_combine_terms_tree<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(part, M, groups, ngroups, mode, G, out);
+  const int G = tree_lanes(max_chunks);
+  k_combine_terms<false><<<(unsigned)((3 * (size_t)M * G + 255) / 256), 256, 0, s>>>(part, nacc, M, groups, ngroups,
+                                                                                    mode, G, out);
 }
 
 void launch_fils_to_rec64(const double* fc, const double* rvc, const double* gam, int64_t N, double* rec,

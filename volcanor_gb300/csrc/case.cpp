@@ -542,13 +542,13 @@ struct Case {
     if (!P) P = s.targets;
     if (!out) out = s.outv;
     if (prec < 0) prec = opt.precision;
+    const bool near = prec == VLM_PREC_FP32_NEAR64;
     const Chunk* ch = dChunks + e.coff;
     if (prec == VLM_PREC_FP64) {
       partial64(e, ch, P, M);
     } else {
-      const bool nearOn = prec == VLM_PREC_FP32_NEAR64;
       launch_partial32(s.rec32, s.rec64, ch, e.nchunks, e.nrec, P, M, s.part, s.err + 2,
-                       nearOn ? s.nearScratch : nullptr, s.nearBytes, s.nacc, stream, s.edgeW, e.shape,
+                       near ? s.nearScratch : nullptr, s.nearBytes, s.nacc, stream, s.edgeW, e.shape,
                        opt.nbody_slots > 0 ? nullptr : &nearOv);  // a batch's cases already run side by side
     }
     if (e.nchunks == 0) {
@@ -556,9 +556,9 @@ struct Case {
       return;
     }
     if (nterms > 0)
-      launch_combine_terms(s.part, M, dGroups + e.goff, e.ngroups, e.maxq, mode, prec == VLM_PREC_FP64, out, stream);
+      launch_combine_terms(s.part, near ? s.nacc : nullptr, M, dGroups + e.goff, e.ngroups, e.maxq, mode, prec == VLM_PREC_FP64, out, stream);
     else if (prec == VLM_PREC_FP64) launch_combine(s.part, M, dGroups + e.goff, e.ngroups, mode, out, stream);
-    else launch_combine_unordered(s.part, M, dGroups + e.goff, e.ngroups, e.maxq, mode, out, stream);
+    else launch_combine_unordered(s.part, near ? s.nacc : nullptr, M, dGroups + e.goff, e.ngroups, e.maxq, mode, out, stream);
   }
 
   // ---- autotuner of the FP32 N-body tile shape and chunking ----------------
@@ -836,7 +836,7 @@ struct Case {
     int dq = 0, dmaxq = 0, mq = 0, mmaxq = 0, mng = 0;
     Group *dG = nullptr, *mG = nullptr;
     Chunk *dC = nullptr, *mC = nullptr;
-    double *dRec = nullptr, *dEw = nullptr, *outD = nullptr, *tPos = nullptr, *tOut = nullptr;
+    double *dRec = nullptr, *dEw = nullptr, *tPos = nullptr, *tOut = nullptr;
     double *dPart = nullptr, *mPart = nullptr;
     long long *dNacc = nullptr, *mNacc = nullptr;
     int* tIdx = nullptr;
@@ -983,7 +983,6 @@ struct Case {
     VLM_CUDA(cudaMemcpy(ip.mC, mch.data(), sizeof(Chunk) * ip.mq, cudaMemcpyHostToDevice));
     ip.dRec = dalloc<double>((size_t)ip.dcap * kRec64, incrOwned);
     ip.dEw = lattice() ? dalloc<double>((size_t)ip.dcap * 4, incrOwned) : nullptr;
-    ip.outD = dalloc<double>((size_t)ip.M * 3, incrOwned);
     ip.tIdx = dalloc<int>((size_t)ip.mcap, incrOwned);
     ip.tPos = dalloc<double>((size_t)ip.mcap * 3, incrOwned);
     ip.tOut = dalloc<double>((size_t)ip.mcap * 3, incrOwned);
@@ -1017,7 +1016,7 @@ struct Case {
     }
     launch_partial32(ip.mRec32, recP, ip.mC, ip.mq, e.nrec, ip.tPos, ip.mcap, ip.mPart, incrCtl, ip.mNear,
                      ip.mNearBytes, ip.mNacc, ms, ew, 0, side ? &incrOv : nullptr);
-    launch_combine_unordered(ip.mPart, ip.mcap, ip.mG, ip.mng, ip.mmaxq, 0, ip.tOut, ms);
+    launch_combine_unordered(ip.mPart, nearOn ? ip.mNacc : nullptr, ip.mcap, ip.mG, ip.mng, ip.mmaxq, 0, ip.tOut, ms);
     if (side) VLM_CUDA(cudaEventRecord(incrJoin, incrStream));
     // the changed records (new +, old -) at every target: the current-wake
     // targets, whose near-field grid the current-wake evaluation left in the
@@ -1028,9 +1027,9 @@ struct Case {
     launch_partial32(s.rec32, ip.dRec, ip.dC, ip.dq, ip.dcap, s.targets, M, ip.dPart, s.err + 2,
                      nearOn ? s.nearScratch : nullptr, s.nearBytes, ip.dNacc, stream, ip.dEw, 0,
                      side ? &nearOv : nullptr, true);
-    launch_combine_unordered(ip.dPart, M, ip.dG, 1, ip.dmaxq, 0, ip.outD, stream);
+    launch_combine_unordered(ip.dPart, nearOn ? ip.dNacc : nullptr, M, ip.dG, 1, ip.dmaxq, 0, s.outv, stream, true);
     if (side) VLM_CUDA(cudaStreamWaitEvent(stream, incrJoin, 0));
-    launch_incr_merge(s.outv, ip.outD, M, ip.tIdx, ip.tOut, incrCnt + 1, ip.mcap, incrCtl, s.err + 2, stream);
+    launch_incr_merge(s.outv, ip.tIdx, ip.tOut, incrCnt + 1, ip.mcap, incrCtl, s.err + 2, stream);
   }
 
   // ---- coupled rotors (nr > 1, vlm_system) ----------------------------------
@@ -1997,6 +1996,9 @@ struct Case {
     VLM_CUDA(cudaEventRecord(ev0, stream));
     for (int r = 0; r < reps; ++r) launch();
     VLM_CUDA(cudaEventRecord(ev1, stream));
+    // no combine took the near-field corrections of these launches
+    if (opt.precision == VLM_PREC_FP32_NEAR64)
+      VLM_CUDA(cudaMemsetAsync(s.nacc, 0, sizeof(long long) * 3 * (size_t)M * pl.node.nchunks, stream));
     VLM_CUDA(cudaStreamSynchronize(stream));
     float ms = 0.f;
     VLM_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
@@ -2232,13 +2234,14 @@ struct Case {
       GatherTargets tg;
       tg.zero[0] = s.err + 3;
       launch_gather(d, t, frame(fi), dg, (int)g.size(), rec, rN, rF, false, nearFactor(), tg, stream);
+      long long* nacc = nullptr;
       if (opt.precision == VLM_PREC_FP64) {
         launch_partial64(rec64, dc, nq, rec, dP, (int)M, part, stream);
       } else {
         const bool nearOn = opt.precision == VLM_PREC_FP32_NEAR64;
         const size_t nb = nearOn ? near_scratch_bytes((int)M, (size_t)std::min<int64_t>(64 * M + (1 << 16), 1 << 26)) : 1;
         unsigned char* ns = dalloc<unsigned char>(nb, tmpOwned);
-        long long* nacc = dalloc<long long>(nearOn ? (size_t)M * nq * 3 : 1, tmpOwned);
+        if (nearOn) nacc = dalloc<long long>((size_t)M * nq * 3, tmpOwned);
         launch_partial32(rec32, rec64, dc, nq, rec, dP, (int)M, part, s.err + 2, nearOn ? ns : nullptr, nb, nacc,
                          stream);
       }
@@ -2246,7 +2249,7 @@ struct Case {
       else {
         int maxq = 0;
         for (const Group& q : g) maxq = std::max(maxq, q.chunk_count);
-        launch_combine_unordered(part, (int)M, dg, (int)g.size(), maxq, 2, dV, stream);
+        launch_combine_unordered(part, nacc, (int)M, dg, (int)g.size(), maxq, 2, dV, stream);
       }
       VLM_CUDA(cudaMemcpyAsync(V, dV, (size_t)M * 3 * sizeof(double), cudaMemcpyDeviceToHost, stream));
       VLM_CUDA(cudaStreamSynchronize(stream));
@@ -2382,7 +2385,7 @@ void rings_device(const double* corners, const double* rvc, const double* gam, i
                        R.nacc, st);
     }
     if (precision == VLM_PREC_FP64) launch_combine(R.part, (int)M, R.group, 1, 2, V, st);
-    else launch_combine_unordered(R.part, (int)M, R.group, 1, nq, 2, V, st);
+    else launch_combine_unordered(R.part, precision == VLM_PREC_FP32_NEAR64 ? R.nacc : nullptr, (int)M, R.group, 1, nq, 2, V, st);
   } else {
     VLM_CUDA(cudaMemsetAsync(V, 0, (size_t)M * 3 * 8, st));
   }

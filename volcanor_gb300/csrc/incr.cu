@@ -191,11 +191,6 @@ __global__ void __launch_bounds__(kDiffThreads)
   if (blockIdx.x == 0 && threadIdx.x == 0 && n > cap) atomicCAS(ctl, 0, 5);
 }
 
-__global__ void k_incr_add(double* __restrict__ out, const double* __restrict__ delta, int n3) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n3) out[i] = out[i] + delta[i];
-}
-
 // also passes the moved targets' evaluation's error code on to the step's
 __global__ void k_incr_put(double* __restrict__ out, const int* __restrict__ idx, const double* __restrict__ v,
                            const int* __restrict__ total, int cap, const int* __restrict__ subCtl,
@@ -242,11 +237,8 @@ void launch_moved_targets(const double* tP, const double* tC, int M, const int* 
   k_moved_targets<<<diff_blocks(M), kDiffThreads, 0, s>>>(tP, tC, M, blockOff, total, idx, pos, cap, ctl);
 }
 
-void launch_incr_merge(double* out, const double* delta, int M, const int* idx, const double* moved,
-                       const int* total, int cap, const int* subCtl, int* ctl, cudaStream_t s) {
-  if (M <= 0) return;
-  count_launch();
-  k_incr_add<<<(3 * M + 255) / 256, 256, 0, s>>>(out, delta, 3 * M);
+void launch_incr_merge(double* out, const int* idx, const double* moved, const int* total, int cap, const int* subCtl,
+                       int* ctl, cudaStream_t s) {
   count_launch();
   k_incr_put<<<(std::max(cap, 1) + 255) / 256, 256, 0, s>>>(out, idx, moved, total, cap, subCtl, ctl);
 }

@@ -170,7 +170,7 @@ extern "C" int vlm_biot_savart_rings_noalloc(const double* corners, const double
       launch_pack32(rec64, (int)N, nearOn ? 4.0 : 0.0, rec32, st);
       launch_partial32(rec32, rec64, chunks, cl.n, (int)N, P, (int)M, part, ctl, nearOn ? near : nullptr, kNearBytes,
                        nacc, st);
-      launch_combine_unordered(part, (int)M, group, 1, cl.n, 2, V, st);
+      launch_combine_unordered(part, nearOn ? nacc : nullptr, (int)M, group, 1, cl.n, 2, V, st);
     }
   } else {
     count_launch();

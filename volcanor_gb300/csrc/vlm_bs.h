@@ -207,18 +207,19 @@ void launch_combine(const double* part, int M, const Group* groups, int ngroups,
                     cudaStream_t s);
 
 // As launch_combine, but each group's chunk partials are added as a fixed
-// tree (up to a warp per target, sized by max_chunks, the largest chunk count
-// of a group) instead of in chunk order: for the FP32 paths, whose chunking
-// is itself free.
-void launch_combine_unordered(const double* part, int M, const Group* groups, int ngroups, int max_chunks, int mode,
-                              double* out, cudaStream_t s);
+// tree (up to a warp per target component, sized by max_chunks, the largest chunk
+// count of a group) instead of in chunk order: for the FP32 paths, whose
+// chunking is itself free.  nacc (or null): launch_partial32's near-field
+// corrections, folded in and zeroed.  add: out = out + the result.
+void launch_combine_unordered(const double* part, long long* nacc, int M, const Group* groups, int ngroups,
+                              int max_chunks, int mode, double* out, cudaStream_t s, bool add = false);
 
 // Coupled rotors: chunk partials -> per-term sums (Group::term).  mode 0:
 // out[m] = sum over terms of (wing + wake), in term order; mode 3:
 // out[t * M + m] = the term's own sum.  ordered: the FP64 chunk order;
-// else the FP32 paths' fixed tree.
-void launch_combine_terms(const double* part, int M, const Group* groups, int ngroups, int max_chunks, int mode,
-                          bool ordered, double* out, cudaStream_t s);
+// else the FP32 paths' fixed tree, with nacc as above.
+void launch_combine_terms(const double* part, long long* nacc, int M, const Group* groups, int ngroups,
+                          int max_chunks, int mode, bool ordered, double* out, cudaStream_t s);
 
 // Incremental predicted-wake evaluation (incr.cu).  Items of two sets that
 // differ bit by bit (records: kRec64 doubles and, with ea/eb, 4 edge weights;
@@ -236,11 +237,10 @@ void launch_delta_records(const double* recP, const double* recC, const double* 
 // The moved targets' indices and positions, padded to cap; ctl = 5 when more than cap moved.
 void launch_moved_targets(const double* tP, const double* tC, int M, const int* blockOff, const int* total, int* idx,
                           double* pos, int cap, int* ctl, cudaStream_t s);
-// out[m] += delta[m] at every target, then out[idx[i]] = moved[i] for the
-// moved ones; a nonzero subCtl[0] (the moved targets' evaluation's launch_partial32
-// code) is passed on to ctl.
-void launch_incr_merge(double* out, const double* delta, int M, const int* idx, const double* moved,
-                       const int* total, int cap, const int* subCtl, int* ctl, cudaStream_t s);
+// out[idx[i]] = moved[i] for the moved targets; a nonzero subCtl[0] (the moved
+// targets' evaluation's launch_partial32 code) is passed on to ctl.
+void launch_incr_merge(double* out, const int* idx, const double* moved, const int* total, int cap, const int* subCtl,
+                       int* ctl, cudaStream_t s);
 
 // Launches a wait that nothing releases, bounded by `limit` polls: 1 if it
 // gave up and reported (the expected outcome), 0 if it did not, -1 on a CUDA
