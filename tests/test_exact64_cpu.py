@@ -50,6 +50,15 @@ int main() {
     for (double d : a)
       if (!div_in_range(d) || !same(divide(d, r, Z), d / s)) return 2;
   }
+  // any divisor: extremes of its significand, quotients next to midpoints, both signs
+  for (int i = 0; i < 1000000; ++i) {
+    const double d = (i & 1 ? -1.0 : 1.0) * number(-200, 200);
+    const double a = i % 3 ? number(-800, 700) : (double)((long double)d * ((long double)number(0, 1) + ldexpl(1, -53)));
+    if (!divisor_in_range(d) || !same(quotient(a, d), a / d) || !same(quotient(0.0, d), 0.0 / d)) return 5;
+  }
+  for (double d : {0.0, -0.0, 1e-310, 1e300, (double)INFINITY, (double)NAN, 3.0})
+    for (double a : {0.0, 1.0, -2e-308, 1e308, (double)INFINITY, (double)NAN})
+      if (!same(quotient(a, d), a / d)) return 6;
   std::uniform_real_distribution<double> U(-1, 1);
   for (int i = 0; i < 200000; ++i) {
     const double sc = i % 7 == 0 ? ldexp(1.0, (int)(g() % 1200) - 600) : 1.0;
@@ -66,6 +75,9 @@ int main() {
       case 6: c[3].y = NAN; break;
     }
     if (!same(vr_vind64(P, c, rv), exact64::vr_vind(Unit{1.0, -0.0}, P, c, rv))) return 3;
+    if (!same(exact64::unit(c[0]), unit3(c[0])) || !same(exact64::proj(P, c[1]), proj3(P, c[1])) ||
+        !same(exact64::noproj(P, c[1]), noproj3(P, c[1])) || !same(exact64::norm(c[2]), norm3(c[2])))
+      return 7;
     if (!same(fil_vind64(P, c[0], c[1], rv[0]), exact64::fil_vind(Unit{1.0, -0.0}, P, c[0], c[1], rv[0]))) return 4;
   }
   return 0;

@@ -396,6 +396,7 @@ struct Case {
     s.bladeForce = dalloc<double>((size_t)nb * 12, owned);
     s.rotorLift = dalloc<double>(6, owned);
     s.ctHist = dalloc<double>((size_t)(nt + 1) * 10, owned);
+    s.loadTmp = dalloc<double>((size_t)9 * nb * npan, owned);
     s.err = dalloc<int>(4, owned);
     s.devIter = dalloc<int>(1, owned);
     s.curFrame = dalloc<double>(d.fl.size, owned);

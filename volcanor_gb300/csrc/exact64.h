@@ -181,6 +181,66 @@ VLM_HD double divide(double a, const Root& r, uint64_t Z) {
   return is_zero(a) ? a : from_bits(w);
 }
 
+// 1/r in FP32, r in [1, 2)
+VLM_HD float rcp32(float r) {
+#if defined(__CUDA_ARCH__)
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(r));
+  return y;
+#elif defined(VLM_RSQRT32_FACTOR)
+  return (1.0f / r) * (VLM_RSQRT32_FACTOR);
+#else
+  return 1.0f / r;
+#endif
+}
+// Any divisor d with |d| in [2^-200, 2^200) (divisor_in_range): as root_of, with
+// one Newton step Y += Y (1 - r Y) in 32 bits (error < 2^-28).
+VLM_HD bool divisor_in_range(double d) {
+  const uint32_t lo = (1023u - 200u) << 20, hi = (1023u + 200u) << 20;
+  return (high(d) & 0x7fffffffu) - lo < hi - lo;
+}
+VLM_HD Root divisor_of(double d) {
+  const uint64_t u = bits(d);
+  Root r;
+  r.N = (u & 0xfffffffffffffull) | 0x10000000000000ull;
+  r.exp = (int32_t)((u >> 52) & 0x7ffu) - 1023;
+  uint32_t rb = bits_float(rcp32(float_bits(0x3f800000u | (uint32_t)((u >> 29) & 0x7fffffu))));
+  rb = rb < 0x3f000000u ? 0x3f000000u : rb;
+  uint32_t Y = rb >= 0x3f800000u ? 0x80000000u : ((rb & 0x7fffffu) | 0x800000u) << 7;
+  const int32_t e = (1 << 30) - (int32_t)mulhi32(Y, (uint32_t)(r.N >> 21));
+  Y += (uint32_t)(mulhi32s((int32_t)((uint32_t)e << 16), (int32_t)(Y >> 1)) >> 13);
+  r.Y = Y;
+  return r;
+}
+VLM_HD double with_sign(double a, double d) { return from_bits(bits(a) ^ (bits(d) & 0x8000000000000000ull)); }
+// a / d
+VLM_HD double quotient(double a, double d) {
+  if (!divisor_in_range(d) || !div_in_range(a)) return a / d;
+  const Root r = divisor_of(d);
+  return with_sign(divide(a, r, reciprocal(r)), d);
+}
+VLM_HD d3 quotient(d3 a, double d) {
+  if (!divisor_in_range(d) || !div_in_range(a.x) || !div_in_range(a.y) || !div_in_range(a.z)) return a / d;
+  const Root r = divisor_of(d);
+  const uint64_t Z = reciprocal(r);
+  return mk3(with_sign(divide(a.x, r, Z), d), with_sign(divide(a.y, r, Z), d), with_sign(divide(a.z, r, Z), d));
+}
+VLM_HD double root(double x) { return in_range(x) ? value(root_of(x)) : sqrt(x); }
+// vlm_math.h's norm3, unit3, proj3, noproj3
+VLM_HD double norm(d3 a) { return root(sumsq3(a)); }
+VLM_HD d3 unit(d3 a) {
+  const double n = norm(a);
+  return n > kEps ? quotient(a, n) : zero3();
+}
+VLM_HD d3 proj(d3 a, d3 d) {
+  const double ns = sumsq3(d);
+  return ns > kEps ? quotient(dot3(a, d) * d, ns) : zero3();
+}
+VLM_HD d3 noproj(d3 a, d3 d) {
+  const double ns = sumsq3(d);
+  return ns > kEps ? a - quotient(dot3(a, d) * d, ns) : a;
+}
+
 // ---- the Biot-Savart functions of vlm_math.h with these roots and divisions ----
 // The same operations in the same order, so the same bits; numbers outside the
 // ranges above (a target on a corner, coordinates beyond 1e60) take
@@ -255,7 +315,6 @@ VLM_HD corner64 make_corner(const Unit& k, d3 P, d3 c) {
   }
   return o;
 }
-VLM_HD double root(double x) { return in_range(x) ? value(root_of(x)) : sqrt(x); }
 VLM_HD d3 vf_vind(const Unit& k, const corner64& a, const corner64& b, double rvc) {
   const d3 r0 = sub(k, a.r, b.r);
   const d3 c = cross(k, a.r, b.r);

@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "exact64.h"
 #include "vlm_math.h"
 #include "vlm_solver.h"
 
@@ -28,8 +29,44 @@ constexpr size_t kSmemMax = 226 * 1024;
 // a - b c, as the reference rounds it in FP64 and fused in FP32
 __device__ __forceinline__ double sub_mul(double a, double b, double c) { return a - b * c; }
 __device__ __forceinline__ float sub_mul(float a, float b, float c) { return fmaf(-b, c, a); }
-__device__ __forceinline__ double mag(double a) { return fabs(a); }
-__device__ __forceinline__ float mag(float a) { return fabsf(a); }
+// |a| as an integer that orders like it (a comparison of doubles takes the FP64
+// unit), -1 for NaN, which no comparison prefers
+__device__ __forceinline__ long long mag(double a) {
+  const long long b = __double_as_longlong(a) & 0x7fffffffffffffffll;
+  return b > 0x7ff0000000000000ll ? -1 : b;
+}
+__device__ __forceinline__ int mag(float a) {
+  const int b = __float_as_int(a) & 0x7fffffff;
+  return b > 0x7f800000 ? -1 : b;
+}
+template <class T>
+struct Mag {
+  typedef long long type;
+};
+template <>
+struct Mag<float> {
+  typedef int type;
+};
+// one divisor for a column's rows
+struct ByDouble {
+  double d;
+  exact64::Root r;
+  uint64_t Z;
+  bool fast;
+  __device__ explicit ByDouble(double x) : d(x), fast(exact64::divisor_in_range(x)) {
+    if (fast) r = exact64::divisor_of(x), Z = exact64::reciprocal(r);
+  }
+  __device__ double operator()(double a) const {
+    return fast && exact64::div_in_range(a) ? exact64::with_sign(exact64::divide(a, r, Z), d) : a / d;
+  }
+};
+struct ByFloat {
+  float d;
+  __device__ explicit ByFloat(float x) : d(x) {}
+  __device__ float operator()(float a) const { return a / d; }
+};
+__device__ __forceinline__ ByDouble by(double d) { return ByDouble(d); }
+__device__ __forceinline__ ByFloat by(float d) { return ByFloat(d); }
 
 template <class T>
 __global__ void k_lu_copy(const double* __restrict__ A, T* __restrict__ LU, size_t n2) {
@@ -51,31 +88,32 @@ __global__ void __launch_bounds__(kPanelThreads) k_lu_panel(T* __restrict__ A, i
                                                            Perm* __restrict__ perm) {
   extern __shared__ __align__(16) unsigned char smem[];
   T* p = reinterpret_cast<T*>(smem);  // [column][row - k0]
-  __shared__ T wv[kPanelThreads / 32];
+  typedef typename Mag<T>::type MagT;
+  __shared__ MagT wv[kPanelThreads / 32];
   __shared__ int wi[kPanelThreads / 32];
   __shared__ int pivots[kPanel];
   const int m = n - k0, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int c = 0; c < nb; ++c)
     for (int i = threadIdx.x; i < m; i += kPanelThreads) p[(size_t)c * m + i] = A[(size_t)(k0 + c) * n + k0 + i];
-  T bv = (T)-1;
+  MagT bv = -1;
   int bi = m;
   for (int i = threadIdx.x; i < m; i += kPanelThreads) {
-    const T v = mag(p[i]);
+    const MagT v = mag(p[i]);
     if (v > bv) bv = v, bi = i;  // a thread's rows come in order: the first of equals stays
   }
   __syncthreads();
   for (int c = 0; c < nb; ++c) {
     for (int o = 16; o > 0; o >>= 1) {
-      const T v = __shfl_xor_sync(0xffffffffu, bv, o);
+      const MagT v = __shfl_xor_sync(0xffffffffu, bv, o);
       const int i = __shfl_xor_sync(0xffffffffu, bi, o);
       if (v > bv || (v == bv && i < bi)) bv = v, bi = i;
     }
     if (lane == 0) wv[warp] = bv, wi[warp] = bi;
     __syncthreads();
-    bv = lane < kPanelThreads / 32 ? wv[lane] : (T)-1;
+    bv = lane < kPanelThreads / 32 ? wv[lane] : (MagT)-1;
     bi = lane < kPanelThreads / 32 ? wi[lane] : m;
     for (int o = 16; o > 0; o >>= 1) {
-      const T v = __shfl_xor_sync(0xffffffffu, bv, o);
+      const MagT v = __shfl_xor_sync(0xffffffffu, bv, o);
       const int i = __shfl_xor_sync(0xffffffffu, bi, o);
       if (v > bv || (v == bv && i < bi)) bv = v, bi = i;
     }
@@ -93,16 +131,20 @@ __global__ void __launch_bounds__(kPanelThreads) k_lu_panel(T* __restrict__ A, i
     __syncthreads();
     const T akk = p[(size_t)c * m + c];
     if (threadIdx.x == 0 && akk == (T)0 && err) atomicExch(err, 10);
-    bv = (T)-1;
+    const auto over = by(akk);
+    bv = -1;
     bi = m;
     for (int i = threadIdx.x; i < m; i += kPanelThreads) {
       if (i <= c) continue;
-      const T l = p[(size_t)c * m + i] / akk;
+      const T l = over(p[(size_t)c * m + i]);
       p[(size_t)c * m + i] = l;
       for (int j = c + 1; j < nb; ++j) {
         const T a = sub_mul(p[(size_t)j * m + i], l, p[(size_t)j * m + c]);
         p[(size_t)j * m + i] = a;
-        if (j == c + 1 && mag(a) > bv) bv = mag(a), bi = i;
+        if (j == c + 1) {
+          const MagT v = mag(a);
+          if (v > bv) bv = v, bi = i;
+        }
       }
     }
   }
@@ -296,7 +338,7 @@ __global__ void __launch_bounds__(kInvThreads) k_inverse64(const double* __restr
         if (i + 1 < n) s = s - u[i + 1] * X[(size_t)(i + 1) * cols + tid];
 #pragma unroll 8
         for (int k = i + 2; k < n; ++k) s = s - p[(size_t)k * cols];
-        X[(size_t)i * cols + tid] = s / u[i];
+        X[(size_t)i * cols + tid] = exact64::quotient(s, u[i]);
       }
     } else {
       // row i - 1's products with what is known: X[i + 1], X[i + 2], ...; row i - 3 of U

@@ -554,10 +554,12 @@ __global__ void k_aic(Dims d, DevState s, const double* fr) {
 // Solve AIC gamVec = -RHS by refinement; records the final relative residual
 // max|b - A x| / max|b| in s.luRes[0] and flags err[1] when it stays above 1e-9.
 // One cluster of kSolveBlocks blocks, a warp per row of the two products (lanes
-// over the columns, then a butterfly), x and r in global memory between them: on
-// one SM the FP64 product alone was n^2 / 2 cycles a pass (290 us at n = 300).
+// over the columns, then a butterfly); x and r go through global memory between
+// them and into every block's shared memory.  On one SM, with the vectors read
+// element by element, it took 290 us at n = 300.
 constexpr int kRefinePasses = 3;
 constexpr int kSolveBlocks = 8;
+inline size_t solve_smem(int n) { return sizeof(double) * n; }
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -568,6 +570,7 @@ __global__ void __cluster_dims__(kSolveBlocks, 1, 1) __launch_bounds__(1024) k_s
   const double* rhs = s.RHS;
   volatile double* x = s.refX;
   volatile double* r = s.refR;
+  extern __shared__ double vec[];  // the vector of the product at hand
   __shared__ double red[32];
   // b = -RHS (under axisymmetry blade 1's for every blade), and its largest magnitude, in every block
   auto b = [&](int i) { return -1.0 * rhs[d.axisym ? i % d.npan : i]; };
@@ -581,23 +584,33 @@ __global__ void __cluster_dims__(kSolveBlocks, 1, 1) __launch_bounds__(1024) k_s
     return v;
   };
   double bmax = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) bmax = fmax(bmax, fabs(b(i)));
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const double v = b(i);
+    vec[i] = v;
+    bmax = fmax(bmax, fabs(v));
+  }
   bmax = block_max(bmax);
   for (int pass = 0; pass < kRefinePasses; ++pass) {
+    if (pass) {
+      for (int i = threadIdx.x; i < n; i += blockDim.x) vec[i] = r[i];
+      __syncthreads();
+    }
     // x += inv32 r  (FP32 products of the FP32-rounded residual, FP64 update); r = b at first
     for (int i = row0; i < n; i += rows) {
       float z = 0.f;
-#pragma unroll 4
-      for (int j = lane; j < n; j += 32) z = fmaf(s.AICinv32[i + (size_t)n * j], (float)(pass ? r[j] : b(j)), z);
+#pragma unroll 8
+      for (int j = lane; j < n; j += 32) z = fmaf(s.AICinv32[i + (size_t)n * j], (float)vec[j], z);
       for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
       if (lane == 0) x[i] = (pass ? x[i] : 0.0) + (double)z;
     }
     cluster_sync();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) vec[i] = x[i];
+    __syncthreads();
     // r = b - A x in FP64
     for (int i = row0; i < n; i += rows) {
       double ax = 0.0;
-#pragma unroll 4
-      for (int j = lane; j < n; j += 32) ax = fma(s.AIC[i + (size_t)n * j], x[j], ax);
+#pragma unroll 8
+      for (int j = lane; j < n; j += 32) ax = fma(s.AIC[i + (size_t)n * j], vec[j], ax);
       for (int o = 16; o > 0; o >>= 1) ax += __shfl_xor_sync(0xffffffffu, ax, o);
       if (lane == 0) r[i] = b(i) - ax;
     }
@@ -662,16 +675,23 @@ struct ChunkAcc1 {
   int C, cnt;
   double tot, part;
   __device__ ChunkAcc1(int c) : C(c), cnt(0), tot(0.0), part(0.0) {}
-  __device__ void add(double x) {
-    if (C <= 0) {
-      tot = tot + x;
-      return;
-    }
-    part = part + x;
-    if (++cnt == C) {
-      tot = tot + part;
-      part = 0.0;
-      cnt = 0;
+  // n values, 3 doubles apart
+  __device__ void add(const exact64::Unit& u, const double* x, int n) {
+    for (int i = 0; i < n;) {
+      const int e = C > 0 ? min(n, i + C - cnt) : n;
+      double p = C > 0 ? part : tot;
+      cnt += e - i;
+#pragma unroll 8
+      for (; i < e; ++i) p = exact64::add(u, p, x[3 * i]);
+      if (C <= 0) {
+        tot = p;
+      } else if (cnt == C) {
+        tot = tot + p;
+        part = 0.0;
+        cnt = 0;
+      } else {
+        part = p;
+      }
     }
   }
   __device__ double result() const { return (C > 0 && cnt > 0) ? tot + part : tot; }
@@ -714,20 +734,21 @@ __device__ void ring_sums(const Dims& d, const DevState& s, const double* fr, d3
         const d3 f3 = exact64::vf_vind(u, c3, c0, rv[3]);
         if (WING) {
           const d3 f0 = exact64::vf_vind(u, c0, c1, rv[0]), f2 = exact64::vf_vind(u, c2, c3, rv[2]);
-          st3(ring + 3 * threadIdx.x, (((f0 + f1) + f2) + f3) * g);
+          st3(ring + 3 * threadIdx.x,
+              exact64::mul(u, exact64::add(u, exact64::add(u, exact64::add(u, f0, f1), f2), f3), g));
         }
-        st3(pair + 3 * threadIdx.x, (f1 + f3) * g);
-        if (p % d.nc == d.nc - 1) st3(te + 3 * (p / d.nc), f1 * g);
+        st3(pair + 3 * threadIdx.x, exact64::mul(u, exact64::add(u, f1, f3), g));
+        if (p % d.nc == d.nc - 1) st3(te + 3 * (p / d.nc), exact64::mul(u, f1, g));
       }
       __syncthreads();
       if (lane < 3) {
-        if (WING && warp == 0)
-          for (int i = 0; i < n; ++i) acc.add(ring[3 * i + lane]);
+        if (WING && warp == 0) acc.add(u, ring + lane, n);
         if (warp == 1) {
-#pragma unroll 4
-          for (int i = 0; i < n; ++i) sb = sb + pair[3 * i + lane];
+#pragma unroll 8
+          for (int i = 0; i < n; ++i) sb = exact64::add(u, sb, pair[3 * i + lane]);
           if (p0 + n == d.npan)
-            for (int j = 0; j < d.ns; ++j) sb = sb - te[3 * j + lane];
+#pragma unroll 8
+            for (int j = 0; j < d.ns; ++j) sb = exact64::sub(u, sb, te[3 * j + lane]);
         }
       }
       __syncthreads();
@@ -902,26 +923,35 @@ __device__ void inv3_doolittle(const double* A, double* X) {
   }
 }
 
-// libMath.f90:577-605
-__device__ double lsq2_dev(double xq, const double* xd, const double* yd, int n) {
-  double s1 = 0, s2 = 0, s3 = 0, s4 = 0, r1 = 0, r2 = 0, r3 = 0;
-  for (int i = 0; i < n; ++i) {
-    const double x = xd[i];
-    s1 = s1 + x;
-    s2 = s2 + x * x;
-    s3 = s3 + (x * x) * x;
-    s4 = s4 + pow4(x);
-    r1 = r1 + yd[i];
-    r2 = r2 + yd[i] * x;
-    r3 = r3 + yd[i] * (x * x);
+// libMath.f90:577-605, for the three components of one section: the normal
+// matrix and its inverse are the stations' alone
+struct Lsq2 {
+  double s1 = 0, s2 = 0, Ai[9];
+  __device__ void stations(const double* xd, int n) {
+    double s3 = 0, s4 = 0;
+    for (int i = 0; i < n; ++i) {
+      const double x = xd[i];
+      s1 = s1 + x;
+      s2 = s2 + x * x;
+      s3 = s3 + (x * x) * x;
+      s4 = s4 + pow4(x);
+    }
+    const double A[9] = {(double)n, s1, s2, s1, s2, s3, s2, s3, s4};
+    inv3_doolittle(A, Ai);
   }
-  const double A[9] = {(double)n, s1, s2, s1, s2, s3, s2, s3, s4};
-  double Ai[9];
-  inv3_doolittle(A, Ai);
-  double c[3];
-  for (int i = 0; i < 3; ++i) c[i] = Ai[i] * r1 + Ai[i + 3] * r2 + Ai[i + 6] * r3;
-  return c[0] + c[1] * xq + (c[2] * xq) * xq;
-}
+  __device__ double at(double xq, const double* xd, const double* yd, int ystride, int n) const {
+    double r1 = 0, r2 = 0, r3 = 0;
+    for (int i = 0; i < n; ++i) {
+      const double x = xd[i], y = yd[i * ystride];
+      r1 = r1 + y;
+      r2 = r2 + y * x;
+      r3 = r3 + y * (x * x);
+    }
+    double c[3];
+    for (int i = 0; i < 3; ++i) c[i] = Ai[i] * r1 + Ai[i + 3] * r2 + Ai[i + 6] * r3;
+    return c[0] + c[1] * xq + (c[2] * xq) * xq;
+  }
+};
 
 constexpr int kMaxNc = 64;
 
@@ -978,46 +1008,52 @@ __device__ double c81_get(const double* T, int c, double alpha, double mach) {
   return num / (A[a2 - 1] - A[a1 - 1]) / (Ma[m2 - 1] - Ma[m1 - 1]);
 }
 
-__global__ void k_loads(Dims d, DevState s, const double* fr, int iter) {
+// One block.  FP64 work is 64 cycles an instruction and its divisions and roots
+// hundreds, so each phase runs over the smallest independent items -- panels,
+// (section, component), sections, (blade, component) -- with the integer
+// divisions; only the ordered sums are serial.  (Over sections alone, with
+// CUDA's divisions, it took 90 us at 75 sections of 4 blades and 84 us at 13
+// sections of 4 panels.)  tmp: 9 doubles a panel.
+constexpr int kLoadsThreads = 512;
+__global__ void __launch_bounds__(kLoadsThreads) k_loads(Dims d, DevState s, const double* fr, int iter) {
   if (iter < 0) iter = s.devIter[0];
-  const int nsec = d.nbC * d.ns;
+  const int nsec = d.nbC * d.ns, npan = d.nbC * d.npan;
   const double iGS = -1.0 * fsign1(d.omega);
+  double* tmp = s.loadTmp;
   // phase A: sectional resultant velocity and lift/drag directions
-  for (int t = threadIdx.x; t < nsec; t += blockDim.x) {
-    const int b = t / d.ns, is = t % d.ns;
-    const double* sec = fr + d.fl.sec + ((size_t)b * d.ns + is) * kSec;
-    const d3 secTauC = ld3(sec), secCP = ld3(sec + 6), pc1 = ld3(sec + 9);
-    d3 rv;
+  for (int gp = threadIdx.x; gp < npan; gp += blockDim.x) {
+    const int b = gp / d.npan, p = gp % d.npan;
+    const double* w = panRec(d, fr, b, p);
+    st3(tmp + 9 * (size_t)gp, exact64::noproj(ld3(s.velCPTotal + 3 * (size_t)gp), ld3(w + 21)));
+    const double* sec = fr + d.fl.sec + ((size_t)b * d.ns + p / d.nc) * kSec;
+    tmp[9 * (size_t)gp + 3] = dot3(ld3(w + 12) - ld3(sec + 9), ld3(sec));
+  }
+  __syncthreads();
+  for (int t3 = threadIdx.x; t3 < 3 * nsec; t3 += blockDim.x) {
+    const int t = t3 / 3, c = t3 % 3, b = t / d.ns, is = t % d.ns;
+    const double* q = tmp + 9 * ((size_t)b * d.npan + (size_t)d.nc * is);
+    double v;
     if (d.nc >= 3) {
-      double xd[kMaxNc], yd[kMaxNc];
-      d3 crv[kMaxNc];
-      for (int ic = 0; ic < d.nc; ++ic) {
-        const int p = ic + d.nc * is;
-        const double* w = panRec(d, fr, b, p);
-        crv[ic] = noproj3(ld3(s.velCPTotal + 3 * ((size_t)b * d.npan + p)), ld3(w + 21));
-        xd[ic] = dot3(ld3(w + 12) - pc1, secTauC);
-      }
-      const double xq = dot3(secCP - pc1, secTauC);
-      double o[3];
-      for (int k = 0; k < 3; ++k) {
-        for (int ic = 0; ic < d.nc; ++ic) yd[ic] = k == 0 ? crv[ic].x : (k == 1 ? crv[ic].y : crv[ic].z);
-        o[k] = lsq2_dev(xq, xd, yd, d.nc);
-      }
-      rv = mk3(o[0], o[1], o[2]);
+      const double* sec = fr + d.fl.sec + ((size_t)b * d.ns + is) * kSec;
+      double xd[kMaxNc];
+      for (int ic = 0; ic < d.nc; ++ic) xd[ic] = q[9 * ic + 3];
+      const double xq = dot3(ld3(sec + 6) - ld3(sec + 9), ld3(sec));
+      Lsq2 fit;
+      fit.stations(xd, d.nc);
+      v = fit.at(xq, xd, q + c, 9, d.nc);
     } else {
-      d3 sum = zero3();
-      for (int ic = 0; ic < d.nc; ++ic) {
-        const int p = ic + d.nc * is;
-        const double* w = panRec(d, fr, b, p);
-        sum = sum + noproj3(ld3(s.velCPTotal + 3 * ((size_t)b * d.npan + p)), ld3(w + 21));
-      }
-      rv = sum / (double)d.nc;
+      double sum = 0.0;
+      for (int ic = 0; ic < d.nc; ++ic) sum = sum + q[9 * ic + c];
+      v = sum / (double)d.nc;
     }
-    st3(s.secResVel + 3 * (size_t)t, rv);
-    const d3 dd = unit3(rv);
-    const d3 yAF = ld3(fr + d.fl.ax + 9 * b + 3);
+    s.secResVel[t3] = v;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < nsec; t += blockDim.x) {
+    const d3 dd = exact64::unit(ld3(s.secResVel + 3 * (size_t)t));
+    const d3 yAF = ld3(fr + d.fl.ax + 9 * (t / d.ns) + 3);
     st3(s.secDragDir + 3 * (size_t)t, dd);
-    st3(s.secLiftDir + 3 * (size_t)t, fsign1(d.omega) * unit3(cross3(dd, yAF)));
+    st3(s.secLiftDir + 3 * (size_t)t, fsign1(d.omega) * exact64::unit(cross3(dd, yAF)));
   }
   __syncthreads();
   // phase B with airfoil tables (forceCalcSwitch 1: blade_calc_force_alpha,
@@ -1055,15 +1091,12 @@ __global__ void k_loads(Dims d, DevState s, const double* fr, int iter) {
     s.secCLu[t] = 0.0;
   }
   // phase B: panel pressures and sectional forces (blade_calc_force)
-  for (int t = threadIdx.x; d.forceCalc != 1 && t < nsec; t += blockDim.x) {
-    const int b = t / d.ns, is = t % d.ns;
-    const d3 liftDir = ld3(s.secLiftDir + 3 * (size_t)t);
-    d3 sFI = zero3(), sL = zero3(), sLU = zero3();
-    for (int ic = 0; ic < d.nc; ++ic) {
-      const int p = ic + d.nc * is;
-      const size_t gp = (size_t)b * d.npan + p;
+  if (d.forceCalc != 1) {
+    for (int gp = threadIdx.x; gp < npan; gp += blockDim.x) {
+      const int b = gp / d.npan, p = gp % d.npan, is = p / d.nc, ic = p % d.nc;
+      const d3 liftDir = ld3(s.secLiftDir + 3 * ((size_t)b * d.ns + is));
       const double* w = panRec(d, fr, b, p);
-      const d3 velCP = ld3(s.velCP + 3 * gp);
+      const d3 velCP = ld3(s.velCP + 3 * (size_t)gp);
       const double vTC = dot3(velCP, ld3(w + 18));
       const double vTS = dot3(velCP, ld3(w + 21));
       const double g = s.wGam[gp];
@@ -1072,81 +1105,79 @@ __global__ void k_loads(Dims d, DevState s, const double* fr, int iter) {
       gEC = iGS * gEC;
       gES = iGS * gES;
       const double gamTrapz = ic > 0 ? (iGS * 0.5) * (g + s.wGam[gp - 1]) : (iGS * 0.5) * g;
-      const double delPU = d.density * (gamTrapz - s.gamPrev[gp]) / d.dt;
-      double delP = delPU + d.density * vTC * gEC / s.panMeanChord[gp];
-      if (d.spanwiseLift != 0) delP = delP + d.density * vTS * gES / s.panMeanSpan[gp];
+      const double delPU = exact64::quotient(d.density * (gamTrapz - s.gamPrev[gp]), d.dt);
+      double delP = delPU + exact64::quotient(d.density * vTC * gEC, s.panMeanChord[gp]);
+      if (d.spanwiseLift != 0) delP = delP + exact64::quotient(d.density * vTS * gES, s.panMeanSpan[gp]);
       s.gamPrev[gp] = gamTrapz;
       const d3 nCap = ld3(w + 15);
       const d3 nF = (delP * s.panArea[gp]) * nCap;
       const d3 nFU = (delPU * s.panArea[gp]) * nCap;
-      sFI = sFI + nF;
-      sL = sL + proj3(nF, liftDir);
-      sLU = sLU + proj3(nFU, liftDir);
+      st3(tmp + 9 * (size_t)gp, nF);
+      st3(tmp + 9 * (size_t)gp + 3, exact64::proj(nF, liftDir));
+      st3(tmp + 9 * (size_t)gp + 6, exact64::proj(nFU, liftDir));
     }
-    const d3 xAF = ld3(fr + d.fl.ax + 9 * b), zAF = ld3(fr + d.fl.ax + 9 * b + 6);
-    st3(s.secForceInertial + 3 * (size_t)t, sFI);
-    st3(s.secLift + 3 * (size_t)t, sL);
-    st3(s.secLiftUnsteady + 3 * (size_t)t, sLU);
-    st3(s.secLiftInPlane + 3 * (size_t)t, iGS * proj3(sL, xAF));
-    st3(s.secLiftOutPlane + 3 * (size_t)t, proj3(sL, zAF));
-    const double m = norm3(ld3(s.secResVel + 3 * (size_t)t));
-    const double q = (0.5 * d.density) * (m * m);
-    const double area = s.secArea[(size_t)b * d.ns + is];
-    if (fabs(q) > kEps) {
-      const double sg = fsign1(dot3(sL, zAF));
-      s.secCL[t] = norm3(sL) * sg / (q * area);
-      s.secCD[t] = 0.0 / (q * area);
-      s.secCLu[t] = norm3(sLU) * sg / (q * area);
-    } else {
-      s.secCL[t] = s.secCD[t] = s.secCLu[t] = 0.0;
+    __syncthreads();
+    for (int t9 = threadIdx.x; t9 < 9 * nsec; t9 += blockDim.x) {
+      const int t = t9 / 9, c = t9 % 9;
+      const double* q = tmp + 9 * ((size_t)(t / d.ns) * d.npan + (size_t)d.nc * (t % d.ns)) + c;
+      double sum = 0.0;
+      for (int ic = 0; ic < d.nc; ++ic) sum = sum + q[9 * ic];
+      double* o = c < 3 ? s.secForceInertial : c < 6 ? s.secLift : s.secLiftUnsteady;
+      o[3 * (size_t)t + c % 3] = sum;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < nsec; t += blockDim.x) {
+      const int b = t / d.ns;
+      const d3 xAF = ld3(fr + d.fl.ax + 9 * b), zAF = ld3(fr + d.fl.ax + 9 * b + 6);
+      const d3 sL = ld3(s.secLift + 3 * (size_t)t), sLU = ld3(s.secLiftUnsteady + 3 * (size_t)t);
+      st3(s.secLiftInPlane + 3 * (size_t)t, iGS * exact64::proj(sL, xAF));
+      st3(s.secLiftOutPlane + 3 * (size_t)t, exact64::proj(sL, zAF));
+      const double m = exact64::norm(ld3(s.secResVel + 3 * (size_t)t));
+      const double q = (0.5 * d.density) * (m * m);
+      const double area = s.secArea[t];
+      if (fabs(q) > kEps) {
+        const double sg = fsign1(dot3(sL, zAF));
+        s.secCL[t] = exact64::quotient(exact64::norm(sL) * sg, q * area);
+        s.secCD[t] = 0.0 / (q * area);
+        s.secCLu[t] = exact64::quotient(exact64::norm(sLU) * sg, q * area);
+      } else {
+        s.secCL[t] = s.secCD[t] = s.secCLu[t] = 0.0;
+      }
     }
   }
   __syncthreads();
-  // phase C: blade sums (blade_sumSecToNetForces)
-  for (int b = threadIdx.x; b < d.nbC; b += blockDim.x) {
-    d3 fi = zero3(), li = zero3(), lu = zero3();
-    for (int is = 0; is < d.ns; ++is) {
-      const size_t t = (size_t)b * d.ns + is;
-      fi = fi + ld3(s.secForceInertial + 3 * t);
-      li = li + ld3(s.secLift + 3 * t);
-      lu = lu + ld3(s.secLiftUnsteady + 3 * t);
-    }
-    st3(s.bladeForce + 12 * (size_t)b, fi);
-    st3(s.bladeForce + 12 * (size_t)b + 3, li);
-    st3(s.bladeForce + 12 * (size_t)b + 6, zero3());
-    st3(s.bladeForce + 12 * (size_t)b + 9, lu);
+  // phase C: blade sums (blade_sumSecToNetForces), one component a thread
+  for (int t9 = threadIdx.x; t9 < 9 * d.nbC; t9 += blockDim.x) {
+    const int b = t9 / 9, c = t9 % 9;
+    const double* q = (c < 3 ? s.secForceInertial : c < 6 ? s.secLift : s.secLiftUnsteady) + 3 * (size_t)b * d.ns + c % 3;
+    double sum = 0.0;
+#pragma unroll 8
+    for (int is = 0; is < d.ns; ++is) sum = sum + q[3 * is];
+    s.bladeForce[12 * (size_t)b + (c < 6 ? c : c + 3)] = sum;
+    if (c < 3) s.bladeForce[12 * (size_t)b + 6 + c] = 0.0;
   }
   __syncthreads();
   // phase D: rotor sums and the CT row (rotor_sumBladeToNetForces, force2file)
-  if (threadIdx.x == 0) {
-    d3 FI = zero3(), L = zero3(), LU = zero3();
+  __shared__ double net[9];  // inertial, lift, unsteady lift
+  if (threadIdx.x < 9) {
+    const int c = threadIdx.x, o = c < 6 ? c : c + 3;
+    double sum = 0.0;
     if (d.axisym) {
-      const double nbd = (double)d.nb;
-      FI = nbd * ld3(s.bladeForce);
-      L = nbd * ld3(s.bladeForce + 3);
-      LU = nbd * ld3(s.bladeForce + 9);
+      sum = (double)d.nb * s.bladeForce[o];
     } else {
-      for (int b = 0; b < d.nbC; ++b) {
-        FI = FI + ld3(s.bladeForce + 12 * (size_t)b);
-        L = L + ld3(s.bladeForce + 12 * (size_t)b + 3);
-        LU = LU + ld3(s.bladeForce + 12 * (size_t)b + 9);
-      }
+      for (int b = 0; b < d.nbC; ++b) sum = sum + s.bladeForce[12 * (size_t)b + o];
     }
-    st3(s.rotorLift, L);
-    st3(s.rotorLift + 3, FI);
+    net[c] = sum;
+    if (c < 6) s.rotorLift[c < 3 ? c + 3 : c - 3] = sum;
+  }
+  __syncthreads();
+  if (threadIdx.x < 10) {
     const double D = d.nonDimDenom;
-    const double sl = fsign1(dot3(L, ld3(fr + d.fl.rot)));
-    double* row = s.ctHist + 10 * (size_t)iter;
-    row[0] = (double)iter;
-    row[1] = sl * norm3(L) / D;
-    row[2] = 0.0 / D;
-    row[3] = norm3(LU) / D;
-    row[4] = 0.0 / D;
-    row[5] = 0.0 / D;
-    row[6] = 0.0 / D;
-    row[7] = FI.x / D;
-    row[8] = FI.y / D;
-    row[9] = FI.z / D;
+    double v = 0.0;
+    if (threadIdx.x == 1) v = fsign1(dot3(ld3(net + 3), ld3(fr + d.fl.rot))) * exact64::norm(ld3(net + 3));
+    if (threadIdx.x == 3) v = exact64::norm(ld3(net + 6));
+    if (threadIdx.x >= 7) v = net[threadIdx.x - 7];
+    s.ctHist[10 * (size_t)iter + threadIdx.x] = threadIdx.x == 0 ? (double)iter : v / D;
   }
 }
 
@@ -1280,11 +1311,17 @@ void launch_aic(const Dims& d, const DevState& s, const double* frame, cudaStrea
   count_launch();
   k_aic<<<nblk(n, 128), 128, 0, st>>>(d, s, frame);
 }
+static void solve_refine(const Dims& d, const DevState& s, cudaStream_t st) {
+  const size_t smem = solve_smem(d.n);
+  if (smem > 40 * 1024)
+    cudaFuncSetAttribute(k_solve_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_smem(8192));
+  k_solve_refine<<<kSolveBlocks, 1024, smem, st>>>(d, s);
+}
 void launch_solve(const Dims& d, const DevState& s, const double* frame, bool withWake, cudaStream_t st) {
   count_launch();
   k_rhs<<<nblk(d.nbC * d.npan, 128), 128, 0, st>>>(d, s, frame, withWake ? 1 : 0);
   count_launch();
-  if (s.LU32) k_solve_refine<<<kSolveBlocks, 1024, 0, st>>>(d, s);
+  if (s.LU32) solve_refine(d, s, st);
   else k_solve<<<1, 1024, 0, st>>>(d, s);
 }
 void launch_step_begin(const Dims& d, const DevState& s, cudaStream_t st) {
@@ -1314,7 +1351,7 @@ void launch_mirror_wake(const Dims& d, const DevState& dst, const DevState& src,
 }
 void launch_solve_only(const Dims& d, const DevState& s, cudaStream_t st) {
   count_launch();
-  if (s.LU32) k_solve_refine<<<kSolveBlocks, 1024, 0, st>>>(d, s);
+  if (s.LU32) solve_refine(d, s, st);
   else k_solve<<<1, 1024, 0, st>>>(d, s);
 }
 // shared memory for up to 8192 stations (the most panels a rotor has)
@@ -1340,7 +1377,7 @@ void launch_loads(const Dims& d, const DevState& s, const double* frame, int sum
   velcp_attr();
   k_velcp_total<<<d.nbC * d.npan, kVcThreads, velcp_smem(d.ns), st>>>(d, s, frame, sumChunk, foreignBound, nrs, self);
   count_launch();
-  k_loads<<<1, 256, 0, st>>>(d, s, frame, iter);
+  k_loads<<<1, kLoadsThreads, 0, st>>>(d, s, frame, iter);
 }
 
 }  // namespace vlm

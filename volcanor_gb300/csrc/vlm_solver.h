@@ -100,6 +100,7 @@ struct DevState {
   double *bladeForce;  // [nb][4][3]: forceInertial, lift, drag(0), liftUnsteady
   double* rotorLift;   // [6] lift (liftPrev of the next step), forceInertial
   double* ctHist;      // [(nt+1) * 10]
+  double* loadTmp;     // [panel][9], the loads' own
   // N-body scratch
   double *rec64, *targets, *part, *outv;
   float* rec32;
