@@ -39,14 +39,61 @@ struct StatusError : std::runtime_error {
     if (e_ != cudaSuccess) throw CudaError(std::string(#x) + ": " + cudaGetErrorString(e_));       \
   } while (0)
 
+// The zeroed device arrays that live and die together.  A case has about 70,
+// most of them a few KB, and a cudaMalloc and a memset each were more of a
+// short run's time than its arithmetic: the small ones share blocks of kBlock
+// bytes (256-byte aligned, one memset a block), an array above a quarter block
+// gets its own allocation.  The 40-step run of a 52-panel wing, creating and
+// freeing its case included: 13.5 -> 12.8 ms.  Each new block is zero before
+// take() returns: the memset runs on the legacy stream, which the cases'
+// non-blocking streams do not wait for.
+class DevArena {
+ public:
+  static constexpr size_t kBlock = 2u << 20, kAlign = 256;
+  DevArena() = default;
+  DevArena(const DevArena&) = delete;
+  DevArena& operator=(const DevArena&) = delete;
+  ~DevArena() { release(); }
+  void* take(size_t bytes) {
+    if (bytes > SIZE_MAX - kAlign) throw CudaError("device allocation too large");
+    bytes = (std::max<size_t>(bytes, 1) + kAlign - 1) & ~(kAlign - 1);
+    if (bytes > kBlock / 4) return block(bytes);
+    if (bytes > left_) {
+      cur_ = static_cast<char*>(block(kBlock));
+      left_ = kBlock;
+    }
+    void* p = cur_;
+    cur_ += bytes;
+    left_ -= bytes;
+    return p;
+  }
+  // the caller has finished every stream that used the arrays
+  void release() {
+    for (void* p : blocks_) cudaFree(p);
+    blocks_.clear();
+    cur_ = nullptr;
+    left_ = 0;
+  }
+
+ private:
+  void* block(size_t bytes) {
+    void* p = nullptr;
+    blocks_.reserve(blocks_.size() + 1);
+    VLM_CUDA(cudaMalloc(&p, bytes));
+    blocks_.push_back(p);
+    VLM_CUDA(cudaMemset(p, 0, bytes));
+    VLM_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+    return p;
+  }
+  std::vector<void*> blocks_;
+  char* cur_ = nullptr;
+  size_t left_ = 0;
+};
+
 template <class T>
-static T* dalloc(size_t n, std::vector<void*>& owned) {
-  void* p = nullptr;
-  if (n == 0) n = 1;
-  VLM_CUDA(cudaMalloc(&p, n * sizeof(T)));
-  VLM_CUDA(cudaMemset(p, 0, n * sizeof(T)));
-  owned.push_back(p);
-  return static_cast<T*>(p);
+static T* dalloc(size_t n, DevArena& owned) {
+  if (n > SIZE_MAX / sizeof(T)) throw CudaError("device allocation too large");
+  return static_cast<T*>(owned.take(n * sizeof(T)));
 }
 
 // Source/target layout of one Biot-Savart evaluation at one step.
@@ -68,7 +115,7 @@ struct Case {
   vlm_options opt{};
   Dims d{};
   DevState s{};
-  std::vector<void*> owned;
+  DevArena owned;
   cudaStream_t stream = nullptr;
   bool ownStream = true;  // false for the rotors of a system after the first (one stream for all)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -101,12 +148,12 @@ struct Case {
 
   ~Case() {
     if (stream) cudaStreamSynchronize(stream);
-    for (void* p : owned) cudaFree(p);
-    for (void* p : scratchOwned) cudaFree(p);
-    for (void* p : surrOwned) cudaFree(p);
+    owned.release();
+    scratchOwned.release();
+    surrOwned.release();
     if (incrStream) cudaStreamSynchronize(incrStream);
     if (incrOv.stream) cudaStreamSynchronize(incrOv.stream);
-    for (void* p : incrOwned) cudaFree(p);
+    incrOwned.release();
     if (incrFork) cudaEventDestroy(incrFork);
     if (incrJoin) cudaEventDestroy(incrJoin);
     if (incrOv.fork) cudaEventDestroy(incrOv.fork);
@@ -115,7 +162,6 @@ struct Case {
     if (incrStream) cudaStreamDestroy(incrStream);
     surr.net.destroy();
     if (gexec) cudaGraphExecDestroy(gexec);
-    if (hIter) cudaFreeHost(hIter);
     if (hFrames) cudaFreeHost(hFrames);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
@@ -308,7 +354,8 @@ struct Case {
     // device memory
     const int nb = d.nb, npan = d.npan, NW = d.NW, NF = d.NF, ns = d.ns;
     s.frames = dalloc<double>(frames.size(), owned);
-    VLM_CUDA(cudaMallocHost(&hFrames, frames.size() * sizeof(double)));
+    VLM_CUDA(cudaMallocHost(&hFrames, (frames.size() + 1) * sizeof(double)));  // + the step counter
+    hIter = reinterpret_cast<int*>(hFrames + frames.size());
     std::memcpy(hFrames, frames.data(), frames.size() * sizeof(double));
     VLM_CUDA(cudaMemcpy(s.frames, hFrames, (size_t)d.fl.size * sizeof(double), cudaMemcpyHostToDevice));
     std::vector<double> rvc((size_t)nb * npan * 4), area((size_t)nb * npan), mc((size_t)nb * npan),
@@ -400,7 +447,6 @@ struct Case {
     s.err = dalloc<int>(4, owned);
     s.devIter = dalloc<int>(1, owned);
     s.curFrame = dalloc<double>(d.fl.size, owned);
-    VLM_CUDA(cudaMallocHost(&hIter, sizeof(int)));
     if (refine) {
       s.LU32 = dalloc<float>((size_t)d.n * d.n, owned);
       s.AICinv32 = dalloc<float>((size_t)d.n * d.n, owned);
@@ -430,10 +476,9 @@ struct Case {
   }
 
   // N-body scratch and plan tables (again after the surrogate adds plans)
-  std::vector<void*> scratchOwned;
+  DevArena scratchOwned;
   void allocScratch() {
-    for (void* p : scratchOwned) cudaFree(p);
-    scratchOwned.clear();
+    scratchOwned.release();
     s.rec64 = dalloc<double>((size_t)maxRecords * kRec64, scratchOwned);
     s.rec32 = opt.precision != VLM_PREC_FP64 ? dalloc<float>((size_t)maxRecords * kRec32, scratchOwned) : nullptr;
     s.edgeW = lattice() ? dalloc<double>((size_t)maxRecords * 4, scratchOwned) : nullptr;
@@ -695,7 +740,7 @@ struct Case {
     constexpr int kReps = 5;
     constexpr int64_t kMaxTunePart = (int64_t)1 << 22;  // (chunks x targets) of a candidate
     constexpr double kMargin = 0.97;                    // a plan must beat the model's by 3 %
-    std::vector<void*> tmp;
+    DevArena tmp;
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     VLM_CUDA(cudaEventCreate(&t0));
     VLM_CUDA(cudaEventCreate(&t1));
@@ -802,7 +847,7 @@ struct Case {
       changed = true;
     }
     VLM_CUDA(cudaStreamSynchronize(stream));
-    for (void* q : tmp) cudaFree(q);
+    tmp.release();
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
     // the timing launches wrote no state; the device error word of the
@@ -849,7 +894,7 @@ struct Case {
   };
   static constexpr int kMaxIncrPlans = 8;
   std::vector<IncrPlan> incr;
-  std::vector<void*> incrOwned;
+  DevArena incrOwned;
   double *recP = nullptr, *ewP = nullptr, *tgtP = nullptr;  // the predicted records, edge weights, targets
   int* incrCnt = nullptr;                                   // [0] changed records, [1] moved targets
   int* incrBlk = nullptr;                                   // per-tile offsets: records, then targets
@@ -1241,7 +1286,7 @@ struct Case {
   };
   Surrogate surr;
   std::vector<SurrPlans> splans;
-  std::vector<void*> surrOwned;
+  DevArena surrOwned;
 
   // lattice form of the near-wake rings for the FP32 precisions
   bool lattice() const { return opt.precision != VLM_PREC_FP64 && opt.lattice != 0; }
@@ -2213,7 +2258,7 @@ struct Case {
     std::vector<Chunk> ch(rec + g.size() + 1);
     const int nq = chunkTable(g.data(), (int)g.size(), (int)M, ch.data(), (int)ch.size());
     if (nq < 0) throw std::runtime_error("chunk table overflow");
-    std::vector<void*> tmpOwned;
+    DevArena tmpOwned;
     Group* dg = dalloc<Group>(g.size(), tmpOwned);
     Chunk* dc = dalloc<Chunk>(nq, tmpOwned);
     double* rec64 = dalloc<double>((size_t)rec * kRec64, tmpOwned);
@@ -2221,44 +2266,35 @@ struct Case {
     double* dP = dalloc<double>((size_t)M * 3, tmpOwned);
     double* dV = dalloc<double>((size_t)M * 3, tmpOwned);
     double* part = dalloc<double>((size_t)M * nq * 3, tmpOwned);
-    auto cleanup = [&]() {
-      for (void* p : tmpOwned) cudaFree(p);
-    };
-    try {
-      VLM_CUDA(cudaMemcpy(dg, g.data(), g.size() * sizeof(Group), cudaMemcpyHostToDevice));
-      VLM_CUDA(cudaMemcpy(dc, ch.data(), nq * sizeof(Chunk), cudaMemcpyHostToDevice));
-      VLM_CUDA(cudaMemcpy(dP, P, (size_t)M * 3 * sizeof(double), cudaMemcpyHostToDevice));
-      DevState t = s;
-      t.rec64 = rec64;
-      t.edgeW = nullptr;  // ring by ring: the probe's record count is not the plans'
-      t.rec32 = opt.precision == VLM_PREC_FP64 ? nullptr : rec32;
-      GatherTargets tg;
-      tg.zero[0] = s.err + 3;
-      launch_gather(d, t, frame(fi), dg, (int)g.size(), rec, rN, rF, false, nearFactor(), tg, stream);
-      long long* nacc = nullptr;
-      if (opt.precision == VLM_PREC_FP64) {
-        launch_partial64(rec64, dc, nq, rec, dP, (int)M, part, stream);
-      } else {
-        const bool nearOn = opt.precision == VLM_PREC_FP32_NEAR64;
-        const size_t nb = nearOn ? near_scratch_bytes((int)M, (size_t)std::min<int64_t>(64 * M + (1 << 16), 1 << 26)) : 1;
-        unsigned char* ns = dalloc<unsigned char>(nb, tmpOwned);
-        if (nearOn) nacc = dalloc<long long>((size_t)M * nq * 3, tmpOwned);
-        launch_partial32(rec32, rec64, dc, nq, rec, dP, (int)M, part, s.err + 2, nearOn ? ns : nullptr, nb, nacc,
-                         stream);
-      }
-      if (opt.precision == VLM_PREC_FP64) launch_combine(part, (int)M, dg, (int)g.size(), 2, dV, stream);
-      else {
-        int maxq = 0;
-        for (const Group& q : g) maxq = std::max(maxq, q.chunk_count);
-        launch_combine_unordered(part, nacc, (int)M, dg, (int)g.size(), maxq, 2, dV, stream);
-      }
-      VLM_CUDA(cudaMemcpyAsync(V, dV, (size_t)M * 3 * sizeof(double), cudaMemcpyDeviceToHost, stream));
-      VLM_CUDA(cudaStreamSynchronize(stream));
-    } catch (...) {
-      cleanup();
-      throw;
+    VLM_CUDA(cudaMemcpy(dg, g.data(), g.size() * sizeof(Group), cudaMemcpyHostToDevice));
+    VLM_CUDA(cudaMemcpy(dc, ch.data(), nq * sizeof(Chunk), cudaMemcpyHostToDevice));
+    VLM_CUDA(cudaMemcpy(dP, P, (size_t)M * 3 * sizeof(double), cudaMemcpyHostToDevice));
+    DevState t = s;
+    t.rec64 = rec64;
+    t.edgeW = nullptr;  // ring by ring: the probe's record count is not the plans'
+    t.rec32 = opt.precision == VLM_PREC_FP64 ? nullptr : rec32;
+    GatherTargets tg;
+    tg.zero[0] = s.err + 3;
+    launch_gather(d, t, frame(fi), dg, (int)g.size(), rec, rN, rF, false, nearFactor(), tg, stream);
+    long long* nacc = nullptr;
+    if (opt.precision == VLM_PREC_FP64) {
+      launch_partial64(rec64, dc, nq, rec, dP, (int)M, part, stream);
+    } else {
+      const bool nearOn = opt.precision == VLM_PREC_FP32_NEAR64;
+      const size_t nb = nearOn ? near_scratch_bytes((int)M, (size_t)std::min<int64_t>(64 * M + (1 << 16), 1 << 26)) : 1;
+      unsigned char* ns = dalloc<unsigned char>(nb, tmpOwned);
+      if (nearOn) nacc = dalloc<long long>((size_t)M * nq * 3, tmpOwned);
+      launch_partial32(rec32, rec64, dc, nq, rec, dP, (int)M, part, s.err + 2, nearOn ? ns : nullptr, nb, nacc,
+                       stream);
     }
-    cleanup();
+    if (opt.precision == VLM_PREC_FP64) launch_combine(part, (int)M, dg, (int)g.size(), 2, dV, stream);
+    else {
+      int maxq = 0;
+      for (const Group& q : g) maxq = std::max(maxq, q.chunk_count);
+      launch_combine_unordered(part, nacc, (int)M, dg, (int)g.size(), maxq, 2, dV, stream);
+    }
+    VLM_CUDA(cudaMemcpyAsync(V, dV, (size_t)M * 3 * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    VLM_CUDA(cudaStreamSynchronize(stream));
   }
 };
 
@@ -2274,7 +2310,11 @@ struct RingScratch {
   int* err = nullptr;
   unsigned char* near = nullptr;
   long long* nacc = nullptr;  // zero between calls
-  size_t cap64 = 0, cap32 = 0, capPart = 0, capChunks = 0, capNear = 0, capNacc = 0;
+  // a small host-buffer call's arrays and tables, packed, and their pinned
+  // image: one copy in, one copy out.  At most kIoMax bytes each.
+  unsigned char *io = nullptr, *hio = nullptr;
+  static constexpr size_t kIoMax = 4u << 20;
+  size_t cap64 = 0, cap32 = 0, capPart = 0, capChunks = 0, capNear = 0, capNacc = 0, capIo = 0;
 };
 static RingScratch g_ring[64];
 
@@ -2282,6 +2322,7 @@ static void grow(void** p, size_t& cap, size_t need) {
   if (need <= cap) return;
   if (*p) cudaFree(*p);
   *p = nullptr;
+  cap = 0;
   VLM_CUDA(cudaMalloc(p, need));
   cap = need;
 }
@@ -2341,64 +2382,162 @@ int64_t ring_sum_chunk(int64_t N, int64_t M, int precision) {
   return c;
 }
 
-// fil: the sources are single filaments (corners = N x [fc1, fc2], rvc and
-// gam one per filament) instead of rings.
-void rings_device(const double* corners, const double* rvc, const double* gam, int64_t N, const double* P, int64_t M,
-                  double* V, int precision, cudaStream_t st, bool fil = false) {
+static void ring_check(int64_t N, int64_t M, int precision) {
   if (precision < 0 || precision > 2) throw StatusError(VLM_ERR_INVALID, "precision must be 0, 1 or 2");
   if (N < 0 || M < 0 || N > (1LL << 30) || M > (1LL << 30)) throw StatusError(VLM_ERR_INVALID, "N and M must be in [0, 2^30]");
+}
+
+// an evaluation's chunk table and the scratch it needs
+struct RingPlan {
+  Group g;
+  std::vector<Chunk> ch;
+  int nq = 0, Q = 1;
+  size_t nearBytes = 1;
+};
+
+// R.mu held
+static RingPlan ring_reserve(RingScratch& R, int64_t N, int64_t M, int precision) {
+  RingPlan p;
+  p.nq = ring_plan(N, M, precision, p.g, p.ch);
+  p.Q = std::max(p.nq, 1);
+  grow((void**)&R.rec64, R.cap64, (size_t)std::max<int64_t>(N, 1) * kRec64 * 8);
+  if (precision != VLM_PREC_FP64) grow((void**)&R.rec32, R.cap32, (size_t)std::max<int64_t>(N, 1) * kRec32 * 4);
+  grow((void**)&R.part, R.capPart, (size_t)M * p.Q * 3 * 8);
+  p.nearBytes = precision == VLM_PREC_FP32_NEAR64 ? near_scratch_bytes((int)M, ring_near_cap(M)) : 1;
+  grow((void**)&R.near, R.capNear, p.nearBytes);
+  if (precision == VLM_PREC_FP32_NEAR64 && (size_t)M * p.Q * 3 * 8 > R.capNacc) {
+    grow((void**)&R.nacc, R.capNacc, (size_t)M * p.Q * 3 * 8);
+    VLM_CUDA(cudaMemset(R.nacc, 0, R.capNacc));
+  }
+  return p;
+}
+
+// fil: the sources are single filaments (corners = N x [fc1, fc2], rvc and
+// gam one per filament) instead of rings.  chunks, group (the plan's) and err
+// (zero) are on the device.  R.mu held.
+static void ring_launch(RingScratch& R, const RingPlan& p, const double* corners, const double* rvc, const double* gam,
+                        int64_t N, const double* P, int64_t M, double* V, int precision, const Chunk* chunks,
+                        const Group* group, int* err, cudaStream_t st, bool fil) {
+  if (N > 0) {
+    if (fil) launch_fils_to_rec64(corners, rvc, gam, N, R.rec64, st);
+    else launch_rings_to_rec64(corners, rvc, gam, N, R.rec64, st);
+    if (precision == VLM_PREC_FP64) {
+      launch_partial64(R.rec64, chunks, p.nq, N, P, (int)M, R.part, st);
+    } else {
+      const bool nearOn = precision == VLM_PREC_FP32_NEAR64;
+      launch_pack32(R.rec64, (int)N, nearOn ? 4.0 : 0.0, R.rec32, st);
+      launch_partial32(R.rec32, R.rec64, chunks, p.nq, (int)N, P, (int)M, R.part, err, nearOn ? R.near : nullptr,
+                       p.nearBytes,
+                       R.nacc, st);
+    }
+    if (precision == VLM_PREC_FP64) launch_combine(R.part, (int)M, group, 1, 2, V, st);
+    else launch_combine_unordered(R.part, precision == VLM_PREC_FP32_NEAR64 ? R.nacc : nullptr, (int)M, group, 1, p.nq, 2, V, st);
+  } else {
+    VLM_CUDA(cudaMemsetAsync(V, 0, (size_t)M * 3 * 8, st));
+  }
+  VLM_CUDA(cudaGetLastError());
+}
+
+static void ring_status(const int* ctl) {
+  if (ctl[0] == 3) throw StatusError(VLM_ERR_CUDA, "near-field pair list overflowed");
+  if (ctl[0] == 4) throw StatusError(VLM_ERR_NONFINITE, "near-field velocity outside the fixed-point range");
+  if (ctl[0]) throw StatusError(VLM_ERR_CUDA, "device wait limit expired in a Biot-Savart tile pipeline");
+}
+
+void rings_device(const double* corners, const double* rvc, const double* gam, int64_t N, const double* P, int64_t M,
+                  double* V, int precision, cudaStream_t st, bool fil = false) {
+  ring_check(N, M, precision);
   if (M == 0) return;
   int dev = 0;
   VLM_CUDA(cudaGetDevice(&dev));
   RingScratch& R = g_ring[dev & 63];
   std::lock_guard<std::mutex> lock(R.mu);
-  Group g;
-  std::vector<Chunk> ch;
-  const int nq = ring_plan(N, M, precision, g, ch);
-  const int Q = std::max(nq, 1);
-  grow((void**)&R.rec64, R.cap64, (size_t)std::max<int64_t>(N, 1) * kRec64 * 8);
-  if (precision != VLM_PREC_FP64) grow((void**)&R.rec32, R.cap32, (size_t)std::max<int64_t>(N, 1) * kRec32 * 4);
-  grow((void**)&R.part, R.capPart, (size_t)M * Q * 3 * 8);
-  grow((void**)&R.chunks, R.capChunks, (size_t)Q * sizeof(Chunk) + sizeof(Group) + 64);
-  R.group = reinterpret_cast<Group*>(R.chunks + Q);
+  const RingPlan p = ring_reserve(R, N, M, precision);
+  grow((void**)&R.chunks, R.capChunks, (size_t)p.Q * sizeof(Chunk) + sizeof(Group) + 64);
+  R.group = reinterpret_cast<Group*>(R.chunks + p.Q);
   if (!R.err) VLM_CUDA(cudaMalloc(&R.err, 4 * sizeof(int)));
-  const size_t nearBytes = precision == VLM_PREC_FP32_NEAR64 ? near_scratch_bytes((int)M, ring_near_cap(M)) : 1;
-  grow((void**)&R.near, R.capNear, nearBytes);
-  if (precision == VLM_PREC_FP32_NEAR64 && (size_t)M * Q * 3 * 8 > R.capNacc) {
-    grow((void**)&R.nacc, R.capNacc, (size_t)M * Q * 3 * 8);
-    VLM_CUDA(cudaMemset(R.nacc, 0, R.capNacc));
-  }
   // the tables are tiny; copy them synchronously with the stream so that the
   // caller's later reuse of the scratch is ordered after this launch
-  VLM_CUDA(cudaMemcpyAsync(R.chunks, ch.data(), sizeof(Chunk) * std::max(nq, 1), cudaMemcpyHostToDevice, st));
-  VLM_CUDA(cudaMemcpyAsync(R.group, &g, sizeof(Group), cudaMemcpyHostToDevice, st));
+  VLM_CUDA(cudaMemcpyAsync(R.chunks, p.ch.data(), sizeof(Chunk) * p.Q, cudaMemcpyHostToDevice, st));
+  VLM_CUDA(cudaMemcpyAsync(R.group, &p.g, sizeof(Group), cudaMemcpyHostToDevice, st));
   VLM_CUDA(cudaMemsetAsync(R.err, 0, 4 * sizeof(int), st));
-  if (N > 0) {
-    if (fil) launch_fils_to_rec64(corners, rvc, gam, N, R.rec64, st);
-    else launch_rings_to_rec64(corners, rvc, gam, N, R.rec64, st);
-    if (precision == VLM_PREC_FP64) {
-      launch_partial64(R.rec64, R.chunks, nq, N, P, (int)M, R.part, st);
-    } else {
-      const bool nearOn = precision == VLM_PREC_FP32_NEAR64;
-      launch_pack32(R.rec64, (int)N, nearOn ? 4.0 : 0.0, R.rec32, st);
-      launch_partial32(R.rec32, R.rec64, R.chunks, nq, (int)N, P, (int)M, R.part, R.err, nearOn ? R.near : nullptr,
-                       nearBytes,
-                       R.nacc, st);
-    }
-    if (precision == VLM_PREC_FP64) launch_combine(R.part, (int)M, R.group, 1, 2, V, st);
-    else launch_combine_unordered(R.part, precision == VLM_PREC_FP32_NEAR64 ? R.nacc : nullptr, (int)M, R.group, 1, nq, 2, V, st);
-  } else {
-    VLM_CUDA(cudaMemsetAsync(V, 0, (size_t)M * 3 * 8, st));
-  }
-  VLM_CUDA(cudaGetLastError());
+  ring_launch(R, p, corners, rvc, gam, N, P, M, V, precision, R.chunks, R.group, R.err, st, fil);
   // the host-side tables above live on this stack frame and the scratch is
   // shared by every call on this device: finish before returning
   int ctl[2] = {0, 0};
   VLM_CUDA(cudaMemcpyAsync(ctl, R.err, sizeof(ctl), cudaMemcpyDeviceToHost, st));
   VLM_CUDA(cudaStreamSynchronize(st));
-  if (ctl[0] == 3) throw StatusError(VLM_ERR_CUDA, "near-field pair list overflowed");
-  if (ctl[0] == 4) throw StatusError(VLM_ERR_NONFINITE, "near-field velocity outside the fixed-point range");
-  if (ctl[0]) throw StatusError(VLM_ERR_CUDA, "device wait limit expired in a Biot-Savart tile pipeline");
+  ring_status(ctl);
+}
+
+// Host-buffer form: nc / nr doubles per source of corners / core radii (rings
+// 12 / 4, filaments 6 / 1).  A call is one panelled wing's worth of work at
+// its smallest, 34 us of kernels, so its cost is the copies and allocations
+// around them: up to RingScratch::kIoMax bytes the arrays, the tables and the
+// control words travel as one pinned copy each way through kept buffers
+// (52 rings at 52 points: 127 -> 58 us); beyond, the copies' own time is what
+// counts and the buffers are allocated for the call.
+void rings_host(const double* corners, const double* rvc, const double* gam, int64_t N, const double* P, int64_t M,
+                double* V, int precision, bool fil) {
+  const size_t nc = fil ? 6 : 12, nr = fil ? 1 : 4;
+  ring_check(N, M, precision);
+  if (M == 0) return;
+  const size_t bc = (size_t)N * nc * 8, br = (size_t)N * nr * 8, bg = (size_t)N * 8, bp = (size_t)M * 3 * 8;
+  const auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
+  const size_t arrays = al(bc) + al(br) + al(bg) + 2 * al(bp);
+  if (arrays > RingScratch::kIoMax / 2) {
+    DevArena own;
+    double* dc = dalloc<double>((size_t)N * nc, own);
+    double* dr = dalloc<double>((size_t)N * nr, own);
+    double* dg = dalloc<double>((size_t)N, own);
+    double* dp = dalloc<double>((size_t)M * 3, own);
+    double* dv = dalloc<double>((size_t)M * 3, own);
+    if (N > 0) {
+      VLM_CUDA(cudaMemcpy(dc, corners, bc, cudaMemcpyHostToDevice));
+      VLM_CUDA(cudaMemcpy(dr, rvc, br, cudaMemcpyHostToDevice));
+      VLM_CUDA(cudaMemcpy(dg, gam, bg, cudaMemcpyHostToDevice));
+    }
+    VLM_CUDA(cudaMemcpy(dp, P, bp, cudaMemcpyHostToDevice));
+    rings_device(dc, dr, dg, N, dp, M, dv, precision, nullptr, fil);
+    VLM_CUDA(cudaMemcpy(V, dv, bp, cudaMemcpyDeviceToHost));
+    return;
+  }
+  int dev = 0;
+  VLM_CUDA(cudaGetDevice(&dev));
+  RingScratch& R = g_ring[dev & 63];
+  std::lock_guard<std::mutex> lock(R.mu);
+  const RingPlan p = ring_reserve(R, N, M, precision);
+  // in: corners, radii, strengths, points, tables, control words; out: control words, velocities
+  const size_t oR = al(bc), oG = oR + al(br), oP = oG + al(bg), oQ = oP + al(bp),
+               oT = oQ + al(sizeof(Chunk) * (size_t)p.Q), oE = oT + al(sizeof(Group)), oV = oE + 256, end = oV + al(bp);
+  if (end > R.capIo) {
+    const size_t want = std::max<size_t>(end, 64u << 10);
+    if (R.hio) cudaFreeHost(R.hio);
+    R.hio = nullptr;
+    grow((void**)&R.io, R.capIo, want);
+    R.capIo = 0;
+    VLM_CUDA(cudaMallocHost((void**)&R.hio, want));
+    R.capIo = want;
+  }
+  if (N > 0) {
+    std::memcpy(R.hio, corners, bc);
+    std::memcpy(R.hio + oR, rvc, br);
+    std::memcpy(R.hio + oG, gam, bg);
+  }
+  std::memcpy(R.hio + oP, P, bp);
+  std::memcpy(R.hio + oQ, p.ch.data(), sizeof(Chunk) * (size_t)p.Q);
+  std::memcpy(R.hio + oT, &p.g, sizeof(Group));
+  std::memset(R.hio + oE, 0, 256);
+  const cudaStream_t st = nullptr;
+  VLM_CUDA(cudaMemcpyAsync(R.io, R.hio, oV, cudaMemcpyHostToDevice, st));
+  int* err = reinterpret_cast<int*>(R.io + oE);
+  const auto at = [&](size_t o) { return reinterpret_cast<double*>(R.io + o); };
+  ring_launch(R, p, at(0), at(oR), at(oG), N, at(oP), M, at(oV), precision, reinterpret_cast<Chunk*>(R.io + oQ),
+              reinterpret_cast<Group*>(R.io + oT), err, st, fil);
+  VLM_CUDA(cudaMemcpyAsync(R.hio + oE, err, oV - oE + bp, cudaMemcpyDeviceToHost, st));
+  VLM_CUDA(cudaStreamSynchronize(st));
+  ring_status(reinterpret_cast<const int*>(R.hio + oE));
+  std::memcpy(V, R.hio + oV, bp);
 }
 
 }  // namespace vlm
@@ -2603,37 +2742,12 @@ int64_t vlm_biot_savart_rings_sum_chunk(int64_t N, int64_t M, int precision) {
   return ring_sum_chunk(N, M, precision);
 }
 
-// Host-buffer form of rings_device: nc / nr doubles per source of corners /
-// core radii (rings 12 / 4, filaments 6 / 1).
 static int sources_host(const double* corners, const double* rvc, const double* gam, int64_t N, const double* P,
                         int64_t M, double* V, int precision, bool fil) {
-  const size_t nc = fil ? 6 : 12, nr = fil ? 1 : 4;
   return guard([&]() {
     if (N < 0 || M < 0) throw StatusError(VLM_ERR_INVALID, "N and M must be non-negative");
     if ((N > 0 && (!corners || !rvc || !gam)) || (M > 0 && (!P || !V))) throw StatusError(VLM_ERR_INVALID, "null array");
-    std::vector<void*> own;
-    auto cleanup = [&]() {
-      for (void* p : own) cudaFree(p);
-    };
-    try {
-      double* dc = dalloc<double>((size_t)std::max<int64_t>(N, 1) * nc, own);
-      double* dr = dalloc<double>((size_t)std::max<int64_t>(N, 1) * nr, own);
-      double* dg = dalloc<double>((size_t)std::max<int64_t>(N, 1), own);
-      double* dp = dalloc<double>((size_t)std::max<int64_t>(M, 1) * 3, own);
-      double* dv = dalloc<double>((size_t)std::max<int64_t>(M, 1) * 3, own);
-      if (N > 0) {
-        VLM_CUDA(cudaMemcpy(dc, corners, (size_t)N * nc * 8, cudaMemcpyHostToDevice));
-        VLM_CUDA(cudaMemcpy(dr, rvc, (size_t)N * nr * 8, cudaMemcpyHostToDevice));
-        VLM_CUDA(cudaMemcpy(dg, gam, (size_t)N * 8, cudaMemcpyHostToDevice));
-      }
-      if (M > 0) VLM_CUDA(cudaMemcpy(dp, P, (size_t)M * 3 * 8, cudaMemcpyHostToDevice));
-      rings_device(dc, dr, dg, N, dp, M, dv, precision, nullptr, fil);
-      if (M > 0) VLM_CUDA(cudaMemcpy(V, dv, (size_t)M * 3 * 8, cudaMemcpyDeviceToHost));
-    } catch (...) {
-      cleanup();
-      throw;
-    }
-    cleanup();
+    rings_host(corners, rvc, gam, N, P, M, V, precision, fil);
   });
 }
 
