@@ -40,6 +40,7 @@
 #include <climits>
 #include <atomic>
 
+#include "launch.h"
 #include "pack32.h"
 #include "vlm_bs.h"
 #include "vlm_math.h"
@@ -351,10 +352,11 @@ constexpr int kBlockW = (kConsumerWarps + 1) * 32;
 // LAT: the records are in lattice form (edges 2 and 3 marked when they carry
 // no circulation); otherwise every record is evaluated as a whole ring.
 template <bool LAT, int kTPT, int kStages, int kMinBlocks>
-__global__ void __launch_bounds__(kBlockW, kMinBlocks) k_partial32(const float* __restrict__ rec32,
-                                                                  const Chunk* __restrict__ chunks,
-                                                                  const double* __restrict__ P, int M,
-                                                                  double* __restrict__ part, int* __restrict__ ctl) {
+__global__ void __launch_bounds__(kBlockW, kMinBlocks) k_partial32(const float* rec32,
+                                                                  const Chunk* chunks,
+                                                                  const double* P, int M,
+                                                                  double* part, int* ctl) {
+  after_previous();
   constexpr int kTargetsPerBlock = kConsumerWarps * 32 * kTPT;
   extern __shared__ __align__(16) float stage[];  // [kStages][kTileW * kRec32]
   __shared__ __align__(8) uint64_t full[kStages];
@@ -535,6 +537,7 @@ __device__ __forceinline__ int cell_slot(const unsigned long long* __restrict__ 
 }
 
 __global__ void k_grid_init(unsigned char* scratch, int T) {
+  after_previous();
   GridHdr* H = reinterpret_cast<GridHdr*>(scratch);
   H->zsum = 0.0;
   H->zcount = 0u;
@@ -554,7 +557,8 @@ __device__ __forceinline__ float ord_value(int c) { return __int_as_float(c >= 0
 
 // Sum and count of the near-zone radii near_factor rvc_k = sqrt([32 + k]) /
 // |e_k| of the active filaments (the cell size is twice their mean).
-__global__ void k_zone_mean(const float* __restrict__ rec32, int nrec, unsigned char* __restrict__ scratch) {
+__global__ void k_zone_mean(const float* rec32, int nrec, unsigned char* scratch) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double z = 0.0;
   unsigned c = 0u;
@@ -590,7 +594,8 @@ __device__ __forceinline__ float grid_h(const GridHdr* H) {
 // PASS 0: insert the target's cell key and count the target in its slot;
 // PASS 1: write the target's FP32 position and index at its slot's cursor.
 template <int PASS>
-__global__ void k_tgrid_insert(const double* __restrict__ P, int M, unsigned char* __restrict__ scratch) {
+__global__ void k_tgrid_insert(const double* P, int M, unsigned char* scratch) {
+  after_previous();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (PASS == 0) {
     // the targets' bounding box: one min and one max per axis and warp
@@ -640,7 +645,8 @@ __global__ void k_tgrid_insert(const double* __restrict__ P, int M, unsigned cha
 // Exclusive scan of the slot counts into start[0..T]; the counts become the
 // fill cursors (= start).  One block of 1024 threads: tiles of 1024 slots,
 // each scanned with warp shuffles, carried from tile to tile.
-__global__ void k_grid_scan(int M, unsigned char* __restrict__ scratch) {
+__global__ void k_grid_scan(int M, unsigned char* scratch) {
+  after_previous();
   const GridLayout L = grid_layout(M);
   const int T = reinterpret_cast<const GridHdr*>(scratch)->T;
   int* count = reinterpret_cast<int*>(scratch + L.count);
@@ -712,11 +718,12 @@ __device__ __forceinline__ d3 fil_near64(d3 p, d3 a, d3 b, double rvc) {
 // every (record, target) pair gets k_near_find's test directly, one thread
 // per pair -- the same pairs without building a grid of the targets or
 // walking every filament through it.
-__global__ void __launch_bounds__(256) k_near_find_small(const float* __restrict__ rec32, int nrec,
-                                                         const Chunk* __restrict__ chunks, int nchunks,
-                                                         const double* __restrict__ P, int M,
-                                                         NearPair* __restrict__ near, int near_cap,
-                                                         int* __restrict__ ctl) {
+__global__ void __launch_bounds__(256) k_near_find_small(const float* rec32, int nrec,
+                                                         const Chunk* chunks, int nchunks,
+                                                         const double* P, int M,
+                                                         NearPair* near, int near_cap,
+                                                         int* ctl) {
+  after_previous();
   const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
@@ -775,11 +782,12 @@ __global__ void __launch_bounds__(256) k_near_find_small(const float* __restrict
   }
 }
 
-__global__ void __launch_bounds__(256, 4) k_near_find(const float* __restrict__ rec32, int nrec,
-                                                   const Chunk* __restrict__ chunks, int nchunks,
-                                                   const double* __restrict__ P, int M,
-                                                   const unsigned char* __restrict__ scratch,
-                                                   NearPair* __restrict__ near, int near_cap, int* __restrict__ ctl) {
+__global__ void __launch_bounds__(256, 4) k_near_find(const float* rec32, int nrec,
+                                                   const Chunk* chunks, int nchunks,
+                                                   const double* P, int M,
+                                                   const unsigned char* scratch,
+                                                   NearPair* near, int near_cap, int* ctl) {
+  after_previous();
   const size_t wid = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wid >= (size_t)nrec * 4) return;  // whole warps leave together
@@ -930,10 +938,11 @@ __global__ void __launch_bounds__(256, 4) k_near_find(const float* __restrict__ 
 // operations, the product taken exactly in FP64), added in fixed point to the
 // accumulator of the target and the record's chunk (order-independent).
 // ctl[0] = 4 flags a correction outside the fixed-point range.
-__global__ void k_near_fix(const NearPair* __restrict__ near, int near_cap, const float* __restrict__ rec32,
-                           const double* __restrict__ rec64, const double* __restrict__ ew,
-                           const double* __restrict__ P, int M, unsigned long long* __restrict__ nacc,
-                           int* __restrict__ ctl) {
+__global__ void k_near_fix(const NearPair* near, int near_cap, const float* rec32,
+                           const double* rec64, const double* ew,
+                           const double* P, int M, unsigned long long* nacc,
+                           int* ctl) {
+  after_previous();
   const int n = min(ctl[1], near_cap);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const NearPair np_ = near[i];
@@ -982,8 +991,9 @@ __global__ void k_wait_probe(uint32_t limit, int* out) {
 }
 
 // FP64 records -> FP32 records, four lanes a record (pack32.h).
-__global__ void k_pack32(const double* __restrict__ rec64, int nrec, double near_factor, float* __restrict__ rec32,
-                         const double* __restrict__ ew) {
+__global__ void k_pack32(const double* rec64, int nrec, double near_factor, float* rec32,
+                         const double* ew) {
+  after_previous();
   const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const bool live = q < (size_t)nrec * 4;
   const size_t i = live ? q >> 2 : 0;
@@ -1003,7 +1013,7 @@ void launch_pack32(const double* rec64, int nrec, double near_factor, float* rec
                    const double* ew) {
   if (nrec <= 0) return;
   count_launch();
-  k_pack32<<<(unsigned)(((size_t)nrec * 4 + 255) / 256), 256, 0, s>>>(rec64, nrec, near_factor, rec32, ew);
+  launch_next(k_pack32, (unsigned)(((size_t)nrec * 4 + 255) / 256), 256, 0, s, rec64, nrec, near_factor, rec32, ew);
 }
 
 // The compiled tile shapes: {targets per thread, stages, blocks per SM}.
@@ -1039,8 +1049,8 @@ template <int V>
 void launch_shape(bool lat, dim3 grid, const float* rec32, const Chunk* chunks, const double* P, int M, double* part,
                   int* ctl, cudaStream_t s) {
   using S = Shape32<V>;
-  if (lat) k_partial32<true, S::tpt, S::stages, S::minb><<<grid, kBlockW, shape_smem<V>(), s>>>(rec32, chunks, P, M, part, ctl);
-  else k_partial32<false, S::tpt, S::stages, S::minb><<<grid, kBlockW, shape_smem<V>(), s>>>(rec32, chunks, P, M, part, ctl);
+  if (lat) launch_next(k_partial32<true, S::tpt, S::stages, S::minb>, grid, kBlockW, shape_smem<V>(), s, rec32, chunks, P, M, part, ctl);
+  else launch_next(k_partial32<false, S::tpt, S::stages, S::minb>, grid, kBlockW, shape_smem<V>(), s, rec32, chunks, P, M, part, ctl);
 }
 
 // the dynamic shared-memory opt-in is per device; set it once on each
@@ -1098,9 +1108,9 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
   if (M <= kNearSmallTargets && (size_t)nrec * M <= ((size_t)1 << 22)) {
     // few targets: every pair tested directly
     count_launches(2);
-    k_near_find_small<<<(unsigned)(((size_t)nrec * M + 255) / 256), 256, 0, ns>>>(rec32, nrec, chunks, nchunks, P, M,
+    launch_next(k_near_find_small, (unsigned)(((size_t)nrec * M + 255) / 256), 256, 0, ns, rec32, nrec, chunks, nchunks, P, M,
                                                                                    list, cap, ctl);
-    k_near_fix<<<4 * sms, 128, 0, ns>>>(list, cap, rec32, rec64, ew, P, M,
+    launch_next(k_near_fix, 4 * sms, 128, 0, ns, list, cap, rec32, rec64, ew, P, M,
                                         reinterpret_cast<unsigned long long*>(nacc), ctl);
     if (ns != s) {
       cudaEventRecord(ov->join, ns);
@@ -1110,18 +1120,18 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
   }
   if (!reuse_grid) {
     count_launches(5);
-    k_grid_init<<<1, 1, 0, ns>>>(g, T);
-    k_zone_mean<<<(nrec + 255) / 256, 256, 0, ns>>>(rec32, nrec, g);
+    launch_next(k_grid_init, 1, 1, 0, ns, g, T);
+    launch_next(k_zone_mean, (nrec + 255) / 256, 256, 0, ns, rec32, nrec, g);
     cudaMemsetAsync(g + L.key, 0xFF, (size_t)T * sizeof(unsigned long long), ns);
     cudaMemsetAsync(g + L.count, 0, (size_t)T * sizeof(int), ns);
-    k_tgrid_insert<0><<<(M + 255) / 256, 256, 0, ns>>>(P, M, g);
-    k_grid_scan<<<1, 1024, 0, ns>>>(M, g);
-    k_tgrid_insert<1><<<(M + 255) / 256, 256, 0, ns>>>(P, M, g);
+    launch_next(k_tgrid_insert<0>, (M + 255) / 256, 256, 0, ns, P, M, g);
+    launch_next(k_grid_scan, 1, 1024, 0, ns, M, g);
+    launch_next(k_tgrid_insert<1>, (M + 255) / 256, 256, 0, ns, P, M, g);
   }
   count_launches(2);
-  k_near_find<<<(unsigned)(((size_t)nrec * 4 * 32 + 255) / 256), 256, 0, ns>>>(rec32, nrec, chunks, nchunks, P, M,
+  launch_next(k_near_find, (unsigned)(((size_t)nrec * 4 * 32 + 255) / 256), 256, 0, ns, rec32, nrec, chunks, nchunks, P, M,
                                                                                g, list, cap, ctl);
-  k_near_fix<<<4 * sms, 128, 0, ns>>>(list, cap, rec32, rec64, ew, P, M, reinterpret_cast<unsigned long long*>(nacc),
+  launch_next(k_near_fix, 4 * sms, 128, 0, ns, list, cap, rec32, rec64, ew, P, M, reinterpret_cast<unsigned long long*>(nacc),
                                       ctl);
   if (ns != s) {
     cudaEventRecord(ov->join, ns);

@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "launch.h"
 #include "exact64.h"
 #include "vlm_bs.h"
 #include "vlm_math.h"
@@ -60,8 +61,9 @@ __device__ __forceinline__ bool same_point(const double* a, const double* b) {
          __double_as_longlong(a[1]) == __double_as_longlong(b[1]) &&
          __double_as_longlong(a[2]) == __double_as_longlong(b[2]);
 }
-__global__ void k_share64(const double* __restrict__ rec, int nrec, const Group* __restrict__ groups, int ngroups,
-                          int L, int* __restrict__ share) {
+__global__ void k_share64(const double* rec, int nrec, const Group* groups, int ngroups,
+                          int L, int* share) {
+  after_previous();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nrec) return;
   int g = 0;
@@ -128,9 +130,10 @@ __device__ __forceinline__ void add_batch64(const exact64::Unit& u, const double
 }
 
 // Grid: (target tiles) x (runs of K consecutive chunks).  lgTT = log2(TT).
-__global__ void __launch_bounds__(kThreads64) k_rings64(const double* __restrict__ rec, const Chunk* __restrict__ chunks,
-                                                       int nchunks, int K, const double* __restrict__ P, int M, int lgTT,
-                                                       double* __restrict__ part) {
+__global__ void __launch_bounds__(kThreads64) k_rings64(const double* rec, const Chunk* chunks,
+                                                       int nchunks, int K, const double* P, int M, int lgTT,
+                                                       double* part) {
+  after_previous();
   __shared__ double C[2][3 * kThreads64];  // contributions of two batches [s][component][t]
   __shared__ double acc[3 * kMaxTT];       // the open chunk's sums [component][t]
   const int TT = 1 << lgTT, S = kThreads64 >> lgTT;
@@ -168,10 +171,11 @@ __global__ void __launch_bounds__(kThreads64) k_rings64(const double* __restrict
 // Between the first barrier of a batch and the second: corners 2 of the batch
 // and the contributions of the one before; between the second and the next
 // first: its edges and the additions of the one before.
-__global__ void __launch_bounds__(kThreadsLattice64) k_lattice64(const double* __restrict__ rec, const int* __restrict__ share,
-                                                         const Chunk* __restrict__ chunks, int nchunks, int K,
-                                                         const double* __restrict__ P, int M, int lgTT, int L,
-                                                         double* __restrict__ part) {
+__global__ void __launch_bounds__(kThreadsLattice64) k_lattice64(const double* rec, const int* share,
+                                                         const Chunk* chunks, int nchunks, int K,
+                                                         const double* P, int M, int lgTT, int L,
+                                                         double* part) {
+  after_previous();
   extern __shared__ double sm[];
   constexpr int NT = kThreadsLattice64;
   constexpr int B = 3 * NT;  // a batch's vectors in doubles, [s][component][t]
@@ -377,8 +381,9 @@ __device__ __forceinline__ double group_sum(const double* __restrict__ part, lon
 // mode 0 (wake nodes): out = 0 + (wing + wake); 1: wake; 2: wing + wake.
 // ADD: out = out + that.
 template <bool ORDERED, bool ADD>
-__global__ void k_combine(const double* __restrict__ part, long long* __restrict__ nacc, int M,
-                          const Group* __restrict__ groups, int ngroups, int mode, int G, double* __restrict__ out) {
+__global__ void k_combine(const double* part, long long* nacc, int M,
+                          const Group* groups, int ngroups, int mode, int G, double* out) {
+  after_previous();
   const size_t gt = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const size_t mc = gt / G;
   const int l = (int)(gt % G);
@@ -405,9 +410,10 @@ __global__ void k_combine(const double* __restrict__ part, long long* __restrict
 // sum each, which the RHS adds to velCP in turn.  With a single term, mode 0
 // equals k_combine's mode 0 bit for bit.
 template <bool ORDERED>
-__global__ void k_combine_terms(const double* __restrict__ part, long long* __restrict__ nacc, int M,
-                                const Group* __restrict__ groups, int ngroups, int mode, int G,
-                                double* __restrict__ out) {
+__global__ void k_combine_terms(const double* part, long long* nacc, int M,
+                                const Group* groups, int ngroups, int mode, int G,
+                                double* out) {
+  after_previous();
   const size_t gt = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const size_t mc = gt / G;
   const int l = (int)(gt % G);
@@ -442,8 +448,9 @@ inline int tree_lanes(int max_chunks) {
   return G;
 }
 
-__global__ void k_rings_to_rec64(const double* __restrict__ corners, const double* __restrict__ rvc,
-                                 const double* __restrict__ gam, int64_t N, double* __restrict__ rec) {
+__global__ void k_rings_to_rec64(const double* corners, const double* rvc,
+                                 const double* gam, int64_t N, double* rec) {
+  after_previous();
   const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= N) return;
   double* R = rec + n * kRec64;
@@ -456,8 +463,9 @@ __global__ void k_rings_to_rec64(const double* __restrict__ corners, const doubl
 // Single filaments fc1 -> fc2 (vf_vind, src/classdef.f90:476-503) as
 // REC_FIL records; no |gam| skip (gridgen sums every filament,
 // src/gridgen.f90:128-136).
-__global__ void k_fils_to_rec64(const double* __restrict__ fc, const double* __restrict__ rvc,
-                                const double* __restrict__ gam, int64_t N, double* __restrict__ rec) {
+__global__ void k_fils_to_rec64(const double* fc, const double* rvc,
+                                const double* gam, int64_t N, double* rec) {
+  after_previous();
   const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (n >= N) return;
   double* R = rec + n * kRec64;
@@ -513,13 +521,13 @@ void launch_rings64(const Tile64& T, const double* rec, const Chunk* chunks, int
                     double* part, cudaStream_t s) {
   int K = 1;
   const dim3 grid = grid64(T, M, nchunks, K);
-  k_rings64<<<grid, kThreads64, 0, s>>>(rec, chunks, nchunks, K, P, M, T.lgTT, part);
+  launch_next(k_rings64, grid, kThreads64, 0, s, rec, chunks, nchunks, K, P, M, T.lgTT, part);
 }
 void launch_lattice64(const Tile64& T, const double* rec, const int* share, const Chunk* chunks, int nchunks, int L,
                       const double* P, int M, double* part, cudaStream_t s) {
   int K = 1;
   const dim3 grid = grid64(T, M, nchunks, K);
-  k_lattice64<<<grid, kThreadsLattice64, lattice_smem64(T.lgTT, L), s>>>(rec, share, chunks, nchunks, K, P, M, T.lgTT,
+  launch_next(k_lattice64, grid, kThreadsLattice64, lattice_smem64(T.lgTT, L), s, rec, share, chunks, nchunks, K, P, M, T.lgTT,
                                                                          L, part);
 }
 }  // namespace
@@ -542,7 +550,7 @@ void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunk
   if (M <= 0 || nchunks <= 0) return;
   lattice_attr64();
   count_launches(2);
-  k_share64<<<(nrec + 255) / 256, 256, 0, s>>>(rec, nrec, groups, ngroups, L, share);
+  launch_next(k_share64, (nrec + 255) / 256, 256, 0, s, rec, nrec, groups, ngroups, L, share);
   launch_lattice64(pick_tile64(M, nchunks, nrec, L, device_sm_count()), rec, share, chunks, nchunks, L, P, M, part, s);
 }
 
@@ -550,7 +558,7 @@ void launch_combine(const double* part, int M, const Group* groups, int ngroups,
                     cudaStream_t s) {
   if (M <= 0) return;
   count_launch();
-  k_combine<true, false><<<(unsigned)((3 * (size_t)M + 127) / 128), 128, 0, s>>>(part, nullptr, M, groups, ngroups,
+  launch_next(k_combine<true, false>, (unsigned)((3 * (size_t)M + 127) / 128), 128, 0, s, part, nullptr, M, groups, ngroups,
                                                                                 mode, 1, out);
 }
 
@@ -560,8 +568,8 @@ void launch_combine_unordered(const double* part, long long* nacc, int M, const 
   const int G = tree_lanes(max_chunks);
   const unsigned blocks = (unsigned)((3 * (size_t)M * G + 255) / 256);
   count_launch();
-  if (add) k_combine<false, true><<<blocks, 256, 0, s>>>(part, nacc, M, groups, ngroups, mode, G, out);
-  else k_combine<false, false><<<blocks, 256, 0, s>>>(part, nacc, M, groups, ngroups, mode, G, out);
+  if (add) launch_next(k_combine<false, true>, blocks, 256, 0, s, part, nacc, M, groups, ngroups, mode, G, out);
+  else launch_next(k_combine<false, false>, blocks, 256, 0, s, part, nacc, M, groups, ngroups, mode, G, out);
 }
 
 void launch_combine_terms(const double* part, long long* nacc, int M, const Group* groups, int ngroups,
@@ -569,12 +577,12 @@ void launch_combine_terms(const double* part, long long* nacc, int M, const Grou
   if (M <= 0 || ngroups <= 0) return;
   count_launch();
   if (ordered) {
-    k_combine_terms<true><<<(unsigned)((3 * (size_t)M + 127) / 128), 128, 0, s>>>(part, nullptr, M, groups, ngroups,
+    launch_next(k_combine_terms<true>, (unsigned)((3 * (size_t)M + 127) / 128), 128, 0, s, part, nullptr, M, groups, ngroups,
                                                                                  mode, 1, out);
     return;
   }
   const int G = tree_lanes(max_chunks);
-  k_combine_terms<false><<<(unsigned)((3 * (size_t)M * G + 255) / 256), 256, 0, s>>>(part, nacc, M, groups, ngroups,
+  launch_next(k_combine_terms<false>, (unsigned)((3 * (size_t)M * G + 255) / 256), 256, 0, s, part, nacc, M, groups, ngroups,
                                                                                     mode, G, out);
 }
 
@@ -582,14 +590,14 @@ void launch_fils_to_rec64(const double* fc, const double* rvc, const double* gam
                           cudaStream_t s) {
   if (N <= 0) return;
   count_launch();
-  k_fils_to_rec64<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(fc, rvc, gam, N, rec);
+  launch_next(k_fils_to_rec64, (unsigned)((N + 255) / 256), 256, 0, s, fc, rvc, gam, N, rec);
 }
 
 void launch_rings_to_rec64(const double* corners, const double* rvc, const double* gam, int64_t N, double* rec,
                            cudaStream_t s) {
   if (N <= 0) return;
   count_launch();
-  k_rings_to_rec64<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(corners, rvc, gam, N, rec);
+  launch_next(k_rings_to_rec64, (unsigned)((N + 255) / 256), 256, 0, s, corners, rvc, gam, N, rec);
 }
 
 }  // namespace vlm

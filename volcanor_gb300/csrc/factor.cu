@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "launch.h"
 #include "exact64.h"
 #include "vlm_math.h"
 #include "vlm_solver.h"
@@ -69,7 +70,8 @@ __device__ __forceinline__ ByDouble by(double d) { return ByDouble(d); }
 __device__ __forceinline__ ByFloat by(float d) { return ByFloat(d); }
 
 template <class T>
-__global__ void k_lu_copy(const double* __restrict__ A, T* __restrict__ LU, size_t n2) {
+__global__ void k_lu_copy(const double* A, T* LU, size_t n2) {
+  after_previous();
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i < n2) LU[i] = (T)A[i];
 }
@@ -83,9 +85,10 @@ struct Perm {
 // divides, updates the row's later columns and has the next column's candidates
 // at hand; the block meets twice a column, for the pivot and after the swap.
 template <class T>
-__global__ void __launch_bounds__(kPanelThreads) k_lu_panel(T* __restrict__ A, int n, int k0, int nb,
-                                                           int* __restrict__ piv, int* __restrict__ err,
-                                                           Perm* __restrict__ perm) {
+__global__ void __launch_bounds__(kPanelThreads) k_lu_panel(T* A, int n, int k0, int nb,
+                                                           int* piv, int* err,
+                                                           Perm* perm) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem[];
   T* p = reinterpret_cast<T*>(smem);  // [column][row - k0]
   typedef typename Mag<T>::type MagT;
@@ -180,8 +183,9 @@ __global__ void __launch_bounds__(kPanelThreads) k_lu_panel(T* __restrict__ A, i
 // Sixteen lanes a column j outside the panel: the panel's interchanges, then,
 // right of the panel, the panel's rows of U (unit lower triangle, k ascending).
 template <class T>
-__global__ void __launch_bounds__(128) k_lu_rows(T* __restrict__ A, int n, int k0, int nb,
-                                                const Perm* __restrict__ perm) {
+__global__ void __launch_bounds__(128) k_lu_rows(T* A, int n, int k0, int nb,
+                                                const Perm* perm) {
+  after_previous();
   __shared__ T L[kPanel][kPanel + 1];
   for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) L[e % nb][e / nb] = A[(size_t)(k0 + e / nb) * n + k0 + e % nb];
   __syncthreads();
@@ -210,7 +214,8 @@ __global__ void __launch_bounds__(128) k_lu_rows(T* __restrict__ A, int n, int k
 
 // The trailing matrix, 32 x 16 elements a block, four a thread.
 template <class T>
-__global__ void __launch_bounds__(128) k_lu_update(T* __restrict__ A, int n, int k0, int nb) {
+__global__ void __launch_bounds__(128) k_lu_update(T* A, int n, int k0, int nb) {
+  after_previous();
   __shared__ T L[kPanel][32], U[kPanel][16];
   const int i0 = k0 + nb + blockIdx.x * 32, j0 = k0 + nb + blockIdx.y * 16;
   for (int e = threadIdx.x; e < nb * 32; e += 128)
@@ -242,21 +247,21 @@ void lu(const double* AIC, T* A, int n, int* piv, int* err, Perm* perm, cudaStre
   }
   const size_t n2 = (size_t)n * n;
   count_launch();
-  k_lu_copy<<<(unsigned)((n2 + 255) / 256), 256, 0, st>>>(AIC, A, n2);
+  launch_next(k_lu_copy<T>, (unsigned)((n2 + 255) / 256), 256, 0, st, AIC, A, n2);
   for (int k0 = 0; k0 < n;) {
     // as many columns as fit shared memory (all kPanel up to 1800 rows)
     const int fit = (int)(kSmemMax / sizeof(T) / (size_t)(n - k0));
     const int nb = std::max(1, std::min(std::min(kPanel, fit), n - k0));
     count_launch();
-    k_lu_panel<T><<<1, kPanelThreads, sizeof(T) * nb * (size_t)(n - k0), st>>>(A, n, k0, nb, piv, err, perm);
+    launch_next(k_lu_panel<T>, 1, kPanelThreads, sizeof(T) * nb * (size_t)(n - k0), st, A, n, k0, nb, piv, err, perm);
     if (n > nb) {
       count_launch();
-      k_lu_rows<T><<<(n - nb + 128 / kPanel - 1) / (128 / kPanel), 128, 0, st>>>(A, n, k0, nb, perm);
+      launch_next(k_lu_rows<T>, (n - nb + 128 / kPanel - 1) / (128 / kPanel), 128, 0, st, A, n, k0, nb, perm);
     }
     const int rest = n - k0 - nb;
     if (rest > 0) {
       count_launch();
-      k_lu_update<T><<<dim3((rest + 31) / 32, (rest + 15) / 16), 128, 0, st>>>(A, n, k0, nb);
+      launch_next(k_lu_update<T>, dim3((rest + 31) / 32, (rest + 15) / 16), 128, 0, st, A, n, k0, nb);
     }
     k0 += nb;
   }
@@ -272,8 +277,9 @@ void lu(const double* AIC, T* A, int n, int* piv, int* err, Perm* perm, cudaStre
 // products and the rows of U were on the chain before: 9.1 ms.
 constexpr int kInvThreads = 128;
 
-__global__ void __launch_bounds__(kInvThreads) k_inverse64(const double* __restrict__ A, const int* __restrict__ piv,
-                                                          int n, int cols, double* __restrict__ inv) {
+__global__ void __launch_bounds__(kInvThreads) k_inverse64(const double* A, const int* piv,
+                                                          int n, int cols, double* inv) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem[];
   double* X = reinterpret_cast<double*>(smem);  // [row][column]
   double* prod = X + (size_t)n * cols;          // [2][k][column]: products of a row's later columns
@@ -361,8 +367,9 @@ __global__ void __launch_bounds__(kInvThreads) k_inverse64(const double* __restr
 
 // The same, a thread per column on global memory: for matrices whose columns do
 // not fit shared memory (over 4100 rows).
-__global__ void k_inverse64_big(const double* __restrict__ A, const int* __restrict__ piv, int n,
-                                double* __restrict__ inv) {
+__global__ void k_inverse64_big(const double* A, const int* piv, int n,
+                                double* inv) {
+  after_previous();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   double* X = inv + (size_t)n * c;
@@ -385,8 +392,9 @@ __global__ void k_inverse64_big(const double* __restrict__ A, const int* __restr
 }
 
 // FP32: a warp per column, lanes over k.
-__global__ void __launch_bounds__(128) k_inverse32(const float* __restrict__ A, const int* __restrict__ piv, int n,
-                                                  float* __restrict__ inv) {
+__global__ void __launch_bounds__(128) k_inverse32(const float* A, const int* piv, int n,
+                                                  float* inv) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const int c = blockIdx.x * wpb + warp;
@@ -416,7 +424,8 @@ __global__ void __launch_bounds__(128) k_inverse32(const float* __restrict__ A, 
 }
 
 // libMath.f90:428-458 (tolerance 1E-04 single precision)
-__global__ void k_is_inverse(const double* __restrict__ A, const double* __restrict__ inv, int n, int* err) {
+__global__ void k_is_inverse(const double* A, const double* inv, int n, int* err) {
+  after_previous();
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (t >= (long)n * n) return;
   const int i = (int)(t % n), j = (int)(t / n);
@@ -439,20 +448,20 @@ void launch_lu_inverse(const Dims& d, const DevState& s, cudaStream_t st) {
   lu<double>(s.AIC, s.LU, n, s.piv, s.err, static_cast<Perm*>(s.luPerm), st);
   count_launch();
   if (inverse_smem(n, 1) > kSmemMax) {
-    k_inverse64_big<<<(n + 63) / 64, 64, 0, st>>>(s.LU, s.piv, n, s.AICinv);
+    launch_next(k_inverse64_big, (n + 63) / 64, 64, 0, st, s.LU, s.piv, n, s.AICinv);
     return;
   }
   // as many columns a block as give every SM one, as far as shared memory holds them
   int cols = std::min(32, std::max(1, (n + device_sm_count() - 1) / device_sm_count()));
   while (cols > 1 && inverse_smem(n, cols) > kSmemMax) --cols;
   cudaFuncSetAttribute(k_inverse64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
-  k_inverse64<<<(n + cols - 1) / cols, kInvThreads, inverse_smem(n, cols), st>>>(s.LU, s.piv, n, cols, s.AICinv);
+  launch_next(k_inverse64, (n + cols - 1) / cols, kInvThreads, inverse_smem(n, cols), st, s.LU, s.piv, n, cols, s.AICinv);
 }
 
 void launch_is_inverse(const Dims& d, const DevState& s, cudaStream_t st) {
   const long n2 = (long)d.n * d.n;
   count_launch();
-  k_is_inverse<<<(unsigned)((n2 + 255) / 256), 256, 0, st>>>(s.AIC, s.AICinv, d.n, s.err);
+  launch_next(k_is_inverse, (unsigned)((n2 + 255) / 256), 256, 0, st, s.AIC, s.AICinv, d.n, s.err);
 }
 
 void launch_lu32(const Dims& d, const DevState& s, cudaStream_t st) {
@@ -461,7 +470,7 @@ void launch_lu32(const Dims& d, const DevState& s, cudaStream_t st) {
   int wpb = 4;
   while (wpb > 1 && sizeof(float) * wpb * (size_t)n > 48 * 1024) --wpb;
   count_launch();
-  k_inverse32<<<(n + wpb - 1) / wpb, 32 * wpb, sizeof(float) * wpb * (size_t)n, st>>>(s.LU32, s.piv32, n, s.AICinv32);
+  launch_next(k_inverse32, (n + wpb - 1) / wpb, 32 * wpb, sizeof(float) * wpb * (size_t)n, st, s.LU32, s.piv32, n, s.AICinv32);
 }
 
 }  // namespace vlm

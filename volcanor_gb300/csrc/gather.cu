@@ -7,6 +7,7 @@
 // the counter: 8 + 12.5 + 1.6 + 1.2 us at 500 records and the launches between.)
 // Only copies and one FP64 subtraction are rounded here, so the unit shares the FP32
 // kernels' compiler options.
+#include "launch.h"
 #include "pack32.h"
 #include "state_dev.h"
 #include "vlm_bs.h"
@@ -51,6 +52,7 @@ __device__ double lattice_weight(const Dims& d, const DevState& s, const double*
 __global__ void __launch_bounds__(256) k_gather(Dims d, DevState s, const double* fr, const Group* groups, int ngroups,
                                                 int nrec, int rowNear, int rowFar, int pred, float nearFactor,
                                                 int recBlocks, GatherTargets tg) {
+  after_previous();
   if ((int)blockIdx.x >= recBlocks) {
     const int m = (blockIdx.x - recBlocks) * blockDim.x + threadIdx.x;
     if (m < tg.M)
@@ -141,7 +143,7 @@ void launch_gather(const Dims& d, const DevState& s, const double* frame, const 
   const int rb = (int)(((long)nrec * 4 + 255) / 256), tb = tg.kind ? (tg.M + 255) / 256 : 0;
   if (rb + tb <= 0) return;
   count_launch();
-  k_gather<<<rb + tb, 256, 0, st>>>(d, s, frame, groups, ngroups, nrec, rowNear, rowFar, pred ? 1 : 0,
+  launch_next(k_gather, rb + tb, 256, 0, st, d, s, frame, groups, ngroups, nrec, rowNear, rowFar, pred ? 1 : 0,
                                     (float)nearFactor, rb, tg);
 }
 

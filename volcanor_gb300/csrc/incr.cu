@@ -17,6 +17,7 @@
 
 #include <algorithm>
 
+#include "launch.h"
 #include "vlm_bs.h"
 
 namespace vlm {
@@ -60,10 +61,11 @@ __device__ __forceinline__ int block_prefix(bool f, int* warpTot, int* total) {
 }
 
 // per block tile of kDiffTile items: the number that changed
-__global__ void __launch_bounds__(kDiffThreads) k_diff_count(const double* __restrict__ a, const double* __restrict__ b,
-                                                             int stride, const double* __restrict__ ea,
-                                                             const double* __restrict__ eb, int n,
-                                                             int* __restrict__ blockCount) {
+__global__ void __launch_bounds__(kDiffThreads) k_diff_count(const double* a, const double* b,
+                                                             int stride, const double* ea,
+                                                             const double* eb, int n,
+                                                             int* blockCount) {
+  after_previous();
   __shared__ int warpTot[kDiffThreads / 32];
   const int base = blockIdx.x * kDiffTile;
   int cnt = 0;
@@ -77,8 +79,9 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_count(const double* __res
 }
 
 // exclusive scan of the block counts in place (one block); *total = their sum
-__global__ void __launch_bounds__(kDiffThreads) k_diff_scan(int* __restrict__ blockCount, int nb,
-                                                            int* __restrict__ total) {
+__global__ void __launch_bounds__(kDiffThreads) k_diff_scan(int* blockCount, int nb,
+                                                            int* total) {
+  after_previous();
   __shared__ int sh[kDiffThreads];
   int carry = 0;
   for (int base = 0; base < nb; base += kDiffThreads) {
@@ -109,10 +112,11 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_scan(int* __restrict__ bl
 // record of zero weights and no near field.  More changed records than half
 // the capacity: ctl = 5 (the step's result is then wrong and reported).
 __global__ void __launch_bounds__(kDiffThreads)
-    k_delta_records(const double* __restrict__ recP, const double* __restrict__ recC, const double* __restrict__ ewP,
-                    const double* __restrict__ ewC, int nrec, const int* __restrict__ blockOff,
-                    const int* __restrict__ total, double* __restrict__ dRec, double* __restrict__ dEw, int cap,
-                    int* __restrict__ ctl) {
+    k_delta_records(const double* recP, const double* recC, const double* ewP,
+                    const double* ewC, int nrec, const int* blockOff,
+                    const int* total, double* dRec, double* dEw, int cap,
+                    int* ctl) {
+  after_previous();
   __shared__ int warpTot[kDiffThreads / 32];
   const int half = cap / 2;
   int off = blockOff[blockIdx.x];
@@ -164,9 +168,10 @@ __global__ void __launch_bounds__(kDiffThreads)
 // slots from min(total, cap) to cap get target 0's position (their results are
 // not used).  More than cap: ctl = 5.
 __global__ void __launch_bounds__(kDiffThreads)
-    k_moved_targets(const double* __restrict__ tP, const double* __restrict__ tC, int M,
-                    const int* __restrict__ blockOff, const int* __restrict__ total, int* __restrict__ idx,
-                    double* __restrict__ pos, int cap, int* __restrict__ ctl) {
+    k_moved_targets(const double* tP, const double* tC, int M,
+                    const int* blockOff, const int* total, int* idx,
+                    double* pos, int cap, int* ctl) {
+  after_previous();
   __shared__ int warpTot[kDiffThreads / 32];
   int off = blockOff[blockIdx.x];
   const int base = blockIdx.x * kDiffTile;
@@ -192,9 +197,10 @@ __global__ void __launch_bounds__(kDiffThreads)
 }
 
 // also passes the moved targets' evaluation's error code on to the step's
-__global__ void k_incr_put(double* __restrict__ out, const int* __restrict__ idx, const double* __restrict__ v,
-                           const int* __restrict__ total, int cap, const int* __restrict__ subCtl,
-                           int* __restrict__ ctl) {
+__global__ void k_incr_put(double* out, const int* idx, const double* v,
+                           const int* total, int cap, const int* subCtl,
+                           int* ctl) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0 && subCtl[0] != 0) atomicCAS(ctl, 0, subCtl[0]);
   if (i >= min(*total, cap)) return;
@@ -216,9 +222,9 @@ void launch_diff_count(const double* a, const double* b, int stride, const doubl
     return;
   }
   count_launch();
-  k_diff_count<<<nb, kDiffThreads, 0, s>>>(a, b, stride, ea, eb, n, blockCount);
+  launch_next(k_diff_count, nb, kDiffThreads, 0, s, a, b, stride, ea, eb, n, blockCount);
   count_launch();
-  k_diff_scan<<<1, kDiffThreads, 0, s>>>(blockCount, nb, total);
+  launch_next(k_diff_scan, 1, kDiffThreads, 0, s, blockCount, nb, total);
 }
 
 void launch_delta_records(const double* recP, const double* recC, const double* ewP, const double* ewC, int nrec,
@@ -226,7 +232,7 @@ void launch_delta_records(const double* recP, const double* recC, const double* 
                           cudaStream_t s) {
   if (nrec <= 0 || cap <= 0) return;
   count_launch();
-  k_delta_records<<<diff_blocks(nrec), kDiffThreads, 0, s>>>(recP, recC, ewP, ewC, nrec, blockOff, total, dRec, dEw,
+  launch_next(k_delta_records, diff_blocks(nrec), kDiffThreads, 0, s, recP, recC, ewP, ewC, nrec, blockOff, total, dRec, dEw,
                                                             cap, ctl);
 }
 
@@ -234,13 +240,13 @@ void launch_moved_targets(const double* tP, const double* tC, int M, const int* 
                           double* pos, int cap, int* ctl, cudaStream_t s) {
   if (M <= 0 || cap <= 0) return;
   count_launch();
-  k_moved_targets<<<diff_blocks(M), kDiffThreads, 0, s>>>(tP, tC, M, blockOff, total, idx, pos, cap, ctl);
+  launch_next(k_moved_targets, diff_blocks(M), kDiffThreads, 0, s, tP, tC, M, blockOff, total, idx, pos, cap, ctl);
 }
 
 void launch_incr_merge(double* out, const int* idx, const double* moved, const int* total, int cap, const int* subCtl,
                        int* ctl, cudaStream_t s) {
   count_launch();
-  k_incr_put<<<(std::max(cap, 1) + 255) / 256, 256, 0, s>>>(out, idx, moved, total, cap, subCtl, ctl);
+  launch_next(k_incr_put, (std::max(cap, 1) + 255) / 256, 256, 0, s, out, idx, moved, total, cap, subCtl, ctl);
 }
 
 }  // namespace vlm

@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "launch.h"
 #include "exact64.h"
 #include "state_dev.h"
 #include "vlm_math.h"
@@ -29,6 +30,7 @@ inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 
 // ---- shed (classdef.f90:4297-4325) ---------------------------------------
 __global__ void k_shed(Dims d, DevState s, const double* fr, int rowNear, int le) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.nb * d.ns) return;
   const int b = t / d.ns, j = t % d.ns;
@@ -49,6 +51,7 @@ __global__ void k_shed(Dims d, DevState s, const double* fr, int rowNear, int le
 
 // ---- age (classdef.f90:4331-4354) -----------------------------------------
 __global__ void k_age(Dims d, DevState s, int rowNear, int rowFar) {
+  after_previous();
   const int rows = d.NW - (rowNear - 1);
   const int nNear = d.nb * rows * d.ns;
   const int nFar = d.nb * max(d.NF - (rowFar - 1), 0);
@@ -69,6 +72,7 @@ __global__ void k_age(Dims d, DevState s, int rowNear, int rowFar) {
 
 // ---- dissipation (classdef.f90:4356-4408) ----------------------------------
 __global__ void k_dissip_a(Dims d, DevState s, int rowNear, int rowFar) {
+  after_previous();
   const int rows = d.NW - (rowNear - 1);
   const int nNear = d.nb * rows * d.ns;
   const int nFar = d.nb * max(d.NF - (rowFar - 1), 0);
@@ -93,6 +97,7 @@ __global__ void k_dissip_a(Dims d, DevState s, int rowNear, int rowFar) {
   }
 }
 __global__ void k_dissip_b(Dims d, DevState s, int rowNear) {
+  after_previous();
   const int rows = d.NW - rowNear;  // rows rowNear+1..NW (1-based)
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (rows <= 0 || t >= d.nb * rows * d.ns) return;
@@ -103,6 +108,7 @@ __global__ void k_dissip_b(Dims d, DevState s, int rowNear) {
 
 // ---- predicted copy (main.f90:1012-1019) -----------------------------------
 __global__ void k_copy_pred(Dims d, DevState s, int rowNear, int rowFar) {
+  after_previous();
   const int rows = d.NW - (rowNear - 1);
   const int nNear = d.nbC * rows * d.ns;
   const int nFar = d.nbC * max(d.NF - (rowFar - 1), 0);
@@ -123,6 +129,7 @@ __global__ void k_copy_pred(Dims d, DevState s, int rowNear, int rowFar) {
 
 // ---- convection shift (classdef.f90:1515-1575) ----------------------------
 __global__ void k_shift(Dims d, DevState s, int rowNear, int rowFar, int pred) {
+  after_previous();
   const int rows = pred ? 1 : d.NW - (rowNear - 1);
   const int i0 = pred ? 0 : rowNear - 1;  // the predicted loop visits row 1 only
   const int nNear = d.nbC * rows * (d.ns + 1);
@@ -146,6 +153,7 @@ __global__ void k_shift(Dims d, DevState s, int rowNear, int rowFar, int pred) {
 
 // ---- continuity (classdef.f90:1609-1702) ----------------------------------
 __global__ void k_continuity(Dims d, DevState s, int rowNear, int rowFar, int pred) {
+  after_previous();
   const int rows = d.NW - (rowNear - 1);
   const int nNear = d.nbC * rows * d.ns;
   const int nFar = d.nbC * max(d.NF - rowFar, 0);
@@ -178,6 +186,7 @@ __global__ void k_continuity(Dims d, DevState s, int rowNear, int rowFar, int pr
 
 // ---- axisymmetric wake copies (classdef.f90:4801-4823) ---------------------
 __global__ void k_axisym(Dims d, DevState s, const double* fr, int rowNear, int rowFar, int pred) {
+  after_previous();
   const int rows = d.NW - (rowNear - 1);
   const int nNear = (d.nb - 1) * rows * d.ns;
   const int rf = max(d.NF - (rowFar - 1), 0);
@@ -217,6 +226,7 @@ __global__ void k_axisym(Dims d, DevState s, const double* fr, int rowNear, int 
 
 // ---- strain (classdef.f90:4410-4422, 505-521) ------------------------------
 __global__ void k_strain(Dims d, DevState s, int rowFar) {
+  after_previous();
   const int rf = d.NF - (rowFar - 1);
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (rf <= 0 || t >= d.nb * rf) return;
@@ -237,6 +247,7 @@ __global__ void k_strain(Dims d, DevState s, int rowFar) {
 // the device's cos/sin/atan2, so the nodes agree with a host evaluation to a
 // few ulps, not bit for bit.
 __global__ void k_presc_update(Dims d, DevState s, const double* fr, int rowFar, int pred) {
+  after_previous();
   const int b = blockIdx.x;
   const int rowStart = d.prescGenNt == 0 ? rowFar : d.NF - d.prescGenNt;
   const int i0 = rowStart - 1, i1 = d.NF - 1, n = i1 - i0 + 1;
@@ -283,6 +294,7 @@ __global__ void k_presc_update(Dims d, DevState s, const double* fr, int rowFar,
 // Axisymmetric copies: blade b's prescribed wake = blade 1's, rotated about
 // the hub by b x 2 pi / nb (the wake copies' rotation).
 __global__ void k_presc_axisym(Dims d, DevState s, const double* fr, int pred) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (d.nb - 1) * kPresc) return;
   const int b = 1 + t / kPresc, i = t % kPresc;
@@ -306,6 +318,7 @@ __global__ void k_presc_axisym(Dims d, DevState s, const double* fr, int pred) {
 // at or above skewLimit both get the chord as core radius.  Only core radii
 // are written, from positions only, so the pairs run in parallel.
 __global__ void k_burst(Dims d, DevState s, int rowFar) {
+  after_previous();
   const int rf = d.NF - (rowFar - 1) - 1;  // pairs (i, i+1)
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (rf <= 0 || t >= d.nb * rf) return;
@@ -322,6 +335,7 @@ __global__ void k_burst(Dims d, DevState s, int rowFar) {
 
 // ---- far-wake shift for truncation (classdef.f90:4500-4513) ----------------
 __global__ void k_far_to_tmp(Dims d, DevState s) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.nb * d.NF) return;
   const int b = t / d.NF, i = t % d.NF;
@@ -336,6 +350,7 @@ __global__ void k_far_to_tmp(Dims d, DevState s) {
   o[11] = i == 0 ? 0.0 : s.fAge[src];
 }
 __global__ void k_far_from_tmp(Dims d, DevState s) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.nb * d.NF) return;
   const double* o = s.fTmp + (size_t)t * 12;
@@ -350,6 +365,7 @@ __global__ void k_far_from_tmp(Dims d, DevState s) {
 
 // ---- rollup (classdef.f90:4515-4605) ---------------------------------------
 __global__ void k_rollup(Dims d, DevState s, int rowFarNext) {
+  after_previous();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= d.nb) return;
   const int NW = d.NW;
@@ -400,6 +416,7 @@ __global__ void k_rollup(Dims d, DevState s, int rowFarNext) {
 
 // ---- near-wake shift after rollup (classdef.f90:4481-4498) -----------------
 __global__ void k_near_to_tmp(Dims d, DevState s) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int per = d.NW * d.ns;
   if (t >= d.nb * per) return;
@@ -413,6 +430,7 @@ __global__ void k_near_to_tmp(Dims d, DevState s) {
   o[17] = i == 0 ? 0.0 : s.nAge[src];
 }
 __global__ void k_near_from_tmp(Dims d, DevState s) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.nb * d.NW * d.ns) return;
   const double* o = s.nTmp + (size_t)t * 18;
@@ -424,6 +442,7 @@ __global__ void k_near_from_tmp(Dims d, DevState s) {
 
 // ---- velocity history algebra (main.f90:844-1406) --------------------------
 __global__ void k_velop(DevState s, long nN, long nF, int op) {
+  after_previous();
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (t >= nN + nF) return;
   const bool nearPart = t < nN;
@@ -472,6 +491,7 @@ __global__ void k_velop(DevState s, long nN, long nF, int op) {
 
 // ---- PC2 averaging (libCommon.f90:213-258) ---------------------------------
 __global__ void k_order2(Dims d, DevState s, int rowNear, int rowFar, int phase) {
+  after_previous();
   const int m = d.NW - (rowNear - 1);
   const int mf = max(d.NF - (rowFar - 1), 0);
   const int nNear = d.nbC * (d.ns + 1) * m * 3;
@@ -518,6 +538,7 @@ __global__ void k_order2(Dims d, DevState s, int rowNear, int rowFar, int phase)
 
 __global__ void k_scatter_nodes(Dims d, DevState s, const double* fr, int rowNear, int rowFar, int pred,
                                 double initWakeVel, int addInit, int M) {
+  after_previous();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= M) return;
   int b, far, i, j;
@@ -534,6 +555,7 @@ __global__ void k_scatter_nodes(Dims d, DevState s, const double* fr, int rowNea
 
 // ---- AIC and its inverse (classdef.f90:4151-4179, libMath.f90:48-83) ---------
 __global__ void k_aic(Dims d, DevState s, const double* fr) {
+  after_previous();
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const long n = d.n;
   if (t >= n * n) return;
@@ -564,6 +586,7 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __global__ void __cluster_dims__(kSolveBlocks, 1, 1) __launch_bounds__(1024) k_solve_refine(Dims d, DevState s) {
+  after_previous();
   const int n = d.n;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = warp * kSolveBlocks + blockIdx.x, rows = 32 * kSolveBlocks;
@@ -641,6 +664,7 @@ __global__ void __cluster_dims__(kSolveBlocks, 1, 1) __launch_bounds__(1024) k_s
 
 // ---- circulation solve (main.f90:522-603) ------------------------------------
 __global__ void k_rhs(Dims d, DevState s, const double* fr, int withWake) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.nbC * d.npan) return;
   const double* w = panRec(d, fr, t / d.npan, t % d.npan);
@@ -650,6 +674,7 @@ __global__ void k_rhs(Dims d, DevState s, const double* fr, int withWake) {
   s.RHS[t] = dot3(v, ld3(w + 15));
 }
 __global__ void k_solve(Dims d, DevState s) {
+  after_previous();
   const int n = d.n;
   if (d.axisym)
     for (int r = d.npan + threadIdx.x; r < n; r += blockDim.x) s.RHS[r] = s.RHS[r % d.npan];
@@ -766,6 +791,7 @@ __device__ void ring_sums(const Dims& d, const DevState& s, const double* fr, d3
 // rotor order + this rotor's wing (src/main.f90:636-652).
 __global__ void __launch_bounds__(kVcThreads) k_velcp_total(Dims d, DevState s, const double* fr, int sumChunk,
                                                             const double* fb, int nrs, int self) {
+  after_previous();
   extern __shared__ double sm[];
   __shared__ double bnd[3];
   const int t = blockIdx.x;
@@ -792,6 +818,7 @@ __global__ void __launch_bounds__(kVcThreads) k_velcp_total(Dims d, DevState s, 
 // (dt, frt), one block per point (a thread per point: 309 us at 16 panels).
 __global__ void __launch_bounds__(kVcThreads) k_bound_foreign(Dims dt, const double* frt, Dims ds, DevState ss,
                                                               const double* frs, double* out) {
+  after_previous();
   extern __shared__ double sm[];
   const int t = blockIdx.x;
   const d3 P = ld3(panRec(dt, frt, t / dt.npan, t % dt.npan) + 12);
@@ -802,7 +829,8 @@ __global__ void __launch_bounds__(kVcThreads) k_bound_foreign(Dims dt, const dou
 
 // ---- image rotors (src/classdef.f90:4990-5131) ------------------------------
 // rotor_mirrorVelCP: the source's velCP with the image-plane component negated
-__global__ void k_mirror_velcp(Dims d, DevState s, const double* __restrict__ src, int plane) {
+__global__ void k_mirror_velcp(Dims d, DevState s, const double* src, int plane) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.nb * d.npan) return;
   for (int c = 0; c < 3; ++c) {
@@ -811,7 +839,8 @@ __global__ void k_mirror_velcp(Dims d, DevState s, const double* __restrict__ sr
   }
 }
 // gamVecPrev = gamVec, rotor_mirrorGamma (gamVec = -source gamVec), map_gam
-__global__ void k_mirror_gamma(Dims d, DevState s, const double* __restrict__ src) {
+__global__ void k_mirror_gamma(Dims d, DevState s, const double* src) {
+  after_previous();
   for (int i = threadIdx.x; i < d.n; i += blockDim.x) {
     s.gamVecPrev[i] = s.gamVec[i];
     s.gamVec[i] = -1.0 * src[i];
@@ -828,6 +857,7 @@ __global__ void k_mirror_gamma(Dims d, DevState s, const double* __restrict__ sr
 // current wake; node coordinates in the image plane and circulation negated
 // (vr_mirror, Fwake_mirror: src/classdef.f90:722-735, 982-993)
 __global__ void k_mirror_wake(Dims d, DevState dst, DevState src, int mode, int rowNear, int rowFar, int plane) {
+  after_previous();
   const int r0 = mode == 2 ? 0 : rowNear - 1, f0 = mode == 2 ? 0 : rowFar - 1;
   const long nNear = (long)d.nb * (d.NW - r0) * d.ns;
   const long nFar = d.NF - f0 > 0 ? (long)d.nb * (d.NF - f0) : 0;
@@ -868,6 +898,7 @@ __global__ void k_mirror_wake(Dims d, DevState dst, DevState src, int mode, int 
 // src/main.f90:549-561, the wake of every rotor and the wing of the others,
 // one per-rotor sum per term); RHS = velCP . nCap
 __global__ void k_rhs_terms(Dims d, DevState s, const double* fr, const double* terms, int nterms, int M) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.nbC * d.npan) return;
   const double* w = panRec(d, fr, t / d.npan, t % d.npan);
@@ -956,6 +987,7 @@ struct Lsq2 {
 constexpr int kMaxNc = 64;
 
 __global__ void k_step_begin(Dims d, DevState s) {
+  after_previous();
   const int it = s.devIter[0] + 1;
   const double* src = s.frames + (size_t)it * d.fl.size;
   for (int i = threadIdx.x; i < d.fl.size; i += blockDim.x) s.curFrame[i] = src[i];
@@ -1016,6 +1048,7 @@ __device__ double c81_get(const double* T, int c, double alpha, double mach) {
 // sections of 4 panels.)  tmp: 9 doubles a panel.
 constexpr int kLoadsThreads = 512;
 __global__ void __launch_bounds__(kLoadsThreads) k_loads(Dims d, DevState s, const double* fr, int iter) {
+  after_previous();
   if (iter < 0) iter = s.devIter[0];
   const int nsec = d.nbC * d.ns, npan = d.nbC * d.npan;
   const double iGS = -1.0 * fsign1(d.omega);
@@ -1186,32 +1219,32 @@ __global__ void __launch_bounds__(kLoadsThreads) k_loads(Dims d, DevState s, con
 // ---------------------------------------------------------------------------
 void launch_shed(const Dims& d, const DevState& s, const double* frame, int rowNear, bool le, cudaStream_t st) {
   count_launch();
-  k_shed<<<nblk(d.nb * d.ns, 128), 128, 0, st>>>(d, s, frame, rowNear, le ? 1 : 0);
+  launch_next(k_shed, nblk(d.nb * d.ns, 128), 128, 0, st, d, s, frame, rowNear, le ? 1 : 0);
 }
 void launch_age(const Dims& d, const DevState& s, int rowNear, int rowFar, cudaStream_t st) {
   const long n = (long)d.nb * (d.NW - (rowNear - 1)) * d.ns + (long)d.nb * (d.NF - (rowFar - 1) > 0 ? d.NF - (rowFar - 1) : 0);
   if (n > 0) {
     count_launch();
-    k_age<<<nblk(n, 256), 256, 0, st>>>(d, s, rowNear, rowFar);
+    launch_next(k_age, nblk(n, 256), 256, 0, st, d, s, rowNear, rowFar);
   }
 }
 void launch_dissipate(const Dims& d, const DevState& s, int rowNear, int rowFar, cudaStream_t st) {
   const long n = (long)d.nb * (d.NW - (rowNear - 1)) * d.ns + (long)d.nb * (d.NF - (rowFar - 1) > 0 ? d.NF - (rowFar - 1) : 0);
   if (n > 0) {
     count_launch();
-    k_dissip_a<<<nblk(n, 256), 256, 0, st>>>(d, s, rowNear, rowFar);
+    launch_next(k_dissip_a, nblk(n, 256), 256, 0, st, d, s, rowNear, rowFar);
   }
   const long n2 = (long)d.nb * (d.NW - rowNear) * d.ns;
   if (n2 > 0) {
     count_launch();
-    k_dissip_b<<<nblk(n2, 256), 256, 0, st>>>(d, s, rowNear);
+    launch_next(k_dissip_b, nblk(n2, 256), 256, 0, st, d, s, rowNear);
   }
 }
 void launch_copy_predicted(const Dims& d, const DevState& s, int rowNear, int rowFar, cudaStream_t st) {
   const long n = (long)d.nbC * (d.NW - (rowNear - 1)) * d.ns + (long)d.nbC * (d.NF - (rowFar - 1) > 0 ? d.NF - (rowFar - 1) : 0);
   if (n > 0) {
     count_launch();
-    k_copy_pred<<<nblk(n, 256), 256, 0, st>>>(d, s, rowNear, rowFar);
+    launch_next(k_copy_pred, nblk(n, 256), 256, 0, st, d, s, rowNear, rowFar);
   }
 }
 void launch_convect(const Dims& d, const DevState& s, const double* frame, int rowNear, int rowFar, bool pred,
@@ -1220,18 +1253,18 @@ void launch_convect(const Dims& d, const DevState& s, const double* frame, int r
   const long n1 = (long)d.nbC * (pred ? 1 : d.NW - (rowNear - 1)) * (d.ns + 1) + (long)d.nbC * rowsF;
   if (n1 > 0) {
     count_launch();
-    k_shift<<<nblk(n1, 256), 256, 0, st>>>(d, s, rowNear, rowFar, pred ? 1 : 0);
+    launch_next(k_shift, nblk(n1, 256), 256, 0, st, d, s, rowNear, rowFar, pred ? 1 : 0);
   }
   const long n2 = (long)d.nbC * (d.NW - (rowNear - 1)) * d.ns + (long)d.nbC * (d.NF - rowFar > 0 ? d.NF - rowFar : 0);
   if (n2 > 0) {
     count_launch();
-    k_continuity<<<nblk(n2, 256), 256, 0, st>>>(d, s, rowNear, rowFar, pred ? 1 : 0);
+    launch_next(k_continuity, nblk(n2, 256), 256, 0, st, d, s, rowNear, rowFar, pred ? 1 : 0);
   }
   if (d.axisym && d.nb > 1) {
     const long n3 = (long)(d.nb - 1) * (d.NW - (rowNear - 1)) * d.ns + (long)(d.nb - 1) * rowsF;
     if (n3 > 0) {
       count_launch();
-      k_axisym<<<nblk(n3, 256), 256, 0, st>>>(d, s, frame, rowNear, rowFar, pred ? 1 : 0);
+      launch_next(k_axisym, nblk(n3, 256), 256, 0, st, d, s, frame, rowNear, rowFar, pred ? 1 : 0);
     }
   }
 }
@@ -1239,24 +1272,24 @@ void launch_presc_update(const Dims& d, const DevState& s, const double* frame, 
                          cudaStream_t st) {
   if (!s.pfC || d.NF - (rowFar - 1) < 1) return;
   count_launch();
-  k_presc_update<<<d.nbC, 256, 0, st>>>(d, s, frame, rowFar, pred ? 1 : 0);
+  launch_next(k_presc_update, d.nbC, 256, 0, st, d, s, frame, rowFar, pred ? 1 : 0);
   if (d.axisym && d.nb > 1) {
     count_launch();
-    k_presc_axisym<<<nblk((long)(d.nb - 1) * kPresc, 256), 256, 0, st>>>(d, s, frame, pred ? 1 : 0);
+    launch_next(k_presc_axisym, nblk((long)(d.nb - 1) * kPresc, 256), 256, 0, st, d, s, frame, pred ? 1 : 0);
   }
 }
 void launch_burst(const Dims& d, const DevState& s, int rowFar, cudaStream_t st) {
   const long n = (long)d.nb * (d.NF - (rowFar - 1) - 1);
   if (n > 0) {
     count_launch();
-    k_burst<<<nblk(n, 256), 256, 0, st>>>(d, s, rowFar);
+    launch_next(k_burst, nblk(n, 256), 256, 0, st, d, s, rowFar);
   }
 }
 void launch_strain(const Dims& d, const DevState& s, int rowFar, cudaStream_t st) {
   const long n = (long)d.nb * (d.NF - (rowFar - 1));
   if (n > 0) {
     count_launch();
-    k_strain<<<nblk(n, 256), 256, 0, st>>>(d, s, rowFar);
+    launch_next(k_strain, nblk(n, 256), 256, 0, st, d, s, rowFar);
   }
 }
 void launch_rollup(const Dims& d, const DevState& s, int rowFar, cudaStream_t st) {
@@ -1264,24 +1297,24 @@ void launch_rollup(const Dims& d, const DevState& s, int rowFar, cudaStream_t st
   if (d.NF > 0 && rowFarNext == 0) {
     const long n = (long)d.nb * d.NF;
     count_launch();
-    k_far_to_tmp<<<nblk(n, 256), 256, 0, st>>>(d, s);
+    launch_next(k_far_to_tmp, nblk(n, 256), 256, 0, st, d, s);
     count_launch();
-    k_far_from_tmp<<<nblk(n, 256), 256, 0, st>>>(d, s);
+    launch_next(k_far_from_tmp, nblk(n, 256), 256, 0, st, d, s);
     rowFarNext = 1;
   }
   count_launch();
-  k_rollup<<<nblk(d.nb, 32), 32, 0, st>>>(d, s, rowFarNext);
+  launch_next(k_rollup, nblk(d.nb, 32), 32, 0, st, d, s, rowFarNext);
   const long n = (long)d.nb * d.NW * d.ns;
   count_launch();
-  k_near_to_tmp<<<nblk(n, 256), 256, 0, st>>>(d, s);
+  launch_next(k_near_to_tmp, nblk(n, 256), 256, 0, st, d, s);
   count_launch();
-  k_near_from_tmp<<<nblk(n, 256), 256, 0, st>>>(d, s);
+  launch_next(k_near_from_tmp, nblk(n, 256), 256, 0, st, d, s);
 }
 void launch_velop(const Dims& d, const DevState& s, VelOp op, cudaStream_t st) {
   const long nN = (long)d.nbC * d.NW * (d.ns + 1) * 3, nF = (long)d.nbC * d.NF * 3;
   if (nN + nF > 0) {
     count_launch();
-    k_velop<<<nblk(nN + nF, 256), 256, 0, st>>>(s, nN, nF, (int)op);
+    launch_next(k_velop, nblk(nN + nF, 256), 256, 0, st, s, nN, nF, (int)op);
   }
 }
 void launch_order2(const Dims& d, const DevState& s, int rowNear, int rowFar, cudaStream_t st) {
@@ -1289,9 +1322,9 @@ void launch_order2(const Dims& d, const DevState& s, int rowNear, int rowFar, cu
                  (long)d.nbC * (d.NF - (rowFar - 1) > 0 ? d.NF - (rowFar - 1) : 0) * 3;
   if (n <= 0) return;
   count_launch();
-  k_order2<<<nblk(n, 256), 256, 0, st>>>(d, s, rowNear, rowFar, 0);
+  launch_next(k_order2, nblk(n, 256), 256, 0, st, d, s, rowNear, rowFar, 0);
   count_launch();
-  k_order2<<<nblk(n, 256), 256, 0, st>>>(d, s, rowNear, rowFar, 1);
+  launch_next(k_order2, nblk(n, 256), 256, 0, st, d, s, rowNear, rowFar, 1);
 }
 int node_target_count(const Dims& d, int rowNear, int rowFar) {
   const int rowsN = d.NW - (rowNear - 1);
@@ -1302,44 +1335,45 @@ void launch_scatter_nodes(const Dims& d, const DevState& s, const double* frame,
                           double initWakeVel, cudaStream_t st) {
   const int M = node_target_count(d, rowNear, rowFar);
   const int addInit = initWakeVel != 0.0 ? 1 : 0;
-  if (M > 0)
+  if (M > 0) {
     count_launch();
-    k_scatter_nodes<<<nblk(M, 256), 256, 0, st>>>(d, s, frame, rowNear, rowFar, pred ? 1 : 0, initWakeVel, addInit, M);
+    launch_next(k_scatter_nodes, nblk(M, 256), 256, 0, st, d, s, frame, rowNear, rowFar, pred ? 1 : 0, initWakeVel, addInit, M);
+  }
 }
 void launch_aic(const Dims& d, const DevState& s, const double* frame, cudaStream_t st) {
   const long n = (long)d.n * d.n;
   count_launch();
-  k_aic<<<nblk(n, 128), 128, 0, st>>>(d, s, frame);
+  launch_next(k_aic, nblk(n, 128), 128, 0, st, d, s, frame);
 }
 static void solve_refine(const Dims& d, const DevState& s, cudaStream_t st) {
   const size_t smem = solve_smem(d.n);
   if (smem > 40 * 1024)
     cudaFuncSetAttribute(k_solve_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_smem(8192));
-  k_solve_refine<<<kSolveBlocks, 1024, smem, st>>>(d, s);
+  launch_next(k_solve_refine, kSolveBlocks, 1024, smem, st, d, s);
 }
 void launch_solve(const Dims& d, const DevState& s, const double* frame, bool withWake, cudaStream_t st) {
   count_launch();
-  k_rhs<<<nblk(d.nbC * d.npan, 128), 128, 0, st>>>(d, s, frame, withWake ? 1 : 0);
+  launch_next(k_rhs, nblk(d.nbC * d.npan, 128), 128, 0, st, d, s, frame, withWake ? 1 : 0);
   count_launch();
   if (s.LU32) solve_refine(d, s, st);
-  else k_solve<<<1, 1024, 0, st>>>(d, s);
+  else launch_next(k_solve, 1, 1024, 0, st, d, s);
 }
 void launch_step_begin(const Dims& d, const DevState& s, cudaStream_t st) {
   count_launch();
-  k_step_begin<<<1, 256, 0, st>>>(d, s);
+  launch_next(k_step_begin, 1, 256, 0, st, d, s);
 }
 void launch_rhs_terms(const Dims& d, const DevState& s, const double* frame, const double* terms, int nterms,
                       cudaStream_t st) {
   count_launch();
-  k_rhs_terms<<<nblk(d.nbC * d.npan, 128), 128, 0, st>>>(d, s, frame, terms, nterms, d.nbC * d.npan);
+  launch_next(k_rhs_terms, nblk(d.nbC * d.npan, 128), 128, 0, st, d, s, frame, terms, nterms, d.nbC * d.npan);
 }
 void launch_mirror_velcp(const Dims& d, const DevState& s, const double* srcVelCP, int plane, cudaStream_t st) {
   count_launch();
-  k_mirror_velcp<<<nblk(d.nb * d.npan, 128), 128, 0, st>>>(d, s, srcVelCP, plane);
+  launch_next(k_mirror_velcp, nblk(d.nb * d.npan, 128), 128, 0, st, d, s, srcVelCP, plane);
 }
 void launch_mirror_gamma(const Dims& d, const DevState& s, const double* srcGamVec, cudaStream_t st) {
   count_launch();
-  k_mirror_gamma<<<1, 1024, 0, st>>>(d, s, srcGamVec);
+  launch_next(k_mirror_gamma, 1, 1024, 0, st, d, s, srcGamVec);
 }
 void launch_mirror_wake(const Dims& d, const DevState& dst, const DevState& src, int mode, int rowNear, int rowFar,
                         int plane, cudaStream_t st) {
@@ -1347,12 +1381,12 @@ void launch_mirror_wake(const Dims& d, const DevState& dst, const DevState& src,
   const long n = (long)d.nb * (d.NW - r0) * d.ns + (d.NF - f0 > 0 ? (long)d.nb * (d.NF - f0) : 0);
   if (n <= 0) return;
   count_launch();
-  k_mirror_wake<<<nblk(n, 256), 256, 0, st>>>(d, dst, src, mode, rowNear, rowFar, plane);
+  launch_next(k_mirror_wake, nblk(n, 256), 256, 0, st, d, dst, src, mode, rowNear, rowFar, plane);
 }
 void launch_solve_only(const Dims& d, const DevState& s, cudaStream_t st) {
   count_launch();
   if (s.LU32) solve_refine(d, s, st);
-  else k_solve<<<1, 1024, 0, st>>>(d, s);
+  else launch_next(k_solve, 1, 1024, 0, st, d, s);
 }
 // shared memory for up to 8192 stations (the most panels a rotor has)
 static void velcp_attr() {
@@ -1369,15 +1403,15 @@ void launch_bound_foreign(const Dims& dt, const double* frameT, const Dims& ds, 
                           const double* frameS, double* out, cudaStream_t st) {
   count_launch();
   velcp_attr();
-  k_bound_foreign<<<dt.nbC * dt.npan, kVcThreads, velcp_smem(ds.ns), st>>>(dt, frameT, ds, ss, frameS, out);
+  launch_next(k_bound_foreign, dt.nbC * dt.npan, kVcThreads, velcp_smem(ds.ns), st, dt, frameT, ds, ss, frameS, out);
 }
 void launch_loads(const Dims& d, const DevState& s, const double* frame, int sumChunk, int iter, cudaStream_t st,
                   const double* foreignBound, int nrs, int self) {
   count_launch();
   velcp_attr();
-  k_velcp_total<<<d.nbC * d.npan, kVcThreads, velcp_smem(d.ns), st>>>(d, s, frame, sumChunk, foreignBound, nrs, self);
+  launch_next(k_velcp_total, d.nbC * d.npan, kVcThreads, velcp_smem(d.ns), st, d, s, frame, sumChunk, foreignBound, nrs, self);
   count_launch();
-  k_loads<<<1, kLoadsThreads, 0, st>>>(d, s, frame, iter);
+  launch_next(k_loads, 1, kLoadsThreads, 0, st, d, s, frame, iter);
 }
 
 }  // namespace vlm

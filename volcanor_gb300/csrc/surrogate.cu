@@ -13,6 +13,7 @@
 // treat as inner targets; the case passes 0.)
 #include <cuda_runtime.h>
 
+#include "launch.h"
 #include "vlm_math.h"
 #include "vlm_solver.h"
 
@@ -37,6 +38,7 @@ __device__ __forceinline__ size_t ringI(const Dims& d, int b, int i, int j) {
 // `young` youngest far-wake nodes, in the node evaluations' order
 __global__ void k_surr_targets(Dims d, DevState s, const double* fr, int rowNear, int rowFar, int young, int stride,
                                int offset, int nNodes, double* P) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int ncp = d.nbC * d.npan;
   if (t >= ncp + nNodes) return;
@@ -64,6 +66,7 @@ __global__ void k_surr_targets(Dims d, DevState s, const double* fr, int rowNear
 // old far-wake nodes (rows rowFar + young .. NF) of the convecting blades,
 // blade-major, oldest last
 __global__ void k_surr_far_targets(Dims d, DevState s, int rowFar, int young, int pred, double* P) {
+  after_previous();
   const int rowsF = d.NF - (rowFar - 1);
   const int nOld = rowsF - young;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -81,6 +84,7 @@ __global__ void k_surr_far_targets(Dims d, DevState s, int rowFar, int young, in
 // desc[3] = its mean |circulation| over the wing's largest |circulation|.
 __global__ void k_surr_descriptor(Dims d, DevState s, const double* fr, int rowFar, int young, int pred, double invR,
                                   double* desc) {
+  after_previous();
   __shared__ double red[4][256];
   const double* rot = fr + d.fl.rot;
   const double* fc = pred ? s.fCP : s.fC;
@@ -128,6 +132,7 @@ __global__ void k_surr_descriptor(Dims d, DevState s, const double* fr, int rowF
 // descriptor (centroid about the hub / R, relative mean |circulation|)
 __global__ void k_surr_features(Dims d, const double* fr, const double* P, int M, double invR, double fill,
                                 const double* desc, float* X) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= M) return;
   const double* rot = fr + d.fl.rot;
@@ -155,6 +160,7 @@ __global__ void k_surr_features(Dims d, const double* fr, const double* P, int M
 
 // outv[m] += scale * Y[m] for m < M
 __global__ void k_surr_add(int M, const float* Y, const double* scale, double* outv) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= M) return;
   const double sc = scale[0];
@@ -166,6 +172,7 @@ __global__ void k_surr_add(int M, const float* Y, const double* scale, double* o
 // sum of the old-far-target evaluation
 __global__ void k_surr_merge_nodes(Dims d, int rowNear, int rowFar, int young, int M, const float* Y,
                                    const double* scale, const double* outFar, double* outv) {
+  after_previous();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= M) return;
   const int rowsN = d.NW - (rowNear - 1);
@@ -184,6 +191,7 @@ __global__ void k_surr_merge_nodes(Dims d, int rowNear, int rowFar, int young, i
 
 // training samples: X rows as they are, T = direct far-wake velocity (FP32)
 __global__ void k_surr_append(int n, const float* Xs, const double* V, float* X, float* T) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   for (int k = 0; k < kSurrFeatures; ++k) X[(size_t)t * kSurrFeatures + k] = Xs[(size_t)t * kSurrFeatures + k];
@@ -193,6 +201,7 @@ __global__ void k_surr_append(int n, const float* Xs, const double* V, float* X,
 // audit sums (one block, fixed order): out[0] = sum |scale Y - V|^2,
 // out[1] = sum |V|^2
 __global__ void k_surr_audit(int n, const float* Y, const double* scale, const double* V, double* out) {
+  after_previous();
   __shared__ double r0[256], r1[256];
   double a = 0.0, b = 0.0;
   const double sc = scale[0];
@@ -226,42 +235,42 @@ void launch_surr_targets(const Dims& d, const DevState& s, const double* fr, int
   const int n = d.nbC * d.npan + nNodes;
   if (n <= 0) return;
   count_launch();
-  k_surr_targets<<<nblk(n, 256), 256, 0, st>>>(d, s, fr, rowNear, rowFar, young, stride, offset, nNodes, P);
+  launch_next(k_surr_targets, nblk(n, 256), 256, 0, st, d, s, fr, rowNear, rowFar, young, stride, offset, nNodes, P);
 }
 void launch_surr_far_targets(const Dims& d, const DevState& s, int rowFar, int young, bool pred, double* P,
                              cudaStream_t st) {
   const int n = d.nbC * (d.NF - (rowFar - 1) - young);
   if (n <= 0) return;
   count_launch();
-  k_surr_far_targets<<<nblk(n, 256), 256, 0, st>>>(d, s, rowFar, young, pred ? 1 : 0, P);
+  launch_next(k_surr_far_targets, nblk(n, 256), 256, 0, st, d, s, rowFar, young, pred ? 1 : 0, P);
 }
 void launch_surr_features(const Dims& d, const DevState& s, const double* fr, const double* P, int M, double invR,
                           double fill, int rowFar, int young, bool pred, double* desc, float* X, cudaStream_t st) {
   if (M <= 0) return;
   count_launch();
-  k_surr_descriptor<<<1, 256, 0, st>>>(d, s, fr, rowFar, young, pred ? 1 : 0, invR, desc);
+  launch_next(k_surr_descriptor, 1, 256, 0, st, d, s, fr, rowFar, young, pred ? 1 : 0, invR, desc);
   count_launch();
-  k_surr_features<<<nblk(M, 256), 256, 0, st>>>(d, fr, P, M, invR, fill, desc, X);
+  launch_next(k_surr_features, nblk(M, 256), 256, 0, st, d, fr, P, M, invR, fill, desc, X);
 }
 void launch_surr_add(int M, const float* Y, const double* scale, double* outv, cudaStream_t st) {
   if (M <= 0) return;
   count_launch();
-  k_surr_add<<<nblk(M, 256), 256, 0, st>>>(M, Y, scale, outv);
+  launch_next(k_surr_add, nblk(M, 256), 256, 0, st, M, Y, scale, outv);
 }
 void launch_surr_merge_nodes(const Dims& d, int rowNear, int rowFar, int young, int M, const float* Y,
                              const double* scale, const double* outFar, double* outv, cudaStream_t st) {
   if (M <= 0) return;
   count_launch();
-  k_surr_merge_nodes<<<nblk(M, 256), 256, 0, st>>>(d, rowNear, rowFar, young, M, Y, scale, outFar, outv);
+  launch_next(k_surr_merge_nodes, nblk(M, 256), 256, 0, st, d, rowNear, rowFar, young, M, Y, scale, outFar, outv);
 }
 void launch_surr_append(int n, const float* Xs, const double* V, float* X, float* T, cudaStream_t st) {
   if (n <= 0) return;
   count_launch();
-  k_surr_append<<<nblk(n, 256), 256, 0, st>>>(n, Xs, V, X, T);
+  launch_next(k_surr_append, nblk(n, 256), 256, 0, st, n, Xs, V, X, T);
 }
 void launch_surr_audit(int n, const float* Y, const double* scale, const double* V, double* out, cudaStream_t st) {
   count_launch();
-  k_surr_audit<<<1, 256, 0, st>>>(n, Y, scale, V, out);
+  launch_next(k_surr_audit, 1, 256, 0, st, n, Y, scale, V, out);
 }
 
 }  // namespace vlm
