@@ -343,9 +343,6 @@ __device__ __forceinline__ void rec_lat_packed(const float4* __restrict__ R4, co
 // per SM) are template arguments; kPartial32Shapes lists the compiled ones,
 // among which the case autotuner picks per evaluation.
 constexpr int kTileW = 128;                 // records per stage (24 KB)
-// evaluations with at most this many targets (and at most 2^22 record-target
-// pairs) find their near pairs by testing every pair (k_near_find_small)
-constexpr int kNearSmallTargets = 1024;
 constexpr int kConsumerWarps = 8;
 constexpr int kBlockW = (kConsumerWarps + 1) * 32;
 
@@ -701,6 +698,99 @@ __device__ __forceinline__ d3 fil_near64(d3 p, d3 a, d3 b, double rvc) {
   return c * (d * rsqrt(s2 * s2 + c2 * c2) * kInv4Pi);
 }
 
+// Near pairs of a small evaluation (collocation points, the moved targets of an
+// incremental one): every filament against every target, two filaments a
+// thread (edges k and k + 2 of a record, of which a lattice record has only the
+// first) and up to kNearTile targets of shared memory a block (fewer while that
+// leaves SMs without one) -- the same pairs as k_near_find's without a grid of
+// the targets.  Bound by FP32 issue, about 16 instructions a test, so it stays
+// below the grid's chain of eight launches (45 us and the walk) up to
+// kNearSmallPairs record-target pairs.  It took the grid's place for the moved
+// targets of a hover step (12500 records, 512 targets; 8 steps 7.24 -> 7.02 ms
+// with k_combine_tree), and a thread per record-target pair's for collocation
+// points.  A block's pairs are gathered in shared memory and appended with one
+// atomic; an atomic of global memory for each warp and target with a pair took
+// longer than the tests (8 coaxial rotor-steps 2.86 ms, now 2.43).
+constexpr int kNearTile = 64;
+constexpr int kNearBuf = 768;
+constexpr size_t kNearSmallPairs = (size_t)1 << 24;
+__global__ void __launch_bounds__(256) k_near_find_small(const float* rec32, int nrec, const Chunk* chunks, int nchunks,
+                                                         const double* P, int M, int tile, int tiles, NearPair* near,
+                                                         int near_cap, int* ctl) {
+  after_previous();
+  __shared__ float4 target[kNearTile];
+  __shared__ NearPair buf[kNearBuf];
+  __shared__ int found, slot0;
+  const int m0 = (int)(blockIdx.x % tiles) * tile, nt = min(tile, M - m0);
+  if (threadIdx.x == 0) found = 0;
+  if ((int)threadIdx.x < nt) {
+    const double* p = P + 3 * (size_t)(m0 + threadIdx.x);
+    target[threadIdx.x] = make_float4((float)p[0], (float)p[1], (float)p[2], 0.f);
+  }
+  __syncthreads();
+  const size_t t = (blockIdx.x / tiles) * (size_t)blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const bool live = t < 2 * (size_t)nrec;
+  const int r = live ? (int)(t >> 1) : 0;
+  const float* R = rec32 + (size_t)r * kRec32;
+  auto chunk_of = [&](int rec) {
+    int lo = 0, hi = nchunks - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (chunks[mid].rec_begin <= rec) lo = mid;
+      else hi = mid - 1;
+    }
+    return lo;
+  };
+  auto append = [&](NearPair np_, int slot) {
+    np_.q = chunk_of(np_.rec);
+    if (slot < near_cap) near[slot] = np_;
+    else atomicExch(ctl, 3);
+  };
+  for (int k = (int)(t & 1); k < 4; k += 2) {
+    const float thr = R[32 + k];
+    const int j = (k + 1) & 3;
+    const float ax = R[3 * k], ay = R[3 * k + 1], az = R[3 * k + 2];
+    const float ex = R[3 * j] - ax, ey = R[3 * j + 1] - ay, ez = R[3 * j + 2] - az;
+    const float ee = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+    const bool active = live && thr >= 0.f && ee > 0.f && R[24 + k] != 0.f;
+    if (!__any_sync(kFull, active)) continue;
+    const float len = sqrtf(ee);
+    const float z = sqrtf(thr) / len;
+    const float iee = 1.f / ee, z2 = active ? z * z : -1.f, tlo = -z * len, thi = fmaf(z, len, ee);
+    for (int i = 0; i < nt; ++i) {
+      const float4 p = target[i];
+      const float dx = p.x - ax, dy = p.y - ay, dz = p.z - az;
+      const float tr = fmaf(dx, ex, fmaf(dy, ey, dz * ez));
+      const float tn = tr * iee;
+      const float qx = fmaf(-tn, ex, dx), qy = fmaf(-tn, ey, dy), qz = fmaf(-tn, ez, dz);
+      const bool isnear = fmaf(qx, qx, fmaf(qy, qy, qz * qz)) < z2 && tr > tlo && tr < thi;
+      const unsigned mask = __ballot_sync(kFull, isnear);
+      if (mask) {
+        int base = 0;
+        if (lane == 0) base = atomicAdd(&found, __popc(mask));
+        base = __shfl_sync(kFull, base, 0);
+        if (isnear) {
+          NearPair np_;
+          np_.m = m0 + i;
+          np_.q = 0;
+          np_.rec = r;
+          np_.k = k;
+          const int at = base + __popc(mask & lt);
+          if (at < kNearBuf) buf[at] = np_;
+          else append(np_, atomicAdd(ctl + 1, 1));
+        }
+      }
+    }
+  }
+  __syncthreads();
+  const int n = min(found, kNearBuf);
+  if (threadIdx.x == 0 && n) slot0 = atomicAdd(ctl + 1, n);
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) append(buf[i], slot0 + i);
+}
+
 // Detection, one warp per filament (record r, edge k).  A filament with a near zone
 // (radius z = near_factor rvc_k, from [32 + k]) is cut into np pieces no
 // longer than a cell; the lanes take the cells of each piece's box (grown by
@@ -714,74 +804,6 @@ __device__ __forceinline__ d3 fil_near64(d3 p, d3 a, d3 b, double rvc) {
 // near_factor rvc, on the FP32 kernel's own FP32 values -- is appended to the
 // near list (one atomic per warp and batch; ctl[1] counts, ctl[0] = 3 if the
 // list is full).
-// Near pairs of an evaluation with few targets (the collocation points):
-// every (record, target) pair gets k_near_find's test directly, one thread
-// per pair -- the same pairs without building a grid of the targets or
-// walking every filament through it.
-__global__ void __launch_bounds__(256) k_near_find_small(const float* rec32, int nrec,
-                                                         const Chunk* chunks, int nchunks,
-                                                         const double* P, int M,
-                                                         NearPair* near, int near_cap,
-                                                         int* ctl) {
-  after_previous();
-  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  const bool live = t < (size_t)nrec * M;
-  const int r = live ? (int)(t / M) : 0, m = live ? (int)(t % M) : 0;
-  const float px = (float)P[3 * (size_t)m], py = (float)P[3 * (size_t)m + 1], pz = (float)P[3 * (size_t)m + 2];
-  const float* R = rec32 + (size_t)r * kRec32;
-  int q = 0;
-  {
-    int hi = nchunks - 1;
-    while (q < hi) {
-      const int mid = (q + hi + 1) >> 1;
-      if (chunks[mid].rec_begin <= r) q = mid;
-      else hi = mid - 1;
-    }
-  }
-  for (int k = 0; k < 4; ++k) {
-    bool isnear = false;
-    const float thr = R[32 + k];
-    if (live && thr >= 0.f) {
-      const int j = (k + 1) & 3;
-      const float ax = R[3 * k], ay = R[3 * k + 1], az = R[3 * k + 2];
-      const float ex = R[3 * j] - ax, ey = R[3 * j + 1] - ay, ez = R[3 * j + 2] - az;
-      const float eev = R[24 + k];
-      const float ee = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-      if (ee > 0.f && eev != 0.f) {
-        const float len = sqrtf(ee);
-        const float z = sqrtf(thr) / len;
-        const float iee = 1.f / ee, z2 = z * z, tlo = -z * len, thi = fmaf(z, len, ee);
-        const float dx = px - ax, dy = py - ay, dz = pz - az;
-        const float tr = fmaf(dx, ex, fmaf(dy, ey, dz * ez));
-        const float tn = tr * iee;
-        const float qx = fmaf(-tn, ex, dx), qy = fmaf(-tn, ey, dy), qz = fmaf(-tn, ez, dz);
-        isnear = fmaf(qx, qx, fmaf(qy, qy, qz * qz)) < z2 && tr > tlo && tr < thi;
-      }
-    }
-    const unsigned mask = __ballot_sync(kFull, isnear);
-    if (mask) {
-      int base_slot = 0;
-      if (lane == 0) base_slot = atomicAdd(ctl + 1, __popc(mask));
-      base_slot = __shfl_sync(kFull, base_slot, 0);
-      if (isnear) {
-        const int slot = base_slot + __popc(mask & lt);
-        if (slot < near_cap) {
-          NearPair np_;
-          np_.m = m;
-          np_.q = q;
-          np_.rec = r;
-          np_.k = k;
-          near[slot] = np_;
-        } else {
-          atomicExch(ctl, 3);
-        }
-      }
-    }
-  }
-}
-
 __global__ void __launch_bounds__(256, 4) k_near_find(const float* rec32, int nrec,
                                                    const Chunk* chunks, int nchunks,
                                                    const double* P, int M,
@@ -1072,7 +1094,7 @@ int partial32_targets_per_block(int shape) { return kConsumerWarps * 32 * (shape
 void launch_partial32(const float* rec32, const double* rec64, const Chunk* chunks, int nchunks, int nrec,
                       const double* P, int M, double* part, int* ctl, void* near_scratch, size_t near_bytes,
                       long long* nacc, cudaStream_t s, const double* ew, int shape, const NearOverlap* ov,
-                      bool reuse_grid) {
+                      int grid_records) {
   if (M <= 0 || nchunks <= 0) return;
   ensure_smem_attrs();
   const int tpb = partial32_targets_per_block(shape);
@@ -1105,11 +1127,14 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
   const GridLayout L = grid_layout(M);
   const int T = grid_buckets(M);
   const int sms = device_sm_count();
-  if (M <= kNearSmallTargets && (size_t)nrec * M <= ((size_t)1 << 22)) {
-    // few targets: every pair tested directly
+  if ((size_t)std::max(nrec, grid_records) * M <= kNearSmallPairs) {
     count_launches(2);
-    launch_next(k_near_find_small, (unsigned)(((size_t)nrec * M + 255) / 256), 256, 0, ns, rec32, nrec, chunks, nchunks, P, M,
-                                                                                   list, cap, ctl);
+    const size_t rb = (2 * (size_t)nrec + 255) / 256;
+    int tile = kNearTile;
+    auto tiles = [&]() { return ((size_t)M + tile - 1) / tile; };
+    while (tile > 8 && tiles() * rb < 2 * (size_t)sms) tile >>= 1;
+    launch_next(k_near_find_small, (unsigned)(tiles() * rb), 256, 0, ns, rec32, nrec, chunks, nchunks, P, M, tile,
+                (int)tiles(), list, cap, ctl);
     launch_next(k_near_fix, 4 * sms, 128, 0, ns, list, cap, rec32, rec64, ew, P, M,
                                         reinterpret_cast<unsigned long long*>(nacc), ctl);
     if (ns != s) {
@@ -1118,7 +1143,7 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
     }
     return;
   }
-  if (!reuse_grid) {
+  if (grid_records == 0) {
     count_launches(5);
     launch_next(k_grid_init, 1, 1, 0, ns, g, T);
     launch_next(k_zone_mean, (nrec + 255) / 256, 256, 0, ns, rec32, nrec, g);

@@ -331,74 +331,39 @@ Tile64 pick_tile64(int M, int nchunks, int64_t nrec, int L, int sms) {
   return T;
 }
 
-// One component of a target's chunk partials -> group sums -> the result, a
-// thread (ORDERED) or G lanes per (target, component).
-//
-// ORDERED (FP64): each group's partials in chunk order, loads 16 at a time (a
-// collocation-point evaluation has few targets and hundreds of chunks).
-// Else (FP32 paths, whose summation order is free): G a power of two <= 32;
-// lane l adds partials l, l + G, ... in order, then a butterfly over the G
-// lanes.  The tree has a fixed shape, so the result is reproducible run to
-// run.  nacc: the near field's fixed-point corrections of the same partials,
-// folded in on the way and zeroed (a pass of their own over the partials before).
-// (One lane's 3 components in turn were 16 us at 16 targets, an FP64 addition
-// being 64 cycles; each component has its own lanes now.)
-template <bool ORDERED>
-__device__ __forceinline__ double group_sum(const double* __restrict__ part, long long* __restrict__ nacc, int M,
-                                            const Group& g, size_t mc, int l, int G, bool live) {
+// FP64: each group's partials in chunk order, one component of a target a
+// thread, loads 16 at a time (a collocation-point evaluation has few targets
+// and hundreds of chunks).
+__device__ __forceinline__ double group_sum(const double* part, int M, const Group& g, size_t mc) {
   const size_t stride = 3 * (size_t)M;
   double s = 0.0;
-  if (ORDERED) {
-    const double* p = part + g.chunk_begin * stride + mc;
-    int q = 0;
-    constexpr int kB = 16;
-    for (; q + kB <= g.chunk_count; q += kB, p += kB * stride) {
-      double buf[kB];
+  const double* p = part + g.chunk_begin * stride + mc;
+  int q = 0;
+  constexpr int kB = 16;
+  for (; q + kB <= g.chunk_count; q += kB, p += kB * stride) {
+    double buf[kB];
 #pragma unroll
-      for (int i = 0; i < kB; ++i) buf[i] = p[i * stride];
+    for (int i = 0; i < kB; ++i) buf[i] = p[i * stride];
 #pragma unroll
-      for (int i = 0; i < kB; ++i) s = s + buf[i];
-    }
-    for (; q < g.chunk_count; ++q, p += stride) s = s + p[0];
-    return s;
+    for (int i = 0; i < kB; ++i) s = s + buf[i];
   }
-  if (live)
-    for (int q = g.chunk_begin + l; q < g.chunk_begin + g.chunk_count; q += G) {
-      double p = part[q * stride + mc];
-      if (nacc) {
-        const long long a = nacc[q * stride + mc];
-        if (a != 0) {
-          p += (double)a * (1.0 / kNearScale);
-          nacc[q * stride + mc] = 0;
-        }
-      }
-      s = s + p;
-    }
-  for (int o = G >> 1; o > 0; o >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, o, G);
+  for (; q < g.chunk_count; ++q, p += stride) s = s + p[0];
   return s;
 }
 
 // mode 0 (wake nodes): out = 0 + (wing + wake); 1: wake; 2: wing + wake.
-// ADD: out = out + that.
-template <bool ORDERED, bool ADD>
-__global__ void k_combine(const double* part, long long* nacc, int M,
-                          const Group* groups, int ngroups, int mode, int G, double* out) {
+__global__ void k_combine(const double* part, int M, const Group* groups, int ngroups, int mode, double* out) {
   after_previous();
-  const size_t gt = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  const size_t mc = gt / G;
-  const int l = (int)(gt % G);
-  const bool live = mc < 3 * (size_t)M;  // dead lanes still take part in the shuffles
-  if (ORDERED && !live) return;
+  const size_t mc = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (mc >= 3 * (size_t)M) return;
   double wing = 0.0, wake = 0.0;
   for (int g = 0; g < ngroups; ++g) {
     const Group gr = groups[g];
-    const double s = group_sum<ORDERED>(part, nacc, M, gr, mc, l, G, live);
+    const double s = group_sum(part, M, gr, mc);
     if (gr.kind == 0) wing = wing + s;
     else wake = wake + s;
   }
-  if (!live || l != 0) return;
-  const double v = mode == 0 ? 0.0 + (wing + wake) : mode == 1 ? wake : wing + wake;
-  out[mc] = ADD ? out[mc] + v : v;
+  out[mc] = mode == 0 ? 0.0 + (wing + wake) : mode == 1 ? wake : wing + wake;
 }
 
 // Coupled rotors: the groups carry the index of the sum they belong to
@@ -409,21 +374,15 @@ __global__ void k_combine(const double* part, long long* nacc, int M,
 // out[t][m] = 0 + the term's groups in order, one per-rotor wake or wing
 // sum each, which the RHS adds to velCP in turn.  With a single term, mode 0
 // equals k_combine's mode 0 bit for bit.
-template <bool ORDERED>
-__global__ void k_combine_terms(const double* part, long long* nacc, int M,
-                                const Group* groups, int ngroups, int mode, int G,
-                                double* out) {
+__global__ void k_combine_terms(const double* part, int M, const Group* groups, int ngroups, int mode, double* out) {
   after_previous();
-  const size_t gt = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  const size_t mc = gt / G;
-  const int l = (int)(gt % G);
-  const bool live = mc < 3 * (size_t)M;
-  if (ORDERED && !live) return;
+  const size_t mc = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (mc >= 3 * (size_t)M) return;
   double v = 0.0, wing = 0.0, wake = 0.0, ts = 0.0;
   int t = groups[0].term;
   auto done = [&]() {
     if (mode == 0) v = v + (wing + wake);
-    else if (live && l == 0) out[3 * (size_t)M * t + mc] = ts;
+    else out[3 * (size_t)M * t + mc] = ts;
     wing = wake = ts = 0.0;
   };
   for (int g = 0; g < ngroups; ++g) {
@@ -432,19 +391,85 @@ __global__ void k_combine_terms(const double* part, long long* nacc, int M,
       done();
       t = gr.term;
     }
-    const double s = group_sum<ORDERED>(part, nacc, M, gr, mc, l, G, live);
+    const double s = group_sum(part, M, gr, mc);
     if (mode != 0) ts = ts + s;
     else if (gr.kind == 0) wing = wing + s;
     else wake = wake + s;
   }
   done();
-  if (mode == 0 && live && l == 0) out[mc] = v;
+  if (mode == 0) out[mc] = v;
+}
+
+// FP32 paths, whose summation order is free: the partials of a target
+// component, whatever their group, over G lanes (a power of two <= 32; lane l
+// adds chunks l, l + G, ...), then a butterfly; the tree has a fixed shape, so
+// the result is reproducible run to run.  nacc: the near field's fixed-point
+// corrections of the same partials, zeroed on the way and added as the integers
+// that they are, with one conversion at the end (those of 64 and more, of
+// which a lane's few thousand could overflow, one by one): conversions and
+// additions run on the FP64 unit, 16 cycles a warp and SM, and bound the kernel.
+// Group by group, each with its own butterfly and a conversion a partial, 13500
+// targets of 24 chunks took 33 us, now 15; 48 of 300 took 12, now 7.  mode 3: term blockIdx.y's groups alone, into its part of out; mode 1
+// leaves the wings' chunks out.
+template <bool ADD>
+__global__ void __launch_bounds__(256) k_combine_tree(const double* part, long long* nacc, int M, const Group* groups,
+                                                      int ngroups, int mode, int G, double* out) {
+  after_previous();
+  const size_t gt = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const size_t mc = gt / G, stride = 3 * (size_t)M;
+  const int l = (int)(gt % G);
+  const bool live = mc < stride;  // dead lanes still take part in the shuffles
+  double s = 0.0;
+  long long sum = 0;
+  auto range = [&](int a, int b, bool use) {
+    constexpr int kB = 4;
+    for (int q = a + l; q < b; q += kB * G) {
+      double p[kB];
+      long long n[kB];
+#pragma unroll
+      for (int i = 0; i < kB; ++i) {
+        const bool in = q + i * G < b;
+        p[i] = in && use ? part[(q + i * G) * stride + mc] : 0.0;
+        n[i] = in && nacc ? nacc[(q + i * G) * stride + mc] : 0;
+      }
+#pragma unroll
+      for (int i = 0; i < kB; ++i) {
+        if (q + i * G < b) s = s + p[i];
+        if (n[i] != 0) {
+          nacc[(q + i * G) * stride + mc] = 0;
+          if (!use) continue;
+          constexpr long long kBig = (long long)1 << 50;
+          if ((unsigned long long)(n[i] + kBig) < 2ull * kBig) sum += n[i];
+          else s = s + (double)n[i] * (1.0 / kNearScale);
+        }
+      }
+    }
+  };
+  if (live) {
+    int g0 = 0, g1 = ngroups;
+    if (mode == 3) {
+      while (g0 < ngroups && groups[g0].term < (int)blockIdx.y) ++g0;
+      g1 = g0;
+      while (g1 < ngroups && groups[g1].term == (int)blockIdx.y) ++g1;
+    }
+    if (mode == 1) {
+      for (int g = g0; g < g1; ++g)
+        range(groups[g].chunk_begin, groups[g].chunk_begin + groups[g].chunk_count, groups[g].kind != 0);
+    } else if (g0 < g1) {
+      range(groups[g0].chunk_begin, groups[g1 - 1].chunk_begin + groups[g1 - 1].chunk_count, true);
+    }
+  }
+  if (sum != 0) s = s + (double)sum * (1.0 / kNearScale);
+  for (int o = G >> 1; o > 0; o >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, o, G);
+  if (!live || l != 0) return;
+  if (mode == 3) out += stride * blockIdx.y;
+  out[mc] = ADD ? out[mc] + s : s;
 }
 
 // lanes per (target, component): about 8 chunk partials each, at most a warp
-inline int tree_lanes(int max_chunks) {
+inline int tree_lanes(int nchunks) {
   int G = 1;
-  while (G < 32 && G * 8 < max_chunks) G <<= 1;
+  while (G < 32 && G * 8 < nchunks) G <<= 1;
   return G;
 }
 
@@ -558,32 +583,30 @@ void launch_combine(const double* part, int M, const Group* groups, int ngroups,
                     cudaStream_t s) {
   if (M <= 0) return;
   count_launch();
-  launch_next(k_combine<true, false>, (unsigned)((3 * (size_t)M + 127) / 128), 128, 0, s, part, nullptr, M, groups, ngroups,
-                                                                                mode, 1, out);
+  launch_next(k_combine, (unsigned)((3 * (size_t)M + 127) / 128), 128, 0, s, part, M, groups, ngroups, mode, out);
 }
 
 void launch_combine_unordered(const double* part, long long* nacc, int M, const Group* groups, int ngroups,
-                              int max_chunks, int mode, double* out, cudaStream_t s, bool add) {
+                              int nchunks, int mode, double* out, cudaStream_t s, bool add) {
   if (M <= 0) return;
-  const int G = tree_lanes(max_chunks);
+  const int G = tree_lanes(nchunks);
   const unsigned blocks = (unsigned)((3 * (size_t)M * G + 255) / 256);
   count_launch();
-  if (add) launch_next(k_combine<false, true>, blocks, 256, 0, s, part, nacc, M, groups, ngroups, mode, G, out);
-  else launch_next(k_combine<false, false>, blocks, 256, 0, s, part, nacc, M, groups, ngroups, mode, G, out);
+  if (add) launch_next(k_combine_tree<true>, blocks, 256, 0, s, part, nacc, M, groups, ngroups, mode, G, out);
+  else launch_next(k_combine_tree<false>, blocks, 256, 0, s, part, nacc, M, groups, ngroups, mode, G, out);
 }
 
 void launch_combine_terms(const double* part, long long* nacc, int M, const Group* groups, int ngroups,
-                          int max_chunks, int mode, bool ordered, double* out, cudaStream_t s) {
+                          int nchunks, int nterms, int mode, bool ordered, double* out, cudaStream_t s) {
   if (M <= 0 || ngroups <= 0) return;
   count_launch();
   if (ordered) {
-    launch_next(k_combine_terms<true>, (unsigned)((3 * (size_t)M + 127) / 128), 128, 0, s, part, nullptr, M, groups, ngroups,
-                                                                                 mode, 1, out);
+    launch_next(k_combine_terms, (unsigned)((3 * (size_t)M + 127) / 128), 128, 0, s, part, M, groups, ngroups, mode, out);
     return;
   }
-  const int G = tree_lanes(max_chunks);
-  launch_next(k_combine_terms<false>, (unsigned)((3 * (size_t)M * G + 255) / 256), 256, 0, s, part, nacc, M, groups, ngroups,
-                                                                                    mode, G, out);
+  const int per = mode == 3 ? nterms : 1, G = tree_lanes((nchunks + per - 1) / per);
+  launch_next(k_combine_tree<false>, dim3((unsigned)((3 * (size_t)M * G + 255) / 256), per), 256, 0, s, part, nacc, M, groups,
+              ngroups, mode, G, out);
 }
 
 void launch_fils_to_rec64(const double* fc, const double* rvc, const double* gam, int64_t N, double* rec,

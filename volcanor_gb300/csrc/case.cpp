@@ -101,7 +101,6 @@ struct EvalPlan {
   int goff = 0, ngroups = 0;  // into the step plan's group table
   int coff = 0, nchunks = 0;  // into the chunk table
   int nrec = 0;
-  int maxq = 0;   // most chunks of one group
   int shape = 0;  // FP32 kernel tile shape (launch_partial32)
   int rows = 0;   // rows of its near-wake sheets (0: it has none)
 };
@@ -228,7 +227,6 @@ struct Case {
     if (nq < 0) throw std::runtime_error("chunk table overflow");
     hChunks.insert(hChunks.end(), tmp.begin(), tmp.begin() + nq);
     e.nchunks = nq;
-    for (int g = e.goff; g < e.goff + e.ngroups; ++g) e.maxq = std::max(e.maxq, hGroups[g].chunk_count);
     maxRecords = std::max(maxRecords, rec);
     maxChunks = std::max(maxChunks, nq);
     maxPart = std::max(maxPart, (int64_t)std::max(nq, 1) * M);
@@ -602,9 +600,9 @@ struct Case {
       return;
     }
     if (nterms > 0)
-      launch_combine_terms(s.part, near ? s.nacc : nullptr, M, dGroups + e.goff, e.ngroups, e.maxq, mode, prec == VLM_PREC_FP64, out, stream);
+      launch_combine_terms(s.part, near ? s.nacc : nullptr, M, dGroups + e.goff, e.ngroups, e.nchunks, nterms, mode, prec == VLM_PREC_FP64, out, stream);
     else if (prec == VLM_PREC_FP64) launch_combine(s.part, M, dGroups + e.goff, e.ngroups, mode, out, stream);
-    else launch_combine_unordered(s.part, near ? s.nacc : nullptr, M, dGroups + e.goff, e.ngroups, e.maxq, mode, out, stream);
+    else launch_combine_unordered(s.part, near ? s.nacc : nullptr, M, dGroups + e.goff, e.ngroups, e.nchunks, mode, out, stream);
   }
 
   // ---- autotuner of the FP32 N-body tile shape and chunking ----------------
@@ -655,8 +653,6 @@ struct Case {
     if (nq < 0) throw std::runtime_error("chunk table overflow");
     const int off = (int)hChunks.size();
     hChunks.insert(hChunks.end(), ch.begin(), ch.begin() + nq);
-    int maxq = 0;
-    for (const Group& x : g) maxq = std::max(maxq, x.chunk_count);
     for (int kk = k; kk <= W.nt; ++kk) {
       StepPlan& p2 = plans[kk];
       if (p2.rowNear != pl.rowNear || p2.rowFar != pl.rowFar) continue;
@@ -664,7 +660,6 @@ struct Case {
       e2.shape = shape;
       e2.coff = off;
       e2.nchunks = nq;
-      e2.maxq = maxq;
       for (int gi = 0; gi < e2.ngroups; ++gi) {
         hGroups[e2.goff + gi].chunk_begin = g[gi].chunk_begin;
         hGroups[e2.goff + gi].chunk_count = g[gi].chunk_count;
@@ -708,8 +703,6 @@ struct Case {
         hChunks.insert(hChunks.end(), ch.begin(), ch.begin() + nq);
         e.nchunks = nq;
         e.shape = sh;
-        e.maxq = 0;
-        for (int gi = 0; gi < e.ngroups; ++gi) e.maxq = std::max(e.maxq, g[gi].chunk_count);
         maxChunks = std::max(maxChunks, nq);
         maxPart = std::max(maxPart, (int64_t)std::max(nq, 1) * M);
       }
@@ -879,7 +872,7 @@ struct Case {
     bool on = false;
     int nrec = 0, M = 0, changed = 0, moved = 0;
     int dcap = 0, mcap = 0;           // delta records (2 per changed record + inert), moved targets
-    int dq = 0, dmaxq = 0, mq = 0, mmaxq = 0, mng = 0;
+    int dq = 0, mq = 0, mng = 0;
     Group *dG = nullptr, *mG = nullptr;
     Chunk *dC = nullptr, *mC = nullptr;
     double *dRec = nullptr, *dEw = nullptr, *tPos = nullptr, *tOut = nullptr;
@@ -1008,7 +1001,6 @@ struct Case {
     std::vector<Chunk> dch((size_t)ip.dcap + 2);
     const int dn = plan_count32(&g, 1, ip.M, slots, ip.dcap + 2, tpb);
     ip.dq = build_chunks32(&g, 1, std::max(dn, 1), dch.data(), ip.dcap + 2);
-    ip.dmaxq = g.chunk_count;
     // the moved targets: the node evaluation's groups re-chunked for mcap targets
     std::vector<Group> mg(hGroups.begin() + e.goff, hGroups.begin() + e.goff + e.ngroups);
     const int mcapCh = e.nrec + e.ngroups + 1;
@@ -1017,8 +1009,6 @@ struct Case {
     ip.mq = build_chunks32(mg.data(), e.ngroups, std::max(mn, 1), mch.data(), mcapCh);
     if (ip.dq <= 0 || ip.mq <= 0) throw std::runtime_error("chunk table overflow");
     ip.mng = e.ngroups;
-    ip.mmaxq = 0;
-    for (const Group& x : mg) ip.mmaxq = std::max(ip.mmaxq, x.chunk_count);
     ip.dG = dalloc<Group>(1, incrOwned);
     ip.dC = dalloc<Chunk>((size_t)ip.dq, incrOwned);
     ip.mG = dalloc<Group>((size_t)e.ngroups, incrOwned);
@@ -1062,7 +1052,7 @@ struct Case {
     }
     launch_partial32(ip.mRec32, recP, ip.mC, ip.mq, e.nrec, ip.tPos, ip.mcap, ip.mPart, incrCtl, ip.mNear,
                      ip.mNearBytes, ip.mNacc, ms, ew, 0, side ? &incrOv : nullptr);
-    launch_combine_unordered(ip.mPart, nearOn ? ip.mNacc : nullptr, ip.mcap, ip.mG, ip.mng, ip.mmaxq, 0, ip.tOut, ms);
+    launch_combine_unordered(ip.mPart, nearOn ? ip.mNacc : nullptr, ip.mcap, ip.mG, ip.mng, ip.mq, 0, ip.tOut, ms);
     if (side) VLM_CUDA(cudaEventRecord(incrJoin, incrStream));
     // the changed records (new +, old -) at every target: the current-wake
     // targets, whose near-field grid the current-wake evaluation left in the
@@ -1072,8 +1062,8 @@ struct Case {
     launch_pack32(ip.dRec, ip.dcap, nf, s.rec32, stream, ip.dEw);
     launch_partial32(s.rec32, ip.dRec, ip.dC, ip.dq, ip.dcap, s.targets, M, ip.dPart, s.err + 2,
                      nearOn ? s.nearScratch : nullptr, s.nearBytes, ip.dNacc, stream, ip.dEw, 0,
-                     side ? &nearOv : nullptr, true);
-    launch_combine_unordered(ip.dPart, nearOn ? ip.dNacc : nullptr, M, ip.dG, 1, ip.dmaxq, 0, s.outv, stream, true);
+                     side ? &nearOv : nullptr, e.nrec);
+    launch_combine_unordered(ip.dPart, nearOn ? ip.dNacc : nullptr, M, ip.dG, 1, ip.dq, 0, s.outv, stream, true);
     if (side) VLM_CUDA(cudaStreamWaitEvent(stream, incrJoin, 0));
     launch_incr_merge(s.outv, ip.tIdx, ip.tOut, incrCnt + 1, ip.mcap, incrCtl, s.err + 2, stream);
   }
@@ -1177,7 +1167,6 @@ struct Case {
     if (nq < 0) throw std::runtime_error("chunk table overflow");
     hChunks.insert(hChunks.end(), tmp.begin(), tmp.begin() + nq);
     e.nchunks = nq;
-    for (int g = e.goff; g < e.goff + e.ngroups; ++g) e.maxq = std::max(e.maxq, hGroups[g].chunk_count);
     maxRecords = std::max(maxRecords, rec);
     maxChunks = std::max(maxChunks, nq);
     maxPart = std::max(maxPart, (int64_t)std::max(nq, 1) * M);
@@ -2289,9 +2278,7 @@ struct Case {
     }
     if (opt.precision == VLM_PREC_FP64) launch_combine(part, (int)M, dg, (int)g.size(), 2, dV, stream);
     else {
-      int maxq = 0;
-      for (const Group& q : g) maxq = std::max(maxq, q.chunk_count);
-      launch_combine_unordered(part, nacc, (int)M, dg, (int)g.size(), maxq, 2, dV, stream);
+      launch_combine_unordered(part, nacc, (int)M, dg, (int)g.size(), nq, 2, dV, stream);
     }
     VLM_CUDA(cudaMemcpyAsync(V, dV, (size_t)M * 3 * sizeof(double), cudaMemcpyDeviceToHost, stream));
     VLM_CUDA(cudaStreamSynchronize(stream));

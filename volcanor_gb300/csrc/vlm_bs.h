@@ -182,9 +182,9 @@ void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunk
 // by ew[4 rec + k] instead of the record's circulation), or null.
 // A second stream and two events on which launch_partial32 runs the
 // near-field detection and correction alongside the pair kernel.
-// reuse_grid: near_scratch already holds the target grid of these M targets P
-// (built by the previous near-field evaluation at the same targets, whose
-// records set its cell size), so only the pair search over these records runs.
+// grid_records: the records of the near-field evaluation before, at the same M
+// targets P and not fewer: near_scratch holds the target grid that it built, so
+// only the pair search over these records runs.  0: none.
 struct NearOverlap {
   cudaStream_t stream;
   cudaEvent_t fork, join;
@@ -192,7 +192,7 @@ struct NearOverlap {
 void launch_partial32(const float* rec32, const double* rec64, const Chunk* chunks, int nchunks, int nrec,
                       const double* P, int M, double* part, int* ctl, void* near_scratch, size_t near_bytes,
                       long long* nacc, cudaStream_t s, const double* ew = nullptr, int shape = 0,
-                      const NearOverlap* ov = nullptr, bool reuse_grid = false);
+                      const NearOverlap* ov = nullptr, int grid_records = 0);
 // Converts FP64 records to FP32 records (near_factor <= 0 disables near-field);
 // ew as above (null: every active filament of a record carries its gam).
 void launch_pack32(const double* rec64, int nrec, double near_factor, float* rec32, cudaStream_t s,
@@ -206,20 +206,20 @@ void launch_pack32(const double* rec64, int nrec, double near_factor, float* rec
 void launch_combine(const double* part, int M, const Group* groups, int ngroups, int mode, double* out,
                     cudaStream_t s);
 
-// As launch_combine, but each group's chunk partials are added as a fixed
-// tree (up to a warp per target component, sized by max_chunks, the largest chunk
-// count of a group) instead of in chunk order: for the FP32 paths, whose
+// As launch_combine, but the chunk partials of all groups added as one fixed
+// tree (up to a warp per target component, sized by nchunks, the chunks of all
+// groups) instead of group by group in chunk order: for the FP32 paths, whose
 // chunking is itself free.  nacc (or null): launch_partial32's near-field
 // corrections, folded in and zeroed.  add: out = out + the result.
 void launch_combine_unordered(const double* part, long long* nacc, int M, const Group* groups, int ngroups,
-                              int max_chunks, int mode, double* out, cudaStream_t s, bool add = false);
+                              int nchunks, int mode, double* out, cudaStream_t s, bool add = false);
 
-// Coupled rotors: chunk partials -> per-term sums (Group::term).  mode 0:
-// out[m] = sum over terms of (wing + wake), in term order; mode 3:
-// out[t * M + m] = the term's own sum.  ordered: the FP64 chunk order;
+// Coupled rotors: chunk partials -> per-term sums (Group::term, nterms of
+// them).  mode 0: out[m] = sum over terms of (wing + wake), in term order;
+// mode 3: out[t * M + m] = the term's own sum.  ordered: the FP64 chunk order;
 // else the FP32 paths' fixed tree, with nacc as above.
 void launch_combine_terms(const double* part, long long* nacc, int M, const Group* groups, int ngroups,
-                          int max_chunks, int mode, bool ordered, double* out, cudaStream_t s);
+                          int nchunks, int nterms, int mode, bool ordered, double* out, cudaStream_t s);
 
 // Incremental predicted-wake evaluation (incr.cu).  Items of two sets that
 // differ bit by bit (records: kRec64 doubles and, with ea/eb, 4 edge weights;
