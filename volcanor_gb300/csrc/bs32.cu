@@ -533,8 +533,15 @@ __device__ __forceinline__ int cell_slot(const unsigned long long* __restrict__ 
   return -1;
 }
 
-__global__ void k_grid_init(unsigned char* scratch, int T) {
+// an empty grid of T slots (a kernel, not fills: those keep no priority in a graph)
+__global__ void k_grid_clear(unsigned char* scratch, GridLayout L, int T) {
   after_previous();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < T) {
+    reinterpret_cast<unsigned long long*>(scratch + L.key)[i] = kEmptyKey;
+    reinterpret_cast<int*>(scratch + L.count)[i] = 0;
+  }
+  if (i != 0) return;
   GridHdr* H = reinterpret_cast<GridHdr*>(scratch);
   H->zsum = 0.0;
   H->zcount = 0u;
@@ -1108,16 +1115,23 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
   }
   // With ov, the near-field detection and FP64 correction (which read only
   // the records and targets) run on ov->stream alongside the pair kernel;
-  // what follows on s (the fold into the partial sums) waits for both.
+  // what follows on s (the fold into the partial sums) waits for both.  The
+  // pair kernel's blocks fill every SM for several waves, so the chain goes
+  // first and on a stream of high priority: its blocks take the slots that a
+  // wave leaves, and its FP64 runs under the FP32 of the next.  Behind the
+  // last wave it was 55 of 720 us of a hover step.
   cudaStream_t ns = s;
   if (nearOn && ov) {
     cudaEventRecord(ov->fork, s);
     cudaStreamWaitEvent(ov->stream, ov->fork, 0);
     ns = ov->stream;
   }
-  count_launch();
-  if (shape == 1) launch_shape<1>(ew != nullptr, grid, rec32, chunks, P, M, part, ctl, s);
-  else launch_shape<0>(ew != nullptr, grid, rec32, chunks, P, M, part, ctl, s);
+  auto pairs = [&]() {
+    count_launch();
+    if (shape == 1) launch_shape<1>(ew != nullptr, grid, rec32, chunks, P, M, part, ctl, s);
+    else launch_shape<0>(ew != nullptr, grid, rec32, chunks, P, M, part, ctl, s);
+  };
+  if (!nearOn || ns == s) pairs();
   if (!nearOn) return;
   // near field: targets binned in a grid, near pairs listed, FP64
   // corrections of the listed pairs, corrections folded into the partials
@@ -1138,6 +1152,7 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
     launch_next(k_near_fix, 4 * sms, 128, 0, ns, list, cap, rec32, rec64, ew, P, M,
                                         reinterpret_cast<unsigned long long*>(nacc), ctl);
     if (ns != s) {
+      pairs();
       cudaEventRecord(ov->join, ns);
       cudaStreamWaitEvent(s, ov->join, 0);
     }
@@ -1145,10 +1160,8 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
   }
   if (grid_records == 0) {
     count_launches(5);
-    launch_next(k_grid_init, 1, 1, 0, ns, g, T);
+    launch_next(k_grid_clear, (T + 255) / 256, 256, 0, ns, g, L, T);
     launch_next(k_zone_mean, (nrec + 255) / 256, 256, 0, ns, rec32, nrec, g);
-    cudaMemsetAsync(g + L.key, 0xFF, (size_t)T * sizeof(unsigned long long), ns);
-    cudaMemsetAsync(g + L.count, 0, (size_t)T * sizeof(int), ns);
     launch_next(k_tgrid_insert<0>, (M + 255) / 256, 256, 0, ns, P, M, g);
     launch_next(k_grid_scan, 1, 1024, 0, ns, M, g);
     launch_next(k_tgrid_insert<1>, (M + 255) / 256, 256, 0, ns, P, M, g);
@@ -1159,6 +1172,7 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
   launch_next(k_near_fix, 4 * sms, 128, 0, ns, list, cap, rec32, rec64, ew, P, M, reinterpret_cast<unsigned long long*>(nacc),
                                       ctl);
   if (ns != s) {
+    pairs();
     cudaEventRecord(ov->join, ns);
     cudaStreamWaitEvent(s, ov->join, 0);
   }

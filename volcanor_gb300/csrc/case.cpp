@@ -90,6 +90,16 @@ class DevArena {
   size_t left_ = 0;
 };
 
+// a stream whose kernels are to be scheduled before those of the case's own (the
+// chains beside a pair kernel that fills the device); a captured graph keeps the
+// priorities only when instantiated with kGraphFlags
+static void createNearStream(cudaStream_t* st) {
+  int least = 0, greatest = 0;
+  VLM_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+  VLM_CUDA(cudaStreamCreateWithPriority(st, cudaStreamNonBlocking, greatest));
+}
+static constexpr unsigned long long kGraphFlags = cudaGraphInstantiateFlagUseNodePriority;
+
 template <class T>
 static T* dalloc(size_t n, DevArena& owned) {
   if (n > SIZE_MAX / sizeof(T)) throw CudaError("device allocation too large");
@@ -297,7 +307,7 @@ struct Case {
     VLM_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
     VLM_CUDA(cudaEventCreateWithFlags(&evFork, cudaEventDisableTiming));
     VLM_CUDA(cudaEventCreateWithFlags(&evJoin, cudaEventDisableTiming));
-    VLM_CUDA(cudaStreamCreateWithFlags(&nearOv.stream, cudaStreamNonBlocking));
+    createNearStream(&nearOv.stream);
     VLM_CUDA(cudaEventCreateWithFlags(&nearOv.fork, cudaEventDisableTiming));
     VLM_CUDA(cudaEventCreateWithFlags(&nearOv.join, cudaEventDisableTiming));
 
@@ -540,7 +550,7 @@ struct Case {
     }
     replaying = false;
     VLM_CUDA(cudaStreamEndCapture(stream, &g));
-    const cudaError_t e = cudaGraphInstantiate(&gexec, g, 0);
+    const cudaError_t e = cudaGraphInstantiate(&gexec, g, kGraphFlags);
     cudaGraphDestroy(g);
     VLM_CUDA(e);
     graphKernels = launch_count() - l0;
@@ -891,8 +901,8 @@ struct Case {
   double *recP = nullptr, *ewP = nullptr, *tgtP = nullptr;  // the predicted records, edge weights, targets
   int* incrCnt = nullptr;                                   // [0] changed records, [1] moved targets
   int* incrBlk = nullptr;                                   // per-tile offsets: records, then targets
-  cudaStream_t incrStream = nullptr;                        // the moved targets' evaluation
-  NearOverlap incrOv{nullptr, nullptr, nullptr};            // its near-field chain
+  cudaStream_t incrStream = nullptr;                        // the changed records' evaluation
+  NearOverlap incrOv{nullptr, nullptr, nullptr};            // the moved targets' near-field chain
   cudaEvent_t incrFork = nullptr, incrJoin = nullptr;
   int* incrCtl = nullptr;  // the moved targets' evaluation's error code and near-pair cursor
 
@@ -936,7 +946,7 @@ struct Case {
     incrCnt = dalloc<int>(2, incrOwned);
     incrCtl = dalloc<int>(2, incrOwned);
     incrBlk = dalloc<int>((size_t)incr_diff_blocks(maxRecords) + incr_diff_blocks(maxTargets) + 2, incrOwned);
-    VLM_CUDA(cudaStreamCreateWithFlags(&incrStream, cudaStreamNonBlocking));
+    createNearStream(&incrStream);
     VLM_CUDA(cudaStreamCreateWithFlags(&incrOv.stream, cudaStreamNonBlocking));
     VLM_CUDA(cudaEventCreateWithFlags(&incrOv.fork, cudaEventDisableTiming));
     VLM_CUDA(cudaEventCreateWithFlags(&incrOv.join, cudaEventDisableTiming));
@@ -1040,30 +1050,31 @@ struct Case {
     const double nf = nearOn ? opt.near_factor : 0.0;
     incrDiff(k, M, ip.mRec32);
     const double* ew = s.edgeW ? ewP : nullptr;
-    launch_moved_targets(tgtP, s.targets, M, incrBlk + incr_diff_blocks(e.nrec), incrCnt + 1, ip.tIdx, ip.tPos,
-                         ip.mcap, s.err + 2, stream);
-    // every predicted record at the moved targets, on its own streams (a
-    // batch's case on its own stream: the batch's cases already run side by side)
+    // the two evaluations side by side (a batch's case has one stream: the
+    // batch's cases already run side by side), the longer chain first and on the
+    // stream of higher priority
     const bool side = opt.nbody_slots <= 0;
-    cudaStream_t ms = side ? incrStream : stream;
+    cudaStream_t ds = side ? incrStream : stream;
     if (side) {
       VLM_CUDA(cudaEventRecord(incrFork, stream));
       VLM_CUDA(cudaStreamWaitEvent(incrStream, incrFork, 0));
     }
-    launch_partial32(ip.mRec32, recP, ip.mC, ip.mq, e.nrec, ip.tPos, ip.mcap, ip.mPart, incrCtl, ip.mNear,
-                     ip.mNearBytes, ip.mNacc, ms, ew, 0, side ? &incrOv : nullptr);
-    launch_combine_unordered(ip.mPart, nearOn ? ip.mNacc : nullptr, ip.mcap, ip.mG, ip.mng, ip.mq, 0, ip.tOut, ms);
-    if (side) VLM_CUDA(cudaEventRecord(incrJoin, incrStream));
     // the changed records (new +, old -) at every target: the current-wake
     // targets, whose near-field grid the current-wake evaluation left in the
     // scratch (the moved targets' results are replaced below)
-    launch_delta_records(recP, s.rec64, ew, s.edgeW, e.nrec, incrBlk, incrCnt, ip.dRec, ip.dEw, ip.dcap, s.err + 2,
-                         stream);
-    launch_pack32(ip.dRec, ip.dcap, nf, s.rec32, stream, ip.dEw);
+    launch_delta_records(recP, s.rec64, ew, s.edgeW, e.nrec, incrBlk, incrCnt, ip.dRec, ip.dEw, ip.dcap, s.err + 2, ds);
+    launch_pack32(ip.dRec, ip.dcap, nf, s.rec32, ds, ip.dEw);
     launch_partial32(s.rec32, ip.dRec, ip.dC, ip.dq, ip.dcap, s.targets, M, ip.dPart, s.err + 2,
-                     nearOn ? s.nearScratch : nullptr, s.nearBytes, ip.dNacc, stream, ip.dEw, 0,
+                     nearOn ? s.nearScratch : nullptr, s.nearBytes, ip.dNacc, ds, ip.dEw, 0,
                      side ? &nearOv : nullptr, e.nrec);
-    launch_combine_unordered(ip.dPart, nearOn ? ip.dNacc : nullptr, M, ip.dG, 1, ip.dq, 0, s.outv, stream, true);
+    launch_combine_unordered(ip.dPart, nearOn ? ip.dNacc : nullptr, M, ip.dG, 1, ip.dq, 0, s.outv, ds, true);
+    if (side) VLM_CUDA(cudaEventRecord(incrJoin, incrStream));
+    // every predicted record at the moved targets
+    launch_moved_targets(tgtP, s.targets, M, incrBlk + incr_diff_blocks(e.nrec), incrCnt + 1, ip.tIdx, ip.tPos,
+                         ip.mcap, s.err + 2, stream);
+    launch_partial32(ip.mRec32, recP, ip.mC, ip.mq, e.nrec, ip.tPos, ip.mcap, ip.mPart, incrCtl, ip.mNear,
+                     ip.mNearBytes, ip.mNacc, stream, ew, 0, side ? &incrOv : nullptr);
+    launch_combine_unordered(ip.mPart, nearOn ? ip.mNacc : nullptr, ip.mcap, ip.mG, ip.mng, ip.mq, 0, ip.tOut, stream);
     if (side) VLM_CUDA(cudaStreamWaitEvent(stream, incrJoin, 0));
     launch_incr_merge(s.outv, ip.tIdx, ip.tOut, incrCnt + 1, ip.mcap, incrCtl, s.err + 2, stream);
   }
@@ -2829,7 +2840,7 @@ struct vlm_batch {
       throw;
     }
     VLM_CUDA(cudaStreamEndCapture(origin, &g));
-    const cudaError_t e = cudaGraphInstantiate(&gexec, g, 0);
+    const cudaError_t e = cudaGraphInstantiate(&gexec, g, kGraphFlags);
     cudaGraphDestroy(g);
     VLM_CUDA(e);
     graphKernels = launch_count() - l0;
