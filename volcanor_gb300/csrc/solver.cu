@@ -575,25 +575,38 @@ __global__ void k_aic(Dims d, DevState s, const double* fr) {
 // gains ~7 digits.
 // Solve AIC gamVec = -RHS by refinement; records the final relative residual
 // max|b - A x| / max|b| in s.luRes[0] and flags err[1] when it stays above 1e-9.
-// One cluster of kSolveBlocks blocks, a warp per row of the two products (lanes
-// over the columns, then a butterfly); x and r go through global memory between
-// them and into every block's shared memory.  On one SM, with the vectors read
-// element by element, it took 290 us at n = 300.
+// One cluster of kSolveBlocks blocks, each with n / kSolveBlocks consecutive rows
+// of the two products.  A thread takes a row and every S-th column of it, so that
+// neighbouring threads read neighbouring rows of a column (the matrices are
+// column-major); a warp then adds a row's S sums.  x and r go through global
+// memory between the products and into every block's shared memory.  Bound by
+// latency: six products of a few loads each and the cluster's barriers between
+// them.  With a warp per row, each load of it 32 columns apart, 62 us at n = 300,
+// now 42; on one SM it was 290.
 constexpr int kRefinePasses = 3;
 constexpr int kSolveBlocks = 8;
-inline size_t solve_smem(int n) { return sizeof(double) * n; }
+constexpr int kSolveThreads = 1024;
+inline int solve_rows(int n) { return (n + kSolveBlocks - 1) / kSolveBlocks; }
+inline int solve_slices(int n) { return std::max(1, std::min(n, kSolveThreads / solve_rows(n))); }
+inline size_t solve_smem(int n) {
+  return sizeof(double) * ((size_t)n + (size_t)solve_rows(n) * solve_slices(n)) + sizeof(float) * (size_t)n;
+}
+constexpr size_t kSolveSmemMax = sizeof(double) * (8192 + 1024) + sizeof(float) * 8192;  // at the most panels of a rotor
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__global__ void __cluster_dims__(kSolveBlocks, 1, 1) __launch_bounds__(1024) k_solve_refine(Dims d, DevState s) {
+__global__ void __cluster_dims__(kSolveBlocks, 1, 1) __launch_bounds__(kSolveThreads) k_solve_refine(Dims d, DevState s, int R,
+                                                                                                    int S) {
   after_previous();
   const int n = d.n;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row0 = warp * kSolveBlocks + blockIdx.x, rows = 32 * kSolveBlocks;
+  const int row0 = blockIdx.x * R, rows = max(0, min(R, n - row0));
   const double* rhs = s.RHS;
   volatile double* x = s.refX;
   volatile double* r = s.refR;
-  extern __shared__ double vec[];  // the vector of the product at hand
+  extern __shared__ double vec[];   // the vector of the product at hand
+  double* sums = vec + n;           // [slice][row]
+  float* vec32 = reinterpret_cast<float*>(sums + R * S);
   __shared__ double red[32];
   // b = -RHS (under axisymmetry blade 1's for every blade), and its largest magnitude, in every block
   auto b = [&](int i) { return -1.0 * rhs[d.axisym ? i % d.npan : i]; };
@@ -606,36 +619,53 @@ __global__ void __cluster_dims__(kSolveBlocks, 1, 1) __launch_bounds__(1024) k_s
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
   };
+  const int mr = threadIdx.x % R, ms = threadIdx.x / R;
+  const bool mine = ms < S && mr < rows;
   double bmax = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double v = b(i);
-    vec[i] = v;
+    vec32[i] = (float)v;
     bmax = fmax(bmax, fabs(v));
   }
   bmax = block_max(bmax);
   for (int pass = 0; pass < kRefinePasses; ++pass) {
     if (pass) {
-      for (int i = threadIdx.x; i < n; i += blockDim.x) vec[i] = r[i];
+      for (int i = threadIdx.x; i < n; i += blockDim.x) vec32[i] = (float)r[i];
       __syncthreads();
     }
     // x += inv32 r  (FP32 products of the FP32-rounded residual, FP64 update); r = b at first
-    for (int i = row0; i < n; i += rows) {
+    float* sums32 = reinterpret_cast<float*>(sums);
+    if (mine) {
+      const float* a = s.AICinv32 + row0 + mr;
       float z = 0.f;
 #pragma unroll 8
-      for (int j = lane; j < n; j += 32) z = fmaf(s.AICinv32[i + (size_t)n * j], (float)vec[j], z);
+      for (int j = ms; j < n; j += S) z = fmaf(a[(size_t)n * j], vec32[j], z);
+      sums32[ms * R + mr] = z;
+    }
+    __syncthreads();
+    for (int i = warp; i < rows; i += 32) {
+      float z = 0.f;
+      for (int k = lane; k < S; k += 32) z += sums32[k * R + i];
       for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-      if (lane == 0) x[i] = (pass ? x[i] : 0.0) + (double)z;
+      if (lane == 0) x[row0 + i] = (pass ? x[row0 + i] : 0.0) + (double)z;
     }
     cluster_sync();
     for (int i = threadIdx.x; i < n; i += blockDim.x) vec[i] = x[i];
     __syncthreads();
     // r = b - A x in FP64
-    for (int i = row0; i < n; i += rows) {
+    if (mine) {
+      const double* a = s.AIC + row0 + mr;
       double ax = 0.0;
 #pragma unroll 8
-      for (int j = lane; j < n; j += 32) ax = fma(s.AIC[i + (size_t)n * j], vec[j], ax);
+      for (int j = ms; j < n; j += S) ax = fma(a[(size_t)n * j], vec[j], ax);
+      sums[ms * R + mr] = ax;
+    }
+    __syncthreads();
+    for (int i = warp; i < rows; i += 32) {
+      double ax = 0.0;
+      for (int k = lane; k < S; k += 32) ax += sums[k * R + i];
       for (int o = 16; o > 0; o >>= 1) ax += __shfl_xor_sync(0xffffffffu, ax, o);
-      if (lane == 0) r[i] = b(i) - ax;
+      if (lane == 0) r[row0 + i] = b(row0 + i) - ax;
     }
     cluster_sync();
   }
@@ -1348,8 +1378,8 @@ void launch_aic(const Dims& d, const DevState& s, const double* frame, cudaStrea
 static void solve_refine(const Dims& d, const DevState& s, cudaStream_t st) {
   const size_t smem = solve_smem(d.n);
   if (smem > 40 * 1024)
-    cudaFuncSetAttribute(k_solve_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_smem(8192));
-  launch_next(k_solve_refine, kSolveBlocks, 1024, smem, st, d, s);
+    cudaFuncSetAttribute(k_solve_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSolveSmemMax);
+  launch_next(k_solve_refine, kSolveBlocks, kSolveThreads, smem, st, d, s, solve_rows(d.n), solve_slices(d.n));
 }
 void launch_solve(const Dims& d, const DevState& s, const double* frame, bool withWake, cudaStream_t st) {
   count_launch();
