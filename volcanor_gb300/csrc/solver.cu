@@ -753,63 +753,138 @@ struct ChunkAcc1 {
 };
 
 // Sums over the rings of a rotor's blades at one collocation point, one block
-// per point: every thread evaluates a ring (the four edges in vr_vind's order)
+// per point.  Every thread evaluates a ring (the four edges in vr_vind's order)
 // and leaves its terms in shared memory -- the ring's (((f0 + f1) + f2) + f3) gam,
-// its bound pair's (f1 + f3) gam and, on the trailing edge, f1 gam -- and the
-// first lanes of two warps add them in the reference's order, one component a
-// lane, so that only additions are serial.  (Formed by three threads between the
-// additions, those terms were two thirds of the kernel: 340 us at 300 points.)
+// its bound pair's (f1 + f3) gam and, on the trailing edge, f1 gam -- and lanes of
+// eight warps add them in the reference's order, a lane per component and blade,
+// so that only additions are serial.  A batch is up to kVcThreads rings: as many
+// whole blades as fit (kVcBlades at most), or part of one.
 //   bound: per blade s = 0, s + the pair's term panel by panel (spanwise
 //          stations outer), s - the trailing-edge terms; blades added to 0
 //          (rotor_vind_bywing_boundVortices, src/classdef.f90:1376-1393, 4445-4457)
 //   wing:  per blade the rings' terms in summation blocks; blades added to 0
-constexpr int kVcThreads = 256;
-inline size_t velcp_smem(int ns) { return sizeof(double) * 3 * (2 * (size_t)kVcThreads + ns); }
+// Neighbouring rings of a blade share corners and edges where these hold bit for
+// bit, as in a wake sheet: panel p's corner 3 and edge 3 are panel p - 1's corner
+// 2 and edge 1, its corner 1 and edge 0 panel p - nc's corner 2 and edge 2, and
+// an edge run backwards has the negated velocity.
+// Bound by the FP64 unit at many points (300 points x 300 panels: 89 us with every
+// ring on its own and the blades in turn, now 65), by one evaluation's chain and
+// the longest blade's additions at few (16 points, two blades of 8: 37, now 28).
+constexpr int kVcThreads = 256, kVcBlades = 32;
+inline int velcp_blades(int npan) { return npan > kVcThreads ? 1 : std::min(kVcBlades, kVcThreads / npan); }
+// of `te`: a group of blades has at most kVcThreads stations, one blade any number
+inline size_t velcp_smem(int npan, int ns) {
+  return sizeof(double) * 3 * (5 * (size_t)kVcThreads + 2 * kVcBlades + (size_t)velcp_blades(npan) * ns);
+}
+__device__ __forceinline__ bool same64(double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); }
+__device__ __forceinline__ bool same_point(const double* a, const double* b) {
+  return same64(a[0], b[0]) && same64(a[1], b[1]) && same64(a[2], b[2]);
+}
+__device__ __forceinline__ d3 negated(const double* a) { return mk3(-a[0], -a[1], -a[2]); }
 template <bool WING>
-__device__ void ring_sums(const Dims& d, const DevState& s, const double* fr, d3 P, int sumChunk, double* sm,
+__device__ void ring_sums(const Dims& d, const DevState& s, const double* fr, d3 P, int sumChunk, int group, double* sm,
                           double& bound, double& wing) {
-  double* ring = sm;                      // [ring of the batch][component]
-  double* pair = ring + 3 * kVcThreads;
-  double* te = pair + 3 * kVcThreads;     // [station][component]
+  constexpr int N = 3 * kVcThreads;
+  double* ring = sm;             // [ring of the batch][component]
+  double* pair = ring + N;
+  double* U2 = pair + N;         // corner 2's unit vectors
+  double* E1 = U2 + N;
+  double* E2 = E1 + N;
+  double* res = E2 + N;          // [bound, wing][blade of the group][component]
+  double* te = res + 6 * kVcBlades;  // [blade of the group][station][component]
   const exact64::Unit u = exact64::load_unit();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int npan = d.npan, nc = d.nc;
   bound = wing = 0.0;
-  for (int b = 0; b < d.nb; ++b) {
+  for (int b0 = 0; b0 < d.nb; b0 += group) {
+    const int blades = min(group, d.nb - b0), total = blades * npan;
     double sb = 0.0;
     ChunkAcc1 acc(sumChunk);
-    for (int p0 = 0; p0 < d.npan; p0 += kVcThreads) {
-      const int n = min(kVcThreads, d.npan - p0), p = p0 + (int)threadIdx.x;
-      if (p < d.npan) {
-        const double* w = panRec(d, fr, b, p);
-        const double* rv = s.wRvc + 4 * ((size_t)b * d.npan + p);
-        const double g = s.wGam[(size_t)b * d.npan + p];
-        const corner64 c1 = exact64::make_corner(u, P, ld3(w + 3)), c2 = exact64::make_corner(u, P, ld3(w + 6));
-        const d3 f1 = exact64::vf_vind(u, c1, c2, rv[1]);
-        const corner64 c0 = exact64::make_corner(u, P, ld3(w)), c3 = exact64::make_corner(u, P, ld3(w + 9));
-        const d3 f3 = exact64::vf_vind(u, c3, c0, rv[3]);
-        if (WING) {
-          const d3 f0 = exact64::vf_vind(u, c0, c1, rv[0]), f2 = exact64::vf_vind(u, c2, c3, rv[2]);
-          st3(ring + 3 * threadIdx.x,
-              exact64::mul(u, exact64::add(u, exact64::add(u, exact64::add(u, f0, f1), f2), f3), g));
-        }
-        st3(pair + 3 * threadIdx.x, exact64::mul(u, exact64::add(u, f1, f3), g));
-        if (p % d.nc == d.nc - 1) st3(te + 3 * (p / d.nc), exact64::mul(u, f1, g));
+    for (int q0 = 0; q0 < total; q0 += kVcThreads) {
+      const int n = min(kVcThreads, total - q0), t = threadIdx.x;
+      const bool live = t < n;
+      const int k = live ? (q0 + t) / npan : 0, p = live ? (q0 + t) % npan : 0;
+      const double* w = panRec(d, fr, b0 + k, p);
+      const double* rv = s.wRvc + 4 * ((size_t)(b0 + k) * npan + p);
+      corner64 c1, c2, c3;
+      if (live) {
+        c2 = exact64::make_corner(u, P, ld3(w + 6));
+        st3(U2 + 3 * t, c2.u);
       }
       __syncthreads();
-      if (lane < 3) {
-        if (WING && warp == 0) acc.add(u, ring + lane, n);
-        if (warp == 1) {
-#pragma unroll 8
-          for (int i = 0; i < n; ++i) sb = exact64::add(u, sb, pair[3 * i + lane]);
-          if (p0 + n == d.npan)
-#pragma unroll 8
-            for (int j = 0; j < d.ns; ++j) sb = exact64::sub(u, sb, te[3 * j + lane]);
+      bool s1 = false, s3 = false;  // corner 1 is panel p - nc's corner 2, corner 3 panel p - 1's
+      d3 f1, f2;
+      if (live) {
+        const d3 p1 = ld3(w + 3), p3 = ld3(w + 9);
+        s1 = p >= nc && t >= nc && same_point(w + 3, panRec(d, fr, b0 + k, p - nc) + 6);
+        s3 = p % nc != 0 && t >= 1 && same_point(w + 9, panRec(d, fr, b0 + k, p - 1) + 6);
+        if (s1) {
+          c1.r = exact64::sub(u, P, p1);
+          c1.u = ld3(U2 + 3 * (t - nc));
+        } else {
+          c1 = exact64::make_corner(u, P, p1);
+        }
+        f1 = exact64::vf_vind(u, c1, c2, rv[1]);
+        st3(E1 + 3 * t, f1);
+        if (s3) {
+          c3.r = exact64::sub(u, P, p3);
+          c3.u = ld3(U2 + 3 * (t - 1));
+        } else {
+          c3 = exact64::make_corner(u, P, p3);
+        }
+        if (WING) {
+          f2 = exact64::vf_vind(u, c2, c3, rv[2]);
+          st3(E2 + 3 * t, f2);
         }
       }
+      __syncthreads();
+      if (live) {
+        const double g = s.wGam[(size_t)(b0 + k) * npan + p];
+        const bool e0 = s1 && same_point(w, panRec(d, fr, b0 + k, p - nc) + 9) && same64(rv[0], rv[2 - 4 * nc]);
+        const bool e3 = s3 && same_point(w, panRec(d, fr, b0 + k, p - 1) + 3) && same64(rv[3], rv[1 - 4]);
+        corner64 c0;
+        if (!e3 || (WING && !e0)) c0 = exact64::make_corner(u, P, ld3(w));
+        const d3 f3 = e3 ? negated(E1 + 3 * (t - 1)) : exact64::vf_vind(u, c3, c0, rv[3]);
+        if (WING) {
+          const d3 f0 = e0 ? negated(E2 + 3 * (t - nc)) : exact64::vf_vind(u, c0, c1, rv[0]);
+          st3(ring + 3 * t, exact64::mul(u, exact64::add(u, exact64::add(u, exact64::add(u, f0, f1), f2), f3), g));
+        }
+        st3(pair + 3 * t, exact64::mul(u, exact64::add(u, f1, f3), g));
+        if (p % nc == nc - 1) st3(te + 3 * (k * d.ns + p / nc), exact64::mul(u, f1, g));
+      }
+      __syncthreads();
+      // the blades' sums: bound by warps 0 to 3, wing by 4 to 7, every fourth blade each
+      if (lane < 3 && (WING || warp < 4))
+        for (int kb = warp & 3; kb < blades; kb += 4) {
+          const int first = max(kb * npan, q0) - q0, last = min((kb + 1) * npan, q0 + n) - q0;
+          if (first >= last) continue;
+          const bool end = q0 + last == (kb + 1) * npan;
+          if (warp >= 4) {
+            acc.add(u, ring + 3 * first + lane, last - first);
+            if (end) {
+              res[3 * (kVcBlades + kb) + lane] = acc.result();
+              acc = ChunkAcc1(sumChunk);
+            }
+          } else {
+#pragma unroll 8
+            for (int i = first; i < last; ++i) sb = exact64::add(u, sb, pair[3 * i + lane]);
+            if (end) {
+              const double* q = te + 3 * (size_t)kb * d.ns + lane;
+#pragma unroll 8
+              for (int j = 0; j < d.ns; ++j) sb = exact64::sub(u, sb, q[3 * j]);
+              res[3 * kb + lane] = sb;
+              sb = 0.0;
+            }
+          }
+        }
       __syncthreads();
     }
-    if (warp == 1) bound = bound + sb;
-    wing = wing + acc.result();
+    if (lane < 3)
+      for (int kb = 0; kb < blades; ++kb) {
+        bound = bound + res[3 * kb + lane];
+        if (WING) wing = wing + res[3 * (kVcBlades + kb) + lane];
+      }
+    __syncthreads();
   }
 }
 
@@ -820,24 +895,21 @@ __device__ void ring_sums(const Dims& d, const DevState& s, const double* fr, d3
 // rotor (self) is computed here.  velCPTotal = velCP - bound of every rotor in
 // rotor order + this rotor's wing (src/main.f90:636-652).
 __global__ void __launch_bounds__(kVcThreads) k_velcp_total(Dims d, DevState s, const double* fr, int sumChunk,
-                                                            const double* fb, int nrs, int self) {
+                                                            const double* fb, int nrs, int self, int group) {
   after_previous();
   extern __shared__ double sm[];
-  __shared__ double bnd[3];
   const int t = blockIdx.x;
   const d3 P = ld3(panRec(d, fr, t / d.npan, t % d.npan) + 12);
   double bound, wing;
-  ring_sums<true>(d, s, fr, P, sumChunk, sm, bound, wing);
-  if (threadIdx.x >= 32 && threadIdx.x < 35) bnd[threadIdx.x - 32] = bound;
-  __syncthreads();
+  ring_sums<true>(d, s, fr, P, sumChunk, group, sm, bound, wing);
   const int c = threadIdx.x;
   if (c < 3) {
     double v = s.velCP[3 * (size_t)t + c];
     if (fb) {
       const size_t M = (size_t)d.nbC * d.npan;
-      for (int jr = 0; jr < nrs; ++jr) v = v - (jr == self ? bnd[c] : fb[3 * (jr * M + t) + c]);
+      for (int jr = 0; jr < nrs; ++jr) v = v - (jr == self ? bound : fb[3 * (jr * M + t) + c]);
     } else {
-      v = v - bnd[c];
+      v = v - bound;
     }
     v = v + wing;
     s.velCPTotal[3 * (size_t)t + c] = v;
@@ -847,14 +919,14 @@ __global__ void __launch_bounds__(kVcThreads) k_velcp_total(Dims d, DevState s, 
 // Bound vortices of rotor (ds, ss, frs) at the collocation points of rotor
 // (dt, frt), one block per point (a thread per point: 309 us at 16 panels).
 __global__ void __launch_bounds__(kVcThreads) k_bound_foreign(Dims dt, const double* frt, Dims ds, DevState ss,
-                                                              const double* frs, double* out) {
+                                                              const double* frs, double* out, int group) {
   after_previous();
   extern __shared__ double sm[];
   const int t = blockIdx.x;
   const d3 P = ld3(panRec(dt, frt, t / dt.npan, t % dt.npan) + 12);
   double bound, wing;
-  ring_sums<false>(ds, ss, frs, P, 0, sm, bound, wing);
-  if (threadIdx.x >= 32 && threadIdx.x < 35) out[3 * (size_t)t + threadIdx.x - 32] = bound;
+  ring_sums<false>(ds, ss, frs, P, 0, group, sm, bound, wing);
+  if (threadIdx.x < 3) out[3 * (size_t)t + threadIdx.x] = bound;
 }
 
 // ---- image rotors (src/classdef.f90:4990-5131) ------------------------------
@@ -1424,7 +1496,7 @@ static void velcp_attr() {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && attr[dev].load(std::memory_order_acquire)) return;
-  const int most = (int)velcp_smem(8192);
+  const int most = (int)velcp_smem(8192, 8192);
   cudaFuncSetAttribute(k_velcp_total, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   cudaFuncSetAttribute(k_bound_foreign, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   if (dev >= 0 && dev < 64) attr[dev].store(true, std::memory_order_release);
@@ -1433,13 +1505,15 @@ void launch_bound_foreign(const Dims& dt, const double* frameT, const Dims& ds, 
                           const double* frameS, double* out, cudaStream_t st) {
   count_launch();
   velcp_attr();
-  launch_next(k_bound_foreign, dt.nbC * dt.npan, kVcThreads, velcp_smem(ds.ns), st, dt, frameT, ds, ss, frameS, out);
+  launch_next(k_bound_foreign, dt.nbC * dt.npan, kVcThreads, velcp_smem(ds.npan, ds.ns), st, dt, frameT, ds, ss, frameS, out,
+              velcp_blades(ds.npan));
 }
 void launch_loads(const Dims& d, const DevState& s, const double* frame, int sumChunk, int iter, cudaStream_t st,
                   const double* foreignBound, int nrs, int self) {
   count_launch();
   velcp_attr();
-  launch_next(k_velcp_total, d.nbC * d.npan, kVcThreads, velcp_smem(d.ns), st, d, s, frame, sumChunk, foreignBound, nrs, self);
+  launch_next(k_velcp_total, d.nbC * d.npan, kVcThreads, velcp_smem(d.npan, d.ns), st, d, s, frame, sumChunk, foreignBound, nrs, self,
+              velcp_blades(d.npan));
   count_launch();
   launch_next(k_loads, 1, kLoadsThreads, 0, st, d, s, frame, iter);
 }
