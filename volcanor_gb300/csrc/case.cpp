@@ -1256,13 +1256,22 @@ struct Case {
     }
   }
   // the loads with every rotor's bound vortices (src/main.f90:632-652)
-  void sysLoads(int k) {
+  void sysLoads(int k, cudaStream_t st) {
     const int Mcp = d.nbC * d.npan;
     for (int jr = 0; jr < (int)sys.size(); ++jr)
       if (jr != self)
-        launch_bound_foreign(d, frame(k), sys[jr]->d, sys[jr]->s, sys[jr]->frame(k), sysBound + 3 * (size_t)jr * Mcp,
-                             stream);
-    launch_loads(d, s, frame(k), chunk64, k, stream, sysBound, (int)sys.size(), self);
+        launch_bound_foreign(d, frame(k), sys[jr]->d, sys[jr]->s, sys[jr]->frame(k), sysBound + 3 * (size_t)jr * Mcp, st);
+    launch_loads(d, s, frame(k), chunk64, k, st, sysBound, (int)sys.size(), self);
+  }
+  // As a lone case's (enqueueStepBody): each rotor's loads on its side stream
+  // beside the wake update, joined at the step's end, before the next solutions
+  // replace what they read.  One after the other on the system's stream they were
+  // half of a step of two small rotors (8 rotor-steps 2.23 ms, now 1.80).
+  void forkSysLoads(int k) {
+    VLM_CUDA(cudaEventRecord(evFork, stream));
+    VLM_CUDA(cudaStreamWaitEvent(side, evFork, 0));
+    sysLoads(k, side);
+    VLM_CUDA(cudaEventRecord(evJoin, side));
   }
 
   // ---- learned far-wake surrogate ----------------------------------------
@@ -2613,7 +2622,7 @@ struct vlm_system {
     }
     for (auto& c : r) launch_shed(c->c.d, c->c.s, c->c.frame(0), c->c.d.NW + 1, false, st);
     if (rotor(0).W.sw.rotorForcePlot != 0)
-      for (auto& c : r) c->c.sysLoads(0);
+      for (auto& c : r) c->c.sysLoads(0, st);
     VLM_CUDA(cudaGetLastError());
     for (auto& c : r) c->c.finishSteps(0, nullptr);
     for (auto& c : r) {
@@ -2644,14 +2653,17 @@ struct vlm_system {
         if (c->c.imgSrc) c->c.imageMirrorGamma();
         else launch_solve_only(c->c.d, c->c.s, st);
       }
-      if (sw.rotorForcePlot != 0 && k % sw.rotorForcePlot == 0)
-        for (auto& c : r) c->c.sysLoads(k);
+      const bool loads = sw.rotorForcePlot != 0 && k % sw.rotorForcePlot == 0;
+      if (loads)
+        for (auto& c : r) c->c.forkSysLoads(k);
       if (sw.wakeSuppress == 0)
         for (int stg = 0; stg < 4; ++stg)
           for (auto& c : r) {
             if (c->c.imgSrc) c->c.imageWakeStage(k, stg);
             else c->c.wakeStage(k, stg);
           }
+      if (loads)
+        for (auto& c : r) VLM_CUDA(cudaStreamWaitEvent(st, c->c.evJoin, 0));
     }
     VLM_CUDA(cudaEventRecord(c0.ev1, st));
     VLM_CUDA(cudaGetLastError());
