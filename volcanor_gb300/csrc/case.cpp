@@ -1509,7 +1509,17 @@ struct Case {
       evalNodesFull(k, pred, M);
     }
     const double iwv = k < W.sw.initWakeVelNt ? W.P.initWakeVel : 0.0;
-    launch_scatter_nodes(d, s, stepFrame(k), pl.rowNear, pl.rowFar, pred, iwv, stream);
+    launch_scatter_nodes(d, s, stepFrame(k), pl.rowNear, pl.rowFar, pred, iwv, nodeOp(k, pred), stream);
+  }
+  // the scheme's operation on the node velocities just evaluated
+  int nodeOp(int k, bool pred) const {
+    switch (W.sw.fdScheme) {
+      case 2: return !pred && k != 1 ? (int)VOP_AB2 : -1;
+      case 3: return pred ? (int)VOP_AM2_CORR : k != 1 ? (int)VOP_AM2_PRED : -1;
+      case 4: return pred ? (int)VOP_AM3_CORR : k != 2 ? (int)VOP_AM3_PRED : -1;
+      case 5: return pred ? (int)VOP_AM4_CORR : k > 3 ? (int)VOP_AM4_PRED : -1;
+      default: return -1;
+    }
   }
   void evalNodesFull(int k, bool pred, int M) {
     const StepPlan& pl = plans[k];
@@ -1571,7 +1581,7 @@ struct Case {
     if (started) throw StatusError(VLM_ERR_STATE, "case already started");
     aicFactor();
     launch_solve(d, s, frame(0), false, stream);
-    if (d.NW > 0) launch_shed(d, s, frame(0), d.NW + 1, false, stream);
+    if (d.NW > 0) launch_shed(d, s, frame(0), d.NW + 1, stream);
     if (W.sw.rotorForcePlot != 0) launch_loads(d, s, frame(0), chunk64, 0, stream);
     VLM_CUDA(cudaGetLastError());
     VLM_CUDA(cudaStreamSynchronize(stream));
@@ -1632,9 +1642,7 @@ struct Case {
     const double* fr = stepFrame(k);
     const bool wake = d.NW > 0 && W.sw.wakeSuppress == 0;
     if (wake) {
-      launch_shed(d, s, fr, rN, true, stream);
-      launch_age(d, s, rN, rF, stream);
-      if (W.sw.wakeDissipation == 1) launch_dissipate(d, s, rN, rF, stream);
+      launch_wake_begin(d, s, fr, rN, rF, W.sw.wakeDissipation == 1, stream);
       if (W.sw.wakeBurst != 0 && k % W.sw.wakeBurst == 0) launch_burst(d, s, rF, stream);
     }
   }
@@ -1684,83 +1692,47 @@ struct Case {
       if (predicts(k)) evalNodes(k, true);
       return;
     }
+    // axisymmetric copies and the prescribed far wake follow a convection in place
+    const bool fused = !d.axisym && d.prescNt == 0;
     if (st == 1) {
-      switch (W.sw.fdScheme) {
-        case 0:
-          convect(k, fr, rN, rF, false);
-          break;
-        case 1:
+      if (predicts(k)) {
+        if (fused) {
+          launch_predict(d, s, rN, rF, stream);
+        } else {
           launch_copy_predicted(d, s, rN, rF, stream);
           convect(k, fr, rN, rF, true);
-          break;
+        }
+        return;
+      }
+      convect(k, fr, rN, rF, false);
+      switch (W.sw.fdScheme) {
         case 2:
-          if (k == 1) {
-            convect(k, fr, rN, rF, false);
-            launch_velop(d, s, VOP_COPY_0_TO_1, stream);
-          } else {
-            launch_velop(d, s, VOP_AB2, stream);
-            convect(k, fr, rN, rF, false);
-          }
-          break;
         case 3:
-          if (k == 1) {
-            convect(k, fr, rN, rF, false);
-            launch_velop(d, s, VOP_COPY_0_TO_1, stream);
-          } else {
-            launch_copy_predicted(d, s, rN, rF, stream);
-            launch_velop(d, s, VOP_AM2_PRED, stream);
-            convect(k, fr, rN, rF, true);
-          }
+          if (k == 1) launch_velop(d, s, VOP_COPY_0_TO_1, stream);
           break;
         case 4:
-          if (k == 2) {
-            convect(k, fr, rN, rF, false);
-            launch_velop(d, s, VOP_COPY_0_TO_2, stream);
-          } else {
-            launch_copy_predicted(d, s, rN, rF, stream);
-            launch_velop(d, s, VOP_AM3_PRED, stream);
-            convect(k, fr, rN, rF, true);
-          }
+          launch_velop(d, s, VOP_COPY_0_TO_2, stream);
           break;
         case 5:
-          if (k <= 3) {
-            convect(k, fr, rN, rF, false);
-            launch_velop(d, s, k == 1 ? VOP_COPY_0_TO_1 : (k == 2 ? VOP_COPY_0_TO_2 : VOP_COPY_0_TO_3), stream);
-          } else {
-            launch_copy_predicted(d, s, rN, rF, stream);
-            launch_velop(d, s, VOP_AM4_PRED, stream);
-            convect(k, fr, rN, rF, true);
-          }
+          launch_velop(d, s, k == 1 ? VOP_COPY_0_TO_1 : (k == 2 ? VOP_COPY_0_TO_2 : VOP_COPY_0_TO_3), stream);
           break;
       }
       return;
     }
     if (predicts(k)) {
-      switch (W.sw.fdScheme) {
-        case 1:
-          launch_order2(d, s, rN, rF, stream);
-          convect(k, fr, rN, rF, false);
-          break;
-        case 3:
-          launch_velop(d, s, VOP_AM2_CORR, stream);
-          convect(k, fr, rN, rF, false);
-          launch_velop(d, s, VOP_STEP_TO_1, stream);
-          break;
-        case 4:
-          launch_velop(d, s, VOP_AM3_CORR, stream);
-          convect(k, fr, rN, rF, false);
-          launch_velop(d, s, VOP_AM3_SHIFT, stream);
-          break;
-        case 5:
-          launch_velop(d, s, VOP_AM4_CORR, stream);
-          convect(k, fr, rN, rF, false);
-          launch_velop(d, s, VOP_AM4_SHIFT, stream);
-          break;
+      const int fd = W.sw.fdScheme;
+      const int op = fd == 3 ? (int)VOP_STEP_TO_1 : fd == 4 ? (int)VOP_AM3_SHIFT : fd == 5 ? (int)VOP_AM4_SHIFT : -1;
+      if (fd == 1) launch_order2(d, s, rN, rF, stream);
+      if (fused) {
+        launch_correct(d, s, fr, rN, rF, W.sw.wakeStrain == 1, op, stream);
+        return;
       }
+      convect(k, fr, rN, rF, false);
+      if (op >= 0) launch_velop(d, s, (VelOp)op, stream);
     }
     if (W.sw.wakeStrain == 1) launch_strain(d, s, rF, stream);
     if (rN == 1) launch_rollup(d, s, rF, stream);
-    launch_shed(d, s, fr, rN, false, stream);
+    launch_shed(d, s, fr, rN, stream);
   }
 
   // ---- the time loop: inputs in, steps enqueued, results out ---------------
@@ -2620,7 +2592,7 @@ struct vlm_system {
       if (c->c.imgSrc) c->c.imageMirrorGamma();
       else launch_solve_only(c->c.d, c->c.s, st);
     }
-    for (auto& c : r) launch_shed(c->c.d, c->c.s, c->c.frame(0), c->c.d.NW + 1, false, st);
+    for (auto& c : r) launch_shed(c->c.d, c->c.s, c->c.frame(0), c->c.d.NW + 1, st);
     if (rotor(0).W.sw.rotorForcePlot != 0)
       for (auto& c : r) c->c.sysLoads(0, st);
     VLM_CUDA(cudaGetLastError());

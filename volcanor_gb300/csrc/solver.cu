@@ -29,28 +29,25 @@ __device__ __forceinline__ m33 frameT(const Dims& d, const double* fr, int b) {
 inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 
 // ---- shed (classdef.f90:4297-4325) ---------------------------------------
-__global__ void k_shed(Dims d, DevState s, const double* fr, int rowNear, int le) {
+// the trailing-edge row (the leading edge's: k_wake_begin)
+__global__ void k_shed(Dims d, DevState s, const double* fr, int rowNear) {
   after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.nb * d.ns) return;
   const int b = t / d.ns, j = t % d.ns;
   const int p = (d.nc - 1) + d.nc * j;
   const double* w = panRec(d, fr, b, p);
-  if (le) {
-    double* c = s.nC + ringI(d, b, rowNear - 1, j) * 12;
-    st3(c + 0, ld3(w + 3));
-    st3(c + 9, ld3(w + 6));
-    s.nGam[ringI(d, b, rowNear - 1, j)] = s.wGam[(size_t)b * d.npan + p];
-  } else {
-    const int r = max(rowNear - 1, 1) - 1;
-    double* c = s.nC + ringI(d, b, r, j) * 12;
-    st3(c + 3, ld3(w + 3));
-    st3(c + 6, ld3(w + 6));
-  }
+  const int r = max(rowNear - 1, 1) - 1;
+  double* c = s.nC + ringI(d, b, r, j) * 12;
+  st3(c + 3, ld3(w + 3));
+  st3(c + 6, ld3(w + 6));
 }
 
-// ---- age (classdef.f90:4331-4354) -----------------------------------------
-__global__ void k_age(Dims d, DevState s, int rowNear, int rowFar) {
+// ---- start of a step: the leading-edge row shed (classdef.f90:4297-4325), age
+// (:4331-4354) and dissipation (:4356-4408), a ring or far filament a thread.
+// A ring's third edge takes the new core radius of the row before: that row's
+// thread writes it.  (Four kernels, 9 us of a hover step, now 4.)
+__global__ void k_wake_begin(Dims d, DevState s, const double* fr, int rowNear, int rowFar, int dissip) {
   after_previous();
   const int rows = d.NW - (rowNear - 1);
   const int nNear = d.nb * rows * d.ns;
@@ -60,18 +57,120 @@ __global__ void k_age(Dims d, DevState s, int rowNear, int rowFar) {
     const int b = t / (rows * d.ns), l = t % (rows * d.ns);
     const int j = l / rows, i = rowNear - 1 + l % rows;
     const size_t r = ringI(d, b, i, j);
+    double g = s.nGam[r];
+    if (i == rowNear - 1) {
+      const int p = (d.nc - 1) + d.nc * j;
+      const double* w = panRec(d, fr, b, p);
+      st3(s.nC + r * 12, ld3(w + 3));
+      st3(s.nC + r * 12 + 9, ld3(w + 6));
+      g = s.wGam[(size_t)b * d.npan + p];
+    }
     s.nAge[r] = s.nAge[r] + d.dt;
+    if (dissip) {
+      double* rv = s.nRvc + 4 * r;
+      const double c = sqrt(rv[0] * rv[0] + d.dissipAdd), e = sqrt(rv[1] * rv[1] + d.dissipAdd);
+      rv[0] = c;
+      rv[2] = c;
+      rv[1] = e;
+      if (i + 1 < d.NW) rv[4 + 3] = e;
+      g = g * d.decay;
+    }
+    s.nGam[r] = g;
   } else if (t < nNear + nFar) {
     const int l = t - nNear;
     const int rf = d.NF - (rowFar - 1);
     const int b = l / rf, i = rowFar - 1 + l % rf;
     const size_t r = (size_t)b * d.NF + i;
     s.fAge[r] = s.fAge[r] + d.dt;
+    if (dissip) {
+      s.fRvc[r] = sqrt(s.fRvc[r] * s.fRvc[r] + d.dissipAdd);
+      s.fGam[r] = s.fGam[r] * d.decay;
+    }
   }
 }
 
-// ---- dissipation (classdef.f90:4356-4408) ----------------------------------
-__global__ void k_dissip_a(Dims d, DevState s, int rowNear, int rowFar) {
+// ---- predictor and corrector ------------------------------------------------
+// Convection moves corner 1 of every ring (and corner 2 of a row's last) by its
+// node's velocity and then copies the corners that neighbours share
+// (classdef.f90:1515-1575, 1609-1702).  These kernels form a ring's or filament's
+// new corners from the old ones of itself and its neighbours and write them
+// elsewhere, so that one pass does what the copy, the shift and the continuity
+// did one after the other.
+// node (i, j) after convection; the predicted wake moves row 1 alone
+__device__ __forceinline__ d3 moved_node(const Dims& d, const DevState& s, int b, int i, int j, bool moves) {
+  const d3 p = j < d.ns ? ld3(s.nC + ringI(d, b, i, j) * 12 + 3) : ld3(s.nC + ringI(d, b, i, d.ns - 1) * 12 + 6);
+  return moves ? p + ld3(s.vN[0] + 3 * velI(d, b, i, j)) * d.dt : p;
+}
+struct Ring4 {
+  d3 c0, c1, c2, c3;
+};
+__device__ __forceinline__ Ring4 convected(const Dims& d, const DevState& s, int b, int i, int j, int rowNear, bool pred) {
+  Ring4 o;
+  const double* c = s.nC + ringI(d, b, i, j) * 12;
+  const bool moves = !pred || i == 0, above = !pred || i - 1 == 0;
+  o.c1 = moved_node(d, s, b, i, j, moves);
+  o.c2 = moved_node(d, s, b, i, j + 1, moves);
+  if (i > rowNear - 1) {
+    o.c0 = moved_node(d, s, b, i - 1, j, above);
+    o.c3 = moved_node(d, s, b, i - 1, j + 1, above);
+  } else {
+    o.c0 = ld3(c);
+    o.c3 = ld3(c + 9);
+  }
+  return o;
+}
+// a far filament's ends after convection: the second is its predecessor's first
+__device__ __forceinline__ void convected_far(const Dims& d, const DevState& s, int b, int i, int rowFar, d3& a, d3& e) {
+  const size_t f = (size_t)b * d.NF + i;
+  a = ld3(s.fC + 6 * f) + ld3(s.vF[0] + 3 * f) * d.dt;
+  e = i > rowFar - 1 ? ld3(s.fC + 6 * (f - 1)) + ld3(s.vF[0] + 3 * (f - 1)) * d.dt : ld3(s.fC + 6 * f + 3);
+}
+__device__ __forceinline__ void put_ring(double* c, const Ring4& r) {
+  st3(c, r.c0);
+  st3(c + 3, r.c1);
+  st3(c + 6, r.c2);
+  st3(c + 9, r.c3);
+}
+
+// The predicted wake (main.f90:1012-1019 and its convection).  (Copy, shift and
+// continuity: 10 us of a hover step, now 3.4.)
+__global__ void k_predict(Dims d, DevState s, int rowNear, int rowFar) {
+  after_previous();
+  const int rows = d.NW - (rowNear - 1);
+  const int nNear = d.nb * rows * d.ns;
+  const int nFar = d.nb * max(d.NF - (rowFar - 1), 0);
+  const int nRow1 = rowNear > 1 ? d.nb * d.ns : 0;  // row 1 moves even where it is not in use
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < nNear) {
+    const int b = t / (rows * d.ns), l = t % (rows * d.ns);
+    const int j = l / rows, i = rowNear - 1 + l % rows;
+    put_ring(s.nCP + ringI(d, b, i, j) * 12, convected(d, s, b, i, j, rowNear, true));
+    return;
+  }
+  t -= nNear;
+  if (t < nFar) {
+    const int rf = d.NF - (rowFar - 1);
+    const int b = t / rf, i = rowFar - 1 + t % rf;
+    d3 a, e;
+    convected_far(d, s, b, i, rowFar, a, e);
+    double* c = s.fCP + ((size_t)b * d.NF + i) * 6;
+    st3(c, a);
+    st3(c + 3, e);
+    return;
+  }
+  t -= nFar;
+  if (t < nRow1) {
+    const int b = t / d.ns, j = t % d.ns;
+    double* c = s.nCP + ringI(d, b, 0, j) * 12;
+    st3(c + 3, ld3(c + 3) + ld3(s.vN[0] + 3 * velI(d, b, 0, j)) * d.dt);
+    if (j == d.ns - 1) st3(c + 6, ld3(c + 6) + ld3(s.vN[0] + 3 * velI(d, b, 0, d.ns)) * d.dt);
+  }
+}
+
+// The corrector's convection, out of place, with the far wake's strain
+// (classdef.f90:4410-4422, 505-521): rings into nTmp (18 doubles: corners,
+// circulation, core radii, age), far filaments into fTmp (12).
+__global__ void k_correct(Dims d, DevState s, int rowNear, int rowFar, int strain) {
   after_previous();
   const int rows = d.NW - (rowNear - 1);
   const int nNear = d.nb * rows * d.ns;
@@ -81,29 +180,142 @@ __global__ void k_dissip_a(Dims d, DevState s, int rowNear, int rowFar) {
     const int b = t / (rows * d.ns), l = t % (rows * d.ns);
     const int j = l / rows, i = rowNear - 1 + l % rows;
     const size_t r = ringI(d, b, i, j);
-    double* rv = s.nRvc + 4 * r;
-    const double a = sqrt(rv[0] * rv[0] + d.dissipAdd);
-    rv[0] = a;
-    rv[2] = a;
-    s.nGam[r] = s.nGam[r] * d.decay;
-    rv[1] = sqrt(rv[1] * rv[1] + d.dissipAdd);
+    double* o = s.nTmp + r * 18;
+    put_ring(o, convected(d, s, b, i, j, rowNear, false));
+    o[12] = s.nGam[r];
+    for (int k = 0; k < 4; ++k) o[13 + k] = s.nRvc[4 * r + k];
+    o[17] = s.nAge[r];
   } else if (t < nNear + nFar) {
     const int l = t - nNear;
     const int rf = d.NF - (rowFar - 1);
     const int b = l / rf, i = rowFar - 1 + l % rf;
-    const size_t r = (size_t)b * d.NF + i;
-    s.fRvc[r] = sqrt(s.fRvc[r] * s.fRvc[r] + d.dissipAdd);
-    s.fGam[r] = s.fGam[r] * d.decay;
+    const size_t f = (size_t)b * d.NF + i;
+    double* o = s.fTmp + f * 12;
+    d3 a, e;
+    convected_far(d, s, b, i, rowFar, a, e);
+    st3(o, a);
+    st3(o + 3, e);
+    double rv = s.fRvc[f], lc = s.fLc[f];
+    if (strain) {
+      lc = norm3(a - e);
+      rv = s.fRvc0[f] * sqrt(s.fL0[f] / lc);
+    }
+    o[6] = s.fGam[f];
+    o[7] = rv;
+    o[8] = s.fRvc0[f];
+    o[9] = s.fL0[f];
+    o[10] = lc;
+    o[11] = s.fAge[f];
   }
 }
-__global__ void k_dissip_b(Dims d, DevState s, int rowNear) {
+
+__device__ __forceinline__ void velop(const DevState& s, bool nearPart, long e, int op);
+
+// Back into the state: with row 1 in use the last row is rolled up into the far
+// wake (classdef.f90:4515-4605) and every row moves on by one (:4481-4498), the far
+// wake too when it is full (:4500-4513); the trailing-edge row is shed; the
+// velocity history moves on.  The rollup has a warp per blade: a lane for each
+// sum (the leading and trailing corner's components, the circulation, the core
+// radius), so that only the additions of one are serial.  (Convection, velocity
+// algebra, rollup, row moves and shedding in ten kernels: 36 us of a hover
+// step, now 10.)
+__global__ void k_correct_back(Dims d, DevState s, const double* fr, int rowNear, int rowFar, int op, int rollBlocks) {
   after_previous();
-  const int rows = d.NW - rowNear;  // rows rowNear+1..NW (1-based)
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (rows <= 0 || t >= d.nb * rows * d.ns) return;
-  const int b = t / (rows * d.ns), l = t % (rows * d.ns);
-  const int j = l / rows, i = rowNear + l % rows;
-  s.nRvc[4 * ringI(d, b, i, j) + 3] = s.nRvc[4 * ringI(d, b, i - 1, j) + 1];
+  const bool roll = rowNear == 1, full = roll && d.NF > 0 && rowFar == 1;
+  const int rowNext = full ? 1 : rowFar - 1;  // the far row that the rollup fills
+  if ((int)blockIdx.x < rollBlocks) {
+    const int lane = threadIdx.x & 31, b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (b >= d.nb) return;
+    auto ring = [&](int j) { return s.nTmp + ringI(d, b, d.NW - 1, j) * 18; };
+    double gamRollup = ring(d.ns - 1)[12];
+    const bool posSense = fsign1(d.omega * d.theta0) > kEps;
+    double sum = 0.0;
+    const int c = lane < 3 ? 9 + lane : lane < 6 ? 3 + lane : lane == 6 ? 12 : 15;  // of the ring's 18
+#pragma unroll 4
+    for (int is = d.rollupStart; is <= d.rollupEnd; ++is) {
+      const double* q = ring(is - 1);
+      const double g = q[12], x = q[c];
+      sum = lane == 6 ? sum + g : sum + x * g;
+      if (posSense ? g < gamRollup : g > gamRollup) gamRollup = g;
+    }
+    const double gamSum = __shfl_sync(0xffffffffu, sum, 6);
+    if (fabs(gamSum) > kEps) {
+      sum = sum / gamSum;
+    } else {
+      const double* q = ring(d.rollupEnd - 1);
+      sum = lane < 3 ? q[3 + lane] : lane < 6 ? q[3 + lane] : q[15];
+    }
+    const double x = __shfl_sync(0xffffffffu, sum, lane < 3 ? lane + 3 : lane);  // cTE
+    const double df = x - sum;                                                   // cTE - cLE, lanes 0 to 2
+    const d3 dv = mk3(__shfl_sync(0xffffffffu, df, 0), __shfl_sync(0xffffffffu, df, 1), __shfl_sync(0xffffffffu, df, 2));
+    if (d.suppressFwake == 1) gamRollup = 0.0;
+    const size_t f = (size_t)b * d.NF + (rowNext - 1);
+    if (lane < 3) {
+      s.fC[6 * f + 3 + lane] = sum;
+      s.fC[6 * f + lane] = x;
+      if (rowNext < d.NF) s.fC[6 * (f + 1) + 3 + lane] = x;
+    }
+    if (lane == 7) {
+      s.fGam[f] = gamRollup;
+      s.fAge[f] = ring(d.ns - 1)[17];
+      s.fRvc0[f] = sum;
+      s.fRvc[f] = sum;
+      const double lc = norm3(dv);
+      s.fLc[f] = lc;
+      s.fL0[f] = lc;
+    }
+    return;
+  }
+  long t = (long)(blockIdx.x - rollBlocks) * blockDim.x + threadIdx.x;
+  const int rows = d.NW - (rowNear - 1), nNear = d.nb * rows * d.ns;
+  if (t < nNear) {
+    const int b = (int)t / (rows * d.ns), l = (int)t % (rows * d.ns);
+    const int j = l / rows, i = rowNear - 1 + l % rows;
+    const size_t r = ringI(d, b, i, j);
+    const double* o = s.nTmp + (roll && i > 0 ? r - 1 : r) * 18;
+    double* c = s.nC + 12 * r;
+    const double* w = roll && i == 0 ? panRec(d, fr, b, (d.nc - 1) + d.nc * j) : nullptr;  // the shed row's trailing edge
+    st3(c, ld3(o));
+    st3(c + 3, ld3(w ? w + 3 : o + 3));
+    st3(c + 6, ld3(w ? w + 6 : o + 6));
+    st3(c + 9, ld3(o + 9));
+    if (roll) {
+      s.nGam[r] = o[12];
+      for (int k = 0; k < 4; ++k) s.nRvc[4 * r + k] = o[13 + k];
+      s.nAge[r] = i == 0 ? 0.0 : o[17];
+    }
+    return;
+  }
+  t -= nNear;
+  const int rf = max(d.NF - (rowFar - 1), 0), nFar = d.nb * rf;
+  if (t < nFar) {
+    const int b = (int)t / rf, i = rowFar - 1 + (int)t % rf;
+    const size_t f = (size_t)b * d.NF + i;
+    if (full && i == 0) return;  // the rollup's
+    const double* o = s.fTmp + (full ? f - 1 : f) * 12;
+    st3(s.fC + 6 * f, ld3(o));
+    if (!(roll && i == rowNext)) st3(s.fC + 6 * f + 3, ld3(o + 3));  // row rowNext + 1's second end is the rollup's
+    s.fGam[f] = o[6];
+    s.fRvc[f] = o[7];
+    s.fRvc0[f] = o[8];
+    s.fL0[f] = o[9];
+    s.fLc[f] = o[10];
+    s.fAge[f] = o[11];
+    return;
+  }
+  t -= nFar;
+  const int nShed = roll ? 0 : d.nb * d.ns;
+  if (t < nShed) {
+    const int b = (int)t / d.ns, j = (int)t % d.ns;
+    const double* w = panRec(d, fr, b, (d.nc - 1) + d.nc * j);
+    double* c = s.nC + ringI(d, b, rowNear - 2, j) * 12;
+    st3(c + 3, ld3(w + 3));
+    st3(c + 6, ld3(w + 6));
+    return;
+  }
+  t -= nShed;
+  const long nN = (long)d.nb * d.NW * (d.ns + 1) * 3, nF = (long)d.nb * d.NF * 3;
+  if (op >= 0 && t < nN + nF) velop(s, t < nN, t < nN ? t : t - nN, op);
 }
 
 // ---- predicted copy (main.f90:1012-1019) -----------------------------------
@@ -441,12 +653,7 @@ __global__ void k_near_from_tmp(Dims d, DevState s) {
 }
 
 // ---- velocity history algebra (main.f90:844-1406) --------------------------
-__global__ void k_velop(DevState s, long nN, long nF, int op) {
-  after_previous();
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (t >= nN + nF) return;
-  const bool nearPart = t < nN;
-  const long e = nearPart ? t : t - nN;
+__device__ __forceinline__ void velop(const DevState& s, bool nearPart, long e, int op) {
   double* a[6];
 #pragma unroll
   for (int k = 0; k < 6; ++k) a[k] = nearPart ? s.vN[k] : s.vF[k];
@@ -487,6 +694,11 @@ __global__ void k_velop(DevState s, long nN, long nF, int op) {
       a[3][e] = st;
       break;
   }
+}
+__global__ void k_velop(DevState s, long nN, long nF, int op) {
+  after_previous();
+  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (t < nN + nF) velop(s, t < nN, t < nN ? t : t - nN, op);
 }
 
 // ---- PC2 averaging (libCommon.f90:213-258) ---------------------------------
@@ -537,7 +749,7 @@ __global__ void k_order2(Dims d, DevState s, int rowNear, int rowFar, int phase)
 }
 
 __global__ void k_scatter_nodes(Dims d, DevState s, const double* fr, int rowNear, int rowFar, int pred,
-                                double initWakeVel, int addInit, int M) {
+                                double initWakeVel, int addInit, int op, int M) {
   after_previous();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= M) return;
@@ -549,8 +761,10 @@ __global__ void k_scatter_nodes(Dims d, DevState s, const double* fr, int rowNea
     if (pred || far) v = v - a;
     else v = v + a;
   }
-  double* dst = far ? s.vF[pred ? 4 : 0] + 3 * ((size_t)b * d.NF + i) : s.vN[pred ? 4 : 0] + 3 * velI(d, b, i, j);
-  st3(dst, v);
+  const size_t e = 3 * (far ? (size_t)b * d.NF + i : velI(d, b, i, j));
+  st3((far ? s.vF : s.vN)[pred ? 4 : 0] + e, v);
+  if (op >= 0)
+    for (int c = 0; c < 3; ++c) velop(s, !far, (long)e + c, op);
 }
 
 // ---- AIC and its inverse (classdef.f90:4151-4179, libMath.f90:48-83) ---------
@@ -1319,28 +1533,39 @@ __global__ void __launch_bounds__(kLoadsThreads) k_loads(Dims d, DevState s, con
 }  // namespace
 
 // ---------------------------------------------------------------------------
-void launch_shed(const Dims& d, const DevState& s, const double* frame, int rowNear, bool le, cudaStream_t st) {
+void launch_shed(const Dims& d, const DevState& s, const double* frame, int rowNear, cudaStream_t st) {
   count_launch();
-  launch_next(k_shed, nblk(d.nb * d.ns, 128), 128, 0, st, d, s, frame, rowNear, le ? 1 : 0);
+  launch_next(k_shed, nblk(d.nb * d.ns, 128), 128, 0, st, d, s, frame, rowNear);
 }
-void launch_age(const Dims& d, const DevState& s, int rowNear, int rowFar, cudaStream_t st) {
-  const long n = (long)d.nb * (d.NW - (rowNear - 1)) * d.ns + (long)d.nb * (d.NF - (rowFar - 1) > 0 ? d.NF - (rowFar - 1) : 0);
+static long wake_items(const Dims& d, int rowNear, int rowFar) {
+  return (long)d.nb * (d.NW - (rowNear - 1)) * d.ns + (long)d.nb * std::max(d.NF - (rowFar - 1), 0);
+}
+void launch_wake_begin(const Dims& d, const DevState& s, const double* frame, int rowNear, int rowFar, bool dissipate,
+                       cudaStream_t st) {
+  const long n = wake_items(d, rowNear, rowFar);
+  if (n <= 0) return;
+  count_launch();
+  launch_next(k_wake_begin, nblk(n, 128), 128, 0, st, d, s, frame, rowNear, rowFar, dissipate ? 1 : 0);
+}
+void launch_predict(const Dims& d, const DevState& s, int rowNear, int rowFar, cudaStream_t st) {
+  const long n = wake_items(d, rowNear, rowFar) + (rowNear > 1 ? (long)d.nb * d.ns : 0);
+  if (n <= 0) return;
+  count_launch();
+  launch_next(k_predict, nblk(n, 128), 128, 0, st, d, s, rowNear, rowFar);
+}
+void launch_correct(const Dims& d, const DevState& s, const double* frame, int rowNear, int rowFar, bool strain, int op,
+                    cudaStream_t st) {
+  const long n = wake_items(d, rowNear, rowFar);
   if (n > 0) {
     count_launch();
-    launch_next(k_age, nblk(n, 256), 256, 0, st, d, s, rowNear, rowFar);
+    launch_next(k_correct, nblk(n, 128), 128, 0, st, d, s, rowNear, rowFar, strain ? 1 : 0);
   }
-}
-void launch_dissipate(const Dims& d, const DevState& s, int rowNear, int rowFar, cudaStream_t st) {
-  const long n = (long)d.nb * (d.NW - (rowNear - 1)) * d.ns + (long)d.nb * (d.NF - (rowFar - 1) > 0 ? d.NF - (rowFar - 1) : 0);
-  if (n > 0) {
-    count_launch();
-    launch_next(k_dissip_a, nblk(n, 256), 256, 0, st, d, s, rowNear, rowFar);
-  }
-  const long n2 = (long)d.nb * (d.NW - rowNear) * d.ns;
-  if (n2 > 0) {
-    count_launch();
-    launch_next(k_dissip_b, nblk(n2, 256), 256, 0, st, d, s, rowNear);
-  }
+  const int rollBlocks = rowNear == 1 && d.NF > 0 ? nblk(d.nb, 4) : 0;
+  const long m = n + (rowNear > 1 ? (long)d.nb * d.ns : 0) +
+                 (op >= 0 ? (long)d.nb * d.NW * (d.ns + 1) * 3 + (long)d.nb * d.NF * 3 : 0);
+  if (m + rollBlocks <= 0) return;
+  count_launch();
+  launch_next(k_correct_back, rollBlocks + nblk(m, 128), 128, 0, st, d, s, frame, rowNear, rowFar, op, rollBlocks);
 }
 void launch_copy_predicted(const Dims& d, const DevState& s, int rowNear, int rowFar, cudaStream_t st) {
   const long n = (long)d.nbC * (d.NW - (rowNear - 1)) * d.ns + (long)d.nbC * (d.NF - (rowFar - 1) > 0 ? d.NF - (rowFar - 1) : 0);
@@ -1434,12 +1659,12 @@ int node_target_count(const Dims& d, int rowNear, int rowFar) {
   return d.nbC * (rowsN * (d.ns + 1) + rowsF);
 }
 void launch_scatter_nodes(const Dims& d, const DevState& s, const double* frame, int rowNear, int rowFar, bool pred,
-                          double initWakeVel, cudaStream_t st) {
+                          double initWakeVel, int op, cudaStream_t st) {
   const int M = node_target_count(d, rowNear, rowFar);
   const int addInit = initWakeVel != 0.0 ? 1 : 0;
   if (M > 0) {
     count_launch();
-    launch_next(k_scatter_nodes, nblk(M, 256), 256, 0, st, d, s, frame, rowNear, rowFar, pred ? 1 : 0, initWakeVel, addInit, M);
+    launch_next(k_scatter_nodes, nblk(M, 256), 256, 0, st, d, s, frame, rowNear, rowFar, pred ? 1 : 0, initWakeVel, addInit, op, M);
   }
 }
 void launch_aic(const Dims& d, const DevState& s, const double* frame, cudaStream_t st) {

@@ -121,9 +121,18 @@ struct DevState {
 };
 
 // ---- wake bookkeeping (src/classdef.f90:4297-4605, 1515-1702, 4786-4830) ----
-void launch_shed(const Dims& d, const DevState& s, const double* frame, int rowNear, bool leadingEdge, cudaStream_t st);
-void launch_age(const Dims& d, const DevState& s, int rowNear, int rowFar, cudaStream_t st);
-void launch_dissipate(const Dims& d, const DevState& s, int rowNear, int rowFar, cudaStream_t st);
+// the trailing-edge row of rows rowNear and on
+void launch_shed(const Dims& d, const DevState& s, const double* frame, int rowNear, cudaStream_t st);
+// leading-edge shed row, age and (if asked for) dissipation
+void launch_wake_begin(const Dims& d, const DevState& s, const double* frame, int rowNear, int rowFar, bool dissipate,
+                       cudaStream_t st);
+// Without axisymmetric copies or a prescribed far wake: the predicted wake
+// (launch_copy_predicted and launch_convect in one), and the corrector's
+// convection, strain, rollup, row moves and trailing-edge shedding, with
+// velocity operation op (-1: none) after the convection.
+void launch_predict(const Dims& d, const DevState& s, int rowNear, int rowFar, cudaStream_t st);
+void launch_correct(const Dims& d, const DevState& s, const double* frame, int rowNear, int rowFar, bool strain, int op,
+                    cudaStream_t st);
 void launch_copy_predicted(const Dims& d, const DevState& s, int rowNear, int rowFar, cudaStream_t st);
 // shift (pred: predicted wake with the reference's row-1 loop) + continuity + axisymmetric copies
 void launch_convect(const Dims& d, const DevState& s, const double* frame, int rowNear, int rowFar, bool pred,
@@ -174,8 +183,10 @@ void launch_gather(const Dims& d, const DevState& s, const double* frame, const 
                    int nrec, int rowNear, int rowFar, bool pred, double nearFactor, const GatherTargets& tg,
                    cudaStream_t st);
 // node velocities from outv (0 + v), plus the initial wake velocity terms
+// and velocity operation op at the nodes (-1: none; elsewhere the velocities are
+// zero, which every operation keeps)
 void launch_scatter_nodes(const Dims& d, const DevState& s, const double* frame, int rowNear, int rowFar, bool pred,
-                          double initWakeVel, cudaStream_t st);
+                          double initWakeVel, int op, cudaStream_t st);
 
 // ---- circulation and loads -----------------------------------------------
 void launch_aic(const Dims& d, const DevState& s, const double* frame, cudaStream_t st);
