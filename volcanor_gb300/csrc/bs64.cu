@@ -283,8 +283,11 @@ __global__ void __launch_bounds__(kThreadsLattice64) k_lattice64(const double* r
   }
 }
 
-// TT and K for M targets, nchunks chunks of nrec records in all, in sheets of L
-// rows (0: rings one by one): the least modelled time on a device of `sms` SMs.
+// TT and K for M targets, nchunks chunks of nrec records in all and at most
+// `largest` each, in sheets of L rows (0: rings one by one): the least modelled
+// time on a device of `sms` SMs, a run taken as long as the longest (as long as the
+// mean, a wing's short chunk beside its wake's made blocks of 8 targets of which
+// the wake's were last to end: 124 us at 336 targets of a 40-step wing, now 77).
 // A batch of a block that shares its quarters with w warps takes lat + w slope
 // cycles (fitted to sweeps over TT and K from 52 to 60000 targets and 52 to 12480
 // records; slope is its FP64 instructions, lat the chain of one evaluation),
@@ -300,9 +303,9 @@ inline size_t lattice_smem64(int lgTT, int L) {
   const int TT = 1 << lgTT, nt = kThreadsLattice64;
   return sizeof(double) * (3 * kMaxTT + (size_t)15 * nt + (size_t)6 * TT * (L + nt / TT));
 }
-Tile64 pick_tile64(int M, int nchunks, int64_t nrec, int L, int sms) {
+Tile64 pick_tile64(int M, int nchunks, int64_t nrec, int largest, int L, int sms) {
   const int nt = L > 0 ? kThreadsLattice64 : kThreads64;
-  const double C = (double)nrec / nchunks, wb = nt / 128;
+  const double wb = nt / 128;
   double best = 0.0;
   Tile64 T;
   for (int lg = 0; (1 << lg) <= kMaxTT; ++lg) {
@@ -312,7 +315,8 @@ Tile64 pick_tile64(int M, int nchunks, int64_t nrec, int L, int sms) {
     if (L > 0) bps = std::min<int>(2, (int)(kSmemPerSm64 / (lattice_smem64(lg, L) + 1024)));
     if (bps < 1) break;
     for (int k = 1;; k *= 2) {
-      const double runs = (nchunks + k - 1) / k, recs = std::min(k, nchunks) * C;
+      // a run's records: the longest, which is last to end
+      const double runs = (nchunks + k - 1) / k, recs = (double)std::min<int64_t>(nrec, (int64_t)k * largest);
       const double batches = std::ceil(recs / S) + 0.3;
       const double lat = L > 0 ? 7700 : 11500, slope = L > 0 ? 8000 + 3200 * std::min(1.0, L / recs) : 13600;
       const double add = 90.0 * std::min<double>(S, recs);
@@ -557,26 +561,26 @@ void launch_lattice64(const Tile64& T, const double* rec, const int* share, cons
 }
 }  // namespace
 
-void launch_partial64(const double* rec, const Chunk* chunks, int nchunks, int64_t nrec, const double* P, int M,
+void launch_partial64(const double* rec, const Chunk* chunks, int nchunks, int64_t nrec, int largest, const double* P, int M,
                       double* part, cudaStream_t s) {
   if (M <= 0 || nchunks <= 0) return;
   count_launch();
-  launch_rings64(pick_tile64(M, nchunks, nrec, 0, device_sm_count()), rec, chunks, nchunks, P, M, part, s);
+  launch_rings64(pick_tile64(M, nchunks, nrec, largest, 0, device_sm_count()), rec, chunks, nchunks, P, M, part, s);
 }
 
-void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunks, int nrec, const Group* groups,
+void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunks, int nrec, int largest, const Group* groups,
                               int ngroups, int L, int* share, const double* P, int M, double* part, cudaStream_t s) {
   // a sheet too tall for shared memory even with one target a block has no
   // room for a column's edges
   if (L <= 0 || lattice_smem64(0, L) + 1024 > kSmemPerSm64) {
-    launch_partial64(rec, chunks, nchunks, nrec, P, M, part, s);
+    launch_partial64(rec, chunks, nchunks, nrec, largest, P, M, part, s);
     return;
   }
   if (M <= 0 || nchunks <= 0) return;
   lattice_attr64();
   count_launches(2);
   launch_next(k_share64, (nrec + 255) / 256, 256, 0, s, rec, nrec, groups, ngroups, L, share);
-  launch_lattice64(pick_tile64(M, nchunks, nrec, L, device_sm_count()), rec, share, chunks, nchunks, L, P, M, part, s);
+  launch_lattice64(pick_tile64(M, nchunks, nrec, largest, L, device_sm_count()), rec, share, chunks, nchunks, L, P, M, part, s);
 }
 
 void launch_combine(const double* part, int M, const Group* groups, int ngroups, int mode, double* out,

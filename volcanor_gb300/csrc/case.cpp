@@ -106,11 +106,18 @@ static T* dalloc(size_t n, DevArena& owned) {
   return static_cast<T*>(owned.take(n * sizeof(T)));
 }
 
+static int largest_chunk(const Chunk* ch, int n) {
+  int c = 0;
+  for (int i = 0; i < n; ++i) c = std::max(c, (int)ch[i].rec_count);
+  return c;
+}
+
 // Source/target layout of one Biot-Savart evaluation at one step.
 struct EvalPlan {
   int goff = 0, ngroups = 0;  // into the step plan's group table
   int coff = 0, nchunks = 0;  // into the chunk table
   int nrec = 0;
+  int largest = 0;  // most records of one chunk
   int shape = 0;  // FP32 kernel tile shape (launch_partial32)
   int rows = 0;   // rows of its near-wake sheets (0: it has none)
 };
@@ -237,6 +244,7 @@ struct Case {
     if (nq < 0) throw std::runtime_error("chunk table overflow");
     hChunks.insert(hChunks.end(), tmp.begin(), tmp.begin() + nq);
     e.nchunks = nq;
+    e.largest = largest_chunk(tmp.data(), nq);
     maxRecords = std::max(maxRecords, rec);
     maxChunks = std::max(maxChunks, nq);
     maxPart = std::max(maxPart, (int64_t)std::max(nq, 1) * M);
@@ -572,8 +580,8 @@ struct Case {
 
   // FP64 chunk sums of plan e's gathered records at the M targets P
   void partial64(const EvalPlan& e, const Chunk* ch, const double* P, int M) {
-    if (s.share) launch_partial64_lattice(s.rec64, ch, e.nchunks, e.nrec, dGroups + e.goff, e.ngroups, e.rows, s.share, P, M, s.part, stream);
-    else launch_partial64(s.rec64, ch, e.nchunks, e.nrec, P, M, s.part, stream);
+    if (s.share) launch_partial64_lattice(s.rec64, ch, e.nchunks, e.nrec, e.largest, dGroups + e.goff, e.ngroups, e.rows, s.share, P, M, s.part, stream);
+    else launch_partial64(s.rec64, ch, e.nchunks, e.nrec, e.largest, P, M, s.part, stream);
   }
 
   // near zones of the FP32 records
@@ -1178,6 +1186,7 @@ struct Case {
     if (nq < 0) throw std::runtime_error("chunk table overflow");
     hChunks.insert(hChunks.end(), tmp.begin(), tmp.begin() + nq);
     e.nchunks = nq;
+    e.largest = largest_chunk(tmp.data(), nq);
     maxRecords = std::max(maxRecords, rec);
     maxChunks = std::max(maxChunks, nq);
     maxPart = std::max(maxPart, (int64_t)std::max(nq, 1) * M);
@@ -2259,7 +2268,7 @@ struct Case {
     launch_gather(d, t, frame(fi), dg, (int)g.size(), rec, rN, rF, false, nearFactor(), tg, stream);
     long long* nacc = nullptr;
     if (opt.precision == VLM_PREC_FP64) {
-      launch_partial64(rec64, dc, nq, rec, dP, (int)M, part, stream);
+      launch_partial64(rec64, dc, nq, rec, largest_chunk(ch.data(), nq), dP, (int)M, part, stream);
     } else {
       const bool nearOn = opt.precision == VLM_PREC_FP32_NEAR64;
       const size_t nb = nearOn ? near_scratch_bytes((int)M, (size_t)std::min<int64_t>(64 * M + (1 << 16), 1 << 26)) : 1;
@@ -2401,7 +2410,7 @@ static void ring_launch(RingScratch& R, const RingPlan& p, const double* corners
     if (fil) launch_fils_to_rec64(corners, rvc, gam, N, R.rec64, st);
     else launch_rings_to_rec64(corners, rvc, gam, N, R.rec64, st);
     if (precision == VLM_PREC_FP64) {
-      launch_partial64(R.rec64, chunks, p.nq, N, P, (int)M, R.part, st);
+      launch_partial64(R.rec64, chunks, p.nq, N, largest_chunk(p.ch.data(), p.nq), P, (int)M, R.part, st);
     } else {
       const bool nearOn = precision == VLM_PREC_FP32_NEAR64;
       launch_pack32(R.rec64, (int)N, nearOn ? 4.0 : 0.0, R.rec32, st);

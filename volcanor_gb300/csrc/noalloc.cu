@@ -159,7 +159,7 @@ extern "C" int vlm_biot_savart_rings_noalloc(const double* corners, const double
   if (N > 0) {
     launch_rings_to_rec64(corners, rvc, gam, N, rec64, st);
     if (precision == VLM_PREC_FP64) {
-      launch_partial64(rec64, chunks, 1, N, P, (int)M, part, st);
+      launch_partial64(rec64, chunks, 1, N, (int)N, P, (int)M, part, st);
       launch_combine(part, (int)M, group, 1, 2, V, st);
     } else {
       const bool nearOn = precision == VLM_PREC_FP32_NEAR64;

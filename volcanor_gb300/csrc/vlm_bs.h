@@ -161,13 +161,14 @@ int device_sm_count();
 
 
 // FP64 reference-arithmetic partial sums: part[(q * M + m) * 3 + k].  The
-// chunks follow one another in the record array and hold nrec records in all.
-void launch_partial64(const double* rec, const Chunk* chunks, int nchunks, int64_t nrec, const double* P, int M,
+// chunks follow one another in the record array and hold nrec records in all,
+// `largest` at most.
+void launch_partial64(const double* rec, const Chunk* chunks, int nchunks, int64_t nrec, int largest, const double* P, int M,
                       double* part, cudaStream_t s);
 // The same for groups that hold lattice sheets of L rows (rings column by
 // column): corners and filaments that neighbouring rings share are evaluated
 // once.  share: nrec ints of scratch.
-void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunks, int nrec, const Group* groups,
+void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunks, int nrec, int largest, const Group* groups,
                               int ngroups, int L, int* share, const double* P, int M, double* part, cudaStream_t s);
 // FP32 pairs with FP64 accumulation over the nrec records the chunks cover.
 // When near_scratch is non-null (near_bytes = near_scratch_bytes(M, cap) for a list of cap
