@@ -798,8 +798,13 @@ __global__ void __launch_bounds__(256) k_near_find_small(const float* rec32, int
   for (int i = threadIdx.x; i < n; i += blockDim.x) append(buf[i], slot0 + i);
 }
 
-// Detection, one warp per filament (record r, edge k).  A filament with a near zone
-// (radius z = near_factor rvc_k, from [32 + k]) is cut into np pieces no
+// Detection, one warp for two filaments (edges k and k + 2 of record r; in lattice
+// form the second is mostly absent).  A warp is a chain of dependent loads -- the
+// record, the table's slots, the targets, the list's cursor -- so what counts is
+// how many warps there are and how long the chain.  (A warp per filament, half of
+// them for absent ones, and the chunk looked up before any pair was found: 4 steps
+// of 8 uneven rotors 10.20 ms, now 10.09.)  A filament with a near zone (radius
+// z = near_factor rvc_k, from [32 + k]) is cut into np pieces no
 // longer than a cell; the lanes take the cells of each piece's box (grown by
 // 1.42 z, which holds the zone's cylinder and its extensions past the ends),
 // skip cells whose centre is farther from the piece than sqrt(2) z + half a
@@ -819,11 +824,9 @@ __global__ void __launch_bounds__(256, 4) k_near_find(const float* rec32, int nr
   after_previous();
   const size_t wid = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (wid >= (size_t)nrec * 4) return;  // whole warps leave together
-  const int r = (int)(wid >> 2), k = (int)(wid & 3);
+  if (wid >= (size_t)nrec * 2) return;  // whole warps leave together
+  const int r = (int)(wid >> 1);
   const float* R = rec32 + (size_t)r * kRec32;
-  const float thr = R[32 + k];
-  if (!(thr >= 0.f)) return;
   const GridHdr* H = reinterpret_cast<const GridHdr*>(scratch);
   const float h = grid_h(H);
   if (!(h > 0.f)) return;
@@ -833,25 +836,18 @@ __global__ void __launch_bounds__(256, 4) k_near_find(const float* rec32, int nr
   const unsigned long long* key = reinterpret_cast<const unsigned long long*>(scratch + L.key);
   const int* start = reinterpret_cast<const int*>(scratch + L.start);
   const float4* entry = reinterpret_cast<const float4*>(scratch + L.entry);
-  // the record's chunk (chunks are in record order)
-  int q = 0;
-  {
-    int hi = nchunks - 1;
-    while (q < hi) {
-      const int mid = (q + hi + 1) >> 1;
-      if (chunks[mid].rec_begin <= r) q = mid;
-      else hi = mid - 1;
-    }
-  }
+  int q = -1;  // the record's chunk, looked up when its first pair is found
   const unsigned lt = (1u << lane) - 1u;
-  {
+  for (int k = (int)(wid & 1); k < 4; k += 2) {
+    const float thr = R[32 + k];
+    if (!(thr >= 0.f)) continue;
     const int j = (k + 1) & 3;
     const float ax = R[3 * k], ay = R[3 * k + 1], az = R[3 * k + 2];
     const float bx = R[3 * j], by = R[3 * j + 1], bz = R[3 * j + 2];
     const float eev = R[24 + k];
     const float ex = bx - ax, ey = by - ay, ez = bz - az;
     const float ee = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-    if (!(ee > 0.f) || !(eev != 0.f)) return;
+    if (!(ee > 0.f) || !(eev != 0.f)) continue;
     const float len = sqrtf(ee);
     const float z = sqrtf(thr) / len;
     // near zone: distance to the line < z, projection within the segment
@@ -867,7 +863,7 @@ __global__ void __launch_bounds__(256, 4) k_near_find(const float* rec32, int nr
     if (fmaxf(ax, bx) + grow < ord_value(H->lo[0]) || fminf(ax, bx) - grow > ord_value(H->hi[0]) ||
         fmaxf(ay, by) + grow < ord_value(H->lo[1]) || fminf(ay, by) - grow > ord_value(H->hi[1]) ||
         fmaxf(az, bz) + grow < ord_value(H->lo[2]) || fminf(az, bz) - grow > ord_value(H->hi[2]))
-      return;
+      continue;
     const float reach = 1.4143f * z * 1.0001f + 0.8661f * h + 1e-6f + 4e-7f * amax;
     const float reach2 = reach * reach;
     for (int pc = 0; pc < np; ++pc) {
@@ -939,6 +935,14 @@ __global__ void __launch_bounds__(256, 4) k_near_find(const float* rec32, int nr
           }
           const unsigned mask = __ballot_sync(kFull, isnear);
           if (mask) {
+            if (q < 0) {
+              q = 0;
+              for (int hi = nchunks - 1; q < hi;) {  // chunks are in record order
+                const int mid = (q + hi + 1) >> 1;
+                if (chunks[mid].rec_begin <= r) q = mid;
+                else hi = mid - 1;
+              }
+            }
             int base_slot = 0;
             if (lane == 0) base_slot = atomicAdd(ctl + 1, __popc(mask));
             base_slot = __shfl_sync(kFull, base_slot, 0);
@@ -1167,7 +1171,7 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
     launch_next(k_tgrid_insert<1>, (M + 255) / 256, 256, 0, ns, P, M, g);
   }
   count_launches(2);
-  launch_next(k_near_find, (unsigned)(((size_t)nrec * 4 * 32 + 255) / 256), 256, 0, ns, rec32, nrec, chunks, nchunks, P, M,
+  launch_next(k_near_find, (unsigned)(((size_t)nrec * 2 * 32 + 255) / 256), 256, 0, ns, rec32, nrec, chunks, nchunks, P, M,
                                                                                g, list, cap, ctl);
   launch_next(k_near_fix, 4 * sms, 128, 0, ns, list, cap, rec32, rec64, ew, P, M, reinterpret_cast<unsigned long long*>(nacc),
                                       ctl);
