@@ -539,8 +539,8 @@ def run_reference(args):
 
 def measure_batch(args, n: int, K: int, W: int, budget_s: float = None):
     """Batched sweep: n independent uneven rotor cases (volcanor_gb300/cases.py
-    batch_sweep) advanced together; once every case is in its steady state
-    each batch step is one CUDA-graph launch.  Returns case-timesteps/s."""
+    batch_sweep) advanced together; in its steady state each
+    case replays its own step graph.  Returns case-timesteps/s."""
     from volcanor_gb300 import lib
     prec = {"fp32near": lib.PREC_FP32_NEAR64, "fp32": lib.PREC_FP32, "fp64": lib.PREC_FP64}[args.precision]
     steady = 8 * 72 + 2
@@ -578,10 +578,10 @@ def measure_batch(args, n: int, K: int, W: int, budget_s: float = None):
             "steps": K, "warmup": W, "ms_per_step": round(ms / K, 4),
             "workload": f"{n} independent rotor cases: 2-4 blades, 24-400 rings, collective 2-12 deg, advance ratio "
                         "0-0.3, wakes of 1-8 revolutions (5k-120k filaments), steady state, one CUDA-graph launch "
-                        "per batch step", "precision": args.precision,
+                        "per case and step", "precision": args.precision,
             "e2e": {"value": round(e2e, 2), "unit": "case-timesteps/s", "h2d_bytes_per_step": None,
                     "d2h_bytes_per_step": n * 80},
-            "gpu_launches": int(launches), "graph_launches_per_step": 1, "warmup_wall_s": round(warm_s, 1),
+            "gpu_launches": int(launches), "graph_launches_per_step": n, "warmup_wall_s": round(warm_s, 1),
             "clocks": clk.summary(), "ct_finite": bool(np.all(np.isfinite(rows)))}
 
 

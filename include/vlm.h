@@ -330,11 +330,10 @@ int vlm_case_profile_eval(vlm_case* c, int reps, double* ms_per_launch, double* 
  * The reference has no batch mode (nr > 1 couples rotors aerodynamically);
  * this runs ncases independent cases (each its own case files, precision
  * and options from opt) on one GPU.  A batch step enqueues every case's step
- * on the case's own stream, so their kernels run concurrently; once every
- * case is in its steady state (same near/far rows step after step), one
- * batch step is captured as one CUDA graph and replayed with one launch per
- * step.  Each case's FP32 chunk plan is made for its share of the device
- * (opt->nbody_slots, default all slots / ncases). */
+ * on the case's own stream (replayed from the case's own graph in its steady
+ * state), so their kernels run concurrently, and the steps of one call do not
+ * wait for one another's cases.  Each case's FP32 chunk plan is made for its
+ * share of the device (opt->nbody_slots, default all slots / ncases). */
 typedef struct vlm_batch vlm_batch;
 int vlm_batch_create(int ncases, const char* const* configs, const char* const* geoms, const char* const* base_dirs,
                      const vlm_options* opt, vlm_batch** out);

@@ -2759,25 +2759,20 @@ int vlm_biot_savart_filaments_device(const double* fc, const double* rvc, const 
 
 // ---------------------------------------------------------------------------
 // Batch: many independent cases advanced together.  Each case keeps its own
-// stream; a step of the batch enqueues every case's step on its stream, so
-// the cases' kernels run concurrently.  Once every case is in its steady
-// state, one step of the whole batch is captured as ONE CUDA graph (a fork
-// from the batch stream into every case stream and a join back) and
-// replayed with a single graph launch per step.  Each case's FP32 chunk plan
-// is made for its share of the device's block slots.
+// stream; a step of the batch enqueues every case's step on its stream (its own
+// step graph in its steady state), so the cases' kernels run concurrently, and
+// the steps of a call follow one another on each stream without waiting for the
+// other cases.  Each case's FP32 chunk plan is made for its share of the device's
+// block slots.
 struct vlm_batch {
   std::vector<vlm_case*> cases;
   cudaStream_t origin = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, fork = nullptr;
   std::vector<cudaEvent_t> joins;
-  cudaGraphExec_t gexec = nullptr;
-  std::vector<std::pair<int, int>> gsig;  // (rowNear, rowFar) per case of the captured step
-  long graphKernels = 0;
   double lastMs = 0.0;
 
   ~vlm_batch() {
     if (origin) cudaStreamSynchronize(origin);
-    if (gexec) cudaGraphExecDestroy(gexec);
     for (cudaEvent_t e : joins) cudaEventDestroy(e);
     for (cudaEvent_t e : {ev0, ev1, fork})
       if (e) cudaEventDestroy(e);
@@ -2798,57 +2793,6 @@ struct vlm_batch {
     }
   }
 
-  bool allSteady(int k) const {
-    for (vlm_case* c : cases)
-      if (!c->c.steadyStep(k)) return false;
-    return true;
-  }
-  // a case's first step of a signature measures its incremental predicted-wake plan (not in a graph)
-  bool anyMeasureDue(int k) const {
-    for (vlm_case* c : cases)
-      if (c->c.incrMeasureDue(k)) return true;
-    return false;
-  }
-
-  void capture(int k) {
-    if (gexec) cudaGraphExecDestroy(gexec);
-    gexec = nullptr;
-    cudaGraph_t g = nullptr;
-    const long l0 = launch_count();
-    VLM_CUDA(cudaStreamBeginCapture(origin, cudaStreamCaptureModeThreadLocal));
-    try {
-      forkAll();
-      for (vlm_case* c : cases) {
-        Case& C = c->c;
-        C.replaying = true;
-        launch_step_begin(C.d, C.s, C.stream);
-        C.enqueueStep(k);
-        C.replaying = false;
-      }
-      joinAll();
-    } catch (...) {
-      for (vlm_case* c : cases) c->c.replaying = false;
-      cudaStreamEndCapture(origin, &g);
-      if (g) cudaGraphDestroy(g);
-      throw;
-    }
-    VLM_CUDA(cudaStreamEndCapture(origin, &g));
-    const cudaError_t e = cudaGraphInstantiate(&gexec, g, kGraphFlags);
-    cudaGraphDestroy(g);
-    VLM_CUDA(e);
-    graphKernels = launch_count() - l0;
-    count_launches(-graphKernels);
-    gsig.clear();
-    for (vlm_case* c : cases) gsig.emplace_back(c->c.plans[k].rowNear, c->c.plans[k].rowFar);
-  }
-
-  bool sigMatches(int k) const {
-    if (!gexec || gsig.size() != cases.size()) return false;
-    for (size_t i = 0; i < cases.size(); ++i)
-      if (gsig[i] != std::make_pair(cases[i]->c.plans[k].rowNear, cases[i]->c.plans[k].rowFar)) return false;
-    return true;
-  }
-
   void step(int nsteps, double* ctRows) {
     if (cases.empty()) return;
     cases[0]->c.useDevice();
@@ -2860,26 +2804,13 @@ struct vlm_batch {
     for (vlm_case* c : cases) c->c.uploadFrames(nsteps);
     VLM_CUDA(cudaEventRecord(ev0, origin));
     joinAll();  // the frames are in
-    for (int k = it0 + 1; k <= it0 + nsteps; ++k) {
-      if (allSteady(k) && !anyMeasureDue(k)) {
-        if (!sigMatches(k)) capture(k);
-        // device step counters for replay (the graph advances them)
-        for (vlm_case* c : cases) {
-          Case& C = c->c;
-          if (!C.iterSynced) {
-            *C.hIter = k - 1;
-            VLM_CUDA(cudaMemcpyAsync(C.s.devIter, C.hIter, sizeof(int), cudaMemcpyHostToDevice, origin));
-            C.iterSynced = true;
-          }
-        }
-        VLM_CUDA(cudaGraphLaunch(gexec, origin));
-        count_launches(graphKernels);
-      } else {
-        forkAll();
-        for (vlm_case* c : cases) c->c.enqueueOne(k);
-        joinAll();
-      }
-    }
+    // every case on its own stream, with no meeting point between steps: uneven
+    // cases drift apart and fill each other's small kernels (8 uneven rotors, one graph
+    // for all and a meeting point each step: 4 steps 10.09 ms, now 9.91)
+    forkAll();
+    for (int k = it0 + 1; k <= it0 + nsteps; ++k)
+      for (vlm_case* c : cases) c->c.enqueueOne(k);
+    joinAll();
     forkAll();  // later work on the case streams follows the batch's steps
     VLM_CUDA(cudaEventRecord(ev1, origin));
     VLM_CUDA(cudaGetLastError());

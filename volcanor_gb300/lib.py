@@ -584,8 +584,8 @@ class System:
 
 
 class Batch:
-    """Many independent cases advanced together (one graph launch per step in
-    steady state); cases = [(config_text, geom_text, base_dir), ...]."""
+    """Many independent cases advanced together (each replaying its own
+    step graph in steady state); cases = [(config_text, geom_text, base_dir), ...]."""
 
     def __init__(self, cases, precision: int = PREC_FP64, sum_chunk: Optional[int] = None,
                  nbody_slots: int = 0, use_graph: bool = True, lattice: Optional[bool] = None,
