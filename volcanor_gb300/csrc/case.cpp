@@ -979,9 +979,8 @@ struct Case {
     tg.zero[1] = incrCtl + 1;
     launch_gather(d, sp, stepFrame(k), dGroups + e.goff, e.ngroups, e.nrec, pl.rowNear, pl.rowFar, true, nearFactor(),
                   tg, stream);
-    launch_diff_count(recP, s.rec64, kRec64, sp.edgeW, s.edgeW, e.nrec, incrBlk, incrCnt, stream);
-    launch_diff_count(tgtP, s.targets, 3, nullptr, nullptr, M, incrBlk + incr_diff_blocks(e.nrec), incrCnt + 1,
-                      stream);
+    launch_diff_count(recP, s.rec64, sp.edgeW, s.edgeW, e.nrec, incrBlk, incrCnt, tgtP, s.targets, M,
+                      incrBlk + incr_diff_blocks(e.nrec), incrCnt + 1, stream);
   }
   static int roundUp(int x, int m) { return (x + m - 1) / m * m; }
   void measureIncr(int k, int M) {

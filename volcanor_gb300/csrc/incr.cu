@@ -29,17 +29,20 @@ constexpr int kDiffThreads = 128;
 constexpr int kDiffItems = 2;  // items per thread per block tile
 constexpr int kDiffTile = kDiffThreads * kDiffItems;
 
-__device__ __forceinline__ bool same_bits(const double* a, const double* b, int n) {
-  for (int k = 0; k < n; ++k)
-    if (__double_as_longlong(a[k]) != __double_as_longlong(b[k])) return false;
-  return true;
+// item i of N doubles differs between the two sets
+template <int N>
+__device__ __forceinline__ bool item_differs(const double* a, const double* b, int i) {
+  unsigned long long x = 0;
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    x |= (unsigned long long)__double_as_longlong(a[(size_t)i * N + k]) ^
+         (unsigned long long)__double_as_longlong(b[(size_t)i * N + k]);
+  return x != 0;
 }
-// item i differs between the two sets: its `stride` doubles, or its 4 edge
-// weights when the sets carry them
-__device__ __forceinline__ bool item_changed(const double* a, const double* b, int stride, const double* ea,
-                                             const double* eb, int i) {
-  if (!same_bits(a + (size_t)i * stride, b + (size_t)i * stride, stride)) return true;
-  return ea && !same_bits(ea + 4 * (size_t)i, eb + 4 * (size_t)i, 4);
+// record i differs: its doubles, or its 4 edge weights when the sets carry them
+__device__ __forceinline__ bool record_differs(const double* a, const double* b, const double* ea, const double* eb, int i) {
+  const bool f = item_differs<kRec64>(a, b, i);
+  return ea ? f | item_differs<4>(ea, eb, i) : f;
 }
 
 // exclusive prefix of f over the block's threads in thread order; *total =
@@ -60,29 +63,42 @@ __device__ __forceinline__ int block_prefix(bool f, int* warpTot, int* total) {
   return before + __popc(b & ((1u << lane) - 1u));
 }
 
-// per block tile of kDiffTile items: the number that changed
-__global__ void __launch_bounds__(kDiffThreads) k_diff_count(const double* a, const double* b,
-                                                             int stride, const double* ea,
-                                                             const double* eb, int n,
-                                                             int* blockCount) {
+// Two sets of items compared in one launch: records (with their edge weights, or
+// none) and targets.
+struct DiffSet {
+  const double *a, *b, *ea, *eb;
+  int n, blocks;
+  int *blockCount, *total;
+};
+
+// per block tile of kDiffTile items: the number that changed (the records' tiles
+// first).  All of an item's words are compared, in loads that do not wait for one
+// another; leaving at the first difference made a chain of them (the counts and
+// scans of a hover step's two sets, four launches: 14 us, now two of 6).
+__global__ void __launch_bounds__(kDiffThreads) k_diff_count(DiffSet rec, DiffSet tgt) {
   after_previous();
   __shared__ int warpTot[kDiffThreads / 32];
-  const int base = blockIdx.x * kDiffTile;
+  const bool isRec = (int)blockIdx.x < rec.blocks;
+  const int block = isRec ? blockIdx.x : blockIdx.x - rec.blocks;
   int cnt = 0;
   for (int u = 0; u < kDiffItems; ++u) {
-    const int i = base + u * kDiffThreads + threadIdx.x;
+    const int i = block * kDiffTile + u * kDiffThreads + threadIdx.x;
+    bool f = false;
+    if (isRec) f = i < rec.n && record_differs(rec.a, rec.b, rec.ea, rec.eb, i);
+    else f = i < tgt.n && item_differs<3>(tgt.a, tgt.b, i);
     int tot = 0;
-    block_prefix(i < n && item_changed(a, b, stride, ea, eb, i), warpTot, &tot);
+    block_prefix(f, warpTot, &tot);
     cnt += tot;
   }
-  if (threadIdx.x == 0) blockCount[blockIdx.x] = cnt;
+  if (threadIdx.x == 0) (isRec ? rec : tgt).blockCount[block] = cnt;
 }
 
-// exclusive scan of the block counts in place (one block); *total = their sum
-__global__ void __launch_bounds__(kDiffThreads) k_diff_scan(int* blockCount, int nb,
-                                                            int* total) {
+// exclusive scan of the block counts in place (block 0 the records', 1 the targets'); *total = their sum
+__global__ void __launch_bounds__(kDiffThreads) k_diff_scan(DiffSet rec, DiffSet tgt) {
   after_previous();
   __shared__ int sh[kDiffThreads];
+  int* blockCount = blockIdx.x == 0 ? rec.blockCount : tgt.blockCount;
+  const int nb = blockIdx.x == 0 ? rec.blocks : tgt.blocks;
   int carry = 0;
   for (int base = 0; base < nb; base += kDiffThreads) {
     const int i = base + threadIdx.x;
@@ -100,7 +116,7 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_scan(int* blockCount, int
     carry += sh[kDiffThreads - 1];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *total = carry;
+  if (threadIdx.x == 0) *(blockIdx.x == 0 ? rec.total : tgt.total) = carry;
 }
 
 // The delta record set: changed record r (o-th in index order) -> slot 2o its
@@ -123,7 +139,7 @@ __global__ void __launch_bounds__(kDiffThreads)
   const int base = blockIdx.x * kDiffTile;
   for (int u = 0; u < kDiffItems; ++u) {
     const int r = base + u * kDiffThreads + threadIdx.x;
-    const bool f = r < nrec && item_changed(recP, recC, kRec64, ewP, ewC, r);
+    const bool f = r < nrec && record_differs(recP, recC, ewP, ewC, r);
     int tot = 0;
     const int p = block_prefix(f, warpTot, &tot);
     const int o = off + p;
@@ -177,7 +193,7 @@ __global__ void __launch_bounds__(kDiffThreads)
   const int base = blockIdx.x * kDiffTile;
   for (int u = 0; u < kDiffItems; ++u) {
     const int m = base + u * kDiffThreads + threadIdx.x;
-    const bool f = m < M && item_changed(tP, tC, 3, nullptr, nullptr, m);
+    const bool f = m < M && item_differs<3>(tP, tC, m);
     int tot = 0;
     const int p = block_prefix(f, warpTot, &tot);
     const int o = off + p;
@@ -214,17 +230,16 @@ inline int diff_blocks(int n) { return (n + kDiffTile - 1) / kDiffTile; }
 
 int incr_diff_blocks(int n) { return n > 0 ? diff_blocks(n) : 0; }
 
-void launch_diff_count(const double* a, const double* b, int stride, const double* ea, const double* eb, int n,
-                       int* blockCount, int* total, cudaStream_t s) {
-  const int nb = diff_blocks(n);
-  if (nb <= 0) {
-    cudaMemsetAsync(total, 0, sizeof(int), s);
-    return;
+void launch_diff_count(const double* recA, const double* recB, const double* ea, const double* eb, int nrec, int* blockR,
+                       int* totalR, const double* tA, const double* tB, int M, int* blockT, int* totalT, cudaStream_t s) {
+  const DiffSet rec{recA, recB, ea, eb, nrec, incr_diff_blocks(nrec), blockR, totalR};
+  const DiffSet tgt{tA, tB, nullptr, nullptr, M, incr_diff_blocks(M), blockT, totalT};
+  if (rec.blocks + tgt.blocks > 0) {
+    count_launch();
+    launch_next(k_diff_count, rec.blocks + tgt.blocks, kDiffThreads, 0, s, rec, tgt);
   }
   count_launch();
-  launch_next(k_diff_count, nb, kDiffThreads, 0, s, a, b, stride, ea, eb, n, blockCount);
-  count_launch();
-  launch_next(k_diff_scan, 1, kDiffThreads, 0, s, blockCount, nb, total);
+  launch_next(k_diff_scan, 2, kDiffThreads, 0, s, rec, tgt);
 }
 
 void launch_delta_records(const double* recP, const double* recC, const double* ewP, const double* ewC, int nrec,

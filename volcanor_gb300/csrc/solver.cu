@@ -1687,7 +1687,7 @@ void launch_solve(const Dims& d, const DevState& s, const double* frame, bool wi
 }
 void launch_step_begin(const Dims& d, const DevState& s, cudaStream_t st) {
   count_launch();
-  launch_next(k_step_begin, 1, 256, 0, st, d, s);
+  launch_next(k_step_begin, 1, 1024, 0, st, d, s);
 }
 void launch_rhs_terms(const Dims& d, const DevState& s, const double* frame, const double* terms, int nterms,
                       cudaStream_t st) {

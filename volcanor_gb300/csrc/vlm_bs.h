@@ -223,12 +223,13 @@ void launch_combine_terms(const double* part, long long* nacc, int M, const Grou
                           int nchunks, int nterms, int mode, bool ordered, double* out, cudaStream_t s);
 
 // Incremental predicted-wake evaluation (incr.cu).  Items of two sets that
-// differ bit by bit (records: kRec64 doubles and, with ea/eb, 4 edge weights;
-// targets: 3 doubles): launch_diff_count leaves per-tile exclusive offsets in
-// blockCount (incr_diff_blocks(n) entries) and the number in *total.
+// differ bit by bit, records (kRec64 doubles and, with ea/eb, 4 edge weights) and
+// targets (3 doubles): launch_diff_count leaves per-tile exclusive offsets in
+// blockR and blockT (incr_diff_blocks(n) entries each) and the numbers in *totalR
+// and *totalT.
 int incr_diff_blocks(int n);
-void launch_diff_count(const double* a, const double* b, int stride, const double* ea, const double* eb, int n,
-                       int* blockCount, int* total, cudaStream_t s);
+void launch_diff_count(const double* recA, const double* recB, const double* ea, const double* eb, int nrec, int* blockR,
+                       int* totalR, const double* tA, const double* tB, int M, int* blockT, int* totalT, cudaStream_t s);
 // The delta set of the changed records (predicted +, current with negated
 // circulation -), padded to cap (even) with inert records; ctl = 5 when more
 // than cap / 2 records changed.
