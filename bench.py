@@ -356,7 +356,7 @@ def run_ours(args):
                      "traffic_note": "DRAM bytes per launch from the ncu capture summarised in "
                                      f"profiles/k_partial32_hover2_steady_{args.precision}.txt; the working set "
                                      "(sources, targets, partials) stays in L2",
-                     "kernel": "k_partial32" if prec != lib.PREC_FP64 else "k_partial64",
+                     "kernel": "k_partial32" if prec != lib.PREC_FP64 else "k_lattice64",
                      "ms_per_launch": round(ms_l, 4), "ring_pairs_per_launch": rp, "fil_pairs_per_launch": fp,
                      "near_pairs_per_launch": near_pairs, "chunks": node_chunks, "autotune": tune,
                      "executed_tflops": round(exec_flops / (ms_l / 1e3) / 1e12, 3),
