@@ -364,7 +364,7 @@ int vlm_batch_last_step_ms(vlm_batch* b, double* ms);
  * VLM_ERR_UNSUPPORTED.  Rotor ir > 0
  * is initialised with dt, nt and the switches as rotor ir - 1 left them
  * (rotor_init's intent(inout) arguments, src/classdef.f90:2778-3011).  opt
- * applies to every rotor; all rotors run on one stream; no graph replay.
+ * applies to every rotor; every lifting rotor has a stream; no graph replay.
  * A rotor's vlm_case handle (vlm_system_rotor) serves the getters, files and
  * checkpoint saves; stepping, phase, surrogate, point-query and checkpoint
  * load calls on it return VLM_ERR_STATE. */

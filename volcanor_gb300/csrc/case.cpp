@@ -133,7 +133,8 @@ struct Case {
   DevState s{};
   DevArena owned;
   cudaStream_t stream = nullptr;
-  bool ownStream = true;  // false for the rotors of a system after the first (one stream for all)
+  bool ownStream = true;  // false for a system's image rotors (their source's stream)
+  cudaEvent_t meetEv = nullptr;  // of a system's rotor
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // the loads (CT row) of a step only read the solution and feed no later
   // part of the step: they run on a side stream, joined at the step's end
@@ -184,6 +185,7 @@ struct Case {
     if (side) cudaStreamSynchronize(side);
     if (evFork) cudaEventDestroy(evFork);
     if (evJoin) cudaEventDestroy(evJoin);
+    if (meetEv) cudaEventDestroy(meetEv);
     if (side) cudaStreamDestroy(side);
     if (nearOv.stream) cudaStreamSynchronize(nearOv.stream);
     if (nearOv.fork) cudaEventDestroy(nearOv.fork);
@@ -315,6 +317,7 @@ struct Case {
     VLM_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
     VLM_CUDA(cudaEventCreateWithFlags(&evFork, cudaEventDisableTiming));
     VLM_CUDA(cudaEventCreateWithFlags(&evJoin, cudaEventDisableTiming));
+    VLM_CUDA(cudaEventCreateWithFlags(&meetEv, cudaEventDisableTiming));
     createNearStream(&nearOv.stream);
     VLM_CUDA(cudaEventCreateWithFlags(&nearOv.fork, cudaEventDisableTiming));
     VLM_CUDA(cudaEventCreateWithFlags(&nearOv.join, cudaEventDisableTiming));
@@ -1273,7 +1276,7 @@ struct Case {
   }
   // As a lone case's (enqueueStepBody): each rotor's loads on its side stream
   // beside the wake update, joined at the step's end, before the next solutions
-  // replace what they read.  One after the other on the system's stream they were
+  // replace what they read.  One after the other on the rotors' streams they were
   // half of a step of two small rotors (8 rotor-steps 2.23 ms, now 1.80).
   void forkSysLoads(int k) {
     VLM_CUDA(cudaEventRecord(evFork, stream));
@@ -2537,9 +2540,13 @@ struct vlm_case {
   Case c;
 };
 
-// Coupled rotors (nr > 1): rotor(1..nr) of src/main.f90, each a Case on one
-// stream, advanced with every do-ir loop of the reference's iteration run
-// over the rotors in turn (src/main.f90:400-1452).
+// Coupled rotors (nr > 1): rotor(1..nr) of src/main.f90, each a Case, advanced
+// with every do-ir loop of the reference's iteration run over the rotors in turn
+// (src/main.f90:400-1452).  Within a loop the rotors only read one another, so
+// each lifting rotor has its own stream (an image shares its source's, which it
+// mirrors after it in every loop) and the streams meet between the loops; on one
+// stream the small kernels of the rotors ran one after the
+// other (8 coaxial rotor-steps 1.57 ms, now 1.18).
 struct vlm_system {
   std::vector<std::unique_ptr<vlm_case>> r;
   int iter = 0;
@@ -2548,9 +2555,26 @@ struct vlm_system {
 
   Case& rotor(int i) { return r[i]->c; }
   cudaStream_t stream() { return r[0]->c.stream; }
-  // rotor 0 owns the stream the others use: release them first
+  // the rotors read one another's arrays and images use their source's stream:
+  // every stream finished, then the last rotor first
   ~vlm_system() {
+    for (auto& c : r) {
+      if (c->c.stream) cudaStreamSynchronize(c->c.stream);
+      if (c->c.side) cudaStreamSynchronize(c->c.side);
+    }
     while (!r.empty()) r.pop_back();
+  }
+  // every rotor's later work waits for all rotors' work so far
+  void meet() {
+    int streams = 0;
+    for (auto& c : r) streams += c->c.ownStream;
+    if (streams < 2) return;
+    for (auto& c : r)
+      if (c->c.ownStream) VLM_CUDA(cudaEventRecord(c->c.meetEv, c->c.stream));
+    for (auto& c : r)
+      if (c->c.ownStream)
+        for (auto& o : r)
+          if (o != c && o->c.ownStream) VLM_CUDA(cudaStreamWaitEvent(c->c.stream, o->c.meetEv, 0));
   }
 
   void create(const std::string& cfg, const std::vector<std::string>& geoms, const std::string& base,
@@ -2569,7 +2593,7 @@ struct vlm_system {
         src = &rotor(sr - 1);
       }
       auto c = std::make_unique<vlm_case>();
-      c->c.create(cfg, geoms[ir], base, o, ir ? &rotor(ir - 1) : nullptr, true, ir ? stream() : nullptr, src);
+      c->c.create(cfg, geoms[ir], base, o, ir ? &rotor(ir - 1) : nullptr, true, src ? src->stream : nullptr, src);
       if (c->c.W.nr != nr)
         throw StatusError(VLM_ERR_INVALID, "config.nml nr = " + std::to_string(c->c.W.nr) + " but " +
                                                std::to_string(nr) + " rotor geometries");
@@ -2591,18 +2615,20 @@ struct vlm_system {
     if (started) throw StatusError(VLM_ERR_STATE, "system already started");
     for (auto& c : r)
       if (!c->c.imgSrc) c->c.aicFactor();
-    cudaStream_t st = stream();
     for (auto& c : r) {
       if (c->c.imgSrc) c->c.imageMirrorVelCP();
       else c->c.sysRhsPhase(0);
     }
+    meet();
     for (auto& c : r) {
       if (c->c.imgSrc) c->c.imageMirrorGamma();
-      else launch_solve_only(c->c.d, c->c.s, st);
+      else launch_solve_only(c->c.d, c->c.s, c->c.stream);
     }
-    for (auto& c : r) launch_shed(c->c.d, c->c.s, c->c.frame(0), c->c.d.NW + 1, st);
+    meet();
+    for (auto& c : r) launch_shed(c->c.d, c->c.s, c->c.frame(0), c->c.d.NW + 1, c->c.stream);
     if (rotor(0).W.sw.rotorForcePlot != 0)
-      for (auto& c : r) c->c.sysLoads(0, st);
+      for (auto& c : r) c->c.sysLoads(0, c->c.stream);
+    meet();
     VLM_CUDA(cudaGetLastError());
     for (auto& c : r) c->c.finishSteps(0, nullptr);
     for (auto& c : r) {
@@ -2625,25 +2651,31 @@ struct vlm_system {
     VLM_CUDA(cudaEventRecord(c0.ev0, st));
     for (int k = iter + 1; k <= iter + nsteps; ++k) {
       for (auto& c : r) c->c.prePhase(k);
+      meet();
       for (auto& c : r) {
         if (c->c.imgSrc) c->c.imageMirrorVelCP();
         else c->c.sysRhsPhase(k);
       }
+      meet();
       for (auto& c : r) {
         if (c->c.imgSrc) c->c.imageMirrorGamma();
-        else launch_solve_only(c->c.d, c->c.s, st);
+        else launch_solve_only(c->c.d, c->c.s, c->c.stream);
       }
+      meet();
       const bool loads = sw.rotorForcePlot != 0 && k % sw.rotorForcePlot == 0;
       if (loads)
         for (auto& c : r) c->c.forkSysLoads(k);
       if (sw.wakeSuppress == 0)
-        for (int stg = 0; stg < 4; ++stg)
+        for (int stg = 0; stg < 4; ++stg) {
           for (auto& c : r) {
             if (c->c.imgSrc) c->c.imageWakeStage(k, stg);
             else c->c.wakeStage(k, stg);
           }
+          if (stg < 3) meet();
+        }
       if (loads)
-        for (auto& c : r) VLM_CUDA(cudaStreamWaitEvent(st, c->c.evJoin, 0));
+        for (auto& c : r) VLM_CUDA(cudaStreamWaitEvent(c->c.stream, c->c.evJoin, 0));
+      meet();
     }
     VLM_CUDA(cudaEventRecord(c0.ev1, st));
     VLM_CUDA(cudaGetLastError());
@@ -2981,7 +3013,6 @@ int vlm_system_create_from_dir(const char* case_dir, const vlm_options* opt, vlm
 }
 
 int vlm_system_destroy(vlm_system* y) {
-  if (y && !y->r.empty()) cudaStreamSynchronize(y->stream());
   delete y;
   return VLM_OK;
 }
