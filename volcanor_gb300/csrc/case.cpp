@@ -1090,7 +1090,7 @@ struct Case {
   }
 
   // ---- coupled rotors (nr > 1, vlm_system) ----------------------------------
-  // Every rotor of a system is a Case on the system's one stream.  Its RHS
+  // Every rotor of a system is a Case.  Its RHS
   // and wake-node evaluations sum the records of every rotor: each source
   // rotor's records are gathered from that rotor's state into a segment of
   // this rotor's record array, and the group table carries the per-rotor
