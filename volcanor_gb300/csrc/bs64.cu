@@ -55,43 +55,6 @@ __device__ __forceinline__ bool skipped(const double* R) {
 }
 static_assert(REC_FIL == 1 && REC_SKIP == 2, "flag words");
 
-constexpr int kShareC3 = 1, kShareE3 = 2, kShareC1 = 4, kShareE0 = 8;
-__device__ __forceinline__ bool same_point(const double* a, const double* b) {
-  return __double_as_longlong(a[0]) == __double_as_longlong(b[0]) &&
-         __double_as_longlong(a[1]) == __double_as_longlong(b[1]) &&
-         __double_as_longlong(a[2]) == __double_as_longlong(b[2]);
-}
-__global__ void k_share64(const double* rec, int nrec, const Group* groups, int ngroups,
-                          int L, int* share) {
-  after_previous();
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nrec) return;
-  int g = 0;
-  while (g + 1 < ngroups && r >= groups[g + 1].rec_begin) ++g;
-  const int first = groups[g].rec_begin;
-  const double* R = rec + (size_t)r * kRec64;
-  int b = 0;
-  if (!is_fil(R)) {
-    if (r - 1 >= first) {
-      const double* A = R - kRec64;
-      if (!is_fil(A) && same_point(R + 9, A + 6)) {
-        b |= kShareC3;
-        if (same_point(R, A + 3) && __double_as_longlong(R[15]) == __double_as_longlong(A[13])) b |= kShareE3;
-      }
-    }
-    if (r - L >= first) {
-      const double* A = R - (size_t)L * kRec64;
-      if (!is_fil(A) && same_point(R + 3, A + 6)) {
-        b |= kShareC1;
-        if (same_point(R, A + 9) && __double_as_longlong(R[12]) == __double_as_longlong(A[14])) b |= kShareE0;
-      }
-    }
-  }
-  share[r] = b;
-}
-
-// One record's contribution (velocity times circulation) at target p; zero
-// for a record the reference skips, which leaves an ordered sum unchanged.
 __device__ __forceinline__ d3 contribution64(const exact64::Unit& u, d3 p, const double* __restrict__ R) {
   if (skipped(R)) return zero3();
   d3 v;
@@ -568,8 +531,8 @@ void launch_partial64(const double* rec, const Chunk* chunks, int nchunks, int64
   launch_rings64(pick_tile64(M, nchunks, nrec, largest, 0, device_sm_count()), rec, chunks, nchunks, P, M, part, s);
 }
 
-void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunks, int nrec, int largest, const Group* groups,
-                              int ngroups, int L, int* share, const double* P, int M, double* part, cudaStream_t s) {
+void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunks, int nrec, int largest, int L,
+                              const int* share, const double* P, int M, double* part, cudaStream_t s) {
   // a sheet too tall for shared memory even with one target a block has no
   // room for a column's edges
   if (L <= 0 || lattice_smem64(0, L) + 1024 > kSmemPerSm64) {
@@ -578,8 +541,7 @@ void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunk
   }
   if (M <= 0 || nchunks <= 0) return;
   lattice_attr64();
-  count_launches(2);
-  launch_next(k_share64, (nrec + 255) / 256, 256, 0, s, rec, nrec, groups, ngroups, L, share);
+  count_launch();
   launch_lattice64(pick_tile64(M, nchunks, nrec, largest, L, device_sm_count()), rec, share, chunks, nchunks, L, P, M, part, s);
 }
 

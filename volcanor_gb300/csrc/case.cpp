@@ -583,7 +583,7 @@ struct Case {
 
   // FP64 chunk sums of plan e's gathered records at the M targets P
   void partial64(const EvalPlan& e, const Chunk* ch, const double* P, int M) {
-    if (s.share) launch_partial64_lattice(s.rec64, ch, e.nchunks, e.nrec, e.largest, dGroups + e.goff, e.ngroups, e.rows, s.share, P, M, s.part, stream);
+    if (s.share) launch_partial64_lattice(s.rec64, ch, e.nchunks, e.nrec, e.largest, e.rows, s.share, P, M, s.part, stream);
     else launch_partial64(s.rec64, ch, e.nchunks, e.nrec, e.largest, P, M, s.part, stream);
   }
 
@@ -597,7 +597,7 @@ struct Case {
     tg.P = P;
     tg.M = M;
     tg.zero[0] = s.err + 3;
-    launch_gather(d, s, fr, dGroups + e.goff, e.ngroups, e.nrec, rN, rF, pred, nearFactor(), tg, stream);
+    launch_gather(d, s, fr, dGroups + e.goff, e.ngroups, e.nrec, rN, rF, pred, nearFactor(), e.rows, tg, stream);
   }
 
   // one Biot-Savart evaluation of plan e (its records already gathered) at the
@@ -981,7 +981,7 @@ struct Case {
     tg.zero[0] = s.err + 3;
     tg.zero[1] = incrCtl + 1;
     launch_gather(d, sp, stepFrame(k), dGroups + e.goff, e.ngroups, e.nrec, pl.rowNear, pl.rowFar, true, nearFactor(),
-                  tg, stream);
+                  0, tg, stream);
     launch_diff_count(recP, s.rec64, sp.edgeW, s.edgeW, e.nrec, incrBlk, incrCnt, tgtP, s.targets, M,
                       incrBlk + incr_diff_blocks(e.nrec), incrCnt + 1, stream);
   }
@@ -1222,6 +1222,7 @@ struct Case {
       sj.rec64 = s.rec64 + (size_t)g.recOff * kRec64;
       sj.edgeW = s.edgeW ? s.edgeW + 4 * (size_t)g.recOff : nullptr;
       sj.rec32 = s.rec32 ? s.rec32 + (size_t)g.recOff * kRec32 : nullptr;
+      sj.share = s.share ? s.share + g.recOff : nullptr;
       GatherTargets tg;
       tg.zero[0] = s.err + 3;
       if (g.jr == self) {
@@ -1231,14 +1232,14 @@ struct Case {
         placed = true;
       }
       launch_gather(o.d, sj, o.frame(fk), dGroups + g.lgoff, g.lng, g.nrec, o.plans[k].rowNear, o.plans[k].rowFar,
-                    pred, nearFactor(), tg, stream);
+                    pred, nearFactor(), se.e.rows, tg, stream);
     }
     if (!placed) {  // this rotor is no source (the initial solution): targets alone
       GatherTargets tg;
       tg.kind = kind;
       tg.P = s.targets;
       tg.M = M;
-      launch_gather(d, s, frame(fk), dGroups, 0, 0, plans[k].rowNear, plans[k].rowFar, pred, 0.0, tg, stream);
+      launch_gather(d, s, frame(fk), dGroups, 0, 0, plans[k].rowNear, plans[k].rowFar, pred, 0.0, 0, tg, stream);
     }
   }
   // velCP and the RHS at step k (frame k; k = 0: the initial solution)
@@ -2264,10 +2265,11 @@ struct Case {
     DevState t = s;
     t.rec64 = rec64;
     t.edgeW = nullptr;  // ring by ring: the probe's record count is not the plans'
+    t.share = nullptr;
     t.rec32 = opt.precision == VLM_PREC_FP64 ? nullptr : rec32;
     GatherTargets tg;
     tg.zero[0] = s.err + 3;
-    launch_gather(d, t, frame(fi), dg, (int)g.size(), rec, rN, rF, false, nearFactor(), tg, stream);
+    launch_gather(d, t, frame(fi), dg, (int)g.size(), rec, rN, rF, false, nearFactor(), 0, tg, stream);
     long long* nacc = nullptr;
     if (opt.precision == VLM_PREC_FP64) {
       launch_partial64(rec64, dc, nq, rec, largest_chunk(ch.data(), nq), dP, (int)M, part, stream);

@@ -5,6 +5,8 @@
 // (A thread per record walked 18 doubles and four FP64-compared neighbours, a
 // second kernel packed the records, a third wrote the targets and a fill reset
 // the counter: 8 + 12.5 + 1.6 + 1.2 us at 500 records and the launches between.)
+// In FP64 it also marks what neighbouring rings of a sheet share (a launch of its own
+// before each evaluation took 4.6 us).
 // Only copies and one FP64 subtraction are rounded here, so the unit shares the FP32
 // kernels' compiler options.
 #include "launch.h"
@@ -49,8 +51,25 @@ __device__ double lattice_weight(const Dims& d, const DevState& s, const double*
   return k < 2 ? G - above_eps(s.nGam[o]) : 0.0;
 }
 
+__device__ __forceinline__ bool same_bits(const double* a, const double* b, int n) {
+  bool f = true;
+  for (int k = 0; k < n; ++k) f &= __double_as_longlong(a[k]) == __double_as_longlong(b[k]);
+  return f;
+}
+// What lane k of a ring's four finds it shares with its neighbours, bit for bit
+// (k_lattice64): lane 3 corner 3 and edge 3 with the ring before (corners cb, radii
+// vb), lane 0 corner 1 and edge 0 with the ring L before (ca, va); null: none.
+__device__ __forceinline__ int shared_with(int k, const double* c, const double* v, const double* cb, const double* vb,
+                                           const double* ca, const double* va) {
+  if (k == 3 && cb && same_bits(c + 9, cb + 6, 3))
+    return kShareC3 | (same_bits(c, cb + 3, 3) && same_bits(v + 3, vb + 1, 1) ? kShareE3 : 0);
+  if (k == 0 && ca && same_bits(c + 3, ca + 6, 3))
+    return kShareC1 | (same_bits(c, ca + 9, 3) && same_bits(v, va + 2, 1) ? kShareE0 : 0);
+  return 0;
+}
+
 __global__ void __launch_bounds__(256) k_gather(Dims d, DevState s, const double* fr, const Group* groups, int ngroups,
-                                                int nrec, int rowNear, int rowFar, int pred, float nearFactor,
+                                                int nrec, int rowNear, int rowFar, int pred, float nearFactor, int L,
                                                 int recBlocks, GatherTargets tg) {
   after_previous();
   if ((int)blockIdx.x >= recBlocks) {
@@ -71,13 +90,17 @@ __global__ void __launch_bounds__(256) k_gather(Dims d, DevState s, const double
   const int b = G.blade;
   const double* corner = nullptr;  // the record's corners, or a single filament's ends
   double rv = 0.0, gam, W = 0.0;   // filament k's core radius, the circulation, edge k's weight
-  int flags = 0;
+  int flags = 0, share = 0;
   if (G.kind == 0) {
     const int p = l0;
     corner = panRec(d, fr, b, p);
     rv = s.wRvc[4 * ((size_t)b * d.npan + p) + k];
     gam = s.wGam[(size_t)b * d.npan + p];
     W = gam;  // wing rings: no eps skip
+    if (s.share) {
+      const double* v = s.wRvc + 4 * ((size_t)b * d.npan + p);
+      share = shared_with(k, corner, v, p > 0 ? panRec(d, fr, b, p - 1) : nullptr, v - 4, nullptr, nullptr);
+    }
   } else {
     const int rowsN = d.NW - (rowNear - 1);
     const int nNear = rowsN * d.ns;
@@ -95,6 +118,11 @@ __global__ void __launch_bounds__(256) k_gather(Dims d, DevState s, const double
       gam = s.nGam[r];
       flags = REC_SKIP;
       if (s.edgeW) W = lattice_weight(d, s, nc, b, i, j, k, rowNear);
+      if (s.share) {
+        const size_t a = j > 0 ? ringI(d, b, i, j - 1) : r;
+        share = shared_with(k, corner, s.nRvc + 4 * r, i > rowNear - 1 ? nc + 12 * (r - 1) : nullptr, s.nRvc + 4 * r - 4,
+                            j > 0 && rowsN == L ? nc + 12 * a : nullptr, s.nRvc + 4 * a);
+      }
     } else if (l < nNear + hs) {
       // the horseshoe's closing filaments
       const size_t r = ringI(d, b, d.NW - 1, l - nNear);
@@ -131,6 +159,11 @@ __global__ void __launch_bounds__(256) k_gather(Dims d, DevState s, const double
     if (k == 1) R[17] = (double)flags;
     if (s.edgeW) s.edgeW[4 * (size_t)t + k] = W;
   }
+  if (s.share) {
+    share |= __shfl_xor_sync(0xffffffffu, share, 1);
+    share |= __shfl_xor_sync(0xffffffffu, share, 2);
+    if (live && k == 0) s.share[t] = share;
+  }
   if (s.rec32)
     pack_edge32(p, rv, gam, flags, s.edgeW != nullptr, W, k, nearFactor,
                 live ? s.rec32 + (size_t)t * kRec32 : nullptr);
@@ -139,12 +172,12 @@ __global__ void __launch_bounds__(256) k_gather(Dims d, DevState s, const double
 }  // namespace
 
 void launch_gather(const Dims& d, const DevState& s, const double* frame, const Group* groups, int ngroups, int nrec,
-                   int rowNear, int rowFar, bool pred, double nearFactor, const GatherTargets& tg, cudaStream_t st) {
+                   int rowNear, int rowFar, bool pred, double nearFactor, int L, const GatherTargets& tg, cudaStream_t st) {
   const int rb = (int)(((long)nrec * 4 + 255) / 256), tb = tg.kind ? (tg.M + 255) / 256 : 0;
   if (rb + tb <= 0) return;
   count_launch();
   launch_next(k_gather, rb + tb, 256, 0, st, d, s, frame, groups, ngroups, nrec, rowNear, rowFar, pred ? 1 : 0,
-                                    (float)nearFactor, rb, tg);
+                                    (float)nearFactor, L, rb, tg);
 }
 
 }  // namespace vlm

@@ -167,9 +167,11 @@ void launch_partial64(const double* rec, const Chunk* chunks, int nchunks, int64
                       double* part, cudaStream_t s);
 // The same for groups that hold lattice sheets of L rows (rings column by
 // column): corners and filaments that neighbouring rings share are evaluated
-// once.  share: nrec ints of scratch.
-void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunks, int nrec, int largest, const Group* groups,
-                              int ngroups, int L, int* share, const double* P, int M, double* part, cudaStream_t s);
+// once.  share: per record, what it shares bit for bit with the records r - 1
+// (corner 3, edge 3) and r - L (corner 1, edge 0).
+constexpr int kShareC3 = 1, kShareE3 = 2, kShareC1 = 4, kShareE0 = 8;
+void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunks, int nrec, int largest, int L,
+                              const int* share, const double* P, int M, double* part, cudaStream_t s);
 // FP32 pairs with FP64 accumulation over the nrec records the chunks cover.
 // When near_scratch is non-null (near_bytes = near_scratch_bytes(M, cap) for a list of cap
 // near pairs), the

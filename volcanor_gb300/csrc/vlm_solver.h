@@ -178,9 +178,10 @@ struct GatherTargets {
 };
 // records of the given groups (kind 0 wing, kind 1 wake) into s.rec64, their
 // lattice weights into s.edgeW and their FP32 records, with near zones of
-// nearFactor core radii (0: none), into s.rec32, each where not null
+// nearFactor core radii (0: none), into s.rec32, and what each ring shares with its
+// neighbours in sheets of L rows into s.share, each where not null
 void launch_gather(const Dims& d, const DevState& s, const double* frame, const Group* groups, int ngroups,
-                   int nrec, int rowNear, int rowFar, bool pred, double nearFactor, const GatherTargets& tg,
+                   int nrec, int rowNear, int rowFar, bool pred, double nearFactor, int L, const GatherTargets& tg,
                    cudaStream_t st);
 // node velocities from outv (0 + v), plus the initial wake velocity terms
 // and velocity operation op at the nodes (-1: none; elsewhere the velocities are
