@@ -2399,7 +2399,13 @@ static RingPlan ring_reserve(RingScratch& R, int64_t N, int64_t M, int precision
   grow((void**)&R.near, R.capNear, p.nearBytes);
   if (precision == VLM_PREC_FP32_NEAR64 && (size_t)M * p.Q * 3 * 8 > R.capNacc) {
     grow((void**)&R.nacc, R.capNacc, (size_t)M * p.Q * 3 * 8);
-    VLM_CUDA(cudaMemset(R.nacc, 0, R.capNacc));
+    // zero before the call goes on: the memset runs on the legacy stream, for
+    // which a caller's non-blocking stream does not wait
+    const size_t cap = R.capNacc;
+    R.capNacc = 0;
+    VLM_CUDA(cudaMemset(R.nacc, 0, cap));
+    VLM_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+    R.capNacc = cap;
   }
   return p;
 }
