@@ -131,6 +131,19 @@ for n, m in ((100, 50), (300, 5000)):
     p = [x.ctypes.data for x in a]
     lib.biot_savart_rings_device(p[0], p[1], p[2], n, p[3], m, p[4], lib.PREC_FP32_NEAR64, st)
 """,
+    # the network of a case's surrogate, trained on the case's stream (what the case itself
+    # left behind is waited for first)
+    "surrogate": """
+from volcanor_gb300 import cases as C
+c = C.rotor_2blade_hover(nt=40, n_nwake=10, truncate_nt=30)
+k = lib.Case(c.config, c.geom, precision=lib.PREC_FP32_NEAR64)
+rt.cudaStreamSynchronize(None)
+rt.fake_reset()
+k.set_surrogate(collect_steps=2, sample_stride=2, train_iters=4, batch=64, hidden=16, layers=3, min_far=4, young_far=2)
+k.start()
+k.step(40)
+assert k.surrogate_stats()["trainings"] > 0
+""",
 }
 
 

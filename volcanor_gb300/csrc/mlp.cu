@@ -250,16 +250,17 @@ void Mlp::create(const std::vector<int>& sizes, uint64_t seed, cudaStream_t stre
   MLP_CUDA(cudaMalloc(&m, sizeof(float) * sh.nparam));
   MLP_CUDA(cudaMalloc(&v, sizeof(float) * sh.nparam));
   MLP_CUDA(cudaMalloc(&loss, sizeof(float) * 2));
-  MLP_CUDA(cudaMemcpy(p, h.data(), sizeof(float) * sh.nparam, cudaMemcpyHostToDevice));
-  MLP_CUDA(cudaMemset(g, 0, sizeof(float) * sh.nparam));
-  MLP_CUDA(cudaMemset(m, 0, sizeof(float) * sh.nparam));
-  MLP_CUDA(cudaMemset(v, 0, sizeof(float) * sh.nparam));
+  // on the network's own stream: a case's does not wait for the legacy one
+  MLP_CUDA(cudaMemcpyAsync(p, h.data(), sizeof(float) * sh.nparam, cudaMemcpyHostToDevice, st));
+  MLP_CUDA(cudaMemsetAsync(g, 0, sizeof(float) * sh.nparam, st));
+  MLP_CUDA(cudaMemsetAsync(m, 0, sizeof(float) * sh.nparam, st));
+  MLP_CUDA(cudaMemsetAsync(v, 0, sizeof(float) * sh.nparam, st));
   adamStep = 0;
   tcFits = tc.plan(sh);
   if (tcFits) {
     MLP_CUDA(cudaMalloc(&tcImg, tc.imgBytes));
     MLP_CUDA(cudaMalloc(&tcErr, sizeof(int)));
-    MLP_CUDA(cudaMemset(tcErr, 0, sizeof(int)));
+    MLP_CUDA(cudaMemsetAsync(tcErr, 0, sizeof(int), st));
   }
   useTc = tcFits;
   tcStale = true;
