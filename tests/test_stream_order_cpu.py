@@ -144,6 +144,40 @@ k.start()
 k.step(40)
 assert k.surrogate_stats()["trainings"] > 0
 """,
+    # a case's tables: created, steady (graph and incremental plan), asked for velocities, resumed
+    "case": """
+from volcanor_gb300 import cases as C
+c = C.rotor_2blade_hover(nt=60, n_nwake=10, truncate_nt=16)
+for precision in (lib.PREC_FP64, lib.PREC_FP32, lib.PREC_FP32_NEAR64):
+    k = lib.Case(c.config, c.geom, precision=precision)
+    k.start()
+    k.step(30)
+    k.vind_points(rng.normal(size=(5, 3)))
+    k.step(2)
+    k.checkpoint_save("case.ckpt")
+    k.checkpoint_load("case.ckpt")
+    k.step(2)
+k.checkpoint_load("case.ckpt")
+f = lib.Case(c.config, c.geom, precision=lib.PREC_FP64)
+f.start()
+f.checkpoint_save("case.ckpt")
+k.checkpoint_load("case.ckpt")  # without FP32 factors: made from the restored AIC
+""",
+    "batch": """
+from volcanor_gb300 import cases as C
+c = C.rotor_2blade_hover(nt=40, n_nwake=10, truncate_nt=16)
+b = lib.Batch([(c.config, c.geom, "")] * 3, precision=lib.PREC_FP32_NEAR64)
+b.start()
+b.step(30)
+""",
+    "system": """
+from volcanor_gb300 import cases as C
+sc = C.rotor_pair(nt=20, n_nwake=8, truncate_nt=12)
+for precision in (lib.PREC_FP64, lib.PREC_FP32_NEAR64):
+    y = lib.System(sc.config, sc.geoms, precision=precision)
+    y.start()
+    y.step(20)
+""",
 }
 
 
@@ -163,9 +197,9 @@ def runtime(tmp_path_factory):
 
 
 @pytest.mark.parametrize("program", sorted(PROGRAMS))
-def test_nothing_left_on_the_legacy_stream(runtime, program):
+def test_nothing_left_on_the_legacy_stream(runtime, program, tmp_path):
     code = PRELUDE + PROGRAMS[program] + "\nprint(rt.fake_hazards().decode())"
-    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env={**os.environ, "LD_PRELOAD": str(runtime)},
-                       capture_output=True, text=True, timeout=300)
+    env = {**os.environ, "LD_PRELOAD": str(runtime), "PYTHONPATH": str(ROOT)}
+    r = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
     assert r.stdout.strip() == "", sorted(set(r.stdout.strip().splitlines()))

@@ -106,6 +106,11 @@ static T* dalloc(size_t n, DevArena& owned) {
   return static_cast<T*>(owned.take(n * sizeof(T)));
 }
 
+// cudaMemcpy of a small pageable array returns when it is staged, and the cases'
+// non-blocking streams do not wait for the legacy one that copies it: the arrays
+// are there after this
+static void wait_for_copies() { VLM_CUDA(cudaStreamSynchronize(cudaStreamLegacy)); }
+
 static int largest_chunk(const Chunk* ch, int n) {
   int c = 0;
   for (int i = 0; i < n; ++i) c = std::max(c, (int)ch[i].rec_count);
@@ -515,6 +520,7 @@ struct Case {
       VLM_CUDA(cudaMemcpy(dGroups, hGroups.data(), hGroups.size() * sizeof(Group), cudaMemcpyHostToDevice));
     if (!hChunks.empty())
       VLM_CUDA(cudaMemcpy(dChunks, hChunks.data(), hChunks.size() * sizeof(Chunk), cudaMemcpyHostToDevice));
+    wait_for_copies();
   }
 
   const double* frame(int k) const { return s.frames + (size_t)k * d.fl.size; }
@@ -1037,6 +1043,7 @@ struct Case {
     VLM_CUDA(cudaMemcpy(ip.dC, dch.data(), sizeof(Chunk) * ip.dq, cudaMemcpyHostToDevice));
     VLM_CUDA(cudaMemcpy(ip.mG, mg.data(), sizeof(Group) * e.ngroups, cudaMemcpyHostToDevice));
     VLM_CUDA(cudaMemcpy(ip.mC, mch.data(), sizeof(Chunk) * ip.mq, cudaMemcpyHostToDevice));
+    wait_for_copies();
     ip.dRec = dalloc<double>((size_t)ip.dcap * kRec64, incrOwned);
     ip.dEw = lattice() ? dalloc<double>((size_t)ip.dcap * 4, incrOwned) : nullptr;
     ip.tIdx = dalloc<int>((size_t)ip.mcap, incrOwned);
@@ -1972,6 +1979,7 @@ struct Case {
       // the FP32 factors only matter to a case that refines
       if (i < common || refine) VLM_CUDA(cudaMemcpy(a.first, buf.data(), a.second, cudaMemcpyHostToDevice));
     }
+    wait_for_copies();
     // a refining case restored from a state without FP32 factors factors the
     // restored AIC itself (the same FP32 LU its start would have made)
     if (refine && !fileRefined) {
@@ -2262,6 +2270,7 @@ struct Case {
     VLM_CUDA(cudaMemcpy(dg, g.data(), g.size() * sizeof(Group), cudaMemcpyHostToDevice));
     VLM_CUDA(cudaMemcpy(dc, ch.data(), nq * sizeof(Chunk), cudaMemcpyHostToDevice));
     VLM_CUDA(cudaMemcpy(dP, P, (size_t)M * 3 * sizeof(double), cudaMemcpyHostToDevice));
+    wait_for_copies();
     DevState t = s;
     t.rec64 = rec64;
     t.edgeW = nullptr;  // ring by ring: the probe's record count is not the plans'
