@@ -719,7 +719,7 @@ def main():
     ap.add_argument("--kernel-m", type=int, default=1 << 20)
     ap.add_argument("--forward-step", type=int, default=720)
     ap.add_argument("--workload", default="hover2", choices=["hover2", "batch", "forward4"],
-                    help="hover2: the headline 2-blade hover case; batch: 256 uneven cases in one graph launch")
+                    help="hover2: the headline 2-blade hover case; batch: 256 uneven cases side by side")
     ap.add_argument("--batch-cases", type=int, default=256)
     ap.add_argument("--batch-steps", type=int, default=10, help="timed steps of the batch key")
     # the batched sweep's transient takes ~3 min (581 steps of 256 cases):

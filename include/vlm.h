@@ -15,8 +15,8 @@
  *   - all arrays are caller-owned host memory unless the name ends in
  *     _device; vectors are xyz-contiguous, i.e. a Fortran real(dp) (3, m)
  *     array passes as c_loc(array) without repacking;
- *   - a vlm_case owns its device memory and one CUDA stream; call it from one
- *     host thread at a time.
+ *   - a vlm_case owns its device memory and up to five CUDA streams; call it
+ *     from one host thread at a time.
  */
 #ifndef VLM_GB300_H
 #define VLM_GB300_H

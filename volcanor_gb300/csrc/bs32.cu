@@ -560,7 +560,7 @@ __device__ __forceinline__ int ord_code(float f) {
 __device__ __forceinline__ float ord_value(int c) { return __int_as_float(c >= 0 ? c : c ^ 0x7FFFFFFF); }
 
 // Sum and count of the near-zone radii near_factor rvc_k = sqrt([32 + k]) /
-// |e_k| of the active filaments (the cell size is twice their mean).
+// |e_k| of the active filaments (the cell size is kCellOverZone times their mean).
 __global__ void k_zone_mean(const float* rec32, int nrec, unsigned char* scratch) {
   after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1082,8 +1082,8 @@ template <int V>
 void launch_shape(bool lat, dim3 grid, const float* rec32, const Chunk* chunks, const double* P, int M, double* part,
                   int* ctl, cudaStream_t s) {
   using S = Shape32<V>;
-  if (lat) launch_next(k_partial32<true, S::tpt, S::stages, S::minb>, grid, kBlockW, shape_smem<V>(), s, rec32, chunks, P, M, part, ctl);
-  else launch_next(k_partial32<false, S::tpt, S::stages, S::minb>, grid, kBlockW, shape_smem<V>(), s, rec32, chunks, P, M, part, ctl);
+  const auto kernel = lat ? k_partial32<true, S::tpt, S::stages, S::minb> : k_partial32<false, S::tpt, S::stages, S::minb>;
+  launch_next(kernel, grid, kBlockW, shape_smem<V>(), s, rec32, chunks, P, M, part, ctl);
 }
 
 // the dynamic shared-memory opt-in is per device; set it once on each
@@ -1154,7 +1154,7 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
     launch_next(k_near_find_small, (unsigned)(tiles() * rb), 256, 0, ns, rec32, nrec, chunks, nchunks, P, M, tile,
                 (int)tiles(), list, cap, ctl);
     launch_next(k_near_fix, 4 * sms, 128, 0, ns, list, cap, rec32, rec64, ew, P, M,
-                                        reinterpret_cast<unsigned long long*>(nacc), ctl);
+                reinterpret_cast<unsigned long long*>(nacc), ctl);
     if (ns != s) {
       pairs();
       cudaEventRecord(ov->join, ns);
@@ -1171,10 +1171,10 @@ void launch_partial32(const float* rec32, const double* rec64, const Chunk* chun
     launch_next(k_tgrid_insert<1>, (M + 255) / 256, 256, 0, ns, P, M, g);
   }
   count_launches(2);
-  launch_next(k_near_find, (unsigned)(((size_t)nrec * 2 * 32 + 255) / 256), 256, 0, ns, rec32, nrec, chunks, nchunks, P, M,
-                                                                               g, list, cap, ctl);
-  launch_next(k_near_fix, 4 * sms, 128, 0, ns, list, cap, rec32, rec64, ew, P, M, reinterpret_cast<unsigned long long*>(nacc),
-                                      ctl);
+  launch_next(k_near_find, (unsigned)(((size_t)nrec * 2 * 32 + 255) / 256), 256, 0, ns, rec32, nrec, chunks, nchunks, P,
+              M, g, list, cap, ctl);
+  launch_next(k_near_fix, 4 * sms, 128, 0, ns, list, cap, rec32, rec64, ew, P, M,
+              reinterpret_cast<unsigned long long*>(nacc), ctl);
   if (ns != s) {
     pairs();
     cudaEventRecord(ov->join, ns);

@@ -20,12 +20,15 @@ namespace {
 // for 64 cycles (half a lane a cycle), so the pair evaluations bound every
 // shape here; a few warps on an SM fill the unit, and what a small shape lacks
 // is quarters.  So the evaluations of a chunk are spread over threads and only
-// its additions, which have to stay in record order, are serial: a block takes TT targets and evaluates a batch of S = threads / TT
-// consecutive records of each at once into shared memory; one warp then adds
-// the S contributions of each (target, component) in record order -- the warps
-// take turns -- while all go on with the next batch.  Each contribution and each addition is the reference's own, so the bits are
-// those of one thread per target (blade_vind_bywing / blade_vind_bywake,
-// src/classdef.f90:1342-1513).
+// its additions, which have to stay in record order, are serial: a block takes TT
+// targets and evaluates a batch of S = threads / TT consecutive records of each at
+// once into shared memory; 3 TT lanes, one for each (target, component), then add
+// the S contributions in record order -- one to three warps, which take turns --
+// while all go on with the next batch.  Each contribution and each addition is
+// the reference's own, so the bits are those of one thread per target
+// (blade_vind_bywing / blade_vind_bywake, src/classdef.f90:1342-1513).  The FP64
+// pipe is busy for 90 % of k_rings64's cycles at 2^18 rings and 2048 targets and
+// for 82 % of k_lattice64's at a 3-revolution hover wake.
 //
 // A near-wake sheet's rings are listed column by column (L rows each): ring
 // r's corner 3 and edge 3 are ring r - 1's corner 2 and edge 1, its corner 1 and
@@ -255,7 +258,7 @@ __global__ void __launch_bounds__(kThreadsLattice64) k_lattice64(const double* r
 // cycles (fitted to sweeps over TT and K from 52 to 60000 targets and 52 to 12480
 // records; slope is its FP64 instructions, lat the chain of one evaluation),
 // a run's first column of a sheet's edges a half more, and an ordered addition
-// 90 in the warp whose turn it is.  Few targets and chunks get one target a
+// 90 in each warp whose turn it is.  Few targets and chunks get one target a
 // block (a wing's 52 rings at 52 points: 52 blocks whose threads take a record
 // each, 18 us; 906 us in one block of a thread per target), many get 4 to 16.
 struct Tile64 {
@@ -376,8 +379,8 @@ __global__ void k_combine_terms(const double* part, int M, const Group* groups, 
 // which a lane's few thousand could overflow, one by one): conversions and
 // additions run on the FP64 unit, 16 cycles a warp and SM, and bound the kernel.
 // Group by group, each with its own butterfly and a conversion a partial, 13500
-// targets of 24 chunks took 33 us, now 15; 48 of 300 took 12, now 7.  mode 3: term blockIdx.y's groups alone, into its part of out; mode 1
-// leaves the wings' chunks out.
+// targets of 24 chunks took 33 us, now 15; 48 of 300 took 12, now 7.  mode 3: term
+// blockIdx.y's groups alone, into its part of out; mode 1 leaves the wings' chunks out.
 template <bool ADD>
 __global__ void __launch_bounds__(256) k_combine_tree(const double* part, long long* nacc, int M, const Group* groups,
                                                       int ngroups, int mode, int G, double* out) {
@@ -519,8 +522,8 @@ void launch_lattice64(const Tile64& T, const double* rec, const int* share, cons
                       const double* P, int M, double* part, cudaStream_t s) {
   int K = 1;
   const dim3 grid = grid64(T, M, nchunks, K);
-  launch_next(k_lattice64, grid, kThreadsLattice64, lattice_smem64(T.lgTT, L), s, rec, share, chunks, nchunks, K, P, M, T.lgTT,
-                                                                         L, part);
+  launch_next(k_lattice64, grid, kThreadsLattice64, lattice_smem64(T.lgTT, L), s, rec, share, chunks, nchunks, K, P, M,
+              T.lgTT, L, part);
 }
 }  // namespace
 
@@ -533,8 +536,11 @@ void launch_partial64(const double* rec, const Chunk* chunks, int nchunks, int64
 
 void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunks, int nrec, int largest, int L,
                               const int* share, const double* P, int M, double* part, cudaStream_t s) {
-  // a sheet too tall for shared memory even with one target a block has no
-  // room for a column's edges
+  // A sheet too tall for shared memory even with one target a block (above 3909
+  // rows) has no room for a column's edges.  Sheets of 8 stations, ns a ring and
+  // target: 0.39 at 1488 rows, where an SM still holds two blocks of one target,
+  // 0.45 at 1489, where it holds one, 0.60 at 2500, 0.64 at 3909, and 0.37 ring
+  // by ring at 3910: by time the line would lie at 1488.
   if (L <= 0 || lattice_smem64(0, L) + 1024 > kSmemPerSm64) {
     launch_partial64(rec, chunks, nchunks, nrec, largest, P, M, part, s);
     return;
@@ -542,7 +548,8 @@ void launch_partial64_lattice(const double* rec, const Chunk* chunks, int nchunk
   if (M <= 0 || nchunks <= 0) return;
   lattice_attr64();
   count_launch();
-  launch_lattice64(pick_tile64(M, nchunks, nrec, largest, L, device_sm_count()), rec, share, chunks, nchunks, L, P, M, part, s);
+  launch_lattice64(pick_tile64(M, nchunks, nrec, largest, L, device_sm_count()), rec, share, chunks, nchunks, L, P, M,
+                   part, s);
 }
 
 void launch_combine(const double* part, int M, const Group* groups, int ngroups, int mode, double* out,
@@ -571,8 +578,8 @@ void launch_combine_terms(const double* part, long long* nacc, int M, const Grou
     return;
   }
   const int per = mode == 3 ? nterms : 1, G = tree_lanes((nchunks + per - 1) / per);
-  launch_next(k_combine_tree<false>, dim3((unsigned)((3 * (size_t)M * G + 255) / 256), per), 256, 0, s, part, nacc, M, groups,
-              ngroups, mode, G, out);
+  launch_next(k_combine_tree<false>, dim3((unsigned)((3 * (size_t)M * G + 255) / 256), per), 256, 0, s, part, nacc, M,
+              groups, ngroups, mode, G, out);
 }
 
 void launch_fils_to_rec64(const double* fc, const double* rvc, const double* gam, int64_t N, double* rec,

@@ -627,9 +627,11 @@ struct Case {
       return;
     }
     if (nterms > 0)
-      launch_combine_terms(s.part, near ? s.nacc : nullptr, M, dGroups + e.goff, e.ngroups, e.nchunks, nterms, mode, prec == VLM_PREC_FP64, out, stream);
+      launch_combine_terms(s.part, near ? s.nacc : nullptr, M, dGroups + e.goff, e.ngroups, e.nchunks, nterms, mode,
+                           prec == VLM_PREC_FP64, out, stream);
     else if (prec == VLM_PREC_FP64) launch_combine(s.part, M, dGroups + e.goff, e.ngroups, mode, out, stream);
-    else launch_combine_unordered(s.part, near ? s.nacc : nullptr, M, dGroups + e.goff, e.ngroups, e.nchunks, mode, out, stream);
+    else launch_combine_unordered(s.part, near ? s.nacc : nullptr, M, dGroups + e.goff, e.ngroups, e.nchunks, mode, out,
+                                  stream);
   }
 
   // ---- autotuner of the FP32 N-body tile shape and chunking ----------------
@@ -2438,7 +2440,8 @@ static void ring_launch(RingScratch& R, const RingPlan& p, const double* corners
                        R.nacc, st);
     }
     if (precision == VLM_PREC_FP64) launch_combine(R.part, (int)M, group, 1, 2, V, st);
-    else launch_combine_unordered(R.part, precision == VLM_PREC_FP32_NEAR64 ? R.nacc : nullptr, (int)M, group, 1, p.nq, 2, V, st);
+    else launch_combine_unordered(R.part, precision == VLM_PREC_FP32_NEAR64 ? R.nacc : nullptr, (int)M, group, 1, p.nq, 2, V,
+                                  st);
   } else {
     VLM_CUDA(cudaMemsetAsync(V, 0, (size_t)M * 3 * 8, st));
   }

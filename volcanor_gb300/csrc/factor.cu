@@ -366,7 +366,10 @@ __global__ void __launch_bounds__(kInvThreads) k_inverse64(const double* A, cons
 }
 
 // The same, a thread per column on global memory: for matrices whose columns do
-// not fit shared memory (over 4100 rows).
+// not fit shared memory (over 4100 rows).  By time the line would lie lower, where
+// a block is left with a column or two and the blocks come in waves: AIC, factors
+// and inverse take 0.32 s at 1812 rows, 1.7 at 2800, 7.2 at 3700, and 3.4 this way
+// at 4200 (with LU and inverse each in one launch 1.6, 5.4, 12.0 and 18.3 s).
 __global__ void k_inverse64_big(const double* A, const int* piv, int n,
                                 double* inv) {
   after_previous();
@@ -470,7 +473,8 @@ void launch_lu32(const Dims& d, const DevState& s, cudaStream_t st) {
   int wpb = 4;
   while (wpb > 1 && sizeof(float) * wpb * (size_t)n > 48 * 1024) --wpb;
   count_launch();
-  launch_next(k_inverse32, (n + wpb - 1) / wpb, 32 * wpb, sizeof(float) * wpb * (size_t)n, st, s.LU32, s.piv32, n, s.AICinv32);
+  launch_next(k_inverse32, (n + wpb - 1) / wpb, 32 * wpb, sizeof(float) * wpb * (size_t)n, st, s.LU32, s.piv32, n,
+              s.AICinv32);
 }
 
 }  // namespace vlm

@@ -177,7 +177,7 @@ void launch_gather(const Dims& d, const DevState& s, const double* frame, const 
   if (rb + tb <= 0) return;
   count_launch();
   launch_next(k_gather, rb + tb, 256, 0, st, d, s, frame, groups, ngroups, nrec, rowNear, rowFar, pred ? 1 : 0,
-                                    (float)nearFactor, L, rb, tg);
+              (float)nearFactor, L, rb, tg);
 }
 
 }  // namespace vlm

@@ -1,14 +1,14 @@
 // Launches that follow one another on a stream.
 //
-// A step is a chain of 50 to 70 kernels, most of them a few microseconds
+// A step is a chain of 35 to 45 kernels, most of them a few microseconds
 // long; launched one after the other, each waited 2.7 us more for its
 // predecessor than the arithmetic needs.  launch_next lets a kernel be set up
 // while the kernel before it on the stream still runs (programmatic stream
 // serialization): 60 small kernels in a chain take 1.4 us each instead of 4.1.
 // In a captured graph a launch costs 1.3 to 1.7 us anyway (1.1 to 1.4 this way),
 // and there the blocks set up early hold registers that the kernels of other
-// branches want: with it 8 steps of a 6-revolution hover rotor took 7.6 ms
-// instead of 7.2 and 4 steps of 8 uneven rotors 12.3 instead of 11.7, so a
+// branches want: with it 8 steps of a 6-revolution hover rotor take 6.1 to 6.3 ms
+// instead of 5.95 and 4 steps of 8 uneven rotors 10.8 instead of 10.0, so a
 // stream under capture gets plain launches.
 //
 // Every kernel launched this way begins with after_previous(), in every

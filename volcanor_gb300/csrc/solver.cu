@@ -809,8 +809,8 @@ constexpr size_t kSolveSmemMax = sizeof(double) * (8192 + 1024) + sizeof(float) 
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__global__ void __cluster_dims__(kSolveBlocks, 1, 1) __launch_bounds__(kSolveThreads) k_solve_refine(Dims d, DevState s, int R,
-                                                                                                    int S) {
+__global__ void __cluster_dims__(kSolveBlocks, 1, 1) __launch_bounds__(kSolveThreads)
+    k_solve_refine(Dims d, DevState s, int R, int S) {
   after_previous();
   const int n = d.n;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1684,7 +1684,8 @@ void launch_scatter_nodes(const Dims& d, const DevState& s, const double* frame,
   const int addInit = initWakeVel != 0.0 ? 1 : 0;
   if (M > 0) {
     count_launch();
-    launch_next(k_scatter_nodes, nblk(M, 256), 256, 0, st, d, s, frame, rowNear, rowFar, pred ? 1 : 0, initWakeVel, addInit, op, M);
+    launch_next(k_scatter_nodes, nblk(M, 256), 256, 0, st, d, s, frame, rowNear, rowFar, pred ? 1 : 0, initWakeVel,
+                addInit, op, M);
   }
 }
 void launch_aic(const Dims& d, const DevState& s, const double* frame, cudaStream_t st) {
@@ -1762,8 +1763,8 @@ void launch_loads(const Dims& d, const DevState& s, const double* frame, int sum
                   const double* foreignBound, int nrs, int self) {
   count_launch();
   velcp_attr();
-  launch_next(k_velcp_total, d.nbC * d.npan, kVcThreads, velcp_smem(d.npan, d.ns), st, d, s, frame, sumChunk, foreignBound, nrs, self,
-              velcp_blades(d.npan));
+  launch_next(k_velcp_total, d.nbC * d.npan, kVcThreads, velcp_smem(d.npan, d.ns), st, d, s, frame, sumChunk, foreignBound,
+              nrs, self, velcp_blades(d.npan));
   count_launch();
   launch_next(k_loads, 1, kLoadsThreads, 0, st, d, s, frame, iter);
 }
