@@ -50,7 +50,6 @@ extern "C" {
 const char* fake_hazards() { return hazards.c_str(); }
 void fake_reset() { hazards.clear(); }
 cudaStream_t fake_stream() { cudaStream_t s; make(&s); return s; }
-void fake_legacy_work() { pending.push_back("the caller's work"); }
 cudaError_t cudaMalloc(void** p, size_t n) { *p = malloc(n); memset(*p, 0, n); return cudaSuccess; }
 cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = calloc(n, 1); pinned[(char*)*p] = n; return cudaSuccess; }
